@@ -237,37 +237,29 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
     }
 }
 
-// Merge per-split lists of every split problem: one warp per (problem, query).
-// mlist holds the record indices of the split problems, by merge_begin.
-__global__ void batched_merge_kernel(const BatchProb *__restrict__ probs,
-                                     const int *__restrict__ mlist, int n_split_probs,
-                                     long long n_tasks, int slab_keys) {
-    extern __shared__ unsigned long long msm[];
-    const int wpb = blockDim.x >> 5;
+// Merge per-split lists of every split problem: one warp per (problem, query)
+// (merge_lists).  mlist holds the record indices of the split problems, by
+// merge_begin.
+constexpr int BM_WARPS = 8;
+template <int KCAP>
+__global__ void __launch_bounds__(32 * BM_WARPS)
+    batched_merge_kernel(const BatchProb *__restrict__ probs, const int *__restrict__ mlist,
+                         int n_split_probs, long long n_tasks) {
+    __shared__ unsigned long long lists[BM_WARPS][KCAP], scratch[BM_WARPS][KCAP];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long task = (long long)blockIdx.x * wpb + warp;
+    const long long task = (long long)blockIdx.x * BM_WARPS + warp;
     if (task >= n_tasks) return;
     const int m = find_record(n_split_probs, task,
                               [&](int i) { return probs[mlist[i]].merge_begin; });
     const BatchProb &P = probs[mlist[m]];
     const int q = (int)(task - P.merge_begin);
-    const int S = P.n_splits, k = P.k;
-    unsigned long long *L = msm + (size_t)warp * slab_keys;
-    for (int e = lane; e < S * k; e += 32) {
-        const int t = e / k, j = e - t * k;
-        L[e] = P.part[((size_t)t * P.Q + q) * k + j];
-    }
-    __syncwarp();
-    for (int e = lane; e < S * k; e += 32) {
-        const int t = e / k, j = e - t * k;
-        const unsigned long long x = L[e];
-        int pos = j;
-        for (int u = 0; u < S && pos < k; ++u)
-            if (u != t) pos += rank_sorted(L + (size_t)u * k, k, x);
-        if (pos < k) {
-            P.out_dist[(size_t)pos * P.ld_out + q] = sqrtf(key_dist2(x));
-            P.out_idx[(size_t)pos * P.ld_out + q] = key_index(x);
-        }
+    const int k = P.k;
+    unsigned long long *L = lists[warp];
+    merge_lists<KCAP>(L, scratch[warp], P.part + (size_t)q * k, (size_t)P.Q * k, 0, 1, P.n_splits,
+                      k, lane);
+    for (int j = lane; j < k; j += 32) {
+        P.out_dist[(size_t)j * P.ld_out + q] = sqrtf(key_dist2(L[j]));
+        P.out_idx[(size_t)j * P.ld_out + q] = key_index(L[j]);
     }
 }
 
@@ -277,7 +269,7 @@ using namespace knnb200;
 
 namespace {
 
-constexpr size_t kBatchMergeSmemMax = 200u * 1024u;
+constexpr int kMaxListKeys = 25600;   // split-list keys per query (splits x k)
 
 struct DevMem {
     void *ptr = nullptr;
@@ -306,7 +298,6 @@ struct knnb200_batched_plan {
     int count = 0, n_rows = 0, n_split_probs = 0;   // count: problems of the persistent launch
     std::vector<ExactProblem> lowdim;                // problems routed to the low-d kernel
     long long n_items = 0, n_tasks = 0;
-    int merge_wpb = 1, slab_keys = 0;
     DevMem tables;      // BatchProb[count] | CUtensorMap[2*count] | counter, status | mlist
     DevMem scratch;     // qdup + parts
     BatchProb *probs = nullptr;
@@ -401,8 +392,7 @@ int knnb200_batched_plan_create_config(const knnb200_problem *all, int n_all,
         P.qtiles = (q.query_nb + bq - 1) / bq;
         const long long stages = (long long)P.n_rtiles * P.n_dchunks;
         int S = (int)std::max<long long>(1, (stages + item_stages / 2) / item_stages);
-        // split lists of one query must fit one merge warp's shared slab
-        S = std::min({S, P.n_rtiles, 256, (int)(kBatchMergeSmemMax / (8ull * q.k))});
+        S = std::min({S, P.n_rtiles, 256, kMaxListKeys / q.k});
         P.n_splits = std::max(1, S);
         P.qry = q.query;
         P.ldq = q.query_ld;
@@ -452,7 +442,7 @@ int knnb200_batched_plan_create_config(const knnb200_problem *all, int n_all,
     std::vector<CUtensorMap> maps(2 * count);
     std::vector<int> mlist;
     long long item = 0, task = 0;
-    int row = 0, max_slab = 0;
+    int row = 0;
     unsigned char *sb = static_cast<unsigned char *>(pl->scratch.ptr);
     for (int r = 0; r < count; ++r) {
         const int i = order[r];
@@ -466,7 +456,6 @@ int knnb200_batched_plan_create_config(const knnb200_problem *all, int n_all,
         if (P.n_splits > 1) {
             mlist.push_back(r);
             task += P.Q;
-            max_slab = std::max(max_slab, P.n_splits * P.k);
         }
         P.row_begin = row;
         row += P.d;
@@ -506,10 +495,6 @@ int knnb200_batched_plan_create_config(const knnb200_problem *all, int n_all,
     pl->n_items = item;
     pl->n_tasks = task;
     pl->n_rows = row;
-    pl->slab_keys = max_slab;
-    pl->merge_wpb = max_slab ? (int)std::max<size_t>(
-                                   1, std::min<size_t>(8, kBatchMergeSmemMax / (8ull * max_slab)))
-                             : 1;
     if ((count > 0 &&
          (cudaMemcpy(pl->probs, table.data(), count * sizeof(BatchProb),
                      cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -572,13 +557,13 @@ int knnb200_batched_run(knnb200_batched_plan *pl, void *stream) {
     }
     if (e != cudaSuccess) return KNNB200_ELAUNCH;
     if (pl->n_tasks > 0) {
-        const size_t smem = (size_t)pl->merge_wpb * pl->slab_keys * 8;
-        if (cudaFuncSetAttribute(batched_merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kBatchMergeSmemMax) != cudaSuccess)
-            return KNNB200_ELAUNCH;
-        const long long blocks = (pl->n_tasks + pl->merge_wpb - 1) / pl->merge_wpb;
-        batched_merge_kernel<<<(unsigned)blocks, pl->merge_wpb * 32, smem, st>>>(
-            pl->probs, pl->mlist, pl->n_split_probs, pl->n_tasks, pl->slab_keys);
+        const unsigned blocks = (unsigned)((pl->n_tasks + BM_WARPS - 1) / BM_WARPS);
+        auto merge = pl->kcap == 32    ? batched_merge_kernel<32>
+                     : pl->kcap == 64  ? batched_merge_kernel<64>
+                     : pl->kcap == 128 ? batched_merge_kernel<128>
+                                       : batched_merge_kernel<256>;
+        merge<<<blocks, BM_WARPS * 32, 0, st>>>(pl->probs, pl->mlist, pl->n_split_probs,
+                                                pl->n_tasks);
         if (cudaGetLastError() != cudaSuccess) return KNNB200_ELAUNCH;
     }
     return KNNB200_OK;

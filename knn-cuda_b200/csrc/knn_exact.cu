@@ -36,6 +36,7 @@
 //     order as a single pass.
 #include <algorithm>
 #include <cstdio>
+#include <type_traits>
 
 #include "knn_exact_core.cuh"
 #include "knn_kernels.h"
@@ -164,34 +165,39 @@ __global__ void dup_queries_kernel(const float *__restrict__ src, int Q, long lo
 }
 
 
-// Merge the per-split sorted key lists of each query (one warp per query).
-// An element's output position is the sum of its ranks in every list.
-__global__ void knn_merge_splits_kernel(const unsigned long long *__restrict__ part, int S,
-                                        int Q, int k, float *__restrict__ out_dist,
-                                        int *__restrict__ out_idx, long long ld_out, int row0,
-                                        unsigned long long *__restrict__ lb_out) {
-    extern __shared__ unsigned long long msm[];
-    const int wpb = blockDim.x >> 5;
+// Merge the per-split sorted key lists of each query (merge_lists).  A block of
+// eight warps takes 8 / WPQ consecutive queries, WPQ warps each: one warp a
+// query, or all eight on one (each merges every eighth list, then the first
+// one merges the eight results) where the queries alone do not fill the GPU
+// and the lists are many.
+constexpr int MG_WARPS = 8;
+template <int KCAP, int WPQ>
+__global__ void __launch_bounds__(32 * MG_WARPS)
+    knn_merge_splits_kernel(const unsigned long long *__restrict__ part, int S, int Q, int k,
+                            float *__restrict__ out_dist, int *__restrict__ out_idx,
+                            long long ld_out, int row0, unsigned long long *__restrict__ lb_out) {
+    constexpr int QPB = MG_WARPS / WPQ;
+    __shared__ unsigned long long lists[MG_WARPS][KCAP], scratch[MG_WARPS][KCAP];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int q = blockIdx.x * wpb + warp;
-    if (q >= Q) return;
-    unsigned long long *L = msm + (size_t)warp * S * k;
-    for (int e = lane; e < S * k; e += 32) {
-        const int t = e / k, j = e - t * k;
-        L[e] = part[((size_t)t * Q + q) * k + j];
+    const int q0 = blockIdx.x * QPB, q = q0 + warp / WPQ;
+    if (q < Q) {
+        merge_lists<KCAP>(lists[warp], scratch[warp], part + (size_t)q * k, (size_t)Q * k,
+                          warp % WPQ, WPQ, S, k, lane);
     }
-    __syncwarp();
-    for (int e = lane; e < S * k; e += 32) {
-        const int t = e / k, j = e - t * k;
-        const unsigned long long x = L[e];
-        int pos = j;
-        for (int u = 0; u < S && pos < k; ++u)
-            if (u != t) pos += rank_sorted(L + (size_t)u * k, k, x);
-        if (pos < k) {
-            out_dist[(size_t)(row0 + pos) * ld_out + q] = sqrtf(key_dist2(x));
-            out_idx[(size_t)(row0 + pos) * ld_out + q] = key_index(x);
-            if (lb_out && pos == k - 1) lb_out[q] = x + 1;
-        }
+    __syncthreads();
+    if (WPQ > 1) {
+        if (warp == 0)
+            merge_lists<KCAP>(scratch[0], scratch[1], lists[0], KCAP, 0, 1, WPQ, k, lane);
+        __syncthreads();
+    }
+    // rows of the k x query_nb output, QPB queries wide
+    for (int e = threadIdx.x; e < k * QPB; e += 32 * MG_WARPS) {
+        const int j = e / QPB, qi = e % QPB;
+        if (q0 + qi >= Q) continue;
+        const unsigned long long key = WPQ > 1 ? scratch[0][j] : lists[qi][j];
+        out_dist[(size_t)(row0 + j) * ld_out + q0 + qi] = sqrtf(key_dist2(key));
+        out_idx[(size_t)(row0 + j) * ld_out + q0 + qi] = key_index(key);
+        if (lb_out && j == k - 1) lb_out[q0 + qi] = key + 1;
     }
 }
 
@@ -199,8 +205,6 @@ __global__ void knn_merge_splits_kernel(const unsigned long long *__restrict__ p
 // Host side
 // ---------------------------------------------------------------------------
 namespace {
-
-constexpr size_t kMergeSmemMax = 200u * 1024u;   // dynamic smem limit of the merge kernel
 
 struct ExactShape {
     int qpw, kcap, bq, splits, n_rtiles, n_dchunks;
@@ -236,8 +240,7 @@ bool choose_shape(int N, int Q, int d, int k_all, int num_sms, ExactShape &s) {
     const double warm = 256.0 / (s.n_dchunks * EX_BD);
     int best = 1;
     double best_t = 1e300;
-    // up to 256 splits, while each query's merge input (splits * k keys) fits
-    // one warp's shared-memory slab in the merge kernel
+    // up to 256 splits and 20480 list entries per query
     int max_s = std::min(s.n_rtiles, std::min(256, (160 * 1024) / (8 * k)));
     // keep the per-split partial lists under 1 GiB of scratch
     const long long per_split = (long long)Q * k * 8;
@@ -276,18 +279,25 @@ static long long qdup_pitch2(int Q) { return ((long long)Q + 31) / 32 * 32; }
 int launch_split_merge(const unsigned long long *part, int S, int Q, int k, float *out_dist,
                        int *out_idx, long long ld_out, cudaStream_t st, int row0,
                        unsigned long long *lb_out) {
-    const size_t per_warp = (size_t)S * k * 8;
-    const int wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (160u * 1024u) / per_warp));
-    const size_t smem = per_warp * wpb;
-    if (smem > kMergeSmemMax) return kErrUnsupported;
-    // one fixed limit for every launch: calls from several host threads must
-    // not lower it between another call's set and launch
-    if (cudaFuncSetAttribute(knn_merge_splits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kMergeSmemMax) != cudaSuccess)
-        return kErrLaunch;
-    knn_merge_splits_kernel<<<(Q + wpb - 1) / wpb, wpb * 32, smem, st>>>(
-        part, S, Q, k, out_dist, out_idx, ld_out, row0, lb_out);
-    return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
+    if (k > kPassRanks) return kErrUnsupported;
+    // all eight warps on one query: 14.6 us against 51.9 with one warp a query at
+    // 40 queries and 148 lists of 50 keys, 15.4 against 22.7 at 300 queries and 29
+    // lists of 100; at 1000 queries and 9 lists one warp a query takes 10.7
+    const bool wide = Q <= 1024 && S >= 16;
+    auto go = [&](auto kern, int qpb) {
+        kern<<<(Q + qpb - 1) / qpb, 32 * MG_WARPS, 0, st>>>(part, S, Q, k, out_dist, out_idx,
+                                                            ld_out, row0, lb_out);
+        return cudaGetLastError() == cudaSuccess ? (int)kOk : (int)kErrLaunch;
+    };
+    auto pick = [&](auto cap) {
+        constexpr int C = decltype(cap)::value;
+        return wide ? go(knn_merge_splits_kernel<C, MG_WARPS>, 1)
+                    : go(knn_merge_splits_kernel<C, 1>, MG_WARPS);
+    };
+    if (k <= 32) return pick(std::integral_constant<int, 32>());
+    if (k <= 64) return pick(std::integral_constant<int, 64>());
+    if (k <= 128) return pick(std::integral_constant<int, 128>());
+    return pick(std::integral_constant<int, 256>());
 }
 
 // Scratch of the exact path: the (q, q)-duplicated queries, 256 bytes of

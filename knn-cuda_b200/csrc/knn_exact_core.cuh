@@ -295,15 +295,73 @@ KNN_DI void select_tile(unsigned long long *wl, uint32_t &nb, f32x2_t (&acc)[QPW
     select_tile<QPW, KCAP, false>(wl, nb, acc, rt, N, k, lane, none);
 }
 
-// Number of elements of sorted A[0..n) below x.
-KNN_DI int rank_sorted(const unsigned long long *A, int n, unsigned long long x) {
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (A[mid] < x) lo = mid + 1;
-        else hi = mid;
+// ---------------------------------------------------------------------------
+// Merge of the per-split sorted key lists of one query, by one warp: a running
+// list of the k smallest keys takes one split's list after the other.  Only the
+// keys below the running k-th key (a prefix, since the list is sorted; about
+// k / t keys of the t-th list) are merged: every key's position is its index
+// plus its rank in the other list.  The next list's keys are loaded while this
+// one is merged.
+// ---------------------------------------------------------------------------
+template <int KCAP, int NC>   // the first n <= 32 NC keys of v
+KNN_DI void merge_prefix(unsigned long long *L, unsigned long long *C,
+                         const unsigned long long (&v)[KCAP / 32], int n, int k, int lane) {
+    constexpr int LPL = KCAP / 32;
+    unsigned long long lv[LPL];
+    int lp[LPL], cp[NC];
+#pragma unroll
+    for (int b = 0; b < NC; ++b) C[b * 32 + lane] = b * 32 + lane < n ? v[b] : kKeyInf;
+#pragma unroll
+    for (int a = 0; a < LPL; ++a) lv[a] = L[a * 32 + lane];
+    __syncwarp();
+    // equal keys (entries without a point) keep the running list's first
+#pragma unroll
+    for (int a = 0; a < LPL; ++a) lp[a] = a * 32 + lane + rank_pow2<32 * NC>(C, lv[a]);
+#pragma unroll
+    for (int b = 0; b < NC; ++b) cp[b] = b * 32 + lane + rank_pow2<KCAP>(L, v[b] + 1);
+    __syncwarp();
+#pragma unroll
+    for (int a = 0; a < LPL; ++a)
+        if (lp[a] < k) L[lp[a]] = lv[a];
+#pragma unroll
+    for (int b = 0; b < NC; ++b)
+        if (b * 32 + lane < n && cp[b] < k) L[cp[b]] = v[b];
+    __syncwarp();
+}
+
+// L (KCAP keys) receives the k smallest keys of the lists t0, t0 + step, ...
+// below S; list t starts at src + t * pitch.  C: KCAP keys of scratch.
+template <int KCAP>
+KNN_DI void merge_lists(unsigned long long *L, unsigned long long *C,
+                        const unsigned long long *src, size_t pitch, int t0, int step, int S,
+                        int k, int lane) {
+    constexpr int LPL = KCAP / 32;
+    unsigned long long nxt[LPL], cur[LPL];
+    auto load = [&](unsigned long long (&v)[LPL], int t) {
+#pragma unroll
+        for (int a = 0; a < LPL; ++a) {
+            const int j = a * 32 + lane;
+            v[a] = t < S && j < k ? src[(size_t)t * pitch + j] : kKeyInf;
+        }
+    };
+    load(cur, t0);
+#pragma unroll
+    for (int a = 0; a < LPL; ++a) L[a * 32 + lane] = cur[a];
+    __syncwarp();
+    load(nxt, t0 + step);
+    for (int t = t0 + step; t < S; t += step) {
+#pragma unroll
+        for (int a = 0; a < LPL; ++a) cur[a] = nxt[a];
+        load(nxt, t + step);
+        const unsigned long long tau = L[k - 1];
+        int n = 0;
+#pragma unroll
+        for (int a = 0; a < LPL; ++a)
+            n += __popc(__ballot_sync(0xffffffffu, cur[a] < tau));
+        if (n == 0) continue;
+        if (LPL == 1 || n <= 32) merge_prefix<KCAP, 1>(L, C, cur, n, k, lane);
+        else merge_prefix<KCAP, LPL>(L, C, cur, n, k, lane);
     }
-    return lo;
 }
 
 }  // namespace knnb200
