@@ -34,11 +34,12 @@ struct BatchProb {
     int n_rtiles, n_splits, n_dchunks, qtiles;
     long long item_begin;     // first work item of this problem
     long long merge_begin;    // first merge task (one per query) or -1
-    int row_begin;            // first row of the query-duplication pass
-    const float *qry;
+    int row_begin;            // first row of the query-copy pass (its own rows only
+                              // where the queries are copied)
+    const float *qry;         // the caller's queries
     long long ldq;
-    float2 *qdup;
-    long long ld2;
+    float *qcopy;             // their aligned copy, nullptr where they are read in place
+    long long ldc;
     float *out_dist;
     int *out_idx;
     long long ld_out;
@@ -62,24 +63,24 @@ KNN_DI int find_record(int n, long long x, F key) {
     return lo;
 }
 
-// Query duplication for every problem: one block per (problem, dimension) row.
-__global__ void batched_dup_kernel(const BatchProb *__restrict__ probs, int n_probs,
-                                   int n_rows) {
+// Aligned copies of the query sets that TMA cannot read in place (base or row
+// pitch not a multiple of 16 bytes): one block per (problem, dimension) row.
+__global__ void batched_copy_kernel(const BatchProb *__restrict__ probs, int n_probs,
+                                    int n_rows) {
     const int row = blockIdx.x;
     if (row >= n_rows) return;
     const int p = find_record(n_probs, row, [&](int i) { return (long long)probs[i].row_begin; });
     const BatchProb P = probs[p];
+    if (!P.qcopy) return;
     const int dd = row - P.row_begin;
-    for (int i = threadIdx.x; i < P.Q; i += blockDim.x) {
-        const float v = P.qry[(size_t)dd * P.ldq + i];
-        P.qdup[(size_t)dd * P.ld2 + i] = make_float2(v, v);
-    }
+    for (int i = threadIdx.x; i < P.Q; i += blockDim.x)
+        P.qcopy[(size_t)dd * P.ldc + i] = P.qry[(size_t)dd * P.ldq + i];
 }
 
 template <int QPW, int KCAP>
 struct BatchCfg {
     using C = ExCfg<QPW, KCAP>;
-    static constexpr size_t ITEM_OFFSET = C::BAR_OFFSET + 2 * EX_STAGES * 8 + 64;
+    static constexpr size_t ITEM_OFFSET = C::BAR_OFFSET + 2 * C::STAGES * 8 + 64;
     static constexpr size_t SMEM = 1024 + ITEM_OFFSET + 2 * sizeof(ItemInfo) + 4 * 8 + 64;
     static_assert(SMEM <= 232448, "shared memory per CTA");
 };
@@ -96,17 +97,17 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     float *stages = reinterpret_cast<float *>(base);
     unsigned long long *lists =
-        reinterpret_cast<unsigned long long *>(base + (size_t)EX_STAGES * C::STAGE_BYTES);
+        reinterpret_cast<unsigned long long *>(base + (size_t)C::STAGES * C::STAGE_BYTES);
     uint64_t *full = reinterpret_cast<uint64_t *>(base + C::BAR_OFFSET);
-    uint64_t *empty = full + EX_STAGES;
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(empty + EX_STAGES);
+    uint64_t *empty = full + C::STAGES;
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(empty + C::STAGES);
     ItemInfo *items = reinterpret_cast<ItemInfo *>(base + B::ITEM_OFFSET);
     uint64_t *item_full = reinterpret_cast<uint64_t *>(items + 2);
     uint64_t *item_empty = item_full + 2;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int s = 0; s < EX_STAGES; ++s) {
+        for (int s = 0; s < C::STAGES; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], EX_WARPS);
         }
@@ -151,9 +152,9 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
                 bool ok = true;
                 for (int rt = t0; rt < t1 && ok; ++rt)
                     for (int dc = 0; dc < P.n_dchunks; ++dc, ++it) {
-                        const int s = it % EX_STAGES;
-                        if (it >= EX_STAGES &&
-                            !mbar_wait(&empty[s], ((it / EX_STAGES) - 1) & 1)) {
+                        const int s = it % C::STAGES;
+                        if (it >= C::STAGES &&
+                            !mbar_wait(&empty[s], ((it / C::STAGES) - 1) & 1)) {
                             atomicMax(status, (int)kDevTimeoutEmpty);
                             *abort_flag = 1;
                             ok = false;
@@ -166,14 +167,14 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
                         float *qs = stages + (size_t)s * C::STAGE_FLOATS;
                         float *rs = qs + C::Q_FLOATS;
                         mbar_arrive_expect_tx(&full[s], C::STAGE_BYTES);
-                        tma_load_2d(qs, mq, &full[s], inf.qtile * 2 * C::BQ, dc * EX_BD);
+                        tma_load_2d(qs, mq, &full[s], inf.qtile * C::BQ, dc * EX_BD);
                         tma_load_2d(rs, mr, &full[s], rt * EX_BR, dc * EX_BD);
                         issued = it + 1;
                     }
                 if (!ok) break;
             }
-            for (int i = max(0, issued - EX_STAGES); i < issued; ++i)
-                if (!mbar_wait(&full[i % EX_STAGES], (i / EX_STAGES) & 1))
+            for (int i = max(0, issued - C::STAGES); i < issued; ++i)
+                if (!mbar_wait(&full[i % C::STAGES], (i / C::STAGES) & 1))
                     atomicMax(status, (int)kDevTimeoutDrain);
         }
         return;
@@ -299,7 +300,7 @@ struct knnb200_batched_plan {
     std::vector<ExactProblem> lowdim;                // problems routed to the low-d kernel
     long long n_items = 0, n_tasks = 0;
     DevMem tables;      // BatchProb[count] | CUtensorMap[2*count] | counter, status | mlist
-    DevMem scratch;     // qdup + parts
+    DevMem scratch;     // query copies + parts
     BatchProb *probs = nullptr;
     CUtensorMap *maps = nullptr;
     unsigned long long *counter = nullptr;
@@ -319,6 +320,10 @@ cudaError_t launch_batched_t(const knnb200_batched_plan *pl, cudaStream_t st) {
     kern<<<pl->num_sms, EX_THREADS, B::SMEM, st>>>(pl->maps, pl->probs, pl->count, pl->n_items,
                                                    pl->counter, pl->status);
     return cudaGetLastError();
+}
+
+bool needs_copy(const knnb200_problem &q) {
+    return (reinterpret_cast<uintptr_t>(q.query) & 15) || q.query_ld % 4;
 }
 
 int validate(const knnb200_problem &q) {
@@ -396,7 +401,7 @@ int knnb200_batched_plan_create_config(const knnb200_problem *all, int n_all,
         P.n_splits = std::max(1, S);
         P.qry = q.query;
         P.ldq = q.query_ld;
-        P.ld2 = round_up(q.query_nb, 32);
+        P.ldc = round_up(q.query_nb, 32);
         P.out_dist = q.knn_dist;
         P.out_idx = q.knn_index;
         P.ld_out = q.out_ld;
@@ -407,14 +412,15 @@ int knnb200_batched_plan_create_config(const knnb200_problem *all, int n_all,
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
 
-    // scratch: duplicated queries + per-split lists; then the low-d
+    // scratch: query copies + per-split lists; then the low-d
     // problems' split lists
     size_t sbytes = 0;
-    std::vector<size_t> dup_off(count), part_off(count), low_off(low_idx.size());
+    std::vector<size_t> copy_off(count), part_off(count), low_off(low_idx.size());
     for (int i = 0; i < count; ++i) {
         BatchProb &P = recs[i];
-        dup_off[i] = sbytes;
-        sbytes += round_up((long long)P.d * P.ld2 * sizeof(float2), 256);
+        copy_off[i] = sbytes;
+        if (needs_copy(in[i]))
+            sbytes += round_up((long long)P.d * P.ldc * (long long)sizeof(float), 256);
         part_off[i] = sbytes;
         if (P.n_splits > 1) sbytes += round_up((long long)P.n_splits * P.Q * P.k * 8, 256);
     }
@@ -448,7 +454,7 @@ int knnb200_batched_plan_create_config(const knnb200_problem *all, int n_all,
         const int i = order[r];
         BatchProb P = recs[i];
         const knnb200_problem &q = in[i];
-        P.qdup = reinterpret_cast<float2 *>(sb + dup_off[i]);
+        P.qcopy = needs_copy(q) ? reinterpret_cast<float *>(sb + copy_off[i]) : nullptr;
         P.part = P.n_splits > 1 ? reinterpret_cast<unsigned long long *>(sb + part_off[i]) : nullptr;
         P.item_begin = item;
         item += (long long)P.qtiles * P.n_splits;
@@ -458,11 +464,11 @@ int knnb200_batched_plan_create_config(const knnb200_problem *all, int n_all,
             task += P.Q;
         }
         P.row_begin = row;
-        row += P.d;
+        if (P.qcopy) row += P.d;
         if (!encode_f32_2d(&maps[2 * r], q.ref, (uint64_t)P.N, (uint64_t)P.d, (uint64_t)q.ref_ld,
                            EX_BR, EX_BD) ||
-            !encode_f32_2d(&maps[2 * r + 1], P.qdup, (uint64_t)(2 * P.Q), (uint64_t)P.d,
-                           (uint64_t)(2 * P.ld2), 2 * bq, EX_BD)) {
+            !encode_f32_2d(&maps[2 * r + 1], P.qcopy ? P.qcopy : P.qry, (uint64_t)P.Q,
+                           (uint64_t)P.d, (uint64_t)(P.qcopy ? P.ldc : P.ldq), bq, EX_BD)) {
             delete pl;
             return KNNB200_ETENSORMAP;
         }
@@ -537,8 +543,10 @@ int knnb200_batched_run(knnb200_batched_plan *pl, void *stream) {
     for (const ExactProblem &e : pl->lowdim)
         if (launch_lowdim(e, st) != kOk) return KNNB200_ELAUNCH;
     if (pl->count == 0) return KNNB200_OK;
-    batched_dup_kernel<<<pl->n_rows, 256, 0, st>>>(pl->probs, pl->count, pl->n_rows);
-    if (cudaGetLastError() != cudaSuccess) return KNNB200_ELAUNCH;
+    if (pl->n_rows > 0) {
+        batched_copy_kernel<<<pl->n_rows, 256, 0, st>>>(pl->probs, pl->count, pl->n_rows);
+        if (cudaGetLastError() != cudaSuccess) return KNNB200_ELAUNCH;
+    }
     cudaError_t e;
     if (pl->kcap == 256) {
         e = launch_batched_t<EX_QPW_K256, 256>(pl, st);

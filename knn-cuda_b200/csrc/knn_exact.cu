@@ -53,10 +53,10 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     float *stages = reinterpret_cast<float *>(base);
     unsigned long long *lists =
-        reinterpret_cast<unsigned long long *>(base + (size_t)EX_STAGES * C::STAGE_BYTES);
+        reinterpret_cast<unsigned long long *>(base + (size_t)C::STAGES * C::STAGE_BYTES);
     uint64_t *full = reinterpret_cast<uint64_t *>(base + C::BAR_OFFSET);
-    uint64_t *empty = full + EX_STAGES;
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(empty + EX_STAGES);
+    uint64_t *empty = full + C::STAGES;
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(empty + C::STAGES);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int qtile = blockIdx.x, split = blockIdx.y;
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
     const int total = (t1 - t0) * a.n_dchunks;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < EX_STAGES; ++s) {
+        for (int s = 0; s < C::STAGES; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], EX_WARPS);
         }
@@ -81,8 +81,8 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
             prefetch_tensormap(&tm_qry);
             int issued = 0;
             for (int it = 0; it < total; ++it) {
-                const int s = it % EX_STAGES;
-                if (it >= EX_STAGES && !mbar_wait(&empty[s], ((it / EX_STAGES) - 1) & 1)) {
+                const int s = it % C::STAGES;
+                if (it >= C::STAGES && !mbar_wait(&empty[s], ((it / C::STAGES) - 1) & 1)) {
                     atomicMax(a.status, (int)kDevTimeoutEmpty);
                     *abort_flag = 1;
                     break;
@@ -92,13 +92,13 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
                 float *rs = qs + C::Q_FLOATS;
                 const int rt = t0 + it / a.n_dchunks, dc = it % a.n_dchunks;
                 mbar_arrive_expect_tx(&full[s], C::STAGE_BYTES);
-                tma_load_2d(qs, &tm_qry, &full[s], qtile * 2 * C::BQ, dc * EX_BD);
+                tma_load_2d(qs, &tm_qry, &full[s], qtile * C::BQ, dc * EX_BD);
                 tma_load_2d(rs, &tm_ref, &full[s], rt * EX_BR, dc * EX_BD);
                 issued = it + 1;
             }
             // Never leave with copies in flight: wait for the last issued stages.
-            for (int it = max(0, issued - EX_STAGES); it < issued; ++it)
-                if (!mbar_wait(&full[it % EX_STAGES], (it / EX_STAGES) & 1))
+            for (int it = max(0, issued - C::STAGES); it < issued; ++it)
+                if (!mbar_wait(&full[it % C::STAGES], (it / C::STAGES) & 1))
                     atomicMax(a.status, (int)kDevTimeoutDrain);
         }
         return;
@@ -152,18 +152,14 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
     }
 }
 
-// Duplicate every query value into a (q, q) pair: dst[d][2i] = dst[d][2i+1]
-// = src[d][i].
-__global__ void dup_queries_kernel(const float *__restrict__ src, int Q, long long lds, int d,
-                                   float2 *__restrict__ dst, long long ldd2) {
+// Copy of a query set whose rows TMA cannot read in place (base or row pitch
+// not a multiple of 16 bytes).
+__global__ void copy_queries_kernel(const float *__restrict__ src, int Q, long long lds,
+                                    float *__restrict__ dst, long long ldd) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int dd = blockIdx.y;
-    if (i < Q) {
-        const float v = src[(size_t)dd * lds + i];
-        dst[(size_t)dd * ldd2 + i] = make_float2(v, v);
-    }
+    if (i < Q) dst[(size_t)dd * ldd + i] = src[(size_t)dd * lds + i];
 }
-
 
 // Merge the per-split sorted key lists of each query (merge_lists).  A block of
 // eight warps takes 8 / WPQ consecutive queries, WPQ warps each: one warp a
@@ -273,8 +269,8 @@ cudaError_t launch_t(const CUtensorMap &mr, const CUtensorMap &mq, const ExactAr
 
 }  // namespace
 
-// Row pitch (in float2) of the duplicated query copy.
-static long long qdup_pitch2(int Q) { return ((long long)Q + 31) / 32 * 32; }
+// Row pitch of the query copy, in floats.
+static long long qcopy_pitch(int Q) { return ((long long)Q + 31) / 32 * 32; }
 
 int launch_split_merge(const unsigned long long *part, int S, int Q, int k, float *out_dist,
                        int *out_idx, long long ld_out, cudaStream_t st, int row0,
@@ -300,13 +296,15 @@ int launch_split_merge(const unsigned long long *part, int S, int Q, int k, floa
     return pick(std::integral_constant<int, 256>());
 }
 
-// Scratch of the exact path: the (q, q)-duplicated queries, 256 bytes of
-// alignment, the per-split key lists of one pass when the reference set is
-// split, and for k > 256 the per-query lower-bound keys of the passes.
+// Scratch of the exact path: room for two copies of the queries (one is used,
+// and only when theirs cannot be read in place; the size is what callers of
+// the allocation-free entry plan with), 256 bytes of alignment, the per-split
+// key lists of one pass when the reference set is split, and for k > 256 the
+// per-query lower-bound keys of the passes.
 static size_t exact_need(const ExactShape &s, int Q, int d, int k, size_t *part_off,
                          size_t *lb_off) {
     const int kp = std::min(k, kPassRanks);
-    const size_t dup = (size_t)d * qdup_pitch2(Q) * sizeof(float2);
+    const size_t dup = (size_t)d * qcopy_pitch(Q) * 2 * sizeof(float);
     const size_t off = (dup + 255) & ~size_t(255);
     const size_t part = s.splits > 1 ? (size_t)s.splits * Q * kp * 8 : 0;
     const size_t lb = k > kPassRanks ? (size_t)Q * 8 : 0;
@@ -329,22 +327,29 @@ int launch_exact(const ExactProblem &p, cudaStream_t st) {
     ExactShape s;
     if (!choose_shape(p.N, p.Q, p.d, p.k, p.num_sms, s)) return kErrUnsupported;
     if (p.force_splits > 0) s.splits = std::min(p.force_splits, std::min(s.n_rtiles, 256));
-    const long long ld2 = qdup_pitch2(p.Q);
     size_t part_off = 0, lb_off = 0;
     if (exact_need(s, p.Q, p.d, p.k, &part_off, &lb_off) > p.scratch_bytes) return kErrScratch;
-    float2 *qdup = static_cast<float2 *>(p.scratch);
     unsigned char *sb = static_cast<unsigned char *>(p.scratch);
     unsigned long long *part = reinterpret_cast<unsigned long long *>(sb + part_off);
     unsigned long long *lb = reinterpret_cast<unsigned long long *>(sb + lb_off);
-    dup_queries_kernel<<<dim3((p.Q + 255) / 256, p.d), 256, 0, st>>>(p.qry, p.Q, p.ldq, p.d, qdup,
-                                                                   ld2);
-    if (cudaGetLastError() != cudaSuccess) return kErrLaunch;
+    const float *qry = p.qry;
+    long long ldq = p.ldq;
+    if ((reinterpret_cast<uintptr_t>(qry) & 15) || ldq % 4) {
+        float *copy = static_cast<float *>(p.scratch);
+        ldq = qcopy_pitch(p.Q);
+        // rows on gridDim.y (at most 65535 of them a launch)
+        for (int d0 = 0; d0 < p.d; d0 += 65535) {
+            const dim3 grid((p.Q + 255) / 256, std::min(65535, p.d - d0));
+            copy_queries_kernel<<<grid, 256, 0, st>>>(p.qry + (size_t)d0 * p.ldq, p.Q, p.ldq,
+                                                      copy + (size_t)d0 * ldq, ldq);
+        }
+        if (cudaGetLastError() != cudaSuccess) return kErrLaunch;
+        qry = copy;
+    }
 
     CUtensorMap mr, mq;
-    if (!encode_f32_2d(&mr, p.ref, (uint64_t)p.N, (uint64_t)p.d, (uint64_t)p.ldr, EX_BR, EX_BD))
-        return kErrTensorMap;
-    if (!encode_f32_2d(&mq, qdup, (uint64_t)(2 * p.Q), (uint64_t)p.d, (uint64_t)(2 * ld2),
-                       2 * s.bq, EX_BD))
+    if (!encode_f32_2d(&mr, p.ref, (uint64_t)p.N, (uint64_t)p.d, (uint64_t)p.ldr, EX_BR, EX_BD) ||
+        !encode_f32_2d(&mq, qry, (uint64_t)p.Q, (uint64_t)p.d, (uint64_t)ldq, s.bq, EX_BD))
         return kErrTensorMap;
 
     ExactArgs a;

@@ -14,21 +14,20 @@ constexpr int EX_WARPS = 16;     // consumer warps
 constexpr int EX_QPW = 4;        // queries per warp for k <= 128
 constexpr int EX_QPW_K256 = 2;   // queries per warp for 128 < k <= 256
 constexpr int EX_THREADS = (EX_WARPS + 1) * 32;
-constexpr int EX_STAGES = 4;
 
 template <int QPW, int KCAP>
 struct ExCfg {
     static constexpr int BQ = QPW * EX_WARPS;
-    // query slab of a stage: each query value stored twice, (q, q), so a
-    // 64-bit shared load yields a ready packed operand
-    static constexpr int Q_FLOATS = EX_BD * 2 * BQ;
+    // ring depth: what the lists leave of the shared memory
+    static constexpr int STAGES = KCAP == 128 && QPW == 4 ? 4 : 6;
+    static constexpr int Q_FLOATS = EX_BD * BQ;   // query slab of a stage
     static constexpr int R_FLOATS = EX_BD * EX_BR;
     static constexpr int STAGE_FLOATS = Q_FLOATS + R_FLOATS;
     static constexpr int STAGE_BYTES = STAGE_FLOATS * 4;
     static constexpr int REGION = KCAP + EX_CB;   // keys per query: list + candidates
     static constexpr size_t LIST_BYTES = (size_t)BQ * REGION * 8;
-    static constexpr size_t BAR_OFFSET = (size_t)EX_STAGES * STAGE_BYTES + LIST_BYTES;
-    static constexpr size_t SMEM = 1024 + BAR_OFFSET + 2 * EX_STAGES * 8 + 16;
+    static constexpr size_t BAR_OFFSET = (size_t)STAGES * STAGE_BYTES + LIST_BYTES;
+    static constexpr size_t SMEM = 1024 + BAR_OFFSET + 2 * STAGES * 8 + 16;
     static_assert(STAGE_BYTES % 1024 == 0, "stage alignment");
     static_assert(SMEM <= 232448, "shared memory per CTA");
     static_assert(KCAP % 32 == 0 && (KCAP & (KCAP - 1)) == 0, "KCAP power of two >= 32");
@@ -219,10 +218,29 @@ KNN_DI void select_half(unsigned long long *wl, uint32_t &nb, D2 d2, uint32_t rb
 }
 
 
+// The warp's QPW queries of one dimension (one broadcast load).
+template <int QPW>
+KNN_DI void load_queries(float (&q)[QPW], const float *src) {
+    static_assert(QPW == 4 || QPW == 2, "one vector load");
+    if (QPW == 4) {
+        const float4 v = *reinterpret_cast<const float4 *>(src);
+        q[0] = v.x; q[1] = v.y; q[QPW - 2] = v.z; q[QPW - 1] = v.w;
+    } else {
+        const float2 v = *reinterpret_cast<const float2 *>(src);
+        q[0] = v.x; q[1] = v.y;
+    }
+}
+
 // Consume the n_dchunks pipeline stages of one reference tile: the lane's
 // QPW x 8 block of squared distances accumulates sum_d (r_d - q_d)^2 with a
 // rounded sub and a fused multiply-add per dimension, in increasing d (the
 // order of the reference's compute_distances loop, code/knncuda.cu:77-80).
+// Bound by the FP32 pipe: 32 packed operations a warp and dimension take 16
+// cycles of an SM.  The shared loads return 128 B a cycle whatever lanes share:
+// two loads of references and one of the four queries take 12.  (Queries kept
+// as (q, q) pairs in shared memory saved the register moves but took 16: 298
+// against 289 ms at 2^20 x 16384, d = 256, k = 100, 814 against 764 us at
+// 16384 x 4096, d = 128, k = 16.)
 // `it` is the running stage counter of the CTA's ring.  Returns false (warp-
 // uniformly) if a wait timed out or another warp aborted.
 template <int QPW, int KCAP>
@@ -235,8 +253,8 @@ KNN_DI bool consume_ref_tile(f32x2_t (&acc)[QPW][4], const float *stages, uint64
 #pragma unroll
         for (int p = 0; p < 4; ++p) acc[i][p] = 0ull;
     for (int dc = 0; dc < n_dchunks; ++dc, ++it) {
-        const int s = it % EX_STAGES;
-        const bool got = mbar_wait(&full[s], (it / EX_STAGES) & 1);
+        const int s = it % C::STAGES;
+        const bool got = mbar_wait(&full[s], (it / C::STAGES) & 1);
         // warp-uniform decision: every lane leaves together or none does.
         // No per-stage check of the abort flag: when another warp gives up,
         // the producer stops refilling and this wait ends by its time limit.
@@ -247,7 +265,7 @@ KNN_DI bool consume_ref_tile(f32x2_t (&acc)[QPW][4], const float *stages, uint64
             }
             return false;
         }
-        const float *qs = stages + (size_t)s * C::STAGE_FLOATS + warp * 2 * QPW;
+        const float *qs = stages + (size_t)s * C::STAGE_FLOATS + warp * QPW;
         const float *rs = stages + (size_t)s * C::STAGE_FLOATS + C::Q_FLOATS + lane * 4;
 #pragma unroll
         for (int dd = 0; dd < EX_BD; ++dd) {
@@ -255,10 +273,11 @@ KNN_DI bool consume_ref_tile(f32x2_t (&acc)[QPW][4], const float *stages, uint64
             const ulonglong2 ra = *reinterpret_cast<const ulonglong2 *>(rs + dd * EX_BR);
             const ulonglong2 rb = *reinterpret_cast<const ulonglong2 *>(rs + dd * EX_BR + 128);
             const f32x2_t r0 = ra.x, r1 = ra.y, r2 = rb.x, r3 = rb.y;
-            const f32x2_t *qp = reinterpret_cast<const f32x2_t *>(qs + dd * 2 * C::BQ);
+            float q[QPW];
+            load_queries<QPW>(q, qs + dd * C::BQ);
 #pragma unroll
             for (int i = 0; i < QPW; ++i) {
-                const f32x2_t qq = qp[i];   // (q_i, q_i)
+                const f32x2_t qq = f2_pack(q[i], q[i]);
                 f32x2_t t;
                 t = f2_sub(r0, qq); acc[i][0] = f2_fma(t, t, acc[i][0]);
                 t = f2_sub(r1, qq); acc[i][1] = f2_fma(t, t, acc[i][1]);
