@@ -182,6 +182,9 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
 
     // -------------------- consumer warps ------------------------------------
     unsigned long long *wl = lists + (size_t)warp * QPW * C::REGION;
+    unsigned long long *wt =
+        reinterpret_cast<unsigned long long *>(base + C::TAU_OFFSET) + warp * QPW;
+    const unsigned long long no_lb[QPW] = {};
     int it = 0;
     for (int n = 0;; ++n) {
         const int slot = n & 1;
@@ -198,9 +201,8 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
         if (lane == 0) mbar_arrive(&item_empty[slot]);
         if (inf.idx >= n_items) break;
         const BatchProb P = probs[inf.p];
-        for (int i = lane; i < QPW * C::REGION; i += 32) wl[i] = kKeyInf;
-        __syncwarp();
-        uint32_t nb = 0;   // candidate buffer fills
+        unsigned long long nb;   // buffer fills
+        select_start<QPW>(wt, nb, inf.qtile * C::BQ + warp * QPW, P.Q, lane);
         const int t0 = (int)((long long)P.n_rtiles * inf.split / P.n_splits);
         const int t1 = (int)((long long)P.n_rtiles * (inf.split + 1) / P.n_splits);
         bool alive = true;
@@ -211,30 +213,30 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
                 alive = false;
                 break;
             }
-            select_tile<QPW, KCAP>(wl, nb, acc, rt, P.N, P.k, lane);
+            select_tile<QPW, KCAP, false>(wl, wt, nb, acc, rt, P.N, P.k, lane, no_lb);
         }
-        flush_all<QPW, KCAP>(wl, nb, P.k, lane);
-        consumer_sync();
+        select_finish<QPW, KCAP>(wl, wt, nb, P.k, lane);
         if (!alive || *abort_flag) break;
-        const int q0 = inf.qtile * C::BQ;
+        // each warp writes its own queries, so that no warp waits for the
+        // others at the end of an item
+        const int q0 = inf.qtile * C::BQ + warp * QPW;
+        const int nq = min(QPW, P.Q - q0);
         if (P.n_splits == 1) {
-            for (int e = threadIdx.x; e < P.k * C::BQ; e += EX_WARPS * 32) {
-                const int j = e / C::BQ, qi = e - j * C::BQ, q = q0 + qi;
-                if (q < P.Q) {
-                    const unsigned long long key = lists[(size_t)qi * C::REGION + j];
-                    P.out_dist[(size_t)j * P.ld_out + q] = sqrtf(key_dist2(key));
-                    P.out_idx[(size_t)j * P.ld_out + q] = key_index(key);
+            for (int j = lane; j < P.k; j += 32)
+#pragma unroll
+                for (int i = 0; i < QPW; ++i) {
+                    if (i >= nq) break;
+                    const unsigned long long key = wl[i * C::REGION + j];
+                    P.out_dist[(size_t)j * P.ld_out + q0 + i] = sqrtf(key_dist2(key));
+                    P.out_idx[(size_t)j * P.ld_out + q0 + i] = key_index(key);
                 }
-            }
         } else {
-            for (int i = 0; i < QPW; ++i) {
-                const int q = q0 + warp * QPW + i;
-                if (q >= P.Q) break;
-                unsigned long long *dst = P.part + ((size_t)inf.split * P.Q + q) * P.k;
+            for (int i = 0; i < nq; ++i) {
+                unsigned long long *dst = P.part + ((size_t)inf.split * P.Q + q0 + i) * P.k;
                 for (int j = lane; j < P.k; j += 32) dst[j] = wl[i * C::REGION + j];
             }
         }
-        consumer_sync();   // lists are rewritten by the next item
+        __syncwarp();   // the buffers are rewritten by the next item
     }
 }
 

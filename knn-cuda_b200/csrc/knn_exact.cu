@@ -15,12 +15,12 @@
 //     multiply-add per dimension, in increasing d -- the arithmetic and
 //     order of the reference's compute_distances inner loop
 //     (code/knncuda.cu:77-80), so squared distances are bit-identical to it.
-//   * Selection is warp-local.  Each query keeps its k smallest
-//     (distance, index) keys sorted in shared memory; the k-th key is the
-//     threshold.  After each half tile the warp ballots the keys below it
-//     into a 128-slot candidate buffer, which is merged into the list only
-//     when it would overflow (a register bitonic sort of the buffer, then
-//     every key placed at its index plus its rank in the other array).
+//   * Selection is warp-local.  Each query has an unsorted buffer of candidate
+//     keys (distance, index) and a threshold in shared memory.  After each tile
+//     the warp ballots the keys below the threshold into the buffer; when they
+//     would not fit, a bisection over the buffered distances lowers the
+//     threshold to one that keeps the k smallest and few more (buf_select).
+//     The buffer is sorted once, at the end of the CTA's range.
 //     Ordering by the 64-bit key (distance bits, index) reproduces the
 //     reference's tie rule: equal distances keep the lower index
 //     (code/knncuda.cu:172, :178).
@@ -106,9 +106,10 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
 
     // -------------------- consumer warps ------------------------------------
     unsigned long long *wl = lists + (size_t)warp * QPW * C::REGION;
-    for (int i = lane; i < QPW * C::REGION; i += 32) wl[i] = kKeyInf;
-    __syncwarp();
-    uint32_t nb = 0;   // candidate buffer fills
+    unsigned long long *wt =
+        reinterpret_cast<unsigned long long *>(base + C::TAU_OFFSET) + warp * QPW;
+    unsigned long long nb;   // buffer fills
+    select_start<QPW>(wt, nb, qtile * C::BQ + warp * QPW, a.Q, lane);
     unsigned long long lbk[QPW];
 #pragma unroll
     for (int i = 0; i < QPW; ++i) {
@@ -122,9 +123,9 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
         if (!consume_ref_tile<QPW, KCAP>(acc, stages, full, empty, abort_flag, it, a.n_dchunks,
                                          warp, lane, a.status))
             break;
-        select_tile<QPW, KCAP, LB>(wl, nb, acc, rt, a.N, a.k, lane, lbk);
+        select_tile<QPW, KCAP, LB>(wl, wt, nb, acc, rt, a.N, a.k, lane, lbk);
     }
-    flush_all<QPW, KCAP>(wl, nb, a.k, lane);
+    select_finish<QPW, KCAP>(wl, wt, nb, a.k, lane);
 
     consumer_sync();
     if (*abort_flag) return;

@@ -19,14 +19,17 @@ template <int QPW, int KCAP>
 struct ExCfg {
     static constexpr int BQ = QPW * EX_WARPS;
     // ring depth: what the lists leave of the shared memory
-    static constexpr int STAGES = KCAP == 128 && QPW == 4 ? 4 : 6;
+    static constexpr int STAGES = QPW == 2 || KCAP == 32 ? 6 : KCAP == 64 ? 5 : 4;
     static constexpr int Q_FLOATS = EX_BD * BQ;   // query slab of a stage
     static constexpr int R_FLOATS = EX_BD * EX_BR;
     static constexpr int STAGE_FLOATS = Q_FLOATS + R_FLOATS;
     static constexpr int STAGE_BYTES = STAGE_FLOATS * 4;
-    static constexpr int REGION = KCAP + EX_CB;   // keys per query: list + candidates
+    // key slots per query: k <= KCAP, one half tile and a margin of 32, so that
+    // a selection need not find exactly the k smallest (buf_select)
+    static constexpr int REGION = KCAP + EX_CB + 32;
     static constexpr size_t LIST_BYTES = (size_t)BQ * REGION * 8;
-    static constexpr size_t BAR_OFFSET = (size_t)STAGES * STAGE_BYTES + LIST_BYTES;
+    static constexpr size_t TAU_OFFSET = (size_t)STAGES * STAGE_BYTES + LIST_BYTES;
+    static constexpr size_t BAR_OFFSET = TAU_OFFSET + BQ * 8;
     static constexpr size_t SMEM = 1024 + BAR_OFFSET + 2 * STAGES * 8 + 16;
     static_assert(STAGE_BYTES % 1024 == 0, "stage alignment");
     static_assert(SMEM <= 232448, "shared memory per CTA");
@@ -45,18 +48,19 @@ KNN_DI int rank_pow2(const unsigned long long *L, unsigned long long x) {
     return pos + (L[pos] < x ? 1 : 0);
 }
 
-// Ascending bitonic sort of 128 keys held by one warp, four per lane
+// Ascending bitonic sort of 32 CPL keys held by one warp, CPL per lane
 // (element e = b * 32 + lane in v[b]): lane partners by shuffle, register
 // partners in place.
-KNN_DI void warp_sort128(unsigned long long (&v)[4], int lane) {
+template <int CPL>
+KNN_DI void warp_sort(unsigned long long (&v)[CPL], int lane) {
 #pragma unroll
-    for (int size = 2; size <= 128; size <<= 1) {
+    for (int size = 2; size <= 32 * CPL; size <<= 1) {
 #pragma unroll
         for (int stride = size >> 1; stride > 0; stride >>= 1) {
             if (stride >= 32) {
                 const int rs = stride >> 5;
 #pragma unroll
-                for (int b = 0; b < 4; ++b) {
+                for (int b = 0; b < CPL; ++b) {
                     if (b & rs) continue;
                     const bool up = (((b << 5) | lane) & size) == 0;
                     const unsigned long long x = v[b], y = v[b | rs];
@@ -67,29 +71,22 @@ KNN_DI void warp_sort128(unsigned long long (&v)[4], int lane) {
             } else {
                 const bool lower = (lane & stride) == 0;
 #pragma unroll
-                for (int b = 0; b < 4; ++b) {
+                for (int b = 0; b < CPL; ++b) {
                     const bool up = (((b << 5) | lane) & size) == 0;
                     const unsigned long long x = v[b];
                     const unsigned long long y = __shfl_xor_sync(0xffffffffu, x, stride);
-                    const unsigned long long mn = x < y ? x : y, mx = x < y ? y : x;
-                    v[b] = (lower == up) ? mn : mx;
+                    const bool take = (y < x) == (lower == up);
+                    v[b] = take ? y : x;
                 }
             }
         }
     }
 }
 
-// Merge c (<= EX_CB) unsorted candidate keys (L[KCAP .. KCAP+c)) into the
-// sorted list L[0..k) held by one warp.  The candidates are sorted in
-// registers and written back sorted; then every key's final position is its
-// index plus its rank in the other sorted array (binary search).  Keys are
-// unique (distinct indices), so the positions form a permutation; positions
-// >= k are dropped.
-template <int KCAP>
-KNN_DI void warp_merge(unsigned long long *L, int c, int k, int lane) {
+// warp_merge for c <= 32 CPL candidates.
+template <int KCAP, int CPL>
+KNN_DI void warp_merge_n(unsigned long long *L, int c, int k, int lane) {
     constexpr int LPL = KCAP / 32;
-    constexpr int CPL = EX_CB / 32;
-    static_assert(CPL == 4, "warp_sort128 holds four keys per lane");
     unsigned long long *C = L + KCAP;
     unsigned long long lv[LPL], cv[CPL];
 #pragma unroll
@@ -97,7 +94,7 @@ KNN_DI void warp_merge(unsigned long long *L, int c, int k, int lane) {
         const int t = b * 32 + lane;
         cv[b] = t < c ? C[t] : kKeyInf;
     }
-    warp_sort128(cv, lane);
+    warp_sort<CPL>(cv, lane);
 #pragma unroll
     for (int a = 0; a < LPL; ++a) lv[a] = L[a * 32 + lane];
     __syncwarp();
@@ -106,7 +103,7 @@ KNN_DI void warp_merge(unsigned long long *L, int c, int k, int lane) {
     __syncwarp();
     int lp[LPL], cp[CPL];
 #pragma unroll
-    for (int a = 0; a < LPL; ++a) lp[a] = a * 32 + lane + rank_pow2<EX_CB>(C, lv[a]);
+    for (int a = 0; a < LPL; ++a) lp[a] = a * 32 + lane + rank_pow2<32 * CPL>(C, lv[a]);
 #pragma unroll
     for (int b = 0; b < CPL; ++b) cp[b] = b * 32 + lane + rank_pow2<KCAP>(L, cv[b]);
     __syncwarp();
@@ -119,84 +116,198 @@ KNN_DI void warp_merge(unsigned long long *L, int c, int k, int lane) {
     __syncwarp();
 }
 
-// Buffer fill of query i (warp-uniform), one byte per query.
-KNN_DI int nbuf_get(uint32_t nb, int i) { return (int)((nb >> (8 * i)) & 0xffu); }
-KNN_DI uint32_t nbuf_set(uint32_t nb, int i, int v) {
-    return (nb & ~(0xffu << (8 * i))) | ((uint32_t)v << (8 * i));
+// Merge c (<= EX_CB) unsorted candidate keys (L[KCAP .. KCAP+c)) into the
+// sorted list L[0..k) held by one warp.  The candidates are sorted in
+// registers (32, 64 or 128 of them: a sort of 128 takes 28 exchange steps of
+// four keys a lane, one of 32 takes 15 of one) and written back sorted; then
+// every key's final position is its index plus its rank in the other sorted
+// array (binary search).  Keys are unique (distinct indices), so the positions
+// form a permutation; positions >= k are dropped.
+template <int KCAP>
+KNN_DI void warp_merge(unsigned long long *L, int c, int k, int lane) {
+    static_assert(EX_CB == 128, "at most four keys a lane");
+    if (c <= 32) warp_merge_n<KCAP, 1>(L, c, k, lane);
+    else if (c <= 64) warp_merge_n<KCAP, 2>(L, c, k, lane);
+    else warp_merge_n<KCAP, 4>(L, c, k, lane);
 }
 
-// Merge query i's buffered candidates into its list (whose k-th key is the
-// query's threshold tau).
-template <int QPW, int KCAP>
-KNN_DI void flush_query(unsigned long long *wl, uint32_t &nb, int i, int k, int lane) {
-    constexpr int REGION = KCAP + EX_CB;
-    const int c = nbuf_get(nb, i);
-    if (c > 0) {
-        warp_merge<KCAP>(wl + i * REGION, c, k, lane);
-        nb = nbuf_set(nb, i, 0);
+// ---------------------------------------------------------------------------
+// Selection state of one query: an unsorted buffer of REGION key slots and a
+// threshold tau; keys >= tau are known not to belong to the k smallest.  A half
+// tile's keys below tau are appended; when they would not fit, buf_select finds
+// a lower tau and drops what is above it.  Any tau that keeps between k and
+// KCAP + 32 keys will do, so it is found by bisection over the distances' bits
+// (a count over the buffer for each step, about six steps) instead of sorting:
+// about 250 instructions against the 1300 to 1900 of sorting 128 keys and
+// merging them into a sorted list of k.  tau lags the keys seen, so more points
+// pass, but selections become rare: the gap between them grows geometrically
+// as tau tightens.  The buffer is sorted once, at the end of the range.
+// ---------------------------------------------------------------------------
+
+// Keep the keys of B[0..c) (c > k + slack) below a tau of which there are at
+// least k and at most k + slack, in their order; tau goes to *tau.  Returns
+// their number.  One warp; not inlined: its call sites share one copy.
+template <int KCAP>
+__device__ __noinline__ int buf_select(unsigned long long *B, unsigned long long *tau, int c,
+                                       int k, int slack, int lane) {
+    constexpr int SL = (KCAP + EX_CB + 32) / 32;
+    unsigned long long key[SL];
+    uint32_t lo = 0xffffffffu, up = 0;
+#pragma unroll
+    for (int a = 0; a < SL; ++a) {
+        const int t = a * 32 + lane;
+        key[a] = t < c ? B[t] : kKeyInf;
+        const uint32_t h = (uint32_t)(key[a] >> 32);
+        lo = min(lo, h);
+        up = max(up, t < c ? h : 0u);
     }
+    // invariant: fewer than k keys have a distance below lo, n >= k below up
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    up = __reduce_max_sync(0xffffffffu, up) + 1u;
+    int n = c;
+    while (n > k + slack && up - lo > 1u) {
+        const uint32_t mid = lo + (up - lo) / 2u;
+        int m = 0;
+#pragma unroll
+        for (int a = 0; a < SL; ++a) m += (uint32_t)(key[a] >> 32) < mid ? 1 : 0;
+        m = (int)__reduce_add_sync(0xffffffffu, (unsigned)m);
+        if (m >= k) {
+            up = mid;
+            n = m;
+        } else {
+            lo = mid;
+        }
+    }
+    unsigned long long cut = (unsigned long long)up << 32;
+    if (n > k + slack) {
+        // many keys of the one distance lo: bisection over their indices
+        // (all different) ends with exactly k at the latest
+        unsigned long long a0 = (unsigned long long)lo << 32, a1 = cut;
+        while (n > k + slack) {
+            const unsigned long long mid = a0 + (a1 - a0) / 2;
+            int m = 0;
+#pragma unroll
+            for (int a = 0; a < SL; ++a) m += key[a] < mid ? 1 : 0;
+            m = (int)__reduce_add_sync(0xffffffffu, (unsigned)m);
+            if (m >= k) {
+                a1 = mid;
+                n = m;
+            } else {
+                a0 = mid;
+            }
+        }
+        cut = a1;
+    }
+    __syncwarp();
+    const unsigned lt = (1u << lane) - 1u;
+    int pos = 0;
+#pragma unroll
+    for (int a = 0; a < SL; ++a) {
+        const bool in = key[a] < cut;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (in) B[pos + __popc(m & lt)] = key[a];
+        pos += __popc(m);
+    }
+    if (lane == 0) *tau = cut;
+    __syncwarp();
+    return n;
 }
 
-// Merge every query's buffered candidates (end of a reference range).
-// (Loops over queries are not unrolled: one inlined copy of the merge.)
+// The k smallest keys of B[0..c), ascending, into B[0..k) (kKeyInf where there
+// are fewer).  One warp.
+template <int KCAP>
+__device__ __noinline__ void buf_finish(unsigned long long *B, unsigned long long *tau, int c,
+                                        int k, int lane) {
+    constexpr int LPL = KCAP / 32;
+    if (c > KCAP) c = buf_select<KCAP>(B, tau, c, k, KCAP - k, lane);
+    unsigned long long v[LPL];
+#pragma unroll
+    for (int a = 0; a < LPL; ++a) v[a] = a * 32 + lane < c ? B[a * 32 + lane] : kKeyInf;
+    warp_sort<LPL>(v, lane);
+    __syncwarp();
+#pragma unroll
+    for (int a = 0; a < LPL; ++a) B[a * 32 + lane] = v[a];
+    __syncwarp();
+}
+
+// Buffer fill of query i (warp-uniform), 16 bits per query.
+KNN_DI int nbuf_get(unsigned long long nb, int i) { return (int)((nb >> (16 * i)) & 0xffffu); }
+KNN_DI unsigned long long nbuf_set(unsigned long long nb, int i, int v) {
+    return (nb & ~(0xffffull << (16 * i))) | ((unsigned long long)v << (16 * i));
+}
+
+// Start of a reference range: empty buffers; queries beyond the set have a
+// threshold that nothing passes.
+template <int QPW>
+KNN_DI void select_start(unsigned long long *wt, unsigned long long &nb, int q0, int Q, int lane) {
+    nb = 0;
+    if (lane < QPW) wt[lane] = q0 + lane < Q ? kKeyInf : 0ull;
+    __syncwarp();
+}
+
+// End of a reference range: every query's buffer sorted.  (Not unrolled.)
 template <int QPW, int KCAP>
-KNN_DI void flush_all(unsigned long long *wl, uint32_t &nb, int k, int lane) {
-    static_assert(QPW <= 4 && EX_CB < 256, "buffer fills packed in one word");
+KNN_DI void select_finish(unsigned long long *wl, unsigned long long *wt, unsigned long long nb,
+                          int k, int lane) {
+    static_assert(QPW <= 4, "buffer fills packed in one word");
+    constexpr int REGION = ExCfg<QPW, KCAP>::REGION;
 #pragma unroll 1
-    for (int i = 0; i < QPW; ++i) flush_query<QPW, KCAP>(wl, nb, i, k, lane);
+    for (int i = 0; i < QPW; ++i)
+        buf_finish<KCAP>(wl + i * REGION, wt + i, nbuf_get(nb, i), k, lane);
 }
 
-// Filter one half tile (4 reference points per lane) against each query's
-// threshold tau (the k-th key of its list) and append the survivors to the
-// query's candidate buffer.  The buffer is merged into the list only when
-// this half tile's survivors would not fit: tau then lags the candidates
-// seen, so more points pass, but merges become rare (the gap between them
-// grows geometrically as the list tightens) instead of one per half tile
-// that holds any survivor.  nb packs the warp-uniform buffer fills.
-// d2(i, j) gives the squared distance of query i to the lane's j-th point.
-// With LB, only keys >= lb[i] are selected: pass p of a k > 256 problem keeps
-// the 256 smallest keys above the ones earlier passes returned.
+// Filter one half tile (4 reference points per lane) against the thresholds of
+// the queries in hitq and append the survivors to their buffers.  A query
+// whose buffer was selected here is tested again with its new threshold: of a
+// list's first half tiles, all of whose points pass, later ones then add few.
+// nb packs the warp-uniform buffer fills.  d2(i, j) gives the squared
+// distance of query i to the lane's j-th point.  With LB, only keys >= lb[i]
+// are selected: pass p of a k > 256 problem keeps the 256 smallest keys above
+// the ones earlier passes returned.
 template <int QPW, int KCAP, bool LB, typename D2>
-KNN_DI void select_half_lb(unsigned long long *wl, uint32_t &nb, D2 d2, uint32_t rbase, int N,
-                           int k, int lane, const unsigned long long (&lb)[QPW]) {
-    constexpr int REGION = KCAP + EX_CB;
-    unsigned long long tau[QPW];
-#pragma unroll
-    for (int i = 0; i < QPW; ++i) tau[i] = wl[i * REGION + k - 1];
-    uint32_t pm[QPW];
-    bool any = false;
-#pragma unroll
-    for (int i = 0; i < QPW; ++i) {
-        pm[i] = 0;
+KNN_DI void select_half_lb(unsigned long long *wl, unsigned long long *wt,
+                           unsigned long long &nb, D2 d2, uint32_t rbase, int N, int k, int lane,
+                           uint32_t hitq, const unsigned long long (&lb)[QPW]) {
+    constexpr int REGION = ExCfg<QPW, KCAP>::REGION;
+    auto passing = [&](int i) {
+        const unsigned long long tau = wt[i];
+        uint32_t m = 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const uint32_t idx = rbase + j;
             const unsigned long long key = make_key(d2(i, j), idx);
-            bool p = (idx < (uint32_t)N) && key < tau[i];
+            bool p = (idx < (uint32_t)N) && key < tau;
             if (LB) p = p && key >= lb[i];
-            pm[i] |= (p ? 1u : 0u) << j;
-            any |= p;
+            m |= (p ? 1u : 0u) << j;
         }
-    }
-    if (!__any_sync(0xffffffffu, any)) return;
-    const unsigned lt = (1u << lane) - 1u;
-    // queries whose buffer cannot take this half tile's survivors: merge first
-    uint32_t full_mask = 0;
+        return m;
+    };
+    uint32_t pm[QPW];
+    uint32_t full_mask = 0;   // queries whose buffer cannot take the survivors
 #pragma unroll
     for (int i = 0; i < QPW; ++i) {
+        pm[i] = 0;
+        if (!((hitq >> i) & 1u)) continue;
+        pm[i] = passing(i);
         const int m_i = (int)__reduce_add_sync(0xffffffffu, (unsigned)__popc(pm[i]));
-        if (nbuf_get(nb, i) + m_i > EX_CB) full_mask |= 1u << i;
+        if (nbuf_get(nb, i) + m_i > REGION) full_mask |= 1u << i;
     }
     if (full_mask) {
         __syncwarp();
 #pragma unroll 1
         for (int i = 0; i < QPW; ++i)
-            if ((full_mask >> i) & 1u) flush_query<QPW, KCAP>(wl, nb, i, k, lane);
+            if ((full_mask >> i) & 1u)
+                nb = nbuf_set(nb, i, buf_select<KCAP>(wl + i * REGION, wt + i, nbuf_get(nb, i), k,
+                                                      KCAP + 32 - k, lane));
+#pragma unroll
+        for (int i = 0; i < QPW; ++i)
+            if ((full_mask >> i) & 1u) pm[i] = passing(i);
     }
+    const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
     for (int i = 0; i < QPW; ++i) {
         if (__ballot_sync(0xffffffffu, pm[i] != 0) == 0) continue;
-        unsigned long long *cb = wl + i * REGION + KCAP;
+        unsigned long long *cb = wl + i * REGION;
         int c = nbuf_get(nb, i);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -209,14 +320,6 @@ KNN_DI void select_half_lb(unsigned long long *wl, uint32_t &nb, D2 d2, uint32_t
     }
     __syncwarp();
 }
-
-template <int QPW, int KCAP, typename D2>
-KNN_DI void select_half(unsigned long long *wl, uint32_t &nb, D2 d2, uint32_t rbase, int N,
-                        int k, int lane) {
-    const unsigned long long none[QPW] = {};
-    select_half_lb<QPW, KCAP, false>(wl, nb, d2, rbase, N, k, lane, none);
-}
-
 
 // The warp's QPW queries of one dimension (one broadcast load).
 template <int QPW>
@@ -292,26 +395,33 @@ KNN_DI bool consume_ref_tile(f32x2_t (&acc)[QPW][4], const float *stages, uint64
 }
 
 // Select both halves of a consumed tile (reference points rt*256 + ...).
-template <int QPW, int KCAP, bool LB = false>
-KNN_DI void select_tile(unsigned long long *wl, uint32_t &nb, f32x2_t (&acc)[QPW][4], int rt,
-                        int N, int k, int lane, const unsigned long long (&lb)[QPW]) {
+// Most tiles hold no candidate of most queries, so each lane first compares
+// the smallest of its 8 distances (as bits: the order of the keys, whatever
+// the index) with the threshold's: about one instruction per pair instead of
+// six for the key comparisons of every pair.
+template <int QPW, int KCAP, bool LB>
+KNN_DI void select_tile(unsigned long long *wl, unsigned long long *wt, unsigned long long &nb,
+                        f32x2_t (&acc)[QPW][4], int rt, int N, int k, int lane,
+                        const unsigned long long (&lb)[QPW]) {
+    auto d2 = [&](int i, int j) {
+        return (j & 1) ? f2_hi(acc[i][j >> 1]) : f2_lo(acc[i][j >> 1]);
+    };
+    uint32_t hitq = 0;
+#pragma unroll
+    for (int i = 0; i < QPW; ++i) {
+        uint32_t b[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) b[j] = __float_as_uint(d2(i, j));
+        const uint32_t m = min(min(min(min(b[0], b[1]), b[2]), min(min(b[3], b[4]), b[5])),
+                               min(b[6], b[7]));
+        const uint32_t tau = (uint32_t)(wt[i] >> 32);
+        hitq |= __any_sync(0xffffffffu, m <= tau) ? 1u << i : 0u;
+    }
+    if (!hitq) return;
     const uint32_t rb0 = (uint32_t)rt * EX_BR + lane * 4;
+    select_half_lb<QPW, KCAP, LB>(wl, wt, nb, d2, rb0, N, k, lane, hitq, lb);
     select_half_lb<QPW, KCAP, LB>(
-        wl, nb,
-        [&](int i, int j) { return (j & 1) ? f2_hi(acc[i][j >> 1]) : f2_lo(acc[i][j >> 1]); },
-        rb0, N, k, lane, lb);
-    select_half_lb<QPW, KCAP, LB>(
-        wl, nb,
-        [&](int i, int j) {
-            return (j & 1) ? f2_hi(acc[i][2 + (j >> 1)]) : f2_lo(acc[i][2 + (j >> 1)]);
-        },
-        rb0 + 128, N, k, lane, lb);
-}
-template <int QPW, int KCAP>
-KNN_DI void select_tile(unsigned long long *wl, uint32_t &nb, f32x2_t (&acc)[QPW][4], int rt,
-                        int N, int k, int lane) {
-    const unsigned long long none[QPW] = {};
-    select_tile<QPW, KCAP, false>(wl, nb, acc, rt, N, k, lane, none);
+        wl, wt, nb, [&](int i, int j) { return d2(i, 4 + j); }, rb0 + 128, N, k, lane, hitq, lb);
 }
 
 // ---------------------------------------------------------------------------
