@@ -120,7 +120,9 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
     }
     __syncthreads();
 
-    if (warp == EX_WARPS) {
+    if (warp >= EX_WARPS) {
+        producer_regs();
+        if (warp > EX_WARPS) return;
         // ---------------- producer: pops items, streams their tiles --------
         if (lane == 0) {
             int issued = 0, it = 0;
@@ -181,6 +183,7 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
     }
 
     // -------------------- consumer warps ------------------------------------
+    consumer_regs();
     unsigned long long *wl = lists + (size_t)warp * QPW * C::REGION;
     unsigned long long *wt =
         reinterpret_cast<unsigned long long *>(base + C::TAU_OFFSET) + warp * QPW;
@@ -315,7 +318,8 @@ namespace {
 template <int QPW, int KCAP>
 cudaError_t launch_batched_t(const knnb200_batched_plan *pl, cudaStream_t st) {
     using B = BatchCfg<QPW, KCAP>;
-    auto kern = knn_exact_batched_kernel<QPW, KCAP>;
+    constexpr auto kern = knn_exact_batched_kernel<QPW, KCAP>;
+    if (!launch_regs_ok<kern>()) return cudaErrorLaunchOutOfResources;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)B::SMEM);
     if (e != cudaSuccess) return e;

@@ -74,7 +74,9 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
     }
     __syncthreads();
 
-    if (warp == EX_WARPS) {
+    if (warp >= EX_WARPS) {
+        producer_regs();
+        if (warp > EX_WARPS) return;
         // ---------------- producer warp: one thread issues all TMA loads ----
         if (lane == 0) {
             prefetch_tensormap(&tm_ref);
@@ -105,6 +107,7 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
     }
 
     // -------------------- consumer warps ------------------------------------
+    consumer_regs();
     unsigned long long *wl = lists + (size_t)warp * QPW * C::REGION;
     unsigned long long *wt =
         reinterpret_cast<unsigned long long *>(base + C::TAU_OFFSET) + warp * QPW;
@@ -259,7 +262,8 @@ template <int QPW, int KCAP, bool LB = false>
 cudaError_t launch_t(const CUtensorMap &mr, const CUtensorMap &mq, const ExactArgs &a,
                      int qtiles, cudaStream_t st) {
     using C = ExCfg<QPW, KCAP>;
-    auto kern = knn_exact_kernel<QPW, KCAP, LB>;
+    constexpr auto kern = knn_exact_kernel<QPW, KCAP, LB>;
+    if (!launch_regs_ok<kern>()) return cudaErrorLaunchOutOfResources;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)C::SMEM);
     if (e != cudaSuccess) return e;

@@ -13,7 +13,33 @@ constexpr int EX_CB = 128;       // candidate slots per query (one half tile)
 constexpr int EX_WARPS = 16;     // consumer warps
 constexpr int EX_QPW = 4;        // queries per warp for k <= 128
 constexpr int EX_QPW_K256 = 2;   // queries per warp for 128 < k <= 256
-constexpr int EX_THREADS = (EX_WARPS + 1) * 32;
+// Four warps of consumers to each scheduler and a warpgroup for the producer, of
+// which one thread works.  Each consumer thread takes 112 registers (setmaxnreg):
+// launched with 96, 640 x 96 = 61440 >= 128 x 24 + 512 x 112 = 60416.  With 17
+// warps of 96 the inner loop and the selection spilled: 10.29 -> 10.07 ms at 131072
+// x 4736, d = 256, k = 100; 692 -> 676 us at 16384 x 4096, d = 128, k = 16; 19.3 ->
+// 18.8 ms for a batch of 512.
+constexpr int EX_THREADS = (EX_WARPS + 4) * 32;
+constexpr int EX_LAUNCH_REGS = 96, EX_PRODUCER_REGS = 24, EX_CONSUMER_REGS = 112;
+static_assert(128 * EX_PRODUCER_REGS + EX_WARPS * 32 * EX_CONSUMER_REGS <=
+                  EX_THREADS * EX_LAUNCH_REGS,
+              "the consumers' registers come from the block's own");
+// Whether `kern` is launched with the registers that the split counts on (asked
+// once for each kernel; a build with fewer would leave its consumers waiting).
+template <auto kern>
+bool launch_regs_ok() {
+    static const bool ok = [] {
+        cudaFuncAttributes a;
+        return cudaFuncGetAttributes(&a, kern) == cudaSuccess && a.numRegs >= EX_LAUNCH_REGS;
+    }();
+    return ok;
+}
+KNN_DI void producer_regs() {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(EX_PRODUCER_REGS));
+}
+KNN_DI void consumer_regs() {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(EX_CONSUMER_REGS));
+}
 
 template <int QPW, int KCAP>
 struct ExCfg {
