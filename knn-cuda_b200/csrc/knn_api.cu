@@ -215,6 +215,7 @@ struct Workspace {
     cudaStream_t stream = nullptr;
     cudaEvent_t last_done = nullptr;   // orders device-resident calls on this device
     Buffer ref, qry, dist, idx, scratch, status;
+    Buffer space;                      // spatial search of point clouds (optional)
     Buffer tcref;                      // prepared reference set of the tensor-core path
     TcRefState tc_state;               // its host-side state
     Buffer bound;                      // re-rank bound check (test-only, off by default)
@@ -544,11 +545,15 @@ size_t usable_memory(const Workspace &ws) {
 // is not asked for its free memory: cudaMemGetInfo costs a driver round
 // trip on every call otherwise.
 template <class F>
-int plan_query_chunk(const Workspace &ws, int Q, size_t fixed, F per_chunk) {
+int plan_query_chunk(Workspace &ws, int Q, size_t fixed, F per_chunk) {
     const size_t held = ws.ref.bytes + ws.qry.bytes + ws.dist.bytes + ws.idx.bytes +
                         ws.scratch.bytes + ws.tcref.bytes;
     if (!g_mem_cap && fixed + per_chunk(Q) <= held) return Q;
-    const size_t avail = usable_memory(ws);
+    size_t avail = usable_memory(ws);
+    if (fixed + per_chunk(Q) > avail && ws.space.bytes) {
+        ws.space.release();   // only a speed-up: it makes way first
+        avail = usable_memory(ws);
+    }
     auto fits = [&](int qc) { return fixed + per_chunk(qc) <= avail; };
     if (fits(Q)) return Q;
     int lo = 0, hi = Q;   // fits(lo) (or lo == 0), !fits(hi)
@@ -559,6 +564,20 @@ int plan_query_chunk(const Workspace &ws, int Q, size_t fixed, F per_chunk) {
     }
     if (lo >= 256) lo = lo / 256 * 256;
     return lo;
+}
+
+// Scratch of the spatial search for an exact problem, if it applies and the
+// memory is there beside `planned` bytes of the call; else the problem runs
+// without it.
+void attach_space(Workspace &ws, ExactProblem &p, size_t planned) {
+    const size_t need = space_bytes(p.N, p.Q, p.d, p.k);
+    if (!need) return;
+    if (need > ws.space.bytes || g_mem_cap) {
+        if (planned + grown(need) > usable_memory(ws)) return;
+        if (!ws.space.ensure(need)) return;
+    }
+    p.space = ws.space.ptr;
+    p.space_bytes = ws.space.bytes;
 }
 
 // Device bytes of one query chunk of the host entry: query copy, outputs,
@@ -667,6 +686,9 @@ bool host_entry(int method, const float *ref, int ref_nb, const float *query, in
         p.status = static_cast<int *>(ws->status.ptr);
         p.num_sms = ws->num_sms;
         p.force_splits = 0;
+        if (!tc)
+            attach_space(*ws, p,
+                         fixed + host_chunk_bytes(method, ref_nb, qc, dim, k, ws->num_sms));
         rc = streamed ? enqueue_tc_streamed(*ws, p, ref, pinned, st)
                       : enqueue(*ws, p, method, st, /*ref_prepared=*/q0 > 0);
         if (rc != kOk) {
@@ -808,6 +830,8 @@ int knnb200_knn_device(const float *ref, int ref_nb, long long ref_ld, const flo
         p.status = static_cast<int *>(ws->status.ptr);
         p.num_sms = ws->num_sms;
         p.force_splits = 0;
+        if (!tc)
+            attach_space(*ws, p, grown(scratch_for(method, ref_nb, qc, dim, k, ws->num_sms)));
         rc = enqueue(*ws, p, method, st, /*ref_prepared=*/q0 > 0);
         stats[0] += ws->tc_stats[0];
         stats[1] += ws->tc_stats[1];
@@ -887,6 +911,7 @@ void knnb200_release_workspace(void) {
     ws->dist.release();
     ws->idx.release();
     ws->scratch.release();
+    ws->space.release();
     ws->tcref.release();
 }
 

@@ -175,29 +175,37 @@ template <int KCAP, int WPQ>
 __global__ void __launch_bounds__(32 * MG_WARPS)
     knn_merge_splits_kernel(const unsigned long long *__restrict__ part, int S, int Q, int k,
                             float *__restrict__ out_dist, int *__restrict__ out_idx,
-                            long long ld_out, int row0, unsigned long long *__restrict__ lb_out) {
+                            long long ld_out, int row0, unsigned long long *__restrict__ lb_out,
+                            QuerySubset subset) {
     constexpr int QPB = MG_WARPS / WPQ;
     __shared__ unsigned long long lists[MG_WARPS][KCAP], scratch[MG_WARPS][KCAP];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int q0 = blockIdx.x * QPB, q = q0 + warp / WPQ;
-    if (q < Q) {
-        merge_lists<KCAP>(lists[warp], scratch[warp], part + (size_t)q * k, (size_t)Q * k,
-                          warp % WPQ, WPQ, S, k, lane);
-    }
-    __syncthreads();
-    if (WPQ > 1) {
-        if (warp == 0)
-            merge_lists<KCAP>(scratch[0], scratch[1], lists[0], KCAP, 0, 1, WPQ, k, lane);
+    const int nq = subset.count ? *subset.count : Q;
+    if (subset.count) S = QuerySubset::splits(nq, S);
+    if (subset.count && S == 1) return;   // written without lists
+    for (int q0 = blockIdx.x * QPB; q0 < nq; q0 += gridDim.x * QPB) {
+        const int q = q0 + warp / WPQ;
+        if (q < nq) {
+            merge_lists<KCAP>(lists[warp], scratch[warp], part + (size_t)q * k, (size_t)Q * k,
+                              warp % WPQ, WPQ, S, k, lane);
+        }
         __syncthreads();
-    }
-    // rows of the k x query_nb output, QPB queries wide
-    for (int e = threadIdx.x; e < k * QPB; e += 32 * MG_WARPS) {
-        const int j = e / QPB, qi = e % QPB;
-        if (q0 + qi >= Q) continue;
-        const unsigned long long key = WPQ > 1 ? scratch[0][j] : lists[qi][j];
-        out_dist[(size_t)(row0 + j) * ld_out + q0 + qi] = sqrtf(key_dist2(key));
-        out_idx[(size_t)(row0 + j) * ld_out + q0 + qi] = key_index(key);
-        if (lb_out && j == k - 1) lb_out[q0 + qi] = key + 1;
+        if (WPQ > 1) {
+            if (warp == 0)
+                merge_lists<KCAP>(scratch[0], scratch[1], lists[0], KCAP, 0, 1, WPQ, k, lane);
+            __syncthreads();
+        }
+        // rows of the k x query_nb output, QPB queries wide
+        for (int e = threadIdx.x; e < k * QPB; e += 32 * MG_WARPS) {
+            const int j = e / QPB, qi = q0 + e % QPB;
+            if (qi >= nq) continue;
+            const unsigned long long key = WPQ > 1 ? scratch[0][j] : lists[e % QPB][j];
+            const int col = subset.list ? subset.list[qi] : qi;
+            out_dist[(size_t)(row0 + j) * ld_out + col] = sqrtf(key_dist2(key));
+            out_idx[(size_t)(row0 + j) * ld_out + col] = key_index(key);
+            if (lb_out && j == k - 1) lb_out[col] = key + 1;
+        }
+        __syncthreads();   // the lists are rewritten
     }
 }
 
@@ -279,15 +287,17 @@ static long long qcopy_pitch(int Q) { return ((long long)Q + 31) / 32 * 32; }
 
 int launch_split_merge(const unsigned long long *part, int S, int Q, int k, float *out_dist,
                        int *out_idx, long long ld_out, cudaStream_t st, int row0,
-                       unsigned long long *lb_out) {
+                       unsigned long long *lb_out, const QuerySubset &subset) {
     if (k > kPassRanks) return kErrUnsupported;
     // all eight warps on one query: 14.6 us against 51.9 with one warp a query at
     // 40 queries and 148 lists of 50 keys, 15.4 against 22.7 at 300 queries and 29
     // lists of 100; at 1000 queries and 9 lists one warp a query takes 10.7
     const bool wide = Q <= 1024 && S >= 16;
     auto go = [&](auto kern, int qpb) {
-        kern<<<(Q + qpb - 1) / qpb, 32 * MG_WARPS, 0, st>>>(part, S, Q, k, out_dist, out_idx,
-                                                            ld_out, row0, lb_out);
+        // a subset is usually empty: few blocks, which loop if it is not
+        const int all = (Q + qpb - 1) / qpb, blocks = subset.count ? std::min(all, 592) : all;
+        kern<<<blocks, 32 * MG_WARPS, 0, st>>>(part, S, Q, k, out_dist, out_idx, ld_out, row0,
+                                               lb_out, subset);
         return cudaGetLastError() == cudaSuccess ? (int)kOk : (int)kErrLaunch;
     };
     auto pick = [&](auto cap) {

@@ -94,6 +94,24 @@ struct ExactProblem {
     int num_sms;
     int force_splits;   // 0 = automatic
     PhaseTimer *timer = nullptr;
+    // scratch of the spatial search (space_bytes), where the caller has it:
+    // without it point clouds run the brute-force kernel
+    void *space = nullptr;
+    size_t space_bytes = 0;
+};
+
+// The queries list[0 .. *count) of a problem (device memory).
+struct QuerySubset {
+    const int *list = nullptr;
+    const int *count = nullptr;
+    // Splits of the reference set for nq queries, of at most max_splits: as
+    // many as give 7104 warps (24 an SM, twice) of four queries each.  The
+    // kernels that work on a subset call it with the count they find.
+    static __host__ __device__ int splits(int nq, int max_splits) {
+        const int warps = (nq + 3) / 4;
+        const int s = warps > 0 ? 7104 / warps : 1;
+        return s < 1 ? 1 : s < max_splits ? s : max_splits;
+    }
 };
 
 // Encode a 2-D tensor map (cols = contiguous axis, row pitch ld_elems) with
@@ -113,11 +131,19 @@ bool lowdim_applies(int N, int Q, int d, int k);
 size_t lowdim_scratch_bytes(int N, int Q, int d, int k, int num_sms);
 int lowdim_plan_splits(int N, int Q, int d, int k, int num_sms);
 int launch_lowdim(const ExactProblem &p, cudaStream_t st);
+// Spatial search of large low-dimension problems (knn_space.cu): used by
+// launch_lowdim where it applies and p.space holds space_bytes (0: does not
+// apply).  launch_space leaves the queries it did not answer in *far.
+bool space_applies(int N, int Q, int d, int k);
+size_t space_bytes(int N, int Q, int d, int k);
+int launch_space(const ExactProblem &p, cudaStream_t st, QuerySubset *far);
 // Merge per-split sorted key lists [S][Q][k] into rows row0 .. row0 + k - 1
-// of the output; with lb_out, lb_out[q] = (k-th merged key) + 1.
+// of the output; with lb_out, lb_out[q] = (k-th merged key) + 1.  With a
+// subset, list q is that of the query subset.list[q], q < *subset.count.
 int launch_split_merge(const unsigned long long *part, int S, int Q, int k, float *out_dist,
                        int *out_idx, long long ld_out, cudaStream_t st, int row0 = 0,
-                       unsigned long long *lb_out = nullptr);
+                       unsigned long long *lb_out = nullptr,
+                       const QuerySubset &subset = QuerySubset());
 size_t exact_scratch_bytes(int N, int Q, int d, int k, int num_sms);
 int exact_plan_splits(int N, int Q, int d, int k, int num_sms);
 int launch_exact(const ExactProblem &p, cudaStream_t st);

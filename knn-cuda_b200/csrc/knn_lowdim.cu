@@ -1,209 +1,213 @@
-// knn_lowdim.cu -- exact FP32 k-NN for low dimension (d <= 4) and small k
-// (k <= 16), e.g. 3-D point clouds.
+// knn_lowdim.cu -- exact FP32 brute-force k-NN for low dimension (d <= 4) and
+// small k (k <= 16), e.g. 3-D point clouds.
 //
 // At d = 3 the distance of a pair costs three subtractions and three fused
 // multiply-adds, so the work is dominated by issue, not by data: the tiled
-// kernel's 16-dimension stages would waste 13/16 of its arithmetic.  Here
-// every thread owns QPT queries (packed in pairs for sub.f32x2 / fma.f32x2)
-// and their sorted top-k lists in registers; the CTA streams its range of
-// reference points through a double-buffered shared-memory tile (each
-// coordinate stored twice, (r, r), so a 64-bit load yields a packed operand)
-// and every thread scans the tile in index order.
+// kernel's 16-dimension stages would waste 13/16 of its arithmetic.  Here a
+// warp holds QPW queries; its lanes take four reference points each, 128
+// consecutive ones a step (one 16-byte load per dimension and lane), as packed
+// pairs for sub.f32x2 / fma.f32x2.  A step's distances are first compared with
+// the query's k-th smallest so far (three minima, one compare and one vote for
+// four points); survivors enter the query's sorted list, which lies across the
+// lanes (knn_lane_list.cuh).
 //
 // Arithmetic: acc = fma(t0, t0, 0), acc = fma(t_i, t_i, acc) for i = 1..d-1,
 // t_i = r_i - q_i -- the fused exact kernel's chain (its zero-padded
 // dimensions add exact zeros), so distances are bit-identical to it.
-// Selection: a candidate enters the list iff it is strictly smaller than the
-// k-th distance, and shifts only past strictly larger entries; because each
-// thread scans references in increasing index, equal distances keep the
-// lower index first -- the reference's rule (code/knncuda.cu:172, :178).
+// Selection keeps the smallest (distance, index) keys: equal distances keep
+// the lower index first -- the reference's rule (code/knncuda.cu:172, :178).
+//
+// Bound by the FP32 pipe: 24 lane operations per four points at d = 3.  One
+// thread per query with register lists, the layout before this one, took 29.1
+// ms at 2^20 x 65536, d = 3, k = 8, where this one takes 22.9, and left most of
+// the GPU idle at smaller sizes: 244 -> 126 us at 1000 x 50000, d = 1, k = 8; 855 ->
+// 79 at 7000 x 7000, d = 3, k = 16; 438 -> 71 at 2^20 x 50, d = 1, k = 8.
+//
+// Large clouds are searched in space (knn_space.cu) where the caller has the
+// scratch for it; this kernel then answers the few queries that search leaves
+// over.
 #include <algorithm>
 
-#include "knn_common.cuh"
+#include "knn_exact_core.cuh"
 #include "knn_kernels.h"
+#include "knn_lane_list.cuh"
 
 namespace knnb200 {
 
-constexpr int LD_THREADS = 256;
-constexpr int LD_TILE = 512;   // reference points per shared tile
+constexpr int LD_WARPS = 8;      // warps per block
+constexpr int LD_STEP = 128;     // reference points per step of a warp
+constexpr int LD_MAX_K = 16;
 
-template <int D, int K, int QPT>
-__global__ void __launch_bounds__(LD_THREADS, 2)
+// A block takes LD_WARPS / WPQ groups of QPW queries and one split of the
+// reference set; with WPQ = LD_WARPS its warps share the split of one group
+// and merge their lists.
+template <int D, int QPW, int WPQ>
+__global__ void __launch_bounds__(32 * LD_WARPS)
     knn_lowdim_kernel(const float *__restrict__ ref, int N, long long ldr,
-                      const float *__restrict__ qry, int Q, long long ldq, int k, int n_rtiles,
-                      int n_splits, float *__restrict__ out_dist, int *__restrict__ out_idx,
-                      long long ld_out, unsigned long long *__restrict__ part) {
-    static_assert(QPT % 2 == 0, "queries are processed in pairs");
-    __shared__ float2 tile[2][D][LD_TILE];
-    const int tid = threadIdx.x;
-    const int qtile = blockIdx.x, split = blockIdx.y;
-    const int BQ = LD_THREADS * QPT;
-    // thread's queries: q_base + tid + m * LD_THREADS (coalesced loads)
-    f32x2_t qp[QPT / 2][D];
-    int qid[QPT];
+                      const float *__restrict__ qry, int Q, long long ldq, int k, int n_splits,
+                      float *__restrict__ out_dist, int *__restrict__ out_idx, long long ld_out,
+                      unsigned long long *__restrict__ part, QuerySubset subset) {
+    constexpr int GROUPS = LD_WARPS / WPQ, QPB = GROUPS * QPW;
+    __shared__ unsigned long long lists[LD_WARPS][QPW][32], merged[GROUPS][QPW][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int group = warp / WPQ;
+    // with a subset: its queries, and the blocks loop over the (query block,
+    // split) pairs; otherwise one pair per block
+    const int nq = subset.count ? *subset.count : Q;
+    if (subset.count) n_splits = QuerySubset::splits(nq, n_splits);
+    const long long n_items = (long long)((nq + QPB - 1) / QPB) * n_splits;
+    const long long steps = ((long long)N + LD_STEP - 1) / LD_STEP;
+    for (long long item = blockIdx.x; item < n_items; item += gridDim.x) {
+        const int split = (int)(item % n_splits);
+        const int q0 = (int)(item / n_splits) * QPB + group * QPW;
+        // this warp's steps
+        const long long parts = (long long)n_splits * WPQ;
+        const long long mypart = (long long)split * WPQ + warp % WPQ;
+        const long long s0 = steps * mypart / parts, s1 = steps * (mypart + 1) / parts;
+        float q[QPW][D];
+        unsigned long long mine[QPW], tau[QPW];
 #pragma unroll
-    for (int m = 0; m < QPT; ++m) qid[m] = qtile * BQ + tid + m * LD_THREADS;
+        for (int i = 0; i < QPW; ++i) {
+            const int qi = q0 + i;
+            const int col = qi < nq ? (subset.list ? subset.list[qi] : qi) : -1;
 #pragma unroll
-    for (int pr = 0; pr < QPT / 2; ++pr)
-#pragma unroll
-        for (int dd = 0; dd < D; ++dd) {
-            const int a = qid[2 * pr], b = qid[2 * pr + 1];
-            const float va = a < Q ? qry[(size_t)dd * ldq + a] : 0.f;
-            const float vb = b < Q ? qry[(size_t)dd * ldq + b] : 0.f;
-            qp[pr][dd] = f2_pack(va, vb);
+            for (int dd = 0; dd < D; ++dd) q[i][dd] = col >= 0 ? qry[(size_t)dd * ldq + col] : 0.f;
+            mine[i] = kKeyNone;
+            tau[i] = col >= 0 ? kKeyNone : 0ull;   // nothing passes a query beyond the set
         }
-    float ld[QPT][K];
-    int li[QPT][K];
+        auto load = [&](float4 (&r)[D], long long s) {
+            const long long p = s * LD_STEP + lane * 4;
 #pragma unroll
-    for (int m = 0; m < QPT; ++m)
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-            ld[m][j] = INFINITY;
-            li[m][j] = -1;
-        }
-
-    // this CTA's reference range, in tiles of LD_TILE points
-    const long long t0 = (long long)n_rtiles * split / n_splits;
-    const long long t1 = (long long)n_rtiles * (split + 1) / n_splits;
-    constexpr int PER = LD_TILE / LD_THREADS;   // points per thread per tile load
-    float pre[D][PER];
-    auto fetch = [&](long long t) {
-#pragma unroll
-        for (int dd = 0; dd < D; ++dd)
-#pragma unroll
-            for (int u = 0; u < PER; ++u) {
-                const long long r = t * LD_TILE + u * LD_THREADS + tid;
-                pre[dd][u] = r < N ? ref[(size_t)dd * ldr + r] : 0.f;
-            }
-    };
-    auto stash = [&](int buf) {
-#pragma unroll
-        for (int dd = 0; dd < D; ++dd)
-#pragma unroll
-            for (int u = 0; u < PER; ++u)
-                tile[buf][dd][u * LD_THREADS + tid] = make_float2(pre[dd][u], pre[dd][u]);
-    };
-    if (t0 < t1) {
-        fetch(t0);
-        stash(0);
-    }
-    __syncthreads();
-    for (long long t = t0; t < t1; ++t) {
-        const int buf = (int)((t - t0) & 1);
-        if (t + 1 < t1) fetch(t + 1);
-        const int rbase = (int)(t * LD_TILE);
-        const int valid = (int)std::min<long long>(LD_TILE, (long long)N - rbase);
-        for (int j = 0; j < valid; ++j) {
-            f32x2_t rr[D];
-#pragma unroll
-            for (int dd = 0; dd < D; ++dd)
-                rr[dd] = *reinterpret_cast<const f32x2_t *>(&tile[buf][dd][j]);
-#pragma unroll
-            for (int pr = 0; pr < QPT / 2; ++pr) {
-                f32x2_t tt = f2_sub(rr[0], qp[pr][0]);
-                f32x2_t acc = f2_fma(tt, tt, 0ull);
-#pragma unroll
-                for (int dd = 1; dd < D; ++dd) {
-                    tt = f2_sub(rr[dd], qp[pr][dd]);
-                    acc = f2_fma(tt, tt, acc);
-                }
-                const float da = f2_lo(acc), db = f2_hi(acc);
-                const int ma = 2 * pr, mb = 2 * pr + 1;
-                if (da < ld[ma][K - 1] || db < ld[mb][K - 1]) {
-                    const int id = rbase + j;
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int m = h ? mb : ma;
-                        const float v = h ? db : da;
-                        if (v < ld[m][K - 1]) {
-#pragma unroll
-                            for (int i = K - 1; i > 0; --i) {
-                                const bool past = v < ld[m][i - 1];
-                                const bool here = v < ld[m][i];
-                                ld[m][i] = past ? ld[m][i - 1] : (here ? v : ld[m][i]);
-                                li[m][i] = past ? li[m][i - 1] : (here ? id : li[m][i]);
-                            }
-                            if (v < ld[m][0]) {
-                                ld[m][0] = v;
-                                li[m][0] = id;
-                            }
-                        }
-                    }
+            for (int dd = 0; dd < D; ++dd) {
+                const float *src = ref + (size_t)dd * ldr + p;
+                if (p + 3 < N) {
+                    r[dd] = *reinterpret_cast<const float4 *>(src);
+                } else {
+                    // the set's last points (NaN: never selected)
+                    const float none = __int_as_float(0x7fc00000);
+                    r[dd].x = p < N ? src[0] : none;
+                    r[dd].y = p + 1 < N ? src[1] : none;
+                    r[dd].z = p + 2 < N ? src[2] : none;
+                    r[dd].w = none;
                 }
             }
-        }
-        if (t + 1 < t1) stash(buf ^ 1);
-        __syncthreads();
-    }
-
-    // results (the first k of the K kept): sqrt into the k x Q layout, or
-    // this split's sorted keys for the split merge
+        };
+        float4 nxt[D];
+        if (s0 < s1) load(nxt, s0);
+        for (long long s = s0; s < s1; ++s) {
+            f32x2_t ra[D], rb[D];
 #pragma unroll
-    for (int m = 0; m < QPT; ++m) {
-        const int q = qid[m];
-        if (q >= Q) continue;
+            for (int dd = 0; dd < D; ++dd) {
+                ra[dd] = f2_pack(nxt[dd].x, nxt[dd].y);
+                rb[dd] = f2_pack(nxt[dd].z, nxt[dd].w);
+            }
+            if (s + 1 < s1) load(nxt, s + 1);
 #pragma unroll
-        for (int j = 0; j < K; ++j) {
-            if (j >= k) break;
-            if (n_splits == 1) {
-                out_dist[(size_t)j * ld_out + q] = sqrtf(ld[m][j]);
-                out_idx[(size_t)j * ld_out + q] = li[m][j];
-            } else {
-                part[((size_t)split * Q + q) * k + j] = make_key(ld[m][j], (uint32_t)li[m][j]);
+            for (int i = 0; i < QPW; ++i) {
+                f32x2_t a, b;
+#pragma unroll
+                for (int dd = 0; dd < D; ++dd) {
+                    const f32x2_t qq = f2_pack(q[i][dd], q[i][dd]);
+                    const f32x2_t ta = f2_sub(ra[dd], qq), tb = f2_sub(rb[dd], qq);
+                    a = f2_fma(ta, ta, dd ? a : 0ull);
+                    b = f2_fma(tb, tb, dd ? b : 0ull);
+                }
+                const float d4[4] = {f2_lo(a), f2_hi(a), f2_lo(b), f2_hi(b)};
+                const float m = fminf(fminf(d4[0], d4[1]), fminf(d4[2], d4[3]));
+                // (strictly: a step's indices are above all earlier ones)
+                if (!__any_sync(0xffffffffu, m < key_dist2(tau[i]))) continue;
+                const uint32_t idx = (uint32_t)(s * LD_STEP + lane * 4);
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    lane_list_add(mine[i], tau[i], finite_key(d4[j], idx + j), k, lane);
             }
         }
+        if (WPQ > 1) {
+#pragma unroll
+            for (int i = 0; i < QPW; ++i) lists[warp][i][lane] = mine[i];
+            __syncthreads();
+            if (warp % WPQ == 0) {
+#pragma unroll 1
+                for (int i = 0; i < QPW; ++i) {
+                    merge_lists<32>(merged[group][i], lists[warp][i], &lists[warp][i][0],
+                                    (size_t)QPW * 32, 0, 1, WPQ, k, lane);
+                }
+            }
+            __syncwarp();
+        }
+        // results: sqrt into the k x Q layout, or this split's sorted keys for
+        // the split merge
+        if (warp % WPQ == 0) {
+#pragma unroll
+            for (int i = 0; i < QPW; ++i) {
+                const int qi = q0 + i;
+                if (qi >= nq || lane >= k) continue;
+                const unsigned long long key = WPQ > 1 ? merged[group][i][lane] : mine[i];
+                if (n_splits == 1) {
+                    const int col = subset.list ? subset.list[qi] : qi;
+                    out_dist[(size_t)lane * ld_out + col] = sqrtf(key_dist2(key));
+                    out_idx[(size_t)lane * ld_out + col] = key_index(key);
+                } else {
+                    part[((size_t)split * Q + qi) * k + lane] = key;
+                }
+            }
+        }
+        if (WPQ > 1) __syncthreads();   // the lists are rewritten
     }
 }
 
 namespace {
 
+// Splits that callers' scratch is sized for, and the kernel's own choice.
 struct LowdimShape {
-    int kcap, qpt, bq, n_rtiles, splits;
+    int max_splits;
+    int qpw, wpq, splits;
 };
 
 bool lowdim_shape(int N, int Q, int d, int k, int num_sms, LowdimShape &s) {
-    if (d < 1 || d > 4 || k < 1 || k > 16) return false;
-    s.kcap = k <= 8 ? 8 : 16;
-    s.qpt = s.kcap == 8 ? 4 : 2;
-    s.bq = LD_THREADS * s.qpt;
-    s.n_rtiles = (N + LD_TILE - 1) / LD_TILE;
-    const int qtiles = (Q + s.bq - 1) / s.bq;
-    // two CTAs per SM; splits fill whole waves, each CTA >= 8 tiles
+    if (d < 1 || d > 4 || k < 1 || k > LD_MAX_K) return false;
+    const int bq = 256 * (k <= 8 ? 4 : 2);
+    const int n_rtiles = (N + 511) / 512;
+    const int qtiles = (Q + bq - 1) / bq;
+    // two blocks of bq queries per SM; splits fill whole waves, each >= 8 tiles
     const int slots = 2 * num_sms;
     int best = 1;
     double best_t = 1e300;
-    const int max_s = std::max(1, std::min({256, s.n_rtiles / 8, (160 * 1024) / (8 * k)}));
+    const int max_s = std::max(1, std::min({256, n_rtiles / 8, (160 * 1024) / (8 * k)}));
     for (int S = 1; S <= max_s; ++S) {
         const long long ctas = (long long)qtiles * S;
-        const double t = (double)((ctas + slots - 1) / slots) * ((double)s.n_rtiles / S + 0.5);
+        const double t = (double)((ctas + slots - 1) / slots) * ((double)n_rtiles / S + 0.5);
         if (t < best_t * 0.999) {
             best_t = t;
             best = S;
         }
     }
-    s.splits = best;
+    s.max_splits = best;
+    // four queries a warp share its loads where that still leaves every SM
+    // its warps; few queries take a whole block each
+    const int want = num_sms * 24;   // warps that keep the GPU busy
+    s.qpw = Q >= 4 * want ? 4 : 1;
+    s.wpq = Q < want ? LD_WARPS : 1;
+    const long long warps = ((long long)Q + s.qpw - 1) / s.qpw * s.wpq;
+    s.splits = (int)std::min<long long>(s.max_splits, std::max<long long>(1, 2 * want / warps));
     return true;
 }
 
-template <int D, int K, int QPT>
+template <int D>
 cudaError_t launch_ld(const ExactProblem &p, const LowdimShape &s, unsigned long long *part,
-                      cudaStream_t st) {
-    dim3 grid((p.Q + s.bq - 1) / s.bq, s.splits);
-    knn_lowdim_kernel<D, K, QPT><<<grid, LD_THREADS, 0, st>>>(
-        p.ref, p.N, p.ldr, p.qry, p.Q, p.ldq, p.k, s.n_rtiles, s.splits, p.out_dist, p.out_idx,
-        p.ld_out, part);
-    return cudaGetLastError();
-}
-
-template <int K, int QPT>
-cudaError_t launch_ld_d(const ExactProblem &p, const LowdimShape &s, unsigned long long *part,
-                        cudaStream_t st) {
-    switch (p.d) {
-        case 1: return launch_ld<1, K, QPT>(p, s, part, st);
-        case 2: return launch_ld<2, K, QPT>(p, s, part, st);
-        case 3: return launch_ld<3, K, QPT>(p, s, part, st);
-        default: return launch_ld<4, K, QPT>(p, s, part, st);
-    }
+                      const QuerySubset &subset, cudaStream_t st) {
+    auto go = [&](auto kern, int qpb) {
+        const long long items = (long long)((p.Q + qpb - 1) / qpb) * s.splits;
+        // a subset is usually small or empty: blocks that loop
+        const long long grid = subset.count ? std::min<long long>(items, 4 * p.num_sms) : items;
+        kern<<<(unsigned)grid, 32 * LD_WARPS, 0, st>>>(p.ref, p.N, p.ldr, p.qry, p.Q, p.ldq, p.k,
+                                                       s.splits, p.out_dist, p.out_idx, p.ld_out,
+                                                       part, subset);
+        return cudaGetLastError();
+    };
+    if (s.wpq > 1) return go(knn_lowdim_kernel<D, 1, LD_WARPS>, 1);
+    if (s.qpw == 4) return go(knn_lowdim_kernel<D, 4, 1>, 4 * LD_WARPS);
+    return go(knn_lowdim_kernel<D, 1, 1>, LD_WARPS);
 }
 
 }  // namespace
@@ -216,28 +220,43 @@ bool lowdim_applies(int N, int Q, int d, int k) {
 size_t lowdim_scratch_bytes(int N, int Q, int d, int k, int num_sms) {
     LowdimShape s;
     if (!lowdim_shape(N, Q, d, k, num_sms, s)) return 0;
-    return s.splits > 1 ? (size_t)s.splits * Q * k * 8 : 0;
+    return s.max_splits > 1 ? (size_t)s.max_splits * Q * k * 8 : 0;
 }
 
 int lowdim_plan_splits(int N, int Q, int d, int k, int num_sms) {
     LowdimShape s;
-    return lowdim_shape(N, Q, d, k, num_sms, s) ? s.splits : 0;
+    return lowdim_shape(N, Q, d, k, num_sms, s) ? s.max_splits : 0;
 }
 
 int launch_lowdim(const ExactProblem &p, cudaStream_t st) {
     LowdimShape s;
     if (!lowdim_shape(p.N, p.Q, p.d, p.k, p.num_sms, s)) return kErrUnsupported;
-    if (p.force_splits > 0) s.splits = std::min(p.force_splits, std::min(s.n_rtiles, 256));
+    if (p.force_splits > 0) s.splits = std::min(p.force_splits, std::min((p.N + 511) / 512, 256));
+    // a large cloud is searched in space; the brute force then answers the
+    // queries that search left over
+    QuerySubset sub;
+    if (p.space && space_applies(p.N, p.Q, p.d, p.k)) {
+        const int rc = launch_space(p, st, &sub);
+        if (rc != kOk) return rc;
+        s.qpw = 4;
+        s.wpq = 1;
+        s.splits = s.max_splits;
+    }
     const size_t need = s.splits > 1 ? (size_t)s.splits * p.Q * p.k * 8 : 0;
     if (need > p.scratch_bytes) return kErrScratch;
     unsigned long long *part = static_cast<unsigned long long *>(p.scratch);
-    const cudaError_t e = s.kcap == 8 ? launch_ld_d<8, 4>(p, s, part, st)
-                                      : launch_ld_d<16, 2>(p, s, part, st);
+    cudaError_t e;
+    switch (p.d) {
+        case 1: e = launch_ld<1>(p, s, part, sub, st); break;
+        case 2: e = launch_ld<2>(p, s, part, sub, st); break;
+        case 3: e = launch_ld<3>(p, s, part, sub, st); break;
+        default: e = launch_ld<4>(p, s, part, sub, st); break;
+    }
     if (e != cudaSuccess) return kErrLaunch;
     if (p.timer) p.timer->mark(st, kPhaseExactMain);
     if (s.splits > 1) {
         const int rc = launch_split_merge(part, s.splits, p.Q, p.k, p.out_dist, p.out_idx,
-                                          p.ld_out, st);
+                                          p.ld_out, st, 0, nullptr, sub);
         if (rc != kOk) return rc;
         if (p.timer) p.timer->mark(st, kPhaseExactMerge);
     }

@@ -61,6 +61,7 @@ struct DevBuf {
 struct Slot {
     cudaStream_t stream = nullptr;
     DevBuf scratch, qry, dist, idx, status;
+    DevBuf space;                // spatial search of a point cloud (optional)
     int *host_stats = nullptr;   // pinned, 8 ints
     bool init(int device) {
         if (cudaSetDevice(device) != cudaSuccess) return false;
@@ -73,6 +74,7 @@ struct Slot {
     void destroy() {
         if (stream) cudaStreamSynchronize(stream);
         scratch.release();
+        space.release();
         qry.release();
         dist.release();
         idx.release();
@@ -169,6 +171,10 @@ int run_refset(knnb200_refset *rs, Slot &slot, const float *query, int Q, long l
     p.num_sms = rs->num_sms;
     p.force_splits = 0;
     p.timer = nullptr;
+    if (slot.space.bytes && slot.space.bytes >= space_bytes(p.N, p.Q, p.d, p.k)) {
+        p.space = slot.space.ptr;
+        p.space_bytes = slot.space.bytes;
+    }
     return launch_exact(p, st);
 }
 
@@ -266,6 +272,9 @@ int knnb200_refset_knn(knnb200_refset *rs, const float *query, int query_nb, lon
     if (method < KNNB200_METHOD_GLOBAL || method > KNNB200_METHOD_FP8) return KNNB200_EINVAL;
     std::lock_guard<std::mutex> lock(rs->mu);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    // (a server's slots, whose memory is admitted beforehand, go without it)
+    if (!use_tc_for(rs, method, query_nb, k))
+        rs->slot.space.ensure(space_bytes(rs->N, query_nb, rs->d, k));
     // scratch of the refset's own slot: order this call after its previous one
     int rc = run_refset(rs, rs->slot, query, query_nb, query_ld, k, method, knn_dist, knn_index,
                         out_ld, st);
