@@ -55,6 +55,7 @@
 
 #include "knn_exact_core.cuh"
 #include "knn_kernels.h"
+#include "knn_lane_list.cuh"
 #include "knn_tc.cuh"
 
 namespace knnb200 {
@@ -63,7 +64,6 @@ constexpr int TC_BM = 128;            // rows (queries) per CTA of a pair, point
 constexpr int TC_QT = 2 * TC_BM;      // queries per CTA pair
 constexpr int TC_BK = 64;             // K block: 64 bf16 = 128 B (one swizzle row)
 constexpr int TC_NK = 16;             // norm step: K = 16 (h, m, l, 13 zeros)
-constexpr int TC_KS = 16;             // pass-1 per-row list length
 constexpr int TC_SAMPLE_EVERY = 16;   // point sample: every 16th point (pass 1 takes every m-th of those)
 constexpr uint32_t TC_TMEM_COLS = 512;   // 2 accumulator buffers x 256 columns
 constexpr int kCenterStride = 64;     // the translation is the mean of every 64th tile
@@ -140,6 +140,91 @@ struct PendingCands {
         ++n;
     }
 };
+
+// Pass-1 list of one query row and column half: the KS smallest of the minima
+// of groups of four values (columns e, e + 32, e + 64, e + 96 of the half tile),
+// ascending.  A group's minimum stands for its four: the KS-th smallest minimum
+// is a threshold with a few more sample points below it than KS (KS^2 / 2 over
+// the number of groups), and a quarter of the values need an insertion.  The
+// group's columns lie 32 apart so that neighbours in a set stored cluster by
+// cluster fall into different groups.
+//
+// A list starts empty and takes nearly everything at first, while its warp waits
+// for the row with most insertions.  Tiles with many are merged whole: the 32
+// minima sorted 16 at a time (63 exchanges) and merged into the list (a bitonic
+// merge), about 450 instructions; single ones are inserted one by one at about 75
+// each.  Every value one by one took 61 us for the sample of 2^21 points and 13
+// queries (d = 128), now 29 in the same splits and 18 in more, and 644 us at 2^20 x
+// 16384 (d = 256), now 550; 176 and 98 at 2^18 x 16384 (d = 128).
+constexpr int TC_KS = 16;             // pass-1 per-row list length
+
+KNN_DI void exchange(float &a, float &b) {
+    const float x = a;
+    a = fminf(x, b);
+    b = fmaxf(x, b);
+}
+
+// Ascending sort of 16 values in registers (Batcher's odd-even merge sort).
+KNN_DI void sort16(float (&s)[16]) {
+    constexpr int net[63][2] = {
+        {0, 1}, {2, 3}, {4, 5}, {6, 7}, {8, 9}, {10, 11}, {12, 13}, {14, 15}, {0, 2},
+        {1, 3}, {4, 6}, {5, 7}, {8, 10}, {9, 11}, {12, 14}, {13, 15}, {1, 2}, {5, 6},
+        {9, 10}, {13, 14}, {0, 4}, {1, 5}, {2, 6}, {3, 7}, {8, 12}, {9, 13}, {10, 14},
+        {11, 15}, {2, 4}, {3, 5}, {10, 12}, {11, 13}, {1, 2}, {3, 4}, {5, 6}, {9, 10},
+        {11, 12}, {13, 14}, {0, 8}, {1, 9}, {2, 10}, {3, 11}, {4, 12}, {5, 13}, {6, 14},
+        {7, 15}, {4, 8}, {5, 9}, {6, 10}, {7, 11}, {2, 4}, {3, 5}, {6, 8}, {7, 9},
+        {10, 12}, {11, 13}, {1, 2}, {3, 4}, {5, 6}, {7, 8}, {9, 10}, {11, 12}, {13, 14},
+    };
+#pragma unroll
+    for (int i = 0; i < 63; ++i) exchange(s[net[i][0]], s[net[i][1]]);
+}
+
+// L (ascending) becomes the 16 smallest of L and the ascending s.
+KNN_DI void merge16(float (&L)[16], const float (&s)[16]) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) L[i] = fminf(L[i], s[15 - i]);   // a bitonic sequence
+#pragma unroll
+    for (int st = 8; st > 0; st >>= 1)
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+            if (!(i & st)) exchange(L[i], L[i + st]);
+}
+
+template <int CHUNKS>
+KNN_DI void sample_tile(float (&L)[TC_KS], const uint32_t (&v)[CHUNKS][32]) {
+    static_assert(CHUNKS == 4 && TC_KS == 16, "groups of four, lists of 16");
+    uint32_t g[32];
+#pragma unroll
+    for (int e = 0; e < 32; ++e)
+        g[e] = __float_as_uint(min3f(fminf(__uint_as_float(v[0][e]), __uint_as_float(v[1][e])),
+                                     __uint_as_float(v[2][e]), __uint_as_float(v[3][e])));
+    const float lim = L[TC_KS - 1];
+    if (!__any_sync(0xffffffffu, min32(g) < lim)) return;
+    uint32_t m = below_mask(g, lim);
+    if (__reduce_max_sync(0xffffffffu, (unsigned)__popc(m)) > 5) {
+        float s[16];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) s[i] = __uint_as_float(g[16 * h + i]);
+            sort16(s);
+            merge16(L, s);
+        }
+        return;
+    }
+    while (m) {
+        const int e = __ffs(m) - 1;
+        m &= m - 1;
+        const float x = __uint_as_float(select32(g, e));
+        if (x < L[TC_KS - 1]) {
+            // sorted insertion: L[i] becomes the median of L[i - 1], x, L[i]
+            // (no NaN reaches here)
+#pragma unroll
+            for (int i = TC_KS - 1; i > 0; --i) L[i] = fmaxf(L[i - 1], fminf(x, L[i]));
+            L[0] = fminf(L[0], x);
+        }
+    }
+}
 
 // ---------------------------------------------------------------------------
 // The tensor scan on CTA pairs (cta_group::2): pass 1 (MODE 0, the tiles
@@ -515,36 +600,28 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
             // first reference of this warp
             const int col0 = (a.tile_base + *tile) * TP_BN + hc * TP_COLS;
             const int valid = a.N - col0;
+            if (valid < TP_COLS) {
 #pragma unroll
-            for (int c = 0; c < TP_CHUNKS; ++c) {
-                const int cvalid = valid - c * 32;
-                if (cvalid < 32) {
+                for (int c = 0; c < TP_CHUNKS; ++c)
 #pragma unroll
                     for (int e = 0; e < 32; ++e)
-                        if (e >= cvalid) v[c][e] = 0x7f800000u;   // +inf
-                }
-                const float lim = MODE == 1 ? thr : L[TC_KS - 1];
-                if (!(min32(v[c]) < lim)) continue;
-                uint32_t m = below_mask(v[c], lim);
+                        if (c * 32 + e >= valid) v[c][e] = 0x7f800000u;   // +inf
+            }
+            if (MODE == 0) {
+                sample_tile(L, v);
+                continue;
+            }
+#pragma unroll
+            for (int c = 0; c < TP_CHUNKS; ++c) {
+                if (!(min32(v[c]) < thr)) continue;
+                uint32_t m = below_mask(v[c], thr);
                 const int cbase = col0 + c * 32;
                 while (m) {
                     const int e = __ffs(m) - 1;
                     m &= m - 1;
                     const uint32_t xb = select32(v[c], e);
-                    if (MODE == 1) {
-                        pend.push(((unsigned long long)ord_bits(xb) << 32) | (uint32_t)(cbase + e),
-                                  a.count, a.cand, a.cmax, qrow);
-                    } else {
-                        const float x = __uint_as_float(xb);
-                        if (x < L[TC_KS - 1]) {
-                            // sorted insertion: L[i] becomes the median of
-                            // L[i - 1], x, L[i] (no NaN reaches here)
-#pragma unroll
-                            for (int i = TC_KS - 1; i > 0; --i)
-                                L[i] = fmaxf(L[i - 1], fminf(x, L[i]));
-                            L[0] = fminf(L[0], x);
-                        }
-                    }
+                    pend.push(((unsigned long long)ord_bits(xb) << 32) | (uint32_t)(cbase + e),
+                              a.count, a.cand, a.cmax, qrow);
                 }
             }
         }
@@ -623,61 +700,71 @@ KNN_DI void write_norm_row(__nv_bfloat16 *parts, int p, float s) {
     dst[1] = row[1];
 }
 
-// Squared norm of each point of a dim x n set, translated by -center
-// (sequential FP32 fma over d), and optionally the largest squared norm
-// (non-negative float bits compare as unsigned).
-// With absmax_bits, also the largest |x - c| of any coordinate (FP8 scale).
-__global__ void tc_norms_kernel(const float *__restrict__ x, int n, long long ld, int d,
-                                const float *__restrict__ center, float *__restrict__ nrm,
-                                unsigned *__restrict__ max_bits,
-                                unsigned *__restrict__ absmax_bits = nullptr) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+// Query prep: dim x n (row pitch ld) FP32 -> n x d_pad BF16 of -2 (x - center)
+// (so bf16(-2 y) = -2 bf16(y)), zero-padded in [d, d_pad), with xlo also the lo
+// part bf16(-2 y - hi) of split BF16, the squared norm of x - center (nullptr:
+// not wanted) and, with absmax_bits, the largest |x - center| of any coordinate
+// (FP8 scale).  A block takes 32 queries; warp w transposes the 32-dimension
+// chunks w, w + 8, ... through a tile of its own, each lane adding up its
+// query's part of the norm, and the warps' parts are added in order at the end.
+// (One thread per query and a chain over all dimensions took 109 us at 2001
+// queries, d = 768, and 39 at 16384, d = 256, next to the packing kernel's 5; this
+// one takes 18 and 11.5 for both.)
+constexpr int TC_QP_WARPS = 8;
+__global__ void __launch_bounds__(32 * TC_QP_WARPS, 3)
+    tc_prep_query_kernel(const float *__restrict__ x, int n, long long ld, int d, int d_pad,
+                         const float *__restrict__ center, float *__restrict__ nrm,
+                         unsigned *__restrict__ absmax_bits, __nv_bfloat16 *__restrict__ xb,
+                         __nv_bfloat16 *__restrict__ xlo) {
+    __shared__ float tile_all[TC_QP_WARPS][32][33], part[TC_QP_WARPS][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float(*tile)[33] = tile_all[warp];
+    const int p0 = blockIdx.x * 32, p = p0 + lane;
     float s = 0.f, am = 0.f;
-    if (p < n) {
-        for (int dd = 0; dd < d; ++dd) {
-            const float v = x[(size_t)dd * ld + p] - center[dd];
-            s = fmaf(v, v, s);
-            am = fmaxf(am, fabsf(v));
+    // write-out roles: 8 rounds of 4 queries, lane -> query 4 r + lane / 8,
+    // dimensions 4 (lane % 8) .. + 3
+    const int wp = lane >> 3, wm = lane & 7;
+    for (int d0 = warp * 32; d0 < d_pad; d0 += TC_QP_WARPS * 32) {
+        float v[32];
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+            v[j] = (d0 + j < d && p < n) ? x[(size_t)(d0 + j) * ld + p] : 0.f;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const float y = d0 + j < d && p < n ? v[j] - __ldg(center + d0 + j) : 0.f;
+            s = fmaf(y, y, s);
+            am = fmaxf(am, fabsf(y));
+            tile[j][lane] = y;
         }
-        nrm[p] = s;
-    }
-    unsigned m = __float_as_uint(s), ma = __float_as_uint(am);
+        __syncwarp();
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-        ma = max(ma, __shfl_xor_sync(0xffffffffu, ma, o));
-    }
-    if ((threadIdx.x & 31) == 0 && max_bits) atomicMax(max_bits, m);
-    if ((threadIdx.x & 31) == 0 && absmax_bits) atomicMax(absmax_bits, ma);
-}
-
-// dim x n (row pitch ld) FP32 -> n x d_pad BF16 of scale * (x - center)
-// (scale a power of two, so bf16(scale y) = scale bf16(y)), zero-padded in
-// [d, d_pad); with xlo also the lo part bf16(scale y - hi) of split BF16.
-// 32 x 32 tiles through shared memory.
-__global__ void tc_pack_kernel(const float *__restrict__ x, int n, long long ld, int d,
-                               int d_pad, const float *__restrict__ center, float scale,
-                               __nv_bfloat16 *__restrict__ xb,
-                               __nv_bfloat16 *__restrict__ xlo = nullptr) {
-    __shared__ float tile[32][33];
-    const int p0 = blockIdx.x * 32, d0 = blockIdx.y * 32;
-    const int tx = threadIdx.x, ty = threadIdx.y;
+        for (int r = 0; r < 8; ++r) {
+            const int pp = 4 * r + wp;
+            if (p0 + pp >= n) continue;
+            __nv_bfloat16 hi[4], lo[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int dd = d0 + ty + 8 * i, p = p0 + tx;
-        tile[ty + 8 * i][tx] = (dd < d && p < n) ? x[(size_t)dd * ld + p] : 0.f;
+            for (int e = 0; e < 4; ++e) {
+                const float y = tile[4 * wm + e][pp] * -2.0f;
+                hi[e] = __float2bfloat16_rn(y);
+                lo[e] = __float2bfloat16_rn(y - __bfloat162float(hi[e]));
+            }
+            const size_t at = (size_t)(p0 + pp) * d_pad + d0 + 4 * wm;
+            *reinterpret_cast<uint2 *>(xb + at) = *reinterpret_cast<const uint2 *>(hi);
+            if (xlo) *reinterpret_cast<uint2 *>(xlo + at) = *reinterpret_cast<const uint2 *>(lo);
+        }
+        __syncwarp();
     }
+    if (absmax_bits) {
+        const unsigned ma = __reduce_max_sync(0xffffffffu, __float_as_uint(am));
+        if (lane == 0) atomicMax(absmax_bits, ma);
+    }
+    part[warp][lane] = s;
     __syncthreads();
+    if (warp == 0 && p < n && nrm) {
+        s = 0.f;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int p = p0 + ty + 8 * i, dd = d0 + tx;
-        if (p < n && dd < d_pad) {
-            const float v = dd < d ? tile[tx][ty + 8 * i] - center[dd] : 0.f;
-            const __nv_bfloat16 hi = __float2bfloat16_rn(v * scale);
-            xb[(size_t)p * d_pad + dd] = hi;
-            if (xlo)
-                xlo[(size_t)p * d_pad + dd] = __float2bfloat16_rn(v * scale - __bfloat162float(hi));
-        }
+        for (int w = 0; w < TC_QP_WARPS; ++w) s += part[w][lane];
+        nrm[p] = s;
     }
 }
 
@@ -726,8 +813,7 @@ __global__ void __launch_bounds__(256)
 // four warps per tile).  A warp owns 32 points (one per lane) and walks the
 // dimensions in chunks of 32: each lane loads its point's 32 values of the
 // chunk (coalesced rows, the next chunk's loads in flight meanwhile),
-// accumulates its squared norm in increasing d with FP32 fma (the order
-// tc_norms_kernel uses), and the chunk is transposed through a padded
+// accumulates its squared norm in increasing d with FP32 fma, and the chunk is transposed through a padded
 // shared tile so that every store writes four points' 128-byte rows.
 constexpr int TC_PREP_WARPS = 4;
 constexpr int TC_PREP_LD = 36;   // floats per point row of the transpose tile
@@ -909,7 +995,7 @@ __global__ void tc_pack_ref_f8_kernel(const float *__restrict__ xt, int n, int d
 }
 
 // dim x n FP32 queries -> n x d_pad8 e4m3 of scale (x - c) (scale = -2 s_q),
-// zero-padded; 32 x 32 tiles through shared memory as in tc_pack_kernel.
+// zero-padded; 32 x 32 tiles through shared memory.
 __global__ void tc_pack_f8_kernel(const float *__restrict__ x, int n, long long ld, int d,
                                   int d_pad8, const float *__restrict__ center, float scale,
                                   unsigned char *__restrict__ x8) {
@@ -944,37 +1030,69 @@ __global__ void tc_pack_f8_kernel(const float *__restrict__ x, int n, long long 
 // [L_0, T] holds many times that; n_wide[0] counts them for probe0 (BF16:
 // switch to split BF16), n_wide[1] for probe1 (FP8: whether an FP8 pass 2
 // pays).
-__global__ void tc_threshold_kernel(const float *__restrict__ p1, int S, int Q,
-                                    const float *__restrict__ qn,
-                                    const unsigned *__restrict__ rmax_bits, TcBound bound,
-                                    TcBound probe0, TcBound probe1, float *__restrict__ thr,
-                                    float *__restrict__ thr_raw, int *__restrict__ count,
-                                    int *__restrict__ n_wide) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= Q) return;
-    float L[TC_KS];
+// One warp per query: the lists' values pass through a sorted list of KS keys
+// that lies across its lanes (one thread per query read the up to 148 lists of
+// a small batch one after the other: 33 us at 13 queries, now 6.7).
+constexpr int TC_THR_WARPS = 4;
+__global__ void __launch_bounds__(32 * TC_THR_WARPS)
+    tc_threshold_kernel(const float *__restrict__ p1, int S, int Q, const float *__restrict__ qn,
+                        const unsigned *__restrict__ rmax_bits, TcBound bound, TcBound probe0,
+                        TcBound probe1, float *__restrict__ thr, float *__restrict__ thr_raw,
+                        int *__restrict__ count, int *__restrict__ n_wide) {
+    const int lane = threadIdx.x & 31;
+    const int q = blockIdx.x * TC_THR_WARPS + (threadIdx.x >> 5);
+    bool wide0 = false, wide1 = false;
+    if (q < Q) {
+        unsigned long long mine = kKeyInf, tau = kKeyInf;
+        auto key_of = [&](int s, int i) {
+            if (s >= S) return kKeyInf;
+            const float v = p1[((size_t)s * Q + q) * TC_KS + i];
+            return ((unsigned long long)ord_bits(__float_as_uint(v)) << 32) |
+                   (uint32_t)(s * TC_KS + i);
+        };
+        constexpr int U = 4;   // loads in flight
+        unsigned long long key[U];
+        if (S <= 8) {
+            // few lists: two whole lists a step
 #pragma unroll
-    for (int i = 0; i < TC_KS; ++i) L[i] = INFINITY;
-    for (int s = 0; s < S; ++s) {
-        const float *src = p1 + ((size_t)s * Q + q) * TC_KS;
-        for (int i = 0; i < TC_KS; ++i) {
-            const float v = src[i];
-            if (!(v < L[TC_KS - 1])) break;   // lists are ascending
+            for (int u = 0; u < U; ++u) key[u] = key_of(2 * u + (lane >> 4), lane & 15);
 #pragma unroll
-            for (int t = TC_KS - 1; t > 0; --t)
-                L[t] = v < L[t - 1] ? L[t - 1] : (v < L[t] ? v : L[t]);
-            L[0] = fminf(L[0], v);
+            for (int u = 0; u < U; ++u) lane_list_add(mine, tau, key[u], TC_KS, lane);
+        } else {
+            // many: the lists' first values, then their second ones, ... until
+            // none of a rank passes (the lists are ascending)
+            for (int i = 0; i < TC_KS; ++i) {
+                bool any = false;
+                for (int s0 = 0; s0 < S; s0 += 32 * U) {
+#pragma unroll
+                    for (int u = 0; u < U; ++u) key[u] = key_of(s0 + 32 * u + lane, i);
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        any = any || key[u] < tau;
+                        lane_list_add(mine, tau, key[u], TC_KS, lane);
+                    }
+                }
+                if (!__any_sync(0xffffffffu, any)) break;
+            }
+        }
+        const float T = ord_float((uint32_t)(tau >> 32));
+        const float L0 = ord_float((uint32_t)(__shfl_sync(0xffffffffu, mine, 0) >> 32));
+        if (lane == 0) {
+            const float r2 = __uint_as_float(*rmax_bits);
+            thr[q] = T + tc_error_bound(qn[q], r2, T, bound);
+            thr_raw[q] = T;
+            count[q] = 0;
+            const float spread = T - L0;
+            wide0 = tc_error_bound(qn[q], r2, T, probe0) > spread;
+            wide1 = tc_error_bound(qn[q], r2, T, probe1) > spread;
         }
     }
-    const float T = L[TC_KS - 1];
-    const float r2 = __uint_as_float(*rmax_bits);
-    thr[q] = T + tc_error_bound(qn[q], r2, T, bound);
-    thr_raw[q] = T;
-    count[q] = 0;
     if (n_wide) {
-        const float spread = T - L[0];
-        if (tc_error_bound(qn[q], r2, T, probe0) > spread) atomicAdd(n_wide, 1);
-        if (tc_error_bound(qn[q], r2, T, probe1) > spread) atomicAdd(n_wide + 1, 1);
+        const int n0 = __syncthreads_count(wide0), n1 = __syncthreads_count(wide1);
+        if (threadIdx.x == 0) {
+            if (n0) atomicAdd(n_wide, n0);
+            if (n1) atomicAdd(n_wide + 1, n1);
+        }
     }
 }
 
@@ -1643,9 +1761,11 @@ TcPlan plan_tc(int N, int Q, int d, int k, int num_sms, bool point_sample = fals
         p.p1_rows = (ns + m - 1) / m;
         p.sample = contiguous_tiles((p.p1_rows + TP_BN - 1) / TP_BN);
     }
-    // coarser pass-1 splits amortise each pair's set-up (query tile load,
-    // TMEM allocation, pipeline fill)
-    p.splits1 = choose_splits(p.qtiles, p.sample.units, 16, 8.0, std::max(1, num_sms / 2));
+    // a pair's set-up (query tile load, TMEM allocation, pipeline fill) and its
+    // first tiles' insertions cost about as much as 6 tiles; with splits of 2
+    // tiles and more instead of 16 the sample of 100003 points, 2001 queries, d =
+    // 768 takes 24 us instead of 119, that of 33000 x 100, d = 64, 10 instead of 19
+    p.splits1 = choose_splits(p.qtiles, p.sample.units, 2, 6.0, std::max(1, num_sms / 2));
     return p;
 }
 
@@ -1956,8 +2076,9 @@ int emit_scan(const TcRun &r, cudaStream_t st, int kind, int Q, const float *thr
                                       : (size_t)r.d_pad * 2 * (kind == kTcBf16x3 ? 2 : 1);
     const size_t tile_bytes = (size_t)TP_BN * (row + 32);
     const int max_tiles = (int)std::max<size_t>(1, kSplitBytes / tile_bytes);
+    // (splits of 2 tiles and more: 13.6 us at 33000 x 100, d = 64, 30 with 8)
     const int splits =
-        choose_splits(qtiles, te - tb, 8, 2.0, std::max(1, r.P.num_sms / 2), max_tiles);
+        choose_splits(qtiles, te - tb, 2, 2.0, std::max(1, r.P.num_sms / 2), max_tiles);
     return launch_scan<1>(r, st, kind, r.qB, r.qBlo, r.q8, Q, thr, cmax, tb,
                           contiguous_tiles(te - tb), splits);
 }
@@ -2082,11 +2203,9 @@ int tc_run_begin(const TcProblem &P, const TcRefView &R, cudaStream_t st, TcRun 
 
     // queries: norms (and their largest |q - c|) + BF16 K-major copy of -2 q
     if (cudaMemsetAsync(r.nwide, 0, 4 * sizeof(int), st) != cudaSuccess) return kErrCuda;
-    tc_norms_kernel<<<(P.Q + 255) / 256, 256, 0, st>>>(
-        P.qry, P.Q, P.ldq, P.d, R.center, r.qn, nullptr,
-        fp8 ? reinterpret_cast<unsigned *>(r.nwide + 2) : nullptr);
-    tc_pack_kernel<<<dim3((P.Q + 31) / 32, p.d_pad / 32), dim3(32, 8), 0, st>>>(
-        P.qry, P.Q, P.ldq, P.d, p.d_pad, R.center, -2.0f, r.qB);
+    tc_prep_query_kernel<<<(P.Q + 31) / 32, 32 * TC_QP_WARPS, 0, st>>>(
+        P.qry, P.Q, P.ldq, P.d, p.d_pad, R.center, r.qn,
+        fp8 ? reinterpret_cast<unsigned *>(r.nwide + 2) : nullptr, r.qB, nullptr);
     if (cudaGetLastError() != cudaSuccess) return kErrLaunch;
     r.want_fp8 = false;
     if (fp8) {
@@ -2122,7 +2241,7 @@ int tc_run_pass1(TcRun &r, cudaStream_t st) {
     const bool probe = !forced && P.host_tmp && ((P.adaptive && lo_ok) || r.want_fp8);
     if (probe && cudaMemsetAsync(r.nwide, 0, 2 * sizeof(int), st) != cudaSuccess) return kErrCuda;
     const TcBound b16 = run_bound(r, kTcBf16);
-    tc_threshold_kernel<<<(P.Q + 255) / 256, 256, 0, st>>>(
+    tc_threshold_kernel<<<(P.Q + TC_THR_WARPS - 1) / TC_THR_WARPS, 32 * TC_THR_WARPS, 0, st>>>(
         r.p1, TP_LISTS * r.splits1, P.Q, r.qn, r.R.rmax_bits, b16, b16,
         r.want_fp8 ? run_bound(r, kTcFp8) : b16, r.thr, r.thr_raw, r.count,
         probe ? r.nwide : nullptr);
@@ -2155,8 +2274,8 @@ int tc_run_pass1(TcRun &r, cudaStream_t st) {
             // most lists expected to overflow in BF16: pass 2 runs in split
             // BF16 (thresholds re-derived from the sample)
             if ((rc = ensure_ref_lo(r, st)) != kOk) return rc;
-            tc_pack_kernel<<<dim3((P.Q + 31) / 32, r.d_pad / 32), dim3(32, 8), 0, st>>>(
-                P.qry, P.Q, P.ldq, P.d, r.d_pad, r.R.center, -2.0f, r.qB, r.qBlo);
+            tc_prep_query_kernel<<<(P.Q + 31) / 32, 32 * TC_QP_WARPS, 0, st>>>(
+                P.qry, P.Q, P.ldq, P.d, r.d_pad, r.R.center, nullptr, nullptr, r.qB, r.qBlo);
             tc_rethreshold_kernel<<<(P.Q + 255) / 256, 256, 0, st>>>(
                 r.thr_raw, P.Q, r.qn, r.R.rmax_bits, run_bound(r, kTcBf16x3), b16, 0, r.thr);
             if (cudaGetLastError() != cudaSuccess) return kErrLaunch;
@@ -2260,10 +2379,8 @@ int tc_run_finish(TcRun &r, cudaStream_t st, int *host_stats) {
     if (kind2 == kTcBf16x3 && (rc = ensure_ref_lo(r, st)) != kOk) return rc;
     gather_queries_kernel<<<dim3((nf + 127) / 128, P.d), 128, 0, st>>>(P.qry, P.ldq, P.d, r.fail,
                                                                        nf, r.qsub, r.ldf);
-    tc_norms_kernel<<<(nf + 255) / 256, 256, 0, st>>>(r.qsub, nf, r.ldf, P.d, r.R.center, r.qn,
-                                                      nullptr);
-    tc_pack_kernel<<<dim3((nf + 31) / 32, r.d_pad / 32), dim3(32, 8), 0, st>>>(
-        r.qsub, nf, r.ldf, P.d, r.d_pad, r.R.center, -2.0f, r.qB,
+    tc_prep_query_kernel<<<(nf + 31) / 32, 32 * TC_QP_WARPS, 0, st>>>(
+        r.qsub, nf, r.ldf, P.d, r.d_pad, r.R.center, r.qn, nullptr, r.qB,
         kind2 == kTcBf16x3 ? r.qBlo : nullptr);
     tc_retry_prep_kernel<<<(nf + 255) / 256, 256, 0, st>>>(
         r.fail, nf, r.retry, r.retry_f, r.retry_s, r.qn, r.R.rmax_bits, run_bound(r, kind2), r.thr,
