@@ -480,8 +480,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
         __syncwarp();
     } else if (warp == 1) {
         // ---------------- MMA issuer (even CTA) ----------------
-        if (lead && lane == 0) {
-            bool ok = n_my == 0 || KA == 0 || mbar_wait(a_full, 0);
+        // The whole warp walks the loop, with votes on every wait, and one
+        // elected lane issues: the operands of tcgen05.mma and of the commits
+        // live in uniform registers, which the compiler only keeps them in when
+        // the control flow is uniform.  (With a single lane in the loop every
+        // instruction first moved its descriptors there: 69 cycles an MMA and 230
+        // a commit, 607 for the four MMAs of a K block whose execution takes 512:
+        // the issuing thread bounded the scan.)
+        if (lead) {
+            auto waited = [&](uint64_t *bar, uint32_t parity) {
+                return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0;
+            };
+            bool ok = n_my == 0 || KA == 0 || waited(a_full, 0);
             bool issued_mma = false;
             int ms = 0;          // ring stage of the next item
             uint32_t mph = 0;    // its phase parity
@@ -494,59 +504,57 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
             for (int j = 0; j < n_my && ok; ++j) {
                 const int b = j & 1;
                 const uint32_t acc = tmem + (uint32_t)(b * TP_BN);
-                if (j >= 2 && !mbar_wait(&acc_empty[b], ((j >> 1) - 1) & 1)) {
+                if (j >= 2 && !waited(&acc_empty[b], ((j >> 1) - 1) & 1)) {
                     ok = false;
                     break;
                 }
                 const int ns = j % TP_NSLOTS;
-                if (!mbar_wait(&n_full[ns], (j / TP_NSLOTS) & 1) || *abort_flag) {
+                if (!waited(&n_full[ns], (j / TP_NSLOTS) & 1) ||
+                    __any_sync(0xffffffffu, *abort_flag != 0)) {
                     ok = false;
                     break;
                 }
                 tc_fence_after();
-                tp_mma_norm<KIND>(acc, odesc, umma_desc_sw32(sN + (size_t)ns * TP_NORM_BYTES));
-                umma_commit_pair_mc(&n_empty[ns], 0x3);
+                if (elect_one()) {
+                    tp_mma_norm<KIND>(acc, odesc,
+                                      umma_desc_sw32(sN + (size_t)ns * TP_NORM_BYTES));
+                    umma_commit_pair_mc(&n_empty[ns], 0x3);
+                }
                 issued_mma = true;
                 for (int i = 0; i < ITEMS; ++i) {
                     const int s = ms;
                     const uint32_t ph = mph;
                     if (++ms == NST) { ms = 0; mph ^= 1u; }
                     // (an abort elsewhere ends this wait by its time limit)
-                    if (!mbar_wait(&b_full[s], ph)) {
+                    if (!waited(&b_full[s], ph)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
                     const uint64_t sdesc = s_desc0 + (uint64_t)(s * stage_tiles) * kTileDesc;
                     const uint64_t bdesc = sdesc + (streamed ? kTileDesc : 0);
-                    if (streamed) {
-                        tp_mma_block<KIND>(acc, sdesc, bdesc);
-                    } else if (KIND == kTcBf16x3) {
-                        const int kb = i >> 1;
-                        const uint64_t ahi = a_desc0 + (uint64_t)kb * kTileDesc;
-                        if ((i & 1) == 0) {
-                            // B hi: A hi . B hi + A lo . B hi
-                            tp_mma_block<KIND>(acc, ahi, bdesc);
-                            tp_mma_block<KIND>(acc, a_desc0 + (uint64_t)(KB + kb) * kTileDesc,
-                                               bdesc);
-                        } else {
-                            tp_mma_block<KIND>(acc, ahi, bdesc);   // A hi . B lo
-                        }
-                    } else {
-                        tp_mma_block<KIND>(acc, a_desc0 + (uint64_t)i * kTileDesc, bdesc);
+                    // split BF16: items alternate B hi (A hi . B hi + A lo . B hi)
+                    // and B lo (A hi . B lo) of K block i / 2
+                    const uint64_t adesc =
+                        streamed ? sdesc
+                                 : a_desc0 + (uint64_t)(KIND == kTcBf16x3 ? (i >> 1) : i) * kTileDesc;
+                    if (elect_one()) {
+                        tp_mma_block<KIND>(acc, adesc, bdesc);
+                        if (KIND == kTcBf16x3 && (i & 1) == 0)
+                            tp_mma_block<KIND>(acc, adesc + (uint64_t)KB * kTileDesc, bdesc);
+                        umma_commit_pair_mc(&b_empty[s], 0x3);
                     }
-                    umma_commit_pair_mc(&b_empty[s], 0x3);
                 }
                 if (!ok) break;
-                umma_commit_pair_mc(&acc_full[b], 0x3);
+                if (elect_one()) umma_commit_pair_mc(&acc_full[b], 0x3);
             }
-            if (!ok) {
+            if (!ok && lane == 0) {
                 atomicMax(a.status, (int)kDevTimeoutFull);
                 *abort_flag = 1;
             }
             if (issued_mma) {
-                umma_commit_pair(drain);
-                if (!mbar_wait(drain, 0)) atomicMax(a.status, (int)kDevTimeoutDrain);
+                if (elect_one()) umma_commit_pair(drain);
+                if (!waited(drain, 0) && lane == 0) atomicMax(a.status, (int)kDevTimeoutDrain);
             }
         }
         __syncwarp();

@@ -132,6 +132,16 @@ KNN_DI void umma_f8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// True in one lane of the converged warp (the same one each time).
+KNN_DI bool elect_one() {
+    uint32_t p;
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "elect.sync _|P, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, P;\n\t}"
+        : "=r"(p));
+    return p != 0;
+}
 // Arrive on the mbarrier at this shared-memory offset in every CTA of
 // cta_mask once the pair MMAs issued so far have completed.
 KNN_DI void umma_commit_pair_mc(uint64_t *bar, uint16_t cta_mask) {
