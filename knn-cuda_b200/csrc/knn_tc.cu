@@ -251,7 +251,6 @@ constexpr int TP_COLS = TP_BN / (TP_EPI_WARPS / 4);   // columns per epilogue wa
 constexpr int TP_CHUNKS = TP_COLS / 32;
 constexpr int TP_THREADS = 32 * (2 + TP_EPI_WARPS);   // warp 0 TMA, warp 1 MMA, epilogue
 constexpr int TP_LISTS = TP_EPI_WARPS / 4;             // pass-1 lists per query and split
-constexpr int TP_NSLOTS = 2;          // norm-step ring slots
 
 // Operand kinds of the scan.  Every kind keeps the same epilogue: the
 // accumulator holds a (scaled for FP8) and the threshold test is the same.
@@ -261,30 +260,32 @@ enum TcKind : int {
     kTcFp8 = 2,      // FP8 e4m3 operands (kind::f8f6f4), power-of-two scales
 };
 
-// Shared memory: a region of TP_REGION_TILES operand tiles (128 rows x
-// 128 bytes, 16 KB each) holds the resident query tiles (A) followed by the
-// reference ring (B), or -- when A does not fit, d_pad > 512 in BF16 -- a
-// ring whose stages carry an A tile and a B tile each; then the ones tile,
-// the norm-step ring and the barriers.
+// Shared memory: a pool that holds the resident query tiles (A, 128 rows x 128
+// bytes, 16 KB each), the reference ring (B) -- or, when A does not fit, d_pad >
+// 512 in BF16, a ring whose stages carry an A tile and a B tile each -- and the
+// norm-step slots (tc_op divides it up); then the ones tile and the barriers.
+// The norm rows of a reference tile arrive on the full barrier of its first ring
+// item.  They need no barriers of their own: with NS x items >= stages slots, the
+// ring stage that the first item of tile j waits for was freed after the norm
+// step of tile j - NS.
 constexpr int TP_TILE_BYTES = TC_BM * 128;            // 16 KB
-constexpr int TP_REGION_TILES = 13;
-constexpr int TP_MAX_RESIDENT_A = 8;                   // leaves >= 5 ring stages
-constexpr int TP_MAX_STAGES = TP_REGION_TILES - 1;
 constexpr int TP_NORM_BYTES = TC_BM * 32;              // 4 KB: 32-byte norm-step rows
-constexpr size_t TP_OFF_REGION = 0;
-constexpr size_t TP_OFF_ONES = (size_t)TP_REGION_TILES * TP_TILE_BYTES;   // 208 KB
-constexpr size_t TP_OFF_N = TP_OFF_ONES + TP_NORM_BYTES;                   // +4 KB
-constexpr size_t TP_OFF_BAR = TP_OFF_N + (size_t)TP_NSLOTS * TP_NORM_BYTES;  // +8 KB
-constexpr int TP_NBARS = 1 + 2 * TP_MAX_STAGES + 2 * TP_NSLOTS + 2 + 2 + 1;
+constexpr int TP_POOL_BYTES = 220 * 1024;
+constexpr int TP_MAX_RESIDENT_A = 8;                   // leaves >= 5 ring stages
+constexpr int TP_MAX_STAGES = 12;
+constexpr size_t TP_OFF_ONES = TP_POOL_BYTES;
+constexpr size_t TP_OFF_BAR = TP_OFF_ONES + TP_NORM_BYTES;
+constexpr int TP_NBARS = 1 + 2 * TP_MAX_STAGES + 2 + 2 + 1;
 constexpr size_t TP_SMEM = 1024 + TP_OFF_BAR + TP_NBARS * 8 + 16;
 static_assert(TP_SMEM <= 232448, "pair scan kernel shared memory");
-static_assert(TP_OFF_N % 1024 == 0 && TP_OFF_ONES % 1024 == 0, "tile alignment");
+static_assert(TP_OFF_ONES % 1024 == 0, "tile alignment");
 
 struct TpArgs {
     int N, Q;
     int kb;                 // K blocks per operand row (128 bytes each)
     int ka;                 // resident A tiles (0: A streamed with B)
     int stages;             // ring stages
+    int nslots;             // norm-step slots
     int items;              // ring items per reference tile
     int tile_base, n_splits;
     TileRuns tiles;         // scan tiles tile_base + tiles.tile(u), u < tiles.units
@@ -331,16 +332,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
     extern __shared__ unsigned char smem_raw[];
     unsigned char *base = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    unsigned char *sR = base + TP_OFF_REGION;
+    unsigned char *sR = base;
     unsigned char *sOnes = base + TP_OFF_ONES;
-    unsigned char *sN = base + TP_OFF_N;
     uint64_t *bars = reinterpret_cast<uint64_t *>(base + TP_OFF_BAR);
     uint64_t *a_full = bars;
     uint64_t *b_full = bars + 1;
     uint64_t *b_empty = b_full + TP_MAX_STAGES;
-    uint64_t *n_full = b_empty + TP_MAX_STAGES;
-    uint64_t *n_empty = n_full + TP_NSLOTS;
-    uint64_t *acc_full = n_empty + TP_NSLOTS;
+    uint64_t *acc_full = b_empty + TP_MAX_STAGES;
     uint64_t *acc_empty = acc_full + 2;
     uint64_t *drain = acc_empty + 2;
     uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + TP_NBARS);
@@ -354,6 +352,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
     const bool streamed = KA == 0;
     const int stage_tiles = streamed ? 2 : 1;
     const uint32_t stage_bytes = (uint32_t)(stage_tiles * TP_TILE_BYTES);
+    unsigned char *sN = base + (size_t)(KA + NST * stage_tiles) * TP_TILE_BYTES;
     // K-block width in elements of the operand type (128 bytes)
     const int kx = KIND == kTcFp8 ? 128 : 64;
     // this split's units [u0, u0 + n_my)
@@ -368,10 +367,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
         for (int s = 0; s < NST; ++s) {
             mbar_init(&b_full[s], 1);
             mbar_init(&b_empty[s], 1);
-        }
-        for (int s = 0; s < TP_NSLOTS; ++s) {
-            mbar_init(&n_full[s], 1);
-            mbar_init(&n_empty[s], 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
@@ -402,14 +397,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
 
     if (warp == 0) {
         // ---------------- TMA producer (both CTAs) ----------------
-        if (lane == 0) {
-            int issued = 0, n_issued = 0;
-            int ps = 0;          // ring stage of the next item
-            uint32_t pph = 0;    // its phase parity
-            bool a_issued = false, ok = true;
-            const int half_row = (int)rank * TC_BM;
-            const int qrow0 = qpair * TC_QT + half_row;
-            if (n_my > 0 && KA > 0) {
+        // (uniform control flow with an elected issuer, as the MMA warp)
+        int issued = 0;
+        int ps = 0, ns = 0;  // ring stage and norm slot of the next item
+        uint32_t pph = 0;    // the stage's phase parity
+        bool a_issued = false, ok = true;
+        const int half_row = (int)rank * TC_BM;
+        const int qrow0 = qpair * TC_QT + half_row;
+        if (n_my > 0 && KA > 0) {
+            if (elect_one()) {
                 if (lead) mbar_arrive_expect_tx(a_full, (uint32_t)(2 * KA * TP_TILE_BYTES));
                 const uint32_t bar = mapa_shared(smem_u32(a_full), 0);
                 for (int t = 0; t < KA; ++t) {
@@ -417,65 +413,58 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
                     const CUtensorMap *m = (KIND == kTcBf16x3 && t >= KB) ? &tmA2 : &tmA;
                     tma_load_2d_pair(sR + (size_t)t * TP_TILE_BYTES, m, bar, (t % KB) * kx, qrow0);
                 }
-                a_issued = true;
             }
-            TileRuns::Iter tile = a.tiles.from(u0);
-            // the even CTA's full barriers (shared::cluster addresses) and
-            // the ring's first stage; stage s is 8 B and s stage_bytes on
-            const uint32_t bfull0 = mapa_shared(smem_u32(&b_full[0]), 0);
-            unsigned char *const stage0 = stage_ptr(0);
-            for (int j = 0; j < n_my && ok; ++j, tile.next()) {
-                const int row0 = (a.tile_base + *tile) * TP_BN + half_row;
-                const int ns = j % TP_NSLOTS;
-                if (j >= TP_NSLOTS && !mbar_wait(&n_empty[ns], ((j / TP_NSLOTS) - 1) & 1)) {
+            a_issued = true;
+        }
+        TileRuns::Iter tile = a.tiles.from(u0);
+        // the even CTA's full barriers (shared::cluster addresses) and the
+        // ring's first stage; stage s is 8 B and s stage_bytes on
+        const uint32_t bfull0 = mapa_shared(smem_u32(&b_full[0]), 0);
+        unsigned char *const stage0 = stage_ptr(0);
+        for (int j = 0; j < n_my && ok; ++j, tile.next()) {
+            const int row0 = (a.tile_base + *tile) * TP_BN + half_row;
+            for (int i = 0; i < ITEMS; ++i) {
+                const int it = j * ITEMS + i, s = ps;
+                const uint32_t ph = pph;
+                if (++ps == NST) { ps = 0; pph ^= 1u; }
+                // (an abort elsewhere ends this wait by its time limit)
+                if (it >= NST && !__all_sync(0xffffffffu, mbar_wait(&b_empty[s], ph ^ 1u))) {
                     ok = false;
                     break;
                 }
-                if (*abort_flag) break;
-                if (lead) mbar_arrive_expect_tx(&n_full[ns], 2 * TP_NORM_BYTES);
-                tma_load_2d_pair(sN + (size_t)ns * TP_NORM_BYTES, &tmN,
-                                 mapa_shared(smem_u32(&n_full[ns]), 0), 0, row0);
-                n_issued = j + 1;
-                for (int i = 0; i < ITEMS; ++i) {
-                    const int it = j * ITEMS + i, s = ps;
-                    const uint32_t ph = pph;
-                    if (++ps == NST) { ps = 0; pph ^= 1u; }
-                    if (it >= NST && !mbar_wait(&b_empty[s], ph ^ 1u)) {
-                        ok = false;
-                        break;
-                    }
-                    if (lead) mbar_arrive_expect_tx(&b_full[s], 2 * stage_bytes);
-                    const uint32_t bar = bfull0 + 8u * (uint32_t)s;
-                    unsigned char *dst = stage0 + (size_t)s * stage_bytes;
-                    // split BF16: items alternate hi, lo of K block i / 2
-                    const int kb = KIND == kTcBf16x3 ? (i >> 1) : i;
-                    const CUtensorMap *mb = (KIND == kTcBf16x3 && (i & 1)) ? &tmB2 : &tmB;
-                    if (streamed) {
-                        tma_load_2d_pair(dst, &tmA, bar, kb * kx, qrow0);
-                        dst += TP_TILE_BYTES;
-                    }
-                    tma_load_2d_pair(dst, mb, bar, kb * kx, row0);
-                    issued = it + 1;
+                const uint32_t bar = bfull0 + 8u * (uint32_t)s;
+                unsigned char *dst = stage0 + (size_t)s * stage_bytes;
+                // split BF16: items alternate hi, lo of K block i / 2
+                const int kb = KIND == kTcBf16x3 ? (i >> 1) : i;
+                if (elect_one()) {
+                    if (lead)
+                        mbar_arrive_expect_tx(&b_full[s],
+                                              2 * (stage_bytes + (i == 0 ? TP_NORM_BYTES : 0)));
+                    if (i == 0)
+                        tma_load_2d_pair(sN + (size_t)ns * TP_NORM_BYTES, &tmN, bar, 0, row0);
+                    if (streamed) tma_load_2d_pair(dst, &tmA, bar, kb * kx, qrow0);
+                    tma_load_2d_pair(dst + (streamed ? TP_TILE_BYTES : 0),
+                                     (KIND == kTcBf16x3 && (i & 1)) ? &tmB2 : &tmB, bar, kb * kx,
+                                     row0);
                 }
-                if (*abort_flag) break;
+                issued = it + 1;
             }
-            if (!ok) {
-                atomicMax(a.status, (int)kDevTimeoutEmpty);
-                *abort_flag = 1;
-            }
-            // The even CTA's full barriers count both CTAs' bytes: once its
-            // last phases completed, no TMA write into either CTA is in
-            // flight (the closing cluster barrier orders the odd CTA's exit
-            // after this).
-            if (lead) {
-                for (int it = max(0, issued - NST); it < issued; ++it)
-                    if (!mbar_wait(&b_full[it % NST], (it / NST) & 1))
-                        atomicMax(a.status, (int)kDevTimeoutDrain);
-                for (int j = max(0, n_issued - TP_NSLOTS); j < n_issued; ++j)
-                    if (!mbar_wait(&n_full[j % TP_NSLOTS], (j / TP_NSLOTS) & 1))
-                        atomicMax(a.status, (int)kDevTimeoutDrain);
-                if (a_issued && !mbar_wait(a_full, 0)) atomicMax(a.status, (int)kDevTimeoutDrain);
-            }
+            if (++ns == a.nslots) ns = 0;
+        }
+        if (!ok && lane == 0) {
+            atomicMax(a.status, (int)kDevTimeoutEmpty);
+            *abort_flag = 1;
+        }
+        // The even CTA's full barriers count both CTAs' bytes: once its
+        // last phases completed, no TMA write into either CTA is in
+        // flight (the closing cluster barrier orders the odd CTA's exit
+        // after this).
+        if (lead) {
+            bool drained = true;
+            for (int it = max(0, issued - NST); it < issued; ++it)
+                drained = mbar_wait(&b_full[it % NST], (it / NST) & 1) && drained;
+            if (a_issued) drained = mbar_wait(a_full, 0) && drained;
+            if (!drained && lane == 0) atomicMax(a.status, (int)kDevTimeoutDrain);
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -493,10 +482,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
             };
             bool ok = n_my == 0 || KA == 0 || waited(a_full, 0);
             bool issued_mma = false;
-            int ms = 0;          // ring stage of the next item
-            uint32_t mph = 0;    // its phase parity
+            int ms = 0, ns = 0;  // ring stage and norm slot of the next item
+            uint32_t mph = 0;    // the stage's phase parity
             tc_fence_after();
             const uint64_t odesc = umma_desc_sw32(sOnes);
+            const uint64_t n_desc0 = umma_desc_sw32(sN);
             // descriptors advance by the operand offset in 16-byte units
             const uint64_t a_desc0 = umma_desc_sw128(sR);
             const uint64_t s_desc0 = umma_desc_sw128(stage_ptr(0));
@@ -508,19 +498,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
                     ok = false;
                     break;
                 }
-                const int ns = j % TP_NSLOTS;
-                if (!waited(&n_full[ns], (j / TP_NSLOTS) & 1) ||
-                    __any_sync(0xffffffffu, *abort_flag != 0)) {
-                    ok = false;
-                    break;
-                }
-                tc_fence_after();
-                if (elect_one()) {
-                    tp_mma_norm<KIND>(acc, odesc,
-                                      umma_desc_sw32(sN + (size_t)ns * TP_NORM_BYTES));
-                    umma_commit_pair_mc(&n_empty[ns], 0x3);
-                }
-                issued_mma = true;
                 for (int i = 0; i < ITEMS; ++i) {
                     const int s = ms;
                     const uint32_t ph = mph;
@@ -539,13 +516,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
                         streamed ? sdesc
                                  : a_desc0 + (uint64_t)(KIND == kTcBf16x3 ? (i >> 1) : i) * kTileDesc;
                     if (elect_one()) {
+                        if (i == 0)
+                            tp_mma_norm<KIND>(acc, odesc,
+                                              n_desc0 + (uint64_t)ns * (TP_NORM_BYTES >> 4));
                         tp_mma_block<KIND>(acc, adesc, bdesc);
                         if (KIND == kTcBf16x3 && (i & 1) == 0)
                             tp_mma_block<KIND>(acc, adesc + (uint64_t)KB * kTileDesc, bdesc);
                         umma_commit_pair_mc(&b_empty[s], 0x3);
                     }
+                    issued_mma = true;
                 }
                 if (!ok) break;
+                if (++ns == a.nslots) ns = 0;
                 if (elect_one()) umma_commit_pair_mc(&acc_full[b], 0x3);
             }
             if (!ok && lane == 0) {
@@ -576,7 +558,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
             const int b = j & 1;
             const int pos = MODE == 1 ? pend.reserve(a.count, qrow) : 0;
             const bool got = mbar_wait(&acc_full[b], (j >> 1) & 1);
-            if (__any_sync(0xffffffffu, !got || *abort_flag != 0)) {
+            // (an abort elsewhere ends this wait by its time limit)
+            if (__any_sync(0xffffffffu, !got)) {
                 if (MODE == 1) pend.commit(pos, a.cand, a.cmax, qrow);
                 if (lane == 0) {
                     if (!got) atomicMax(a.status, (int)kDevTimeoutFull);
@@ -1690,7 +1673,7 @@ struct TcPlan {
 // resident A tiles (0: A streams beside B), ring stages and items per
 // reference tile.
 struct TcOp {
-    int kind, kb, ka, stages, items;
+    int kind, kb, ka, stages, items, nslots;
 };
 
 TcOp tc_op(int kind, int d_pad, int d_pad8) {
@@ -1709,7 +1692,14 @@ TcOp tc_op(int kind, int d_pad, int d_pad8) {
         o.ka = o.kb <= TP_MAX_RESIDENT_A ? o.kb : 0;
         o.items = o.kb;
     }
-    o.stages = o.ka > 0 ? TP_REGION_TILES - o.ka : TP_REGION_TILES / 2;
+    // the deepest ring whose norm slots (one for every `items` stages) fit too
+    const int stage_tiles = o.ka > 0 ? 1 : 2;
+    for (o.stages = TP_MAX_STAGES;; --o.stages) {
+        o.nslots = (o.stages + o.items - 1) / o.items;
+        if ((o.ka + o.stages * stage_tiles) * TP_TILE_BYTES + o.nslots * TP_NORM_BYTES <=
+            TP_POOL_BYTES)
+            break;
+    }
     return o;
 }
 
@@ -2038,6 +2028,7 @@ int launch_scan(const TcRun &r, cudaStream_t st, int kind, const __nv_bfloat16 *
     a.kb = op.kb;
     a.ka = op.ka;
     a.stages = op.stages;
+    a.nslots = op.nslots;
     a.items = op.items;
     a.tile_base = tile_base;
     a.tiles = tiles;
