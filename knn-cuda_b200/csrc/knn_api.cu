@@ -214,6 +214,7 @@ struct Workspace {
     int num_sms = 148;
     cudaStream_t stream = nullptr;
     cudaEvent_t last_done = nullptr;   // orders device-resident calls on this device
+    cudaEvent_t probe = nullptr;       // read-back of the tensor path's overflow prediction
     Buffer ref, qry, dist, idx, scratch, status;
     Buffer space;                      // spatial search of point clouds (optional)
     Buffer tcref;                      // prepared reference set of the tensor-core path
@@ -253,6 +254,7 @@ struct Workspace {
         if (cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess) return false;
         if (cudaEventCreateWithFlags(&last_done, cudaEventDisableTiming) != cudaSuccess)
             return false;
+        if (cudaEventCreateWithFlags(&probe, cudaEventDisableTiming) != cudaSuccess) return false;
         if (!status.ensure(sizeof(int))) return false;
         if (cudaMallocHost(reinterpret_cast<void **>(&status_host), sizeof(int)) != cudaSuccess)
             return false;
@@ -330,6 +332,7 @@ int enqueue(Workspace &ws, const ExactProblem &p0, int method, cudaStream_t st,
     t.request = (method == KNNB200_METHOD_FP8 && tc_fp8_supported(p.d)) ? kTcReqFp8 : kTcReqBf16;
     t.force_kind = g_force_kind;
     t.point_sample = true;   // the whole set is prepared before pass 1
+    t.probe_event = ws.probe;
     if (ws.bound_check) {
         if (cudaMemsetAsync(ws.bound.ptr, 0, 16, st) != cudaSuccess) return kErrCuda;
         t.bound_stat = static_cast<unsigned *>(ws.bound.ptr);

@@ -218,6 +218,12 @@ struct TcProblem {
     // of tiles (a set still streaming in): a sample spread over every part
     // of the set, whatever its order
     bool point_sample = false;
+    // event for the read-back of the overflow prediction (launch_tc): with it
+    // the main scan is queued before the host knows whether it runs in BF16
+    cudaEvent_t probe_event = nullptr;
+    // pinned, 2 ints: [0] the device status word, copied with the last
+    // read-back of a run, [1] whether nothing was queued after that copy
+    int *host_status = nullptr;
 };
 
 // A sample of the 256-point tiles: `run` consecutive tiles out of every
@@ -274,8 +280,14 @@ struct TcRun {
     __nv_bfloat16 *qB, *qBlo;
     unsigned char *q8;
     float *qn, *thr, *thr_raw, *retry, *retry_f, *retry_s, *p1, *qsub, *sd;
+    // control words, cleared together at the start: nfail [0] uncertified
+    // queries, [1] overflowing lists; cand_total; nwide [0], [1] predicted
+    // overflows, [2] query max |q - c| bits.  The first four are read back
+    // together.
+    int *ctl;
     int *count, *fail, *fail2, *nfail, *si, *nwide, *nsel;
     unsigned long long *cand_total, *cand;
+    bool undecided;         // the overflow prediction is on its way (probe_event)
     unsigned char *xs;
     size_t xcap;
     // incremental re-rank (tc_run_rerank_piece): running k smallest exact

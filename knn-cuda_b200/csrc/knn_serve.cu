@@ -62,13 +62,18 @@ struct Slot {
     cudaStream_t stream = nullptr;
     DevBuf scratch, qry, dist, idx, status;
     DevBuf space;                // spatial search of a point cloud (optional)
-    int *host_stats = nullptr;   // pinned, 8 ints
+    // pinned, 10 ints: the tensor path's 8, then its host_status
+    int *host_stats = nullptr;
+    cudaEvent_t probe = nullptr; // read-back of the tensor path's overflow prediction
     bool init(int device) {
         if (cudaSetDevice(device) != cudaSuccess) return false;
         if (cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess) return false;
         if (!status.ensure(sizeof(int))) return false;
-        if (cudaMallocHost(reinterpret_cast<void **>(&host_stats), 8 * sizeof(int)) != cudaSuccess)
+        if (cudaMallocHost(reinterpret_cast<void **>(&host_stats), 10 * sizeof(int)) !=
+                cudaSuccess ||
+            cudaEventCreateWithFlags(&probe, cudaEventDisableTiming) != cudaSuccess)
             return false;
+        host_stats[9] = 0;
         return true;
     }
     void destroy() {
@@ -80,7 +85,9 @@ struct Slot {
         idx.release();
         status.release();
         if (host_stats) cudaFreeHost(host_stats);
+        if (probe) cudaEventDestroy(probe);
         if (stream) cudaStreamDestroy(stream);
+        probe = nullptr;
         host_stats = nullptr;
         stream = nullptr;
     }
@@ -129,6 +136,7 @@ int run_refset(knnb200_refset *rs, Slot &slot, const float *query, int Q, long l
                int method, float *dist, int *idx, long long ld_out, cudaStream_t st) {
     if (!exact_supported_k(k)) return kErrUnsupported;
     if (!slot.scratch.ensure(scratch_need(rs, method, Q, k))) return kErrNoMemory;
+    slot.host_stats[9] = 0;
     if (cudaMemsetAsync(slot.status.ptr, 0, sizeof(int), st) != cudaSuccess) return kErrCuda;
     if (use_tc_for(rs, method, Q, k)) {
         TcProblem t;
@@ -151,6 +159,8 @@ int run_refset(knnb200_refset *rs, Slot &slot, const float *query, int Q, long l
         t.request = (method == KNNB200_METHOD_FP8 && tc_fp8_supported(rs->d)) ? kTcReqFp8
                                                                              : kTcReqBf16;
         t.point_sample = true;   // the resident set was prepared as a whole
+        t.probe_event = slot.probe;
+        t.host_status = slot.host_stats + 8;
         return launch_tc(t, rs->tc, st, slot.host_stats);
     }
     ExactProblem p;
@@ -279,6 +289,8 @@ int knnb200_refset_knn(knnb200_refset *rs, const float *query, int query_nb, lon
     int rc = run_refset(rs, rs->slot, query, query_nb, query_ld, k, method, knn_dist, knn_index,
                         out_ld, st);
     if (rc != kOk) return rc;
+    // the tensor path's last read-back brought the status word along
+    if (rs->slot.host_stats[9]) return rs->slot.host_stats[8] ? kErrDeviceTimeout : kOk;
     return slot_status(rs->slot, st);
 }
 

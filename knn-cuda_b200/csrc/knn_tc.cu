@@ -297,6 +297,8 @@ struct TpArgs {
     int *count;             // [Q]
     int cmax;
     int *status;
+    const int *n_wide;      // queries predicted to overflow: the scan does nothing
+                            // when they are more than half (nullptr: always runs)
 };
 
 // Norm step and one ring item's MMAs for each kind, issued by the even
@@ -344,6 +346,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
     uint32_t *tmem_holder = reinterpret_cast<uint32_t *>(bars + TP_NBARS);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_holder + 1);
 
+    // (both CTAs of a pair read the same word: they leave together)
+    if (a.n_wide && 2 * *a.n_wide > a.Q) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const bool lead = rank == 0;
@@ -1986,7 +1990,8 @@ int ensure_ref_f8(const TcRun &r, cudaStream_t st, unsigned *host_tmp) {
 template <int MODE>
 int launch_scan(const TcRun &r, cudaStream_t st, int kind, const __nv_bfloat16 *qB,
                 const __nv_bfloat16 *qBlo, const unsigned char *q8, int Q, const float *thr,
-                int cmax, int tile_base, const TileRuns &tiles, int n_splits) {
+                int cmax, int tile_base, const TileRuns &tiles, int n_splits,
+                const int *n_wide = nullptr) {
     const TcProblem &P = r.P;
     if (!kind_fits(kind, r.d_pad, r.d_pad8)) return kErrUnsupported;
     const TcOp op = tc_op(kind, r.d_pad, r.d_pad8);
@@ -2047,6 +2052,7 @@ int launch_scan(const TcRun &r, cudaStream_t st, int kind, const __nv_bfloat16 *
     a.count = r.count;
     a.cmax = cmax;
     a.status = P.status;
+    a.n_wide = n_wide;
     const dim3 grid(2 * ((Q + TC_QT - 1) / TC_QT), n_splits);
     auto go = [&](auto kern) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2064,7 +2070,7 @@ int launch_scan(const TcRun &r, cudaStream_t st, int kind, const __nv_bfloat16 *
 
 // Emission scan of the reference tiles [tb, te).
 int emit_scan(const TcRun &r, cudaStream_t st, int kind, int Q, const float *thr, int cmax,
-              int tb, int te) {
+              int tb, int te, const int *n_wide = nullptr) {
     const int qtiles = (Q + TC_QT - 1) / TC_QT;
     // reference bytes a tile streams (operand rows + norm-step rows); a
     // split holds at most kSplitBytes of them: measured at 2^20 x 256 BF16
@@ -2079,7 +2085,7 @@ int emit_scan(const TcRun &r, cudaStream_t st, int kind, int Q, const float *thr
     const int splits =
         choose_splits(qtiles, te - tb, 2, 2.0, std::max(1, r.P.num_sms / 2), max_tiles);
     return launch_scan<1>(r, st, kind, r.qB, r.qBlo, r.q8, Q, thr, cmax, tb,
-                          contiguous_tiles(te - tb), splits);
+                          contiguous_tiles(te - tb), splits, n_wide);
 }
 
 TcBound run_bound(const TcRun &r, int kind) {
@@ -2094,7 +2100,9 @@ int rerank(const TcRun &r, cudaStream_t st, int kind, int Q, int cmax, const flo
            long long ldq, const float *qn, const float *thr, const float *thr_raw,
            float *out_dist, int *out_idx, long long ld_out, int *fail, bool final_pass) {
     const TcProblem &P = r.P;
-    if (cudaMemsetAsync(r.nfail, 0, 2 * sizeof(int), st) != cudaSuccess) return kErrCuda;
+    // (clear at the start of a run)
+    if (final_pass && cudaMemsetAsync(r.nfail, 0, 2 * sizeof(int), st) != cudaSuccess)
+        return kErrCuda;
     int cpow = 32;
     while (cpow < cmax) cpow <<= 1;
     const size_t gsmem = tc_rr_gather_bytes(r.d_pad);
@@ -2184,9 +2192,11 @@ int tc_run_begin(const TcProblem &P, const TcRefView &R, cudaStream_t st, TcRun 
     r.fail = cv.take<int>(P.Q);
     r.fail2 = cv.take<int>(P.Q);
     r.nsel = cv.take<int>(P.Q);
-    r.nfail = cv.take<int>(4);
-    r.nwide = cv.take<int>(4);   // [0] predicted overflows, [2] query max |q - c| bits
-    r.cand_total = cv.take<unsigned long long>(1);
+    r.ctl = cv.take<int>(8);
+    r.nfail = r.ctl;
+    r.cand_total = reinterpret_cast<unsigned long long *>(r.ctl + 2);
+    r.nwide = r.ctl + 4;
+    r.undecided = false;
     r.p1 = cv.take<float>((size_t)TP_LISTS * p.splits1 * P.Q * TC_KS);
     r.cand = cv.take<unsigned long long>((size_t)P.Q * p.cmax);
     r.ldf = (P.Q + 3) / 4 * 4;   // second-chance buffers, sized for all queries
@@ -2201,7 +2211,7 @@ int tc_run_begin(const TcProblem &P, const TcRefView &R, cudaStream_t st, TcRun 
     r.done = nullptr;
 
     // queries: norms (and their largest |q - c|) + BF16 K-major copy of -2 q
-    if (cudaMemsetAsync(r.nwide, 0, 4 * sizeof(int), st) != cudaSuccess) return kErrCuda;
+    if (cudaMemsetAsync(r.ctl, 0, 8 * sizeof(int), st) != cudaSuccess) return kErrCuda;
     tc_prep_query_kernel<<<(P.Q + 31) / 32, 32 * TC_QP_WARPS, 0, st>>>(
         P.qry, P.Q, P.ldq, P.d, p.d_pad, R.center, r.qn,
         fp8 ? reinterpret_cast<unsigned *>(r.nwide + 2) : nullptr, r.qB, nullptr);
@@ -2218,8 +2228,22 @@ int tc_run_begin(const TcProblem &P, const TcRefView &R, cudaStream_t st, TcRun 
         r.want_fp8 = true;
     }
     if (P.timer) P.timer->mark(st, kPhaseTcPrepQuery);
-    if (cudaMemsetAsync(r.cand_total, 0, sizeof(unsigned long long), st) != cudaSuccess)
-        return kErrCuda;
+    return kOk;
+}
+
+// Most lists are expected to overflow in BF16: pass 2 runs in split BF16, with
+// thresholds re-derived from the sample.
+static int switch_to_split(TcRun &r, cudaStream_t st) {
+    const TcProblem &P = r.P;
+    const int rc = ensure_ref_lo(r, st);
+    if (rc != kOk) return rc;
+    tc_prep_query_kernel<<<(P.Q + 31) / 32, 32 * TC_QP_WARPS, 0, st>>>(
+        P.qry, P.Q, P.ldq, P.d, r.d_pad, r.R.center, nullptr, nullptr, r.qB, r.qBlo);
+    tc_rethreshold_kernel<<<(P.Q + 255) / 256, 256, 0, st>>>(r.thr_raw, P.Q, r.qn, r.R.rmax_bits,
+                                                            run_bound(r, kTcBf16x3),
+                                                            run_bound(r, kTcBf16), 0, r.thr);
+    if (cudaGetLastError() != cudaSuccess) return kErrLaunch;
+    r.kind = kTcBf16x3;
     return kOk;
 }
 
@@ -2238,7 +2262,6 @@ int tc_run_pass1(TcRun &r, cudaStream_t st) {
     const bool forced = (force == kTcBf16) || (force == kTcBf16x3 && lo_ok) ||
                         (force == kTcFp8 && r.want_fp8);
     const bool probe = !forced && P.host_tmp && ((P.adaptive && lo_ok) || r.want_fp8);
-    if (probe && cudaMemsetAsync(r.nwide, 0, 2 * sizeof(int), st) != cudaSuccess) return kErrCuda;
     const TcBound b16 = run_bound(r, kTcBf16);
     tc_threshold_kernel<<<(P.Q + TC_THR_WARPS - 1) / TC_THR_WARPS, 32 * TC_THR_WARPS, 0, st>>>(
         r.p1, TP_LISTS * r.splits1, P.Q, r.qn, r.R.rmax_bits, b16, b16,
@@ -2247,6 +2270,17 @@ int tc_run_pass1(TcRun &r, cudaStream_t st) {
     if (cudaGetLastError() != cudaSuccess) return kErrLaunch;
     r.kind = kTcBf16;
     int wide16 = 0, wide8 = 0;
+    if (probe && P.probe_event && !r.want_fp8) {
+        // BF16 unless most lists would overflow: launch_tc queues the BF16
+        // scan, which looks at the count itself, before the host knows it
+        if (cudaMemcpyAsync(P.host_tmp, r.nwide, sizeof(int), cudaMemcpyDeviceToHost, st) !=
+                cudaSuccess ||
+            cudaEventRecord(P.probe_event, st) != cudaSuccess)
+            return kErrCuda;
+        r.undecided = true;
+        if (P.timer) P.timer->mark(st, kPhaseTcThreshold);
+        return kOk;
+    }
     if (probe) {
         if ((rc = read_count(r.nwide, P.host_tmp, st, wide16, 2)) != kOk) return rc;
         wide8 = P.host_tmp[1];
@@ -2270,15 +2304,7 @@ int tc_run_pass1(TcRun &r, cudaStream_t st) {
             if (cudaGetLastError() != cudaSuccess) return kErrLaunch;
             r.kind = kTcFp8;
         } else if ((P.adaptive || forced) && lo_ok && 2 * wide16 > P.Q) {
-            // most lists expected to overflow in BF16: pass 2 runs in split
-            // BF16 (thresholds re-derived from the sample)
-            if ((rc = ensure_ref_lo(r, st)) != kOk) return rc;
-            tc_prep_query_kernel<<<(P.Q + 31) / 32, 32 * TC_QP_WARPS, 0, st>>>(
-                P.qry, P.Q, P.ldq, P.d, r.d_pad, r.R.center, nullptr, nullptr, r.qB, r.qBlo);
-            tc_rethreshold_kernel<<<(P.Q + 255) / 256, 256, 0, st>>>(
-                r.thr_raw, P.Q, r.qn, r.R.rmax_bits, run_bound(r, kTcBf16x3), b16, 0, r.thr);
-            if (cudaGetLastError() != cudaSuccess) return kErrLaunch;
-            r.kind = kTcBf16x3;
+            if ((rc = switch_to_split(r, st)) != kOk) return rc;
         }
     }
     if (P.timer) P.timer->mark(st, kPhaseTcThreshold);
@@ -2288,7 +2314,20 @@ int tc_run_pass1(TcRun &r, cudaStream_t st) {
 int tc_run_pass2(TcRun &r, int tile_begin, int tile_end, cudaStream_t st) {
     tile_end = std::min(tile_end, r.n_tiles2);
     if (tile_begin >= tile_end) return kOk;
-    const int rc = emit_scan(r, st, r.kind, r.P.Q, r.thr, r.cmax, tile_begin, tile_end);
+    int rc = kOk;
+    if (r.undecided) {
+        // the host's wait for the prediction hides behind this scan
+        rc = emit_scan(r, st, r.kind, r.P.Q, r.thr, r.cmax, tile_begin, tile_end, r.nwide);
+        if (rc != kOk) return rc;
+        if (cudaEventSynchronize(r.P.probe_event) != cudaSuccess) return kErrCuda;
+        r.undecided = false;
+        const bool wide = 2 * (long long)r.P.host_tmp[0] > r.P.Q;
+        if (!wide || (rc = switch_to_split(r, st)) != kOk) {
+            if (rc == kOk && r.P.timer) r.P.timer->mark(st, kPhaseTcPass2);
+            return rc;
+        }
+    }
+    rc = emit_scan(r, st, r.kind, r.P.Q, r.thr, r.cmax, tile_begin, tile_end);
     if (rc == kOk && r.P.timer) r.P.timer->mark(st, kPhaseTcPass2);
     return rc;
 }
@@ -2342,7 +2381,6 @@ int tc_run_finish(TcRun &r, cudaStream_t st, int *host_stats) {
     int rc = kOk;
     if (r.pieces) {
         // every candidate was re-ranked piece by piece: certify
-        if (cudaMemsetAsync(r.nfail, 0, 2 * sizeof(int), st) != cudaSuccess) return kErrCuda;
         RrBounds rb;
         rb.cur = run_bound(r, r.kind);
         rb.a_scale = 1.f;
@@ -2358,14 +2396,21 @@ int tc_run_finish(TcRun &r, cudaStream_t st, int *host_stats) {
     }
     if (rc != kOk) return rc;
     if (tm) tm->mark(st, kPhaseTcRerank);
-    if (cudaMemcpyAsync(host_stats + 4, r.cand_total, sizeof(unsigned long long),
-                        cudaMemcpyDeviceToHost, st) != cudaSuccess)
-        return kErrCuda;
+    // nfail[0..1] and cand_total land in host_stats[2..5]
+    if (P.host_status) {
+        P.host_status[1] = 0;
+        if (cudaMemcpyAsync(P.host_status, P.status, sizeof(int), cudaMemcpyDeviceToHost, st) !=
+            cudaSuccess)
+            return kErrCuda;
+    }
     int nf = 0;
-    if ((rc = read_count(r.nfail, host_tmp, st, nf, 2)) != kOk) return rc;
+    if ((rc = read_count(r.ctl, host_tmp, st, nf, 4)) != kOk) return rc;
     const int n_over = host_tmp[1];
     host_stats[0] = nf;
-    if (nf == 0) return kOk;
+    if (nf == 0) {
+        if (P.host_status) P.host_status[1] = 1;
+        return kOk;
+    }
 
     // second chance: the uncertified queries, compacted, scanned again with
     // thresholds that certify (list overflows excepted).  Kind: BF16 after
