@@ -280,20 +280,28 @@ bool valid_sizes(int ref_nb, int query_nb, int dim, int k) {
     return ref_nb >= 1 && query_nb >= 1 && dim >= 1 && k >= 1 && k <= ref_nb;
 }
 
-bool use_tc(int method, int N, int Q, int d, int k) {
-    return (method == KNNB200_METHOD_CUBLAS || method == KNNB200_METHOD_FP8) &&
-           tc_supported(N, Q, d, k);
+// The method a call runs with: the expansion methods become the exact one where
+// the tensor path does not apply or does not pay.  Decided once per call, for
+// all its query chunks.
+int route(int method, int N, int Q, int d, int k) {
+    if (method != KNNB200_METHOD_CUBLAS && method != KNNB200_METHOD_FP8) return method;
+    return tc_pays(N, Q, d, k) ? method : KNNB200_METHOD_GLOBAL;
+}
+
+// Whether a routed method runs the tensor path.
+bool use_tc(int method) {
+    return method == KNNB200_METHOD_CUBLAS || method == KNNB200_METHOD_FP8;
 }
 
 size_t scratch_for(int method, int N, int Q, int d, int k, int num_sms) {
-    if (use_tc(method, N, Q, d, k)) return tc_scratch_bytes(N, Q, d, k, num_sms);
+    if (use_tc(method)) return tc_scratch_bytes(N, Q, d, k, num_sms);
     return exact_scratch_bytes(N, Q, d, k, num_sms);
 }
 
 // Queue the computation for one problem whose inputs are on the device.
-// knn_cublas runs the tensor-core expansion path when the shape qualifies
-// (it synchronises the stream once, to recompute uncertified queries);
-// everything else runs the fused exact kernel.
+// A routed expansion method runs the tensor-core path (it synchronises the
+// stream once, to recompute uncertified queries); everything else runs the
+// fused exact kernel.
 // ref_prepared: the tensor-core view of this reference set is already in
 // ws.tcref (a later query chunk of the same call).
 int enqueue(Workspace &ws, const ExactProblem &p0, int method, cudaStream_t st,
@@ -304,7 +312,7 @@ int enqueue(Workspace &ws, const ExactProblem &p0, int method, cudaStream_t st,
     ExactProblem p = p0;
     p.timer = &ws.timer;
     ws.timer.begin(st);
-    if (!use_tc(method, p.N, p.Q, p.d, p.k)) return launch_exact(p, st);
+    if (!use_tc(method)) return launch_exact(p, st);
     if (!ws.tcref.ensure(tc_ref_bytes(p.N, p.d))) return kErrNoMemory;
     // a later chunk of the same call keeps the view (and its prepared copies)
     TcRefView v = tc_carve_ref(ws.tcref.ptr, p.N, p.d, ref_prepared ? nullptr : &ws.tc_state);
@@ -592,16 +600,16 @@ size_t host_chunk_bytes(int method, int N, int qc, int d, int k, int num_sms) {
 }
 
 // The body shared by the three host entry points.
-bool host_entry(int method, const float *ref, int ref_nb, const float *query, int query_nb,
+bool host_entry(int wanted, const float *ref, int ref_nb, const float *query, int query_nb,
                 int dim, int k, float *knn_dist, int *knn_index) {
     if (!ref || !query || !knn_dist || !knn_index) {
-        std::printf("ERROR: %s: null pointer argument\n", method_name(method));
+        std::printf("ERROR: %s: null pointer argument\n", method_name(wanted));
         return false;
     }
     if (!valid_sizes(ref_nb, query_nb, dim, k)) {
         std::printf("ERROR: %s: invalid sizes (ref_nb=%d query_nb=%d dim=%d k=%d; "
                     "need >= 1 and k <= ref_nb)\n",
-                    method_name(method), ref_nb, query_nb, dim, k);
+                    method_name(wanted), ref_nb, query_nb, dim, k);
         return false;
     }
     Workspace *ws = nullptr;
@@ -623,12 +631,22 @@ bool host_entry(int method, const float *ref, int ref_nb, const float *query, in
         return false;
     }
     const long long ldr = round_up(ref_nb, 64);
-    const bool tc = use_tc(method, ref_nb, query_nb, dim, k);
-    const size_t fixed = grown((size_t)dim * ldr * sizeof(float)) +
-                         (tc ? grown(tc_ref_bytes(ref_nb, dim)) : 0);
-    const int qc = plan_query_chunk(*ws, query_nb, fixed, [&](int c) {
-        return host_chunk_bytes(method, ref_nb, c, dim, k, ws->num_sms);
-    });
+    int method = route(wanted, ref_nb, query_nb, dim, k);
+    size_t fixed;
+    auto plan = [&] {
+        fixed = grown((size_t)dim * ldr * sizeof(float)) +
+                (use_tc(method) ? grown(tc_ref_bytes(ref_nb, dim)) : 0);
+        return plan_query_chunk(*ws, query_nb, fixed, [&](int c) {
+            return host_chunk_bytes(method, ref_nb, c, dim, k, ws->num_sms);
+        });
+    };
+    int qc = plan();
+    if (qc < query_nb && use_tc(method) && ref_nb < kTcAlwaysPoints) {
+        // a small set takes the tensor path only where the memory is no question
+        method = KNNB200_METHOD_GLOBAL;
+        qc = plan();
+    }
+    const bool tc = use_tc(method);
     if (qc < 1) {
         std::printf("ERROR: Memory allocation error\n");
         return false;
@@ -800,12 +818,22 @@ int knnb200_knn_device(const float *ref, int ref_nb, long long ref_ld, const flo
     // inputs and outputs are the caller's: only the scratch (and the tensor
     // path's prepared reference set) grow with the call; queries that do not
     // fit in one go run in chunks (column offsets into the caller's arrays)
-    const bool tc = use_tc(method, ref_nb, query_nb, dim, k);
-    const int qc = plan_query_chunk(*ws, query_nb, tc ? grown(tc_ref_bytes(ref_nb, dim)) : 0,
-                                    [&](int c) {
-                                        return grown(scratch_for(method, ref_nb, c, dim, k,
-                                                                 ws->num_sms));
-                                    });
+    method = route(method, ref_nb, query_nb, dim, k);
+    auto plan = [&] {
+        return plan_query_chunk(*ws, query_nb,
+                                use_tc(method) ? grown(tc_ref_bytes(ref_nb, dim)) : 0,
+                                [&](int c) {
+                                    return grown(
+                                        scratch_for(method, ref_nb, c, dim, k, ws->num_sms));
+                                });
+    };
+    int qc = plan();
+    if (qc < query_nb && use_tc(method) && ref_nb < kTcAlwaysPoints) {
+        // a small set takes the tensor path only where the memory is no question
+        method = KNNB200_METHOD_GLOBAL;
+        qc = plan();
+    }
+    const bool tc = use_tc(method);
     if (qc < 1) return KNNB200_ENOMEM;
     g_last_chunks = (query_nb + qc - 1) / qc;
     if (!ws->scratch.ensure(scratch_for(method, ref_nb, qc, dim, k, ws->num_sms)))
@@ -862,8 +890,8 @@ size_t knnb200_call_bytes(int ref_nb, int query_nb, int dim, int k, int method, 
     if (cudaGetDevice(&dev) == cudaSuccess)
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaGetLastError();
-    const bool tc = use_tc(method, ref_nb, query_nb, dim, k);
-    const size_t tcb = tc ? grown(tc_ref_bytes(ref_nb, dim)) : 0;
+    method = route(method, ref_nb, query_nb, dim, k);
+    const size_t tcb = use_tc(method) ? grown(tc_ref_bytes(ref_nb, dim)) : 0;
     if (!host) return tcb + grown(scratch_for(method, ref_nb, query_nb, dim, k, sms));
     return grown((size_t)dim * round_up(ref_nb, 64) * sizeof(float)) + tcb +
            host_chunk_bytes(method, ref_nb, query_nb, dim, k, sms);
@@ -890,7 +918,7 @@ size_t knnb200_scratch_bytes(int ref_nb, int query_nb, int dim, int k, int metho
     if (cudaGetDevice(&dev) == cudaSuccess)
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaGetLastError();
-    return scratch_for(method, ref_nb, query_nb, dim, k, sms);
+    return scratch_for(route(method, ref_nb, query_nb, dim, k), ref_nb, query_nb, dim, k, sms);
 }
 
 int knnb200_plan_splits(int ref_nb, int query_nb, int dim, int k) {

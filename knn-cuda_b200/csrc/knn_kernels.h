@@ -253,7 +253,13 @@ struct TileRuns {
     }
 };
 
+// Shapes the tensor path can run, and those where the entry points that choose
+// between it and the exact kernel for a caller's knn_cublas take it: all that it
+// supports with kTcAlwaysPoints points and more, below that the ones whose exact
+// kernel is expected to take longer.
+constexpr int kTcAlwaysPoints = 32768;
 bool tc_supported(int N, int Q, int d, int k);
+bool tc_pays(int N, int Q, int d, int k);
 bool tc_fp8_supported(int d);
 size_t tc_ref_bytes(int N, int d);
 size_t tc_scratch_bytes(int N, int Q, int d, int k, int num_sms);

@@ -122,7 +122,7 @@ namespace {
 
 bool use_tc_for(const knnb200_refset *rs, int method, int Q, int k) {
     return (method == KNNB200_METHOD_CUBLAS || method == KNNB200_METHOD_FP8) && rs->has_tc &&
-           tc_supported(rs->N, Q, rs->d, k);
+           tc_supported(rs->N, Q, rs->d, k);   // (has_tc: kTcAlwaysPoints or more)
 }
 
 size_t scratch_need(const knnb200_refset *rs, int method, int Q, int k) {
@@ -232,7 +232,7 @@ int knnb200_refset_create(const float *ref, int ref_nb, long long ref_ld, int di
                           st) != cudaSuccess)
         rc = KNNB200_ECUDA;
     // the tensor-core view, when the shape qualifies for any k
-    if (rc == KNNB200_OK && tc_supported(ref_nb, 1, dim, 1)) {
+    if (rc == KNNB200_OK && ref_nb >= kTcAlwaysPoints && tc_supported(ref_nb, 1, dim, 1)) {
         if (!rs->tcmem.ensure(tc_ref_bytes(ref_nb, dim))) {
             rc = KNNB200_ENOMEM;
         } else {

@@ -1737,14 +1737,16 @@ static int choose_splits(int qtiles, int tiles, int min_tiles, double fixed, int
     return best;
 }
 
+// Pass 1 samples one tile in `stride`: the sample must hold about 2.5k points
+// below T_q, KS * stride >= 2.5k.
+int sample_stride(int k) { return std::max(16, (5 * k + 2 * TC_KS - 1) / (2 * TC_KS)); }
+
 TcPlan plan_tc(int N, int Q, int d, int k, int num_sms, bool point_sample = false) {
     TcPlan p;
     p.d_pad = (d + 63) / 64 * 64;
     p.d_pad8 = (d + 127) / 128 * 128;
     p.qtiles = (Q + TC_QT - 1) / TC_QT;
-    // pass 1 samples one tile in `stride`: the sample must hold about 2.5k
-    // points below T_q, KS * stride >= 2.5k
-    const int stride = std::max(16, (5 * k + 2 * TC_KS - 1) / (2 * TC_KS));
+    const int stride = sample_stride(k);
     p.cmax = 4 * TC_KS * stride;
     p.n_tiles2 = (N + TP_BN - 1) / TP_BN;
     // in runs of up to 16 consecutive tiles (one every stride tiles when
@@ -1820,7 +1822,27 @@ float pow2_ceil(double x) { return (float)std::ldexp(1.0, (int)std::ceil(std::lo
 }  // namespace
 
 bool tc_supported(int N, int Q, int d, int k) {
-    return d >= 16 && d <= kTcMaxDim && k >= 1 && k <= kTcMaxK && N >= 32768 && Q >= 1;
+    // (256 sample rows at least: the threshold is the 16th of their minima)
+    return d >= 16 && d <= kTcMaxDim && k >= 1 && k <= kTcMaxK && Q >= 1 &&
+           N >= 16 * 256 * ((sample_stride(k) + TC_SAMPLE_EVERY - 1) / TC_SAMPLE_EVERY);
+}
+
+bool tc_pays(int N, int Q, int d, int k) {
+    if (!tc_supported(N, Q, d, k)) return false;
+    if (N >= kTcAlwaysPoints) return true;
+    // Models in us.  The exact kernel: 13e6 coordinates of pairs a us.  The tensor
+    // path: its launches and read-backs, and for each query the selection and
+    // the gather of about 1.7 k + 20 rows.  Exact / tensor measured at (points,
+    // queries, dimensions, k): 674 / 206 (16384, 4096, 128, 10), 719 / 354 (16384,
+    // 4096, 128, 100), 389 / 343 (8192, 4096, 128, 100), 649 / 280 (4096, 4096, 512,
+    // 10), 2400 / 515 (16384, 16384, 128, 10), 185 / 128 (30000, 1000, 64, 10), 114 /
+    // 126 (30000, 200, 128, 10), 813 / 742 (16384, 16384, 16, 100 and 10).  The line
+    // leaves ties and small gains to the exact kernel, whose time does not
+    // depend on the data.
+    const double exact = 30.0 + (double)N * Q * std::max(d, 32) / 13e6;
+    const double tensor =
+        150.0 + Q * (0.025 + (1.7 * k + 20) * d * 8e-7 + 0.00015 * k);
+    return exact > 1.2 * tensor;
 }
 
 bool tc_fp8_supported(int d) {
