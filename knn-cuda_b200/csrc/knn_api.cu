@@ -165,10 +165,14 @@ class HostPool {
     bool stop_ = false;
 };
 
-// Pinned staging of the streamed host entry for pageable input: two
-// buffers; the host gathers a piece of the reference set into one while the
-// other's copy is in flight.
-constexpr size_t kStageBytes = 32u << 20;
+// Pinned staging of the streamed host entry for pageable input: the host
+// gathers a piece of the reference set into one buffer while the copies out
+// of the others are in flight.  A piece holds several ranges where they are
+// short: with a gather of its own for each 0.25 MB run of the threshold sample
+// the sample of 2^18 x 128 took 3.1 ms and the call 11.3, now 7.5.
+constexpr int kStageSlots = 4;
+constexpr size_t kStageBytes = 16u << 20;
+constexpr size_t kStageMinBytes = 1u << 20;   // smaller input is left to the driver
 
 // count floats from src to a 16-byte aligned dst with non-temporal stores:
 // the staging buffer is read next by the copy engine, not by this core, so
@@ -226,23 +230,29 @@ struct Workspace {
     int *tc_stats = nullptr;           // pinned: [0] second-scan queries, [1] exact fallbacks
     cudaStream_t copy_stream = nullptr;          // host entry: reference copies
     cudaEvent_t copied[1 + kStreamChunks] = {};  // sample, then each chunk
-    float *stage[2] = {nullptr, nullptr};        // pinned staging for pageable input
-    cudaEvent_t stage_done[2] = {};              // the copy out of each stage has ended
+    float *stage[kStageSlots] = {};              // pinned staging for pageable input
+    cudaEvent_t stage_done[kStageSlots] = {};    // the copies out of each stage have ended
     int stage_slot = 0;
     std::unique_ptr<HostPool> pool;              // gathers into the staging buffers
 
-    // Staging buffers and the pool, on first use.
-    bool ensure_staging() {
-        if (stage[0]) return true;
-        for (int i = 0; i < 2; ++i) {
-            if (cudaMallocHost(reinterpret_cast<void **>(&stage[i]), kStageBytes) != cudaSuccess ||
-                cudaEventCreateWithFlags(&stage_done[i], cudaEventDisableTiming) != cudaSuccess) {
-                cudaGetLastError();
-                return false;
-            }
+    // Staging buffer `slot` and the pool, on first use.
+    bool ensure_staging(int slot) {
+        if (!stage_done[slot] &&
+            cudaEventCreateWithFlags(&stage_done[slot], cudaEventDisableTiming) != cudaSuccess) {
+            stage_done[slot] = nullptr;
+            cudaGetLastError();
+            return false;
         }
-        const unsigned hc = std::thread::hardware_concurrency();
-        pool.reset(new HostPool((int)std::max(1u, std::min(16u, hc ? hc : 4u)) - 1));
+        if (!stage[slot] && cudaMallocHost(reinterpret_cast<void **>(&stage[slot]), kStageBytes) !=
+                                cudaSuccess) {
+            stage[slot] = nullptr;
+            cudaGetLastError();
+            return false;
+        }
+        if (!pool) {
+            const unsigned hc = std::thread::hardware_concurrency();
+            pool.reset(new HostPool((int)std::max(1u, std::min(16u, hc ? hc : 4u)) - 1));
+        }
         return true;
     }
 
@@ -348,6 +358,78 @@ int enqueue(Workspace &ws, const ExactProblem &p0, int method, cudaStream_t st,
     return launch_tc(t, v, st, ws.tc_stats);
 }
 
+// A range of columns (points).
+struct Range {
+    size_t c0, len;
+};
+
+// Copy the ranges' columns of every row from pageable host memory through the
+// staging buffers, as many ranges (or as much of one) to a piece as a buffer
+// holds; the host gathers the piece's rows (the pool splits them, long ones in
+// parts) while earlier pieces' copies are in flight.
+int copy_staged(Workspace &ws, const std::vector<Range> &ranges, const float *src, size_t src_ld,
+                float *dst, size_t dst_ld, int rows, cudaStream_t st) {
+    const size_t fb = sizeof(float);
+    // columns of a piece (its ranges start at multiples of 4), rows of a pass
+    const int max_rows = (int)std::min<size_t>(rows, kStageBytes / (64 * fb));
+    for (int r0 = 0; r0 < rows; r0 += max_rows) {
+        const int nr = std::min(max_rows, rows - r0);
+        const size_t cap = kStageBytes / ((size_t)nr * fb) / 4 * 4;
+        std::vector<Range> piece;
+        size_t held = 0;
+        auto flush = [&]() -> int {
+            if (piece.empty()) return kOk;
+            const int slot = ws.stage_slot;
+            if (!ws.ensure_staging(slot)) return kErrNoMemory;
+            ws.stage_slot = (ws.stage_slot + 1) % kStageSlots;
+            if (cudaEventSynchronize(ws.stage_done[slot]) != cudaSuccess) return kErrCuda;
+            float *buf = ws.stage[slot];
+            const size_t pitch = held;
+            // a single long range of few rows: parts of a row
+            const int parts =
+                piece.size() == 1 ? (int)std::max<size_t>(
+                                        1, std::min<size_t>(32 / nr, piece[0].len / 16384))
+                                  : 1;
+            const std::function<void(int)> item = [&](int i) {
+                const int rr = i / parts, part = i % parts;
+                size_t off = 0;
+                for (const Range &g : piece) {
+                    const size_t a = g.len * part / parts / 16 * 16;
+                    const size_t b = part + 1 < parts ? g.len * (part + 1) / parts / 16 * 16
+                                                      : g.len;
+                    stage_row(buf + (size_t)rr * pitch + off + a,
+                              src + (size_t)(r0 + rr) * src_ld + g.c0 + a, b - a);
+                    off += (g.len + 3) / 4 * 4;
+                }
+            };
+            ws.pool->run(nr * parts, item);
+            size_t off = 0;
+            for (const Range &g : piece) {
+                if (cudaMemcpy2DAsync(dst + (size_t)r0 * dst_ld + g.c0, dst_ld * fb, buf + off,
+                                      pitch * fb, g.len * fb, nr, cudaMemcpyHostToDevice,
+                                      st) != cudaSuccess)
+                    return kErrCuda;
+                off += (g.len + 3) / 4 * 4;
+            }
+            piece.clear();
+            held = 0;
+            return cudaEventRecord(ws.stage_done[slot], st) == cudaSuccess ? kOk : kErrCuda;
+        };
+        int rc;
+        for (Range g : ranges)
+            while (g.len > 0) {
+                const size_t n = std::min(cap - held, g.len);
+                piece.push_back(Range{g.c0, n});
+                held += (n + 3) / 4 * 4;
+                g.c0 += n;
+                g.len -= n;
+                if (held >= cap && (rc = flush()) != kOk) return rc;
+            }
+        if ((rc = flush()) != kOk) return rc;
+    }
+    return kOk;
+}
+
 // Calls fn(g0, g1) for each maximal range of tiles [g0, g1) of [tb, te)
 // outside the runs of the sample pattern s.
 template <class F>
@@ -380,7 +462,6 @@ int enqueue_tc_streamed(Workspace &ws, const ExactProblem &p, const float *ref_h
     ws.tc_stats[6] = ws.tc_stats[7] = -1;
     ws.timer.begin(st);
     if (!ws.tcref.ensure(tc_ref_bytes(p.N, p.d))) return kErrNoMemory;
-    if (!pinned && !ws.ensure_staging()) return kErrNoMemory;
     const TcRefView rv = tc_carve_ref(ws.tcref.ptr, p.N, p.d, &ws.tc_state);
     float *ref_d = const_cast<float *>(p.ref);
     const int T = tc_tile_points();
@@ -388,41 +469,22 @@ int enqueue_tc_streamed(Workspace &ws, const ExactProblem &p, const float *ref_h
     const TileRuns sample = tc_sample_runs(p.N, p.Q, p.d, p.k, p.num_sms);
     const size_t fb = sizeof(float);
     cudaStream_t cs = ws.copy_stream;
-    // points [c0, c0 + len) of every dimension from page-locked memory: one
-    // 2-D copy
-    auto copy_direct = [&](size_t c0, size_t len) -> int {
-        return cudaMemcpy2DAsync(ref_d + c0, (size_t)p.ldr * fb, ref_host + c0, (size_t)p.N * fb,
-                                 len * fb, p.d, cudaMemcpyHostToDevice, cs) == cudaSuccess
-                   ? kOk
-                   : kErrCuda;
-    };
-    // the same from pageable memory: through the staging buffers, at most
-    // kStageBytes per piece; the host gathers the piece's rows (the pool
-    // splits them) while the previous piece's copy is in flight
-    auto copy_staged = [&](size_t c0, size_t len) -> int {
-        const size_t cols = std::max<size_t>(1, kStageBytes / ((size_t)p.d * fb));
-        for (size_t q0 = c0; q0 < c0 + len; q0 += cols) {
-            const size_t n = std::min(cols, c0 + len - q0);
-            const int slot = ws.stage_slot;
-            ws.stage_slot ^= 1;
-            if (cudaEventSynchronize(ws.stage_done[slot]) != cudaSuccess) return kErrCuda;
-            float *dst = ws.stage[slot];
-            const std::function<void(int)> rows = [&](int dd) {
-                stage_row(dst + (size_t)dd * n, ref_host + (size_t)dd * p.N + q0, n);
-            };
-            ws.pool->run(p.d, rows);
-            if (cudaMemcpy2DAsync(ref_d + q0, (size_t)p.ldr * fb, dst, n * fb, n * fb, p.d,
-                                  cudaMemcpyHostToDevice, cs) != cudaSuccess ||
-                cudaEventRecord(ws.stage_done[slot], cs) != cudaSuccess)
+    // the ranges' points of every dimension: from page-locked memory one 2-D
+    // copy each, from pageable memory through the staging buffers
+    auto copy_ranges = [&](const std::vector<Range> &ranges) -> int {
+        if (!pinned)
+            return copy_staged(ws, ranges, ref_host, (size_t)p.N, ref_d, (size_t)p.ldr, p.d, cs);
+        for (const Range &g : ranges)
+            if (cudaMemcpy2DAsync(ref_d + g.c0, (size_t)p.ldr * fb, ref_host + g.c0,
+                                  (size_t)p.N * fb, g.len * fb, p.d, cudaMemcpyHostToDevice,
+                                  cs) != cudaSuccess)
                 return kErrCuda;
-        }
         return kOk;
     };
-    // points [t0 T, t1 T) of every dimension
-    auto copy_tiles = [&](int t0, int t1) -> int {
+    // a range of tiles [t0, t1)
+    auto add_tiles = [&](std::vector<Range> &ranges, int t0, int t1) {
         const size_t p0 = (size_t)t0 * T, p1 = std::min<size_t>(p.N, (size_t)t1 * T);
-        if (p0 >= p1) return kOk;
-        return pinned ? copy_direct(p0, p1 - p0) : copy_staged(p0, p1 - p0);
+        if (p0 < p1) ranges.push_back(Range{p0, p1 - p0});
     };
     // the copies start after everything queued so far on the compute stream
     // (an earlier call may still read the reference buffer)
@@ -430,9 +492,10 @@ int enqueue_tc_streamed(Workspace &ws, const ExactProblem &p, const float *ref_h
         cudaStreamWaitEvent(cs, ws.last_done, 0) != cudaSuccess)
         return kErrCuda;
     int rc = kOk;
-    for (int t = 0; t < n_tiles && rc == kOk; t += sample.period)
-        rc = copy_tiles(t, std::min(n_tiles, t + sample.run));
-    if (rc != kOk) return rc;
+    std::vector<Range> ranges;
+    for (int t = 0; t < n_tiles; t += sample.period)
+        add_tiles(ranges, t, std::min(n_tiles, t + sample.run));
+    if ((rc = copy_ranges(ranges)) != kOk) return rc;
     if (cudaEventRecord(ws.copied[0], cs) != cudaSuccess) return kErrCuda;
     int bound[kStreamChunks + 1], wsum = 0;
     for (int c = 0; c < kStreamChunks; ++c) wsum += kStreamWeights[c];
@@ -479,7 +542,12 @@ int enqueue_tc_streamed(Workspace &ws, const ExactProblem &p, const float *ref_h
     // copy's event), so the work of chunk c is on the device while the host
     // gathers chunk c + 1 (pageable input)
     for (int c = 0; c < kStreamChunks; ++c) {
-        if ((rc = for_each_gap(sample, bound[c], bound[c + 1], copy_tiles)) != kOk) return rc;
+        ranges.clear();
+        for_each_gap(sample, bound[c], bound[c + 1], [&](int t0, int t1) {
+            add_tiles(ranges, t0, t1);
+            return (int)kOk;
+        });
+        if ((rc = copy_ranges(ranges)) != kOk) return rc;
         if (cudaEventRecord(ws.copied[1 + c], cs) != cudaSuccess ||
             cudaStreamWaitEvent(st, ws.copied[1 + c], 0) != cudaSuccess)
             return kErrCuda;
@@ -492,15 +560,15 @@ int enqueue_tc_streamed(Workspace &ws, const ExactProblem &p, const float *ref_h
     return tc_run_finish(run, st, ws.tc_stats);
 }
 
-// Page-locked (or registered) host memory: only then do the copies run
-// asynchronously and overlap the scans.
-bool host_pinned(const void *ptr) {
+// Ordinary host memory, neither page-locked, registered nor managed: its copies
+// do not run asynchronously.
+bool host_pageable(const void *ptr) {
     cudaPointerAttributes a;
     if (cudaPointerGetAttributes(&a, ptr) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return true;
     }
-    return a.type == cudaMemoryTypeHost;
+    return a.type == cudaMemoryTypeUnregistered;
 }
 
 int current_workspace(Workspace *&ws) {
@@ -669,11 +737,19 @@ bool host_entry(int wanted, const float *ref, int ref_nb, const float *query, in
     // page-locked input is copied directly, pageable input through the
     // pinned staging buffers
     const bool streamed = tc && qc == query_nb && ref_nb >= kStreamMinPoints;
-    const bool pinned = streamed && host_pinned(ref);
-    cudaError_t e0 = streamed ? cudaSuccess
-                              : cudaMemcpy2DAsync(ref_d, ldr * sizeof(float), ref,
-                                                  ref_nb * sizeof(float), ref_nb * sizeof(float),
-                                                  dim, cudaMemcpyHostToDevice, st);
+    const bool pinned = streamed && !host_pageable(ref);
+    // other input of some size from pageable memory goes through the staging
+    // buffers too: the driver copies it with one thread (8.4 MB in 400 to
+    // 700 us; a call at 16384 x 4096 x 128 takes 0.58 ms instead of 0.83)
+    auto copy_in = [&](const float *src, size_t src_ld, float *dst, size_t dst_ld, size_t cols) {
+        if (cols * dim * sizeof(float) >= kStageMinBytes && host_pageable(src)) {
+            const int r = copy_staged(*ws, {Range{0, cols}}, src, src_ld, dst, dst_ld, dim, st);
+            if (r != kErrNoMemory) return r == kOk ? cudaSuccess : cudaErrorUnknown;
+        }
+        return cudaMemcpy2DAsync(dst, dst_ld * sizeof(float), src, src_ld * sizeof(float),
+                                 cols * sizeof(float), dim, cudaMemcpyHostToDevice, st);
+    };
+    cudaError_t e0 = streamed ? cudaSuccess : copy_in(ref, ref_nb, ref_d, ldr, ref_nb);
     cudaError_t e2 = cudaMemsetAsync(ws->status.ptr, 0, sizeof(int), st);
     if (e0 != cudaSuccess || e2 != cudaSuccess) {
         std::printf("ERROR: Unable to copy data from host to device\n");
@@ -683,9 +759,7 @@ bool host_entry(int wanted, const float *ref, int ref_nb, const float *query, in
     long long stats[3] = {0, 0, 0};   // second scan, exact, candidates over the chunks
     for (int q0 = 0; q0 < query_nb; q0 += qc) {
         const int n = std::min(qc, query_nb - q0);
-        if (cudaMemcpy2DAsync(qry_d, ldq * sizeof(float), query + q0, query_nb * sizeof(float),
-                              n * sizeof(float), dim, cudaMemcpyHostToDevice,
-                              st) != cudaSuccess) {
+        if (copy_in(query + q0, query_nb, qry_d, ldq, n) != cudaSuccess) {
             std::printf("ERROR: Unable to copy data from host to device\n");
             cudaGetLastError();
             return false;

@@ -1,0 +1,31 @@
+"""Host entries on pageable arrays large enough for the staging buffers: many and
+few rows, ragged lengths, more than one buffer's worth, a set whose threshold
+sample is many short runs.  The answers are the device entry's bit for bit."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # (ref_nb, query_nb, dim, k, method)
+    (400003, 300, 3, 4, "global"), (65537, 40, 70, 5, "global"), (9, 5, 70001, 3, "global"),
+    (300001, 262147, 1, 2, "global"), (16385, 4099, 129, 16, "cublas"),
+    (262147, 4100, 40, 10, "cublas"), (300005, 70, 100, 33, "cublas"),
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=["-".join(map(str, c)) for c in CASES])
+def test_pageable_input(knncuda, gpu, case):
+    import torch
+
+    n, q, dim, k, method = case
+    rng = np.random.default_rng(n)
+    ref, query = rng.random((dim, n), dtype=np.float32), rng.random((dim, q), dtype=np.float32)
+    r = torch.zeros((dim, (n + 3) // 4 * 4), device=gpu)[:, :n]
+    x = torch.zeros((dim, (q + 3) // 4 * 4), device=gpu)[:, :q]
+    r.copy_(torch.from_numpy(ref))
+    x.copy_(torch.from_numpy(query))
+    wd, wi = knncuda.knn_device(r, x, k, "global")
+    for _ in range(2):   # the buffers are reused
+        d, i = knncuda.knn(ref, query, k, method)
+        assert np.array_equal(d, wd.cpu().numpy()) and np.array_equal(i, wi.cpu().numpy())
