@@ -731,6 +731,18 @@ bool host_entry(int wanted, const float *ref, int ref_nb, const float *query, in
         return false;
     }
     cudaStream_t st = ws->stream;
+    // The scratch and the status word are shared with the device entry, whose
+    // last call may still be running on its caller's stream: this call waits
+    // for it, and the next one for this call, however it ends.
+    struct Done {
+        Workspace *w;
+        ~Done() { cudaEventRecord(w->last_done, w->stream); }
+    } done{ws};
+    if (cudaStreamWaitEvent(st, ws->last_done, 0) != cudaSuccess) {
+        std::printf("ERROR: Cannot order the call after earlier work\n");
+        cudaGetLastError();
+        return false;
+    }
     float *ref_d = static_cast<float *>(ws->ref.ptr);
     float *qry_d = static_cast<float *>(ws->qry.ptr);
     // the streamed reference copy serves a call that runs as one chunk;

@@ -29,3 +29,28 @@ def test_pageable_input(knncuda, gpu, case):
     for _ in range(2):   # the buffers are reused
         d, i = knncuda.knn(ref, query, k, method)
         assert np.array_equal(d, wd.cpu().numpy()) and np.array_equal(i, wi.cpu().numpy())
+
+
+def test_host_call_waits_for_a_device_call_in_flight(knncuda, gpu):
+    """The host and device entries share the workspace's scratch: a host call made
+    while a device call still runs on another stream must not touch it."""
+    import torch
+
+    rng = np.random.default_rng(9)
+    n, q, dim, k = 16385, 4099, 129, 16
+    ref, query = rng.random((dim, n), dtype=np.float32), rng.random((dim, q), dtype=np.float32)
+    r = torch.zeros((dim, (n + 3) // 4 * 4), device=gpu)[:, :n]
+    x = torch.zeros((dim, (q + 3) // 4 * 4), device=gpu)[:, :q]
+    r.copy_(torch.from_numpy(ref))
+    x.copy_(torch.from_numpy(query))
+    want = [t.cpu() for t in knncuda.knn_device(r, x, k, "global")]
+    knncuda.knn(ref, query, k, "cublas")   # the buffers have their sizes now
+    side = torch.cuda.Stream()
+    for method in ("cublas", "global") * 5:
+        with torch.cuda.stream(side):
+            outs = [knncuda.knn_device(r, x, k, "global") for _ in range(4)]
+        d, i = knncuda.knn(ref, query, k, method)
+        torch.cuda.synchronize()
+        assert np.array_equal(d, want[0].numpy()) and np.array_equal(i, want[1].numpy())
+        for dd, ii in outs:
+            assert torch.equal(dd.cpu(), want[0]) and torch.equal(ii.cpu(), want[1])
