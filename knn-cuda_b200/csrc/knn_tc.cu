@@ -1355,12 +1355,143 @@ KNN_DI void rr_certify(const unsigned long long *keys, int q, float qq, float r2
     }
 }
 
-// Select: reject lists that cannot be re-ranked, find the k-th smallest
-// entry key (the order-preserving bits of a) by an 8-bit radix selection
-// over the list, and compact the entries with a <= the pruning limit to the
-// front of the list (in place: an entry moves only to a position already
+// (buf_select does the same inside the exact kernel, whose call it shares; with
+// this function inside it that kernel came out 0.9 % slower.)
+// Bisection over the high words of the keys key[] (kKeyInf: none; c of them, c >
+// k + slack) of one warp: a cut below which there are at least k and at most k +
+// slack.  Many keys with one high word are told apart by their low words (keys
+// are unique), so that it always ends.
+template <int SL>
+KNN_DI unsigned long long key_cut(const unsigned long long (&key)[SL], int c, int k, int slack) {
+    uint32_t lo = 0xffffffffu, up = 0;
+#pragma unroll
+    for (int a = 0; a < SL; ++a) {
+        const uint32_t h = (uint32_t)(key[a] >> 32);
+        lo = min(lo, h);
+        up = max(up, key[a] != kKeyInf ? h : 0u);
+    }
+    // invariant: fewer than k keys have a high word below lo, n >= k below up
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    up = __reduce_max_sync(0xffffffffu, up) + 1u;
+    int n = c;
+    while (n > k + slack && up - lo > 1u) {
+        const uint32_t mid = lo + (up - lo) / 2u;
+        int m = 0;
+#pragma unroll
+        for (int a = 0; a < SL; ++a) m += (uint32_t)(key[a] >> 32) < mid ? 1 : 0;
+        m = (int)__reduce_add_sync(0xffffffffu, (unsigned)m);
+        if (m >= k) {
+            up = mid;
+            n = m;
+        } else {
+            lo = mid;
+        }
+    }
+    unsigned long long a0 = (unsigned long long)lo << 32, a1 = (unsigned long long)up << 32;
+    while (n > k + slack) {
+        const unsigned long long mid = a0 + (a1 - a0) / 2;
+        int m = 0;
+#pragma unroll
+        for (int a = 0; a < SL; ++a) m += key[a] < mid ? 1 : 0;
+        m = (int)__reduce_add_sync(0xffffffffu, (unsigned)m);
+        if (m >= k) {
+            a1 = mid;
+            n = m;
+        } else {
+            a0 = mid;
+        }
+    }
+    return a1;
+}
+
+// The keys below cut, in their order, to dst; returns their number.
+template <int SL>
+KNN_DI int keep_below(const unsigned long long (&key)[SL], unsigned long long cut,
+                      unsigned long long *dst, int lane) {
+    const unsigned lt = (1u << lane) - 1u;
+    int pos = 0;
+#pragma unroll
+    for (int a = 0; a < SL; ++a) {
+        const bool in = key[a] < cut;
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (in) dst[pos + __popc(m & lt)] = key[a];
+        pos += __popc(m);
+    }
+    return pos;
+}
+
+// Select: reject lists that cannot be re-ranked, find the k-th smallest entry
+// key (a bisection over the order-preserving bits of a, key_cut) and compact the entries with a <= the pruning limit
+// to the front of the list (in place: an entry moves only to a position already
 // read).  nsel[q] = their number, or -1 for a rejected list.
-__global__ void __launch_bounds__(32)
+//
+// The list sits in registers, SL keys a lane.  Against an 8-bit radix selection
+// in shared memory that read the list six times: 66 -> 42 us at 16384 queries of
+// about 370 candidates (two launches), 11.5 -> 6 at 13 queries.
+template <int SL>
+KNN_DI int rr_select(unsigned long long *cq, int c, int k, float qq, float r2, const RrBounds &rb,
+                     int d_pad, int lane) {
+    unsigned long long key[SL];
+#pragma unroll
+    for (int a = 0; a < SL; ++a) key[a] = a * 32 + lane < c ? cq[a * 32 + lane] : kKeyInf;
+    uint32_t top = 0;   // the k-th smallest
+    if (c > k) {
+        const unsigned long long cut = key_cut<SL>(key, c, k, 0);
+#pragma unroll
+        for (int a = 0; a < SL; ++a)
+            top = max(top, key[a] < cut ? (uint32_t)(key[a] >> 32) : 0u);
+    } else {
+#pragma unroll
+        for (int a = 0; a < SL; ++a)
+            top = max(top, key[a] != kKeyInf ? (uint32_t)(key[a] >> 32) : 0u);
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    const float ak = ord_float(top) * rb.a_scale;
+    const float E = tc_error_bound(qq, r2, ak, rb.cur);
+    const float g = tc_fp32_gamma(d_pad);
+    const float lim = (ak + 2.f * E + 2.f * g * (fabsf(ak) + qq + E)) / rb.a_scale;
+    const uint32_t lim_o = ord_bits(__float_as_uint(lim));
+    // (a limit that is no number keeps the whole list)
+    const unsigned long long cut =
+        lim == lim && lim_o >= top ? ((unsigned long long)lim_o << 32) | 0xffffffffull : kKeyInf;
+    __syncwarp();
+    return keep_below<SL>(key, cut, cq, lane);
+}
+
+constexpr int TC_RK_REG = 1024;   // longest list held in registers (32 keys a lane)
+
+// The same for longer lists, which stay in memory.
+KNN_DI int rr_select_long(unsigned long long *cq, int c, int k, float qq, float r2,
+                          const RrBounds &rb, int d_pad, int lane) {
+    uint32_t lo = 0, up = 0xffffffffu;   // fewer than k below lo, at least k below up
+    while (up - lo > 1u) {
+        const uint32_t mid = lo + (up - lo) / 2u;
+        int m = 0;
+        for (int t = lane; t < c; t += 32) m += (uint32_t)(cq[t] >> 32) < mid ? 1 : 0;
+        m = (int)__reduce_add_sync(0xffffffffu, (unsigned)m);
+        if (m >= k) up = mid;
+        else lo = mid;
+    }
+    const float ak = ord_float(lo) * rb.a_scale;
+    const float E = tc_error_bound(qq, r2, ak, rb.cur);
+    const float g = tc_fp32_gamma(d_pad);
+    const float lim = (ak + 2.f * E + 2.f * g * (fabsf(ak) + qq + E)) / rb.a_scale;
+    const uint32_t lim_o = ord_bits(__float_as_uint(lim));
+    if (!(lim == lim) || lim_o < lo) return c;
+    int pos = 0;
+    for (int t0 = 0; t0 < c; t0 += 32) {
+        const int t = t0 + lane;
+        const unsigned long long e = t < c ? cq[t] : kKeyInf;
+        const bool in = t < c && (uint32_t)(e >> 32) <= lim_o;
+        const unsigned b = __ballot_sync(0xffffffffu, in);
+        if (in) cq[pos + __popc(b & ((1u << lane) - 1u))] = e;
+        pos += __popc(b);
+    }
+    return pos;
+}
+
+constexpr int TC_RK_WARPS = 4;   // queries per block of the select and certify kernels
+__global__ void __launch_bounds__(32 * TC_RK_WARPS)
     tc_rerank_select_kernel(unsigned long long *__restrict__ cand, const int *__restrict__ count,
                             int cmax, int Q, int k, const float *__restrict__ qn,
                             const unsigned *__restrict__ rmax_bits,
@@ -1369,11 +1500,16 @@ __global__ void __launch_bounds__(32)
                             int *__restrict__ n_fail, float *__restrict__ retry,
                             float *__restrict__ retry_f, float *__restrict__ retry_s,
                             unsigned long long *__restrict__ cand_total, int *__restrict__ nsel) {
-    __shared__ unsigned hist[256];
-    const int q = blockIdx.x, lane = threadIdx.x;
+    __shared__ unsigned long long total;
+    const int lane = threadIdx.x & 31;
+    const int q = blockIdx.x * TC_RK_WARPS + (threadIdx.x >> 5);
+    if (threadIdx.x == 0) total = 0;
+    __syncthreads();
+    int c = q < Q ? count[q] : 0;
+    if (lane == 0) atomicAdd(&total, (unsigned long long)c);
+    __syncthreads();
+    if (threadIdx.x == 0) atomicAdd(cand_total, total);
     if (q >= Q) return;
-    int c = count[q];
-    if (lane == 0) atomicAdd(cand_total, (unsigned long long)c);
     const float qq = qn[q];
     const float r2 = __uint_as_float(*rmax_bits);
     const float T = thr[q];
@@ -1385,76 +1521,11 @@ __global__ void __launch_bounds__(32)
     }
     if (rj == 2) c = cmax;   // the entries that were kept
     unsigned long long *cq = cand + (size_t)q * cmax;
-    // k-th smallest key, 8 bits per round from the top
-    uint32_t prefix = 0, hmask = 0;
-    unsigned rank = (unsigned)k;   // 1-based rank among the keys matching prefix
-    for (int shift = 24; shift >= 0; shift -= 8) {
-        for (int i = lane; i < 256; i += 32) hist[i] = 0u;
-        __syncwarp();
-        for (int t = lane; t < c; t += 32) {
-            const uint32_t key = (uint32_t)(cq[t] >> 32);
-            if ((key & hmask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
-        }
-        __syncwarp();
-        unsigned h[8], sum = 0;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            h[j] = hist[8 * lane + j];
-            sum += h[j];
-        }
-        unsigned incl = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        const unsigned excl = incl - sum;
-        const unsigned owner = __ballot_sync(0xffffffffu, excl < rank && rank <= incl);
-        const int src = __ffs(owner) - 1;
-        int bin = 0;
-        unsigned below = 0;
-        if (lane == src) {
-            unsigned run = excl;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                if (bin == 0 && run + h[j] >= rank) {
-                    bin = 8 * lane + j + 1;   // +1: found
-                    below = run;
-                }
-                run += h[j];
-            }
-        }
-        bin = __shfl_sync(0xffffffffu, bin, src) - 1;
-        below = __shfl_sync(0xffffffffu, below, src);
-        prefix |= (uint32_t)bin << shift;
-        hmask |= 255u << shift;
-        rank -= below;
-        __syncwarp();
-    }
-    const float ak = ord_float(prefix) * rb.a_scale;
-    const float E = tc_error_bound(qq, r2, ak, rb.cur);
-    const float g = tc_fp32_gamma(d_pad);
-    const float lim = (ak + 2.f * E + 2.f * g * (fabsf(ak) + qq + E)) / rb.a_scale;
-    const uint32_t lim_o = ord_bits(__float_as_uint(lim));
-    int kept = 0;
-    for (int t0 = 0; t0 < c; t0 += 32) {
-        const int t = t0 + lane;
-        kept += __popc(__ballot_sync(0xffffffffu, t < c && (uint32_t)(cq[t] >> 32) <= lim_o));
-    }
-    if (kept >= k) {
-        int pos0 = 0;
-        for (int t0 = 0; t0 < c; t0 += 32) {
-            const int t = t0 + lane;
-            const unsigned long long e = t < c ? cq[t] : kKeyInf;
-            const bool in = t < c && (uint32_t)(e >> 32) <= lim_o;
-            const unsigned b = __ballot_sync(0xffffffffu, in);
-            if (in) cq[pos0 + __popc(b & ((1u << lane) - 1u))] = e;
-            pos0 += __popc(b);
-        }
-    } else {
-        kept = c;   // not reached for finite values (lim >= a_k); keep the whole list
-    }
-    if (lane == 0) nsel[q] = kept;
+    const int n = c <= 256   ? rr_select<8>(cq, c, k, qq, r2, rb, d_pad, lane)
+                  : c <= 512 ? rr_select<16>(cq, c, k, qq, r2, rb, d_pad, lane)
+                  : c <= TC_RK_REG ? rr_select<32>(cq, c, k, qq, r2, rb, d_pad, lane)
+                                   : rr_select_long(cq, c, k, qq, r2, rb, d_pad, lane);
+    if (lane == 0) nsel[q] = n;
 }
 
 // Gather: exact FP32 distances of the nsel[q] selected candidates, keys
@@ -1483,9 +1554,32 @@ __global__ void __launch_bounds__(32)
                              BoundStat{qq, E, rb.a_scale, bound_stat});
 }
 
-// Certify: sort the exact keys of the selected candidates (their k-th is
-// the k-th of all candidates) and certify (rr_certify).
-__global__ void __launch_bounds__(32)
+// Certify: the k smallest of the exact keys of the selected candidates (their
+// k-th is the k-th of all candidates), sorted, and the check (rr_certify).  Up
+// to 1024 keys are held in registers and cut down to KCAP before the sort (140 ->
+// 31 us at 16384 queries, k = 32, and 182 -> 52 at k = 100, against a sort of
+// them all in shared memory); longer lists are sorted in shared memory.
+template <int SL, int KCAP>
+KNN_DI void rr_sorted(const unsigned long long *cq, int n, int k, unsigned long long *L,
+                      int lane) {
+    unsigned long long key[SL];
+#pragma unroll
+    for (int a = 0; a < SL; ++a) key[a] = a * 32 + lane < n ? cq[a * 32 + lane] : kKeyInf;
+    const unsigned long long cut = n > KCAP ? key_cut<SL>(key, n, k, KCAP - k) : kKeyInf;
+    const int m = keep_below<SL>(key, cut, L, lane);
+    __syncwarp();
+    unsigned long long v[KCAP / 32];
+#pragma unroll
+    for (int a = 0; a < KCAP / 32; ++a) v[a] = a * 32 + lane < m ? L[a * 32 + lane] : kKeyInf;
+    warp_sort<KCAP / 32>(v, lane);
+    __syncwarp();
+#pragma unroll
+    for (int a = 0; a < KCAP / 32; ++a) L[a * 32 + lane] = v[a];
+    __syncwarp();
+}
+
+template <int KCAP>
+__global__ void __launch_bounds__(32 * TC_RK_WARPS)
     tc_rerank_certify_kernel(const unsigned long long *__restrict__ cand,
                              const int *__restrict__ nsel, const int *__restrict__ count,
                              int cmax, int Q, int k, int d_pad,
@@ -1495,17 +1589,29 @@ __global__ void __launch_bounds__(32)
                              long long ld_out, int *__restrict__ fail_list,
                              int *__restrict__ n_fail, float *__restrict__ retry,
                              float *__restrict__ retry_f, float *__restrict__ retry_s) {
-    extern __shared__ unsigned long long keys[];
-    const int q = blockIdx.x, lane = threadIdx.x;
+    // KCAP keys per warp; one warp per block with room for cmax keys when lists
+    // may be longer than TC_RK_REG
+    extern __shared__ unsigned long long keys_all[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int q = blockIdx.x * (blockDim.x >> 5) + warp;
     if (q >= Q) return;
     const int n = nsel[q];
     if (n < 0) return;
     const unsigned long long *cq = cand + (size_t)q * cmax;
-    int P = 32;
-    while (P < n) P <<= 1;
-    for (int t = lane; t < P; t += 32) keys[t] = t < n ? cq[t] : kKeyInf;
-    __syncwarp();
-    warp_bitonic_sort(keys, P, lane);
+    unsigned long long *keys = keys_all + (size_t)warp * KCAP;
+    if (n <= 256) {
+        rr_sorted<8, KCAP>(cq, n, k, keys, lane);
+    } else if (n <= 512) {
+        rr_sorted<16, KCAP>(cq, n, k, keys, lane);
+    } else if (n <= TC_RK_REG) {
+        rr_sorted<32, KCAP>(cq, n, k, keys, lane);
+    } else {
+        int P = 32;
+        while (P < n) P <<= 1;
+        for (int t = lane; t < P; t += 32) keys[t] = t < n ? cq[t] : kKeyInf;
+        __syncwarp();
+        warp_bitonic_sort(keys, P, lane);
+    }
     rr_certify(keys, q, qn[q], __uint_as_float(*rmax_bits), thr[q], d_pad, k, rb, out_dist,
                out_idx, ld_out, fail_list, n_fail, retry, retry_f, retry_s, count[q] > cmax,
                lane);
@@ -2125,10 +2231,18 @@ int rerank(const TcRun &r, cudaStream_t st, int kind, int Q, int cmax, const flo
     // (clear at the start of a run)
     if (final_pass && cudaMemsetAsync(r.nfail, 0, 2 * sizeof(int), st) != cudaSuccess)
         return kErrCuda;
-    int cpow = 32;
-    while (cpow < cmax) cpow <<= 1;
+    const int kcap = P.k <= 32 ? 32 : P.k <= 64 ? 64 : P.k <= 128 ? 128 : 256;
+    int cpow = kcap, cwarps = TC_RK_WARPS;   // certify: keys in shared memory, warps
+    if (cmax > TC_RK_REG) {
+        cwarps = 1;
+        while (cpow < cmax) cpow <<= 1;
+    }
     const size_t gsmem = tc_rr_gather_bytes(r.d_pad);
-    const size_t csmem = (size_t)cpow * 8;
+    const size_t csmem = (size_t)cpow * 8 * cwarps;
+    auto certify = kcap == 32    ? tc_rerank_certify_kernel<32>
+                   : kcap == 64  ? tc_rerank_certify_kernel<64>
+                   : kcap == 128 ? tc_rerank_certify_kernel<128>
+                                 : tc_rerank_certify_kernel<256>;
     RrBounds rb;
     rb.cur = run_bound(r, kind);
     rb.a_scale = kind == kTcFp8 ? 1.f / r.scale : 1.f;
@@ -2139,19 +2253,17 @@ int rerank(const TcRun &r, cudaStream_t st, int kind, int Q, int cmax, const flo
     if (gsmem > kRerankSmem || csmem > kRerankSmem ||
         cudaFuncSetAttribute(gather, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kRerankSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(tc_rerank_certify_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(certify, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kRerankSmem) != cudaSuccess)
         return kErrLaunch;
-    tc_rerank_select_kernel<<<Q, 32, 0, st>>>(r.cand, r.count, cmax, Q, P.k, qn, r.R.rmax_bits,
-                                              thr, thr_raw, rb, r.d_pad, final_pass ? 1 : 0, fail,
-                                              r.nfail, r.retry, r.retry_f, r.retry_s, r.cand_total,
-                                              r.nsel);
+    tc_rerank_select_kernel<<<(Q + TC_RK_WARPS - 1) / TC_RK_WARPS, 32 * TC_RK_WARPS, 0, st>>>(
+        r.cand, r.count, cmax, Q, P.k, qn, r.R.rmax_bits, thr, thr_raw, rb, r.d_pad,
+        final_pass ? 1 : 0, fail, r.nfail, r.retry, r.retry_f, r.retry_s, r.cand_total, r.nsel);
     gather<<<Q, 32, gsmem, st>>>(r.R.refT, P.d, r.d_pad, qry, ldq, qn, r.R.rmax_bits, thr, rb,
                                  r.cand, r.nsel, cmax, Q, P.bound_stat);
-    tc_rerank_certify_kernel<<<Q, 32, csmem, st>>>(r.cand, r.nsel, r.count, cmax, Q, P.k,
-                                                   r.d_pad, qn, r.R.rmax_bits, thr, rb, out_dist,
-                                                   out_idx, ld_out, fail, r.nfail, r.retry,
-                                                   r.retry_f, r.retry_s);
+    certify<<<(Q + cwarps - 1) / cwarps, 32 * cwarps, csmem, st>>>(
+        r.cand, r.nsel, r.count, cmax, Q, P.k, r.d_pad, qn, r.R.rmax_bits, thr, rb, out_dist,
+        out_idx, ld_out, fail, r.nfail, r.retry, r.retry_f, r.retry_s);
     return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 
