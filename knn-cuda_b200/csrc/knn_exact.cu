@@ -228,6 +228,13 @@ void shape_of(ExactShape &s) {
     s.smem = C::SMEM;
 }
 
+template <int QPW>
+void shape_for_k(int k, ExactShape &s) {
+    if (k <= 32) shape_of<QPW, 32>(s);
+    else if (k <= 64) shape_of<QPW, 64>(s);
+    else shape_of<QPW, 128>(s);
+}
+
 // Ranks selected by one pass of the kernel: k <= 256 in one pass, larger k
 // in passes of 256 (the last one may be shorter).
 constexpr int kPassRanks = 256;
@@ -235,10 +242,14 @@ constexpr int kPassRanks = 256;
 bool choose_shape(int N, int Q, int d, int k_all, int num_sms, ExactShape &s) {
     if (k_all < 1) return false;
     const int k = std::min(k_all, kPassRanks);
-    if (k <= 32) shape_of<EX_QPW, 32>(s);
-    else if (k <= 64) shape_of<EX_QPW, 64>(s);
-    else if (k <= 128) shape_of<EX_QPW, 128>(s);
-    else shape_of<EX_QPW_K256, 256>(s);
+    // up to 32 queries: tiles of 32 or 16, two or one to a warp, which cut the
+    // arithmetic on padding and the selections a warp makes one after the other:
+    // with tiles of 64, 14.8 us at 1000 x 16 (d = 32, k = 10), now 7.3; 531 at 10^6
+    // x 1 (d = 128, k = 10), now 278; 266 at 200000 x 20 (d = 256, k = 100), now 164
+    if (k > 128) shape_of<EX_QPW_K256, 256>(s);
+    else if (Q <= 16) shape_for_k<1>(k, s);
+    else if (Q <= 32) shape_for_k<2>(k, s);
+    else shape_for_k<EX_QPW>(k, s);
     s.n_rtiles = (N + EX_BR - 1) / EX_BR;
     s.n_dchunks = (d + EX_BD - 1) / EX_BD;
     const int qtiles = (Q + s.bq - 1) / s.bq;
@@ -278,6 +289,16 @@ cudaError_t launch_t(const CUtensorMap &mr, const CUtensorMap &mq, const ExactAr
     dim3 grid(qtiles, a.n_splits);
     kern<<<grid, EX_THREADS, C::SMEM, st>>>(mr, mq, a);
     return cudaGetLastError();
+}
+
+template <int QPW>
+cudaError_t launch_k(int kcap, const CUtensorMap &mr, const CUtensorMap &mq, const ExactArgs &a,
+                     int qtiles, cudaStream_t st) {
+    switch (kcap) {
+        case 32: return launch_t<QPW, 32>(mr, mq, a, qtiles, st);
+        case 64: return launch_t<QPW, 64>(mr, mq, a, qtiles, st);
+        default: return launch_t<QPW, 128>(mr, mq, a, qtiles, st);
+    }
 }
 
 }  // namespace
@@ -394,12 +415,10 @@ int launch_exact(const ExactProblem &p, cudaStream_t st) {
             e = row0 == 0 ? launch_t<EX_QPW_K256, 256, false>(mr, mq, a, qtiles, st)
                           : launch_t<EX_QPW_K256, 256, true>(mr, mq, a, qtiles, st);
         } else {
-            switch (s.kcap) {
-                case 32: e = launch_t<EX_QPW, 32>(mr, mq, a, qtiles, st); break;
-                case 64: e = launch_t<EX_QPW, 64>(mr, mq, a, qtiles, st); break;
-                case 128: e = launch_t<EX_QPW, 128>(mr, mq, a, qtiles, st); break;
-                default: e = launch_t<EX_QPW_K256, 256>(mr, mq, a, qtiles, st); break;
-            }
+            if (s.kcap == 256) e = launch_t<EX_QPW_K256, 256>(mr, mq, a, qtiles, st);
+            else if (s.qpw == 1) e = launch_k<1>(s.kcap, mr, mq, a, qtiles, st);
+            else if (s.qpw == 2) e = launch_k<2>(s.kcap, mr, mq, a, qtiles, st);
+            else e = launch_k<EX_QPW>(s.kcap, mr, mq, a, qtiles, st);
         }
         if (e != cudaSuccess) return kErrLaunch;
         if (p.timer) p.timer->mark(st, kPhaseExactMain);

@@ -45,7 +45,7 @@ template <int QPW, int KCAP>
 struct ExCfg {
     static constexpr int BQ = QPW * EX_WARPS;
     // ring depth: what the lists leave of the shared memory
-    static constexpr int STAGES = QPW == 2 || KCAP == 32 ? 6 : KCAP == 64 ? 5 : 4;
+    static constexpr int STAGES = QPW < 4 || KCAP == 32 ? 6 : KCAP == 64 ? 5 : 4;
     static constexpr int Q_FLOATS = EX_BD * BQ;   // query slab of a stage
     static constexpr int R_FLOATS = EX_BD * EX_BR;
     static constexpr int STAGE_FLOATS = Q_FLOATS + R_FLOATS;
@@ -350,13 +350,15 @@ KNN_DI void select_half_lb(unsigned long long *wl, unsigned long long *wt,
 // The warp's QPW queries of one dimension (one broadcast load).
 template <int QPW>
 KNN_DI void load_queries(float (&q)[QPW], const float *src) {
-    static_assert(QPW == 4 || QPW == 2, "one vector load");
-    if (QPW == 4) {
+    static_assert(QPW == 4 || QPW == 2 || QPW == 1, "one load");
+    if constexpr (QPW == 4) {
         const float4 v = *reinterpret_cast<const float4 *>(src);
-        q[0] = v.x; q[1] = v.y; q[QPW - 2] = v.z; q[QPW - 1] = v.w;
-    } else {
+        q[0] = v.x; q[1] = v.y; q[2] = v.z; q[3] = v.w;
+    } else if constexpr (QPW == 2) {
         const float2 v = *reinterpret_cast<const float2 *>(src);
         q[0] = v.x; q[1] = v.y;
+    } else {
+        q[0] = *src;
     }
 }
 

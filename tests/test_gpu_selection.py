@@ -23,6 +23,9 @@ CASES = [
     (6000, 40, 8, 16, 2), (6000, 40, 8, 100, 2),
     (60000, 5, 8, 10, 30), (60000, 5, 8, 50, 30), (60000, 3, 8, 100, 30), (60000, 3, 8, 200, 30),
     (60000, 1500, 8, 40, 30),
+    # up to 16 and up to 32 queries: smaller query tiles
+    (3000, 16, 9, 50, 9), (3000, 17, 9, 30, 9), (5000, 32, 40, 120, 9), (60000, 30, 8, 64, 30),
+    (700, 1, 5, 128, 4),
 ]
 
 
