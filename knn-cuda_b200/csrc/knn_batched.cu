@@ -211,8 +211,8 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
         bool alive = true;
         for (int rt = t0; rt < t1; ++rt) {
             f32x2_t acc[QPW][4];
-            if (!consume_ref_tile<QPW, KCAP>(acc, stages, full, empty, abort_flag, it,
-                                             P.n_dchunks, warp, lane, status)) {
+            if (!consume_ref_tile<QPW, KCAP, false>(acc, stages, full, empty, abort_flag, it,
+                                             P.n_dchunks, 0, warp, lane, status)) {
                 alive = false;
                 break;
             }

@@ -43,7 +43,7 @@
 
 namespace knnb200 {
 
-template <int QPW, int KCAP, bool LB>
+template <int QPW, int KCAP, bool LB, bool PARTIAL>
 __global__ void __launch_bounds__(EX_THREADS, 1)
     knn_exact_kernel(const __grid_constant__ CUtensorMap tm_ref,
                      const __grid_constant__ CUtensorMap tm_qry, ExactArgs a) {
@@ -121,10 +121,11 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
     }
 
     int it = 0;
+    const int tail = last_stage_groups(a.d);
     for (int rt = t0; rt < t1; ++rt) {
         f32x2_t acc[QPW][4];
-        if (!consume_ref_tile<QPW, KCAP>(acc, stages, full, empty, abort_flag, it, a.n_dchunks,
-                                         warp, lane, a.status))
+        if (!consume_ref_tile<QPW, KCAP, PARTIAL>(acc, stages, full, empty, abort_flag, it, a.n_dchunks,
+                                         tail, warp, lane, a.status))
             break;
         select_tile<QPW, KCAP, LB>(wl, wt, nb, acc, rt, a.N, a.k, lane, lbk);
     }
@@ -277,11 +278,11 @@ bool choose_shape(int N, int Q, int d, int k_all, int num_sms, ExactShape &s) {
     return true;
 }
 
-template <int QPW, int KCAP, bool LB = false>
-cudaError_t launch_t(const CUtensorMap &mr, const CUtensorMap &mq, const ExactArgs &a,
+template <int QPW, int KCAP, bool LB, bool PARTIAL>
+cudaError_t launch_v(const CUtensorMap &mr, const CUtensorMap &mq, const ExactArgs &a,
                      int qtiles, cudaStream_t st) {
     using C = ExCfg<QPW, KCAP>;
-    constexpr auto kern = knn_exact_kernel<QPW, KCAP, LB>;
+    constexpr auto kern = knn_exact_kernel<QPW, KCAP, LB, PARTIAL>;
     if (!launch_regs_ok<kern>()) return cudaErrorLaunchOutOfResources;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)C::SMEM);
@@ -289,6 +290,14 @@ cudaError_t launch_t(const CUtensorMap &mr, const CUtensorMap &mq, const ExactAr
     dim3 grid(qtiles, a.n_splits);
     kern<<<grid, EX_THREADS, C::SMEM, st>>>(mr, mq, a);
     return cudaGetLastError();
+}
+
+template <int QPW, int KCAP, bool LB = false>
+cudaError_t launch_t(const CUtensorMap &mr, const CUtensorMap &mq, const ExactArgs &a,
+                     int qtiles, cudaStream_t st) {
+    return last_stage_groups(a.d) < EX_BD / 4
+               ? launch_v<QPW, KCAP, LB, true>(mr, mq, a, qtiles, st)
+               : launch_v<QPW, KCAP, LB, false>(mr, mq, a, qtiles, st);
 }
 
 template <int QPW>

@@ -362,6 +362,29 @@ KNN_DI void load_queries(float (&q)[QPW], const float *src) {
     }
 }
 
+// One dimension of the lane's QPW x 8 block.
+template <int QPW>
+KNN_DI void consume_dim(f32x2_t (&acc)[QPW][4], const float *rs, const float *qs) {
+    // 16-byte loads straight into packed pairs (x, y), (z, w)
+    const ulonglong2 ra = *reinterpret_cast<const ulonglong2 *>(rs);
+    const ulonglong2 rb = *reinterpret_cast<const ulonglong2 *>(rs + 128);
+    const f32x2_t r0 = ra.x, r1 = ra.y, r2 = rb.x, r3 = rb.y;
+    float q[QPW];
+    load_queries<QPW>(q, qs);
+#pragma unroll
+    for (int i = 0; i < QPW; ++i) {
+        const f32x2_t qq = f2_pack(q[i], q[i]);
+        f32x2_t t;
+        t = f2_sub(r0, qq); acc[i][0] = f2_fma(t, t, acc[i][0]);
+        t = f2_sub(r1, qq); acc[i][1] = f2_fma(t, t, acc[i][1]);
+        t = f2_sub(r2, qq); acc[i][2] = f2_fma(t, t, acc[i][2]);
+        t = f2_sub(r3, qq); acc[i][3] = f2_fma(t, t, acc[i][3]);
+    }
+}
+
+// Groups of four dimensions in the last stage of d dimensions.
+__host__ __device__ inline int last_stage_groups(int d) { return ((d - 1) % EX_BD) / 4 + 1; }
+
 // Consume the n_dchunks pipeline stages of one reference tile: the lane's
 // QPW x 8 block of squared distances accumulates sum_d (r_d - q_d)^2 with a
 // rounded sub and a fused multiply-add per dimension, in increasing d (the
@@ -372,12 +395,16 @@ KNN_DI void load_queries(float (&q)[QPW], const float *src) {
 // as (q, q) pairs in shared memory saved the register moves but took 16: 298
 // against 289 ms at 2^20 x 16384, d = 256, k = 100, 814 against 764 us at
 // 16384 x 4096, d = 128, k = 16.)
+// PARTIAL: the last stage takes only `tail` groups of four dimensions
+// (last_stage_groups); 1143 -> 884 us at 100000 x 4736, d = 20, k = 20, 712 -> 548 at
+// d = 5, 1074 -> 982 at 30000 x 4736, d = 100.  A variant of its own: with the choice made inside, problems of whole
+// stages came out up to 3 % slower.
 // `it` is the running stage counter of the CTA's ring.  Returns false (warp-
 // uniformly) if a wait timed out or another warp aborted.
-template <int QPW, int KCAP>
+template <int QPW, int KCAP, bool PARTIAL>
 KNN_DI bool consume_ref_tile(f32x2_t (&acc)[QPW][4], const float *stages, uint64_t *full,
                              uint64_t *empty, volatile int *abort_flag, int &it, int n_dchunks,
-                             int warp, int lane, int *status) {
+                             int tail, int warp, int lane, int *status) {
     using C = ExCfg<QPW, KCAP>;
 #pragma unroll
     for (int i = 0; i < QPW; ++i)
@@ -398,22 +425,18 @@ KNN_DI bool consume_ref_tile(f32x2_t (&acc)[QPW][4], const float *stages, uint64
         }
         const float *qs = stages + (size_t)s * C::STAGE_FLOATS + warp * QPW;
         const float *rs = stages + (size_t)s * C::STAGE_FLOATS + C::Q_FLOATS + lane * 4;
+        if (!PARTIAL || dc + 1 < n_dchunks) {
 #pragma unroll
-        for (int dd = 0; dd < EX_BD; ++dd) {
-            // 16-byte loads straight into packed pairs (x, y), (z, w)
-            const ulonglong2 ra = *reinterpret_cast<const ulonglong2 *>(rs + dd * EX_BR);
-            const ulonglong2 rb = *reinterpret_cast<const ulonglong2 *>(rs + dd * EX_BR + 128);
-            const f32x2_t r0 = ra.x, r1 = ra.y, r2 = rb.x, r3 = rb.y;
-            float q[QPW];
-            load_queries<QPW>(q, qs + dd * C::BQ);
+            for (int dd = 0; dd < EX_BD; ++dd)
+                consume_dim<QPW>(acc, rs + dd * EX_BR, qs + dd * C::BQ);
+        } else {
+            // the last chunk's dimensions, in fours: the zeros beyond them would
+            // add exact zeros
+#pragma unroll 1
+            for (int g = 0; g < tail; ++g) {
 #pragma unroll
-            for (int i = 0; i < QPW; ++i) {
-                const f32x2_t qq = f2_pack(q[i], q[i]);
-                f32x2_t t;
-                t = f2_sub(r0, qq); acc[i][0] = f2_fma(t, t, acc[i][0]);
-                t = f2_sub(r1, qq); acc[i][1] = f2_fma(t, t, acc[i][1]);
-                t = f2_sub(r2, qq); acc[i][2] = f2_fma(t, t, acc[i][2]);
-                t = f2_sub(r3, qq); acc[i][3] = f2_fma(t, t, acc[i][3]);
+                for (int e = 0; e < 4; ++e)
+                    consume_dim<QPW>(acc, rs + (4 * g + e) * EX_BR, qs + (4 * g + e) * C::BQ);
             }
         }
         __syncwarp();
