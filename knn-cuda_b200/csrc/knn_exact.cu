@@ -295,9 +295,15 @@ cudaError_t launch_v(const CUtensorMap &mr, const CUtensorMap &mq, const ExactAr
 template <int QPW, int KCAP, bool LB = false>
 cudaError_t launch_t(const CUtensorMap &mr, const CUtensorMap &mq, const ExactArgs &a,
                      int qtiles, cudaStream_t st) {
-    return last_stage_groups(a.d) < EX_BD / 4
-               ? launch_v<QPW, KCAP, LB, true>(mr, mq, a, qtiles, st)
-               : launch_v<QPW, KCAP, LB, false>(mr, mq, a, qtiles, st);
+    // Whole stages run either variant.  The one with the test for a short stage
+    // measured faster with lists of 128 keys and four stages or more a tile (277.3
+    // -> 272.2 ms at 2^20 x 16384, d = 256, k = 100; 1440 -> 1434 us at 65536 x 4736, d
+    // = 64) and slower below (867 -> 883 at d = 32; 793 -> 809 with k = 32): the
+    // compiler schedules the stage differently around the branch.
+    const bool partial = last_stage_groups(a.d) < EX_BD / 4 ||
+                         (KCAP == 128 && QPW == EX_QPW && a.n_dchunks >= 4);
+    return partial ? launch_v<QPW, KCAP, LB, true>(mr, mq, a, qtiles, st)
+                   : launch_v<QPW, KCAP, LB, false>(mr, mq, a, qtiles, st);
 }
 
 template <int QPW>

@@ -397,8 +397,7 @@ __host__ __device__ inline int last_stage_groups(int d) { return ((d - 1) % EX_B
 // 16384 x 4096, d = 128, k = 16.)
 // PARTIAL: the last stage takes only `tail` groups of four dimensions
 // (last_stage_groups); 1143 -> 884 us at 100000 x 4736, d = 20, k = 20, 712 -> 548 at
-// d = 5, 1074 -> 982 at 30000 x 4736, d = 100.  A variant of its own: with the choice made inside, problems of whole
-// stages came out up to 3 % slower.
+// d = 5, 1074 -> 982 at 30000 x 4736, d = 100.
 // `it` is the running stage counter of the CTA's ring.  Returns false (warp-
 // uniformly) if a wait timed out or another warp aborted.
 template <int QPW, int KCAP, bool PARTIAL>
@@ -425,7 +424,7 @@ KNN_DI bool consume_ref_tile(f32x2_t (&acc)[QPW][4], const float *stages, uint64
         }
         const float *qs = stages + (size_t)s * C::STAGE_FLOATS + warp * QPW;
         const float *rs = stages + (size_t)s * C::STAGE_FLOATS + C::Q_FLOATS + lane * 4;
-        if (!PARTIAL || dc + 1 < n_dchunks) {
+        if (!PARTIAL || dc + 1 < n_dchunks || tail == EX_BD / 4) {
 #pragma unroll
             for (int dd = 0; dd < EX_BD; ++dd)
                 consume_dim<QPW>(acc, rs + dd * EX_BR, qs + dd * C::BQ);
