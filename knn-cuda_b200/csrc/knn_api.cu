@@ -645,6 +645,19 @@ int plan_query_chunk(Workspace &ws, int Q, size_t fixed, F per_chunk) {
     return lo;
 }
 
+// The scratch of a call.  Where it has to be allocated anyway and no cap is set,
+// it is taken with the room that the exact kernel can make use of (at most 64 MB
+// more); a call that the held scratch is enough for never allocates, so that
+// what was run once can be captured.
+bool ensure_scratch(Workspace &ws, int method, int N, int Q, int d, int k) {
+    const size_t need = scratch_for(method, N, Q, d, k, ws.num_sms);
+    if (need <= ws.scratch.bytes) return true;
+    if (!use_tc(method) && !g_mem_cap &&
+        ws.scratch.ensure(exact_scratch_wanted(N, Q, d, k, ws.num_sms)))
+        return true;
+    return ws.scratch.ensure(need);
+}
+
 // Scratch of the spatial search for an exact problem, if it applies and the
 // memory is there beside `planned` bytes of the call; else the problem runs
 // without it.
@@ -722,11 +735,11 @@ bool host_entry(int wanted, const float *ref, int ref_nb, const float *query, in
     g_last_chunks = (query_nb + qc - 1) / qc;
     const long long ldq = round_up(qc, 64);
     const size_t out_elems = (size_t)k * qc;
-    const size_t scratch = scratch_for(method, ref_nb, qc, dim, k, ws->num_sms);
     if (!ws->ref.ensure((size_t)dim * ldr * sizeof(float)) ||
         !ws->qry.ensure((size_t)dim * ldq * sizeof(float)) ||
         !ws->dist.ensure(out_elems * sizeof(float)) ||
-        !ws->idx.ensure(out_elems * sizeof(int)) || !ws->scratch.ensure(scratch)) {
+        !ws->idx.ensure(out_elems * sizeof(int)) ||
+        !ensure_scratch(*ws, method, ref_nb, qc, dim, k)) {
         std::printf("ERROR: Memory allocation error\n");
         return false;
     }
@@ -922,8 +935,7 @@ int knnb200_knn_device(const float *ref, int ref_nb, long long ref_ld, const flo
     const bool tc = use_tc(method);
     if (qc < 1) return KNNB200_ENOMEM;
     g_last_chunks = (query_nb + qc - 1) / qc;
-    if (!ws->scratch.ensure(scratch_for(method, ref_nb, qc, dim, k, ws->num_sms)))
-        return KNNB200_ENOMEM;
+    if (!ensure_scratch(*ws, method, ref_nb, qc, dim, k)) return KNNB200_ENOMEM;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // Calls on one device share the workspace scratch: order them.
     if (cudaStreamWaitEvent(st, ws->last_done, 0) != cudaSuccess) return KNNB200_ECUDA;

@@ -24,6 +24,8 @@
 //     Ordering by the 64-bit key (distance bits, index) reproduces the
 //     reference's tie rule: equal distances keep the lower index
 //     (code/knncuda.cu:172, :178).
+//   * Where that grid's waves do not come out even, the tiles of all query tiles
+//     are laid end to end and cut into one range a CTA instead (TileRanges).
 //   * With one split the kernel writes sqrt(distance) and the index straight
 //     into the k x query_nb output; with several splits it writes each
 //     split's sorted keys to scratch and knn_merge_splits_kernel merges them.
@@ -43,7 +45,10 @@
 
 namespace knnb200 {
 
-template <int QPW, int KCAP, bool LB, bool PARTIAL>
+// RANGES: the CTA takes the whole tiles [u0, u1) of all query tiles' reference
+// tiles laid end to end (TileRanges), which may cross from one query tile into
+// the next; the ring runs on across the border.
+template <int QPW, int KCAP, bool LB, bool PARTIAL, bool RANGES>
 __global__ void __launch_bounds__(EX_THREADS, 1)
     knn_exact_kernel(const __grid_constant__ CUtensorMap tm_ref,
                      const __grid_constant__ CUtensorMap tm_qry, ExactArgs a) {
@@ -62,7 +67,9 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
     const int qtile = blockIdx.x, split = blockIdx.y;
     const int t0 = (int)((long long)a.n_rtiles * split / a.n_splits);
     const int t1 = (int)((long long)a.n_rtiles * (split + 1) / a.n_splits);
-    const int total = (t1 - t0) * a.n_dchunks;
+    const long long u0 = RANGES ? a.ranges.begin(blockIdx.x) : 0;
+    const long long u1 = RANGES ? a.ranges.begin(blockIdx.x + 1) : 0;
+    const int total = (RANGES ? (int)(u1 - u0) : t1 - t0) * a.n_dchunks;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::STAGES; ++s) {
@@ -92,9 +99,15 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
                 if (*abort_flag) break;
                 float *qs = stages + (size_t)s * C::STAGE_FLOATS;
                 float *rs = qs + C::Q_FLOATS;
-                const int rt = t0 + it / a.n_dchunks, dc = it % a.n_dchunks;
+                int rt = t0 + it / a.n_dchunks, qt = qtile;
+                const int dc = it % a.n_dchunks;
+                if (RANGES) {
+                    const long long u = u0 + it / a.n_dchunks;
+                    qt = (int)(u / a.n_rtiles);
+                    rt = (int)(u % a.n_rtiles);
+                }
                 mbar_arrive_expect_tx(&full[s], C::STAGE_BYTES);
-                tma_load_2d(qs, &tm_qry, &full[s], qtile * C::BQ, dc * EX_BD);
+                tma_load_2d(qs, &tm_qry, &full[s], qt * C::BQ, dc * EX_BD);
                 tma_load_2d(rs, &tm_ref, &full[s], rt * EX_BR, dc * EX_BD);
                 issued = it + 1;
             }
@@ -112,6 +125,35 @@ __global__ void __launch_bounds__(EX_THREADS, 1)
     unsigned long long *wt =
         reinterpret_cast<unsigned long long *>(base + C::TAU_OFFSET) + warp * QPW;
     unsigned long long nb;   // buffer fills
+    if constexpr (RANGES) {
+        const unsigned long long no_lb[QPW] = {};
+        const int tail = last_stage_groups(a.d);
+        int it = 0;
+        for (long long u = u0; u < u1;) {
+            const int qt = (int)(u / a.n_rtiles), r0 = (int)(u % a.n_rtiles);
+            const int r1 = (int)min((long long)a.n_rtiles, r0 + (u1 - u));
+            const int qw = qt * C::BQ + warp * QPW;
+            select_start<QPW>(wt, nb, qw, a.Q, lane);
+            for (int rt = r0; rt < r1; ++rt) {
+                f32x2_t acc[QPW][4];
+                if (!consume_ref_tile<QPW, KCAP, PARTIAL>(acc, stages, full, empty, abort_flag,
+                                                          it, a.n_dchunks, tail, warp, lane,
+                                                          a.status))
+                    return;
+                select_tile<QPW, KCAP, false>(wl, wt, nb, acc, rt, a.N, a.k, lane, no_lb);
+            }
+            select_finish<QPW, KCAP>(wl, wt, nb, a.k, lane);
+            const int slot = (int)blockIdx.x - a.ranges.owner((long long)qt * a.n_rtiles);
+            for (int i = 0; i < QPW; ++i) {
+                if (qw + i >= a.Q) break;
+                unsigned long long *dst = a.part + ((size_t)slot * a.Q + qw + i) * a.k;
+                for (int j = lane; j < a.k; j += 32) dst[j] = wl[i * C::REGION + j];
+            }
+            __syncwarp();   // the buffers are rewritten
+            u += r1 - r0;
+        }
+        return;
+    }
     select_start<QPW>(wt, nb, qtile * C::BQ + warp * QPW, a.Q, lane);
     unsigned long long lbk[QPW];
 #pragma unroll
@@ -177,7 +219,7 @@ __global__ void __launch_bounds__(32 * MG_WARPS)
     knn_merge_splits_kernel(const unsigned long long *__restrict__ part, int S, int Q, int k,
                             float *__restrict__ out_dist, int *__restrict__ out_idx,
                             long long ld_out, int row0, unsigned long long *__restrict__ lb_out,
-                            QuerySubset subset) {
+                            QuerySubset subset, TileRanges ranges) {
     constexpr int QPB = MG_WARPS / WPQ;
     __shared__ unsigned long long lists[MG_WARPS][KCAP], scratch[MG_WARPS][KCAP];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -188,7 +230,7 @@ __global__ void __launch_bounds__(32 * MG_WARPS)
         const int q = q0 + warp / WPQ;
         if (q < nq) {
             merge_lists<KCAP>(lists[warp], scratch[warp], part + (size_t)q * k, (size_t)Q * k,
-                              warp % WPQ, WPQ, S, k, lane);
+                              warp % WPQ, WPQ, ranges.ctas ? ranges.lists(q) : S, k, lane);
         }
         __syncthreads();
         if (WPQ > 1) {
@@ -217,6 +259,8 @@ namespace {
 
 struct ExactShape {
     int qpw, kcap, bq, splits, n_rtiles, n_dchunks;
+    TileRanges ranges;      // ctas = 0: the grid of qtiles x splits
+    int range_lists = 0;    // lists a query of the ranges has, at most
     size_t smem;
 };
 
@@ -275,19 +319,43 @@ bool choose_shape(int N, int Q, int d, int k_all, int num_sms, ExactShape &s) {
         }
     }
     s.splits = best;
+    // The grid leaves SMs idle where its waves do not come out even.  One range
+    // of tiles a CTA (TileRanges) gives every SM the same work, but most CTAs
+    // then hold parts of two query tiles and warm up twice.  Modelled time as
+    // above, in whole tiles; taken where it is less by 3 %.  Measured over 84
+    // shapes of d = 8 to 512 and k = 5 to 100: at a modelled ratio below 0.97 the
+    // ranges take 0.78 to 0.975 of the grid's time (675 -> 609 us at 16384 x 4096, d
+    // = 128, k = 16: 128 CTAs of the grid; 1771 -> 1635 at 17149 x 2865, d = 512),
+    // from 0.97 to 1 they take 0.94 to 1.03, above 1 up to 1.2.
+    s.ranges = TileRanges();
+    const long long units = (long long)qtiles * s.n_rtiles;
+    if (s.qpw != EX_QPW || k_all > 128 || units < num_sms) return true;
+    const long long per = (units + num_sms - 1) / num_sms;
+    const long long parts = (per + s.n_rtiles - 2) / s.n_rtiles + 1;   // query tiles of a CTA
+    const long long waves = ((long long)qtiles * best + num_sms - 1) / num_sms;
+    const double t_grid = (double)waves * ((s.n_rtiles + best - 1) / best + warm);
+    const long long lists = (s.n_rtiles - 1) / (units / num_sms) + 2;   // at most, of a query
+    if (per + parts * warm < 0.97 * t_grid && lists <= max_s &&
+        per * s.n_dchunks < (1ll << 31)) {
+        s.ranges.ctas = num_sms;
+        s.ranges.bq = s.bq;
+        s.ranges.n_rtiles = s.n_rtiles;
+        s.ranges.units = units;
+        s.range_lists = (int)lists;
+    }
     return true;
 }
 
-template <int QPW, int KCAP, bool LB, bool PARTIAL>
+template <int QPW, int KCAP, bool LB, bool PARTIAL, bool RANGES>
 cudaError_t launch_v(const CUtensorMap &mr, const CUtensorMap &mq, const ExactArgs &a,
                      int qtiles, cudaStream_t st) {
     using C = ExCfg<QPW, KCAP>;
-    constexpr auto kern = knn_exact_kernel<QPW, KCAP, LB, PARTIAL>;
+    constexpr auto kern = knn_exact_kernel<QPW, KCAP, LB, PARTIAL, RANGES>;
     if (!launch_regs_ok<kern>()) return cudaErrorLaunchOutOfResources;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)C::SMEM);
     if (e != cudaSuccess) return e;
-    dim3 grid(qtiles, a.n_splits);
+    const dim3 grid = RANGES ? dim3(a.ranges.ctas) : dim3(qtiles, a.n_splits);
     kern<<<grid, EX_THREADS, C::SMEM, st>>>(mr, mq, a);
     return cudaGetLastError();
 }
@@ -302,8 +370,13 @@ cudaError_t launch_t(const CUtensorMap &mr, const CUtensorMap &mq, const ExactAr
     // compiler schedules the stage differently around the branch.
     const bool partial = last_stage_groups(a.d) < EX_BD / 4 ||
                          (KCAP == 128 && QPW == EX_QPW && a.n_dchunks >= 4);
-    return partial ? launch_v<QPW, KCAP, LB, true>(mr, mq, a, qtiles, st)
-                   : launch_v<QPW, KCAP, LB, false>(mr, mq, a, qtiles, st);
+    if constexpr (QPW == EX_QPW && !LB && KCAP <= 128) {
+        if (a.ranges.ctas)
+            return partial ? launch_v<QPW, KCAP, LB, true, true>(mr, mq, a, qtiles, st)
+                           : launch_v<QPW, KCAP, LB, false, true>(mr, mq, a, qtiles, st);
+    }
+    return partial ? launch_v<QPW, KCAP, LB, true, false>(mr, mq, a, qtiles, st)
+                   : launch_v<QPW, KCAP, LB, false, false>(mr, mq, a, qtiles, st);
 }
 
 template <int QPW>
@@ -323,7 +396,8 @@ static long long qcopy_pitch(int Q) { return ((long long)Q + 31) / 32 * 32; }
 
 int launch_split_merge(const unsigned long long *part, int S, int Q, int k, float *out_dist,
                        int *out_idx, long long ld_out, cudaStream_t st, int row0,
-                       unsigned long long *lb_out, const QuerySubset &subset) {
+                       unsigned long long *lb_out, const QuerySubset &subset,
+                       const TileRanges &ranges) {
     if (k > kPassRanks) return kErrUnsupported;
     // all eight warps on one query: 14.6 us against 51.9 with one warp a query at
     // 40 queries and 148 lists of 50 keys, 15.4 against 22.7 at 300 queries and 29
@@ -333,7 +407,7 @@ int launch_split_merge(const unsigned long long *part, int S, int Q, int k, floa
         // a subset is usually empty: few blocks, which loop if it is not
         const int all = (Q + qpb - 1) / qpb, blocks = subset.count ? std::min(all, 592) : all;
         kern<<<blocks, 32 * MG_WARPS, 0, st>>>(part, S, Q, k, out_dist, out_idx, ld_out, row0,
-                                               lb_out, subset);
+                                               lb_out, subset, ranges);
         return cudaGetLastError() == cudaSuccess ? (int)kOk : (int)kErrLaunch;
     };
     auto pick = [&](auto cap) {
@@ -371,6 +445,25 @@ size_t exact_scratch_bytes(int N, int Q, int d, int k, int num_sms) {
     return exact_need(s, Q, d, k, nullptr, nullptr);
 }
 
+// Scratch of the ranges: their lists, after the copy of the queries if there is
+// one.  The room of the copies holds them in most cases.
+static size_t ranges_need(const ExactShape &s, int Q, int d, int k, bool copied,
+                          size_t *part_off) {
+    const size_t off = copied ? ((size_t)d * qcopy_pitch(Q) * sizeof(float) + 255) & ~size_t(255)
+                              : 0;
+    if (part_off) *part_off = off;
+    return off + (size_t)s.range_lists * Q * k * 8;
+}
+
+size_t exact_scratch_wanted(int N, int Q, int d, int k, int num_sms) {
+    const size_t need = exact_scratch_bytes(N, Q, d, k, num_sms);
+    ExactShape s;
+    if (lowdim_applies(N, Q, d, k) || !choose_shape(N, Q, d, k, num_sms, s) || !s.ranges.ctas)
+        return need;
+    const size_t want = ranges_need(s, Q, d, k, true, nullptr);
+    return want > need + (size_t(64) << 20) ? need : std::max(need, want);
+}
+
 bool exact_supported_k(int k) { return k >= 1; }
 
 int launch_exact(const ExactProblem &p, cudaStream_t st) {
@@ -380,12 +473,24 @@ int launch_exact(const ExactProblem &p, cudaStream_t st) {
     if (p.force_splits > 0) s.splits = std::min(p.force_splits, std::min(s.n_rtiles, 256));
     size_t part_off = 0, lb_off = 0;
     if (exact_need(s, p.Q, p.d, p.k, &part_off, &lb_off) > p.scratch_bytes) return kErrScratch;
+    const bool copied = (reinterpret_cast<uintptr_t>(p.qry) & 15) || p.ldq % 4;
+    if (s.ranges.ctas) {
+        // not where the split is given, or the scratch has no room for the lists
+        size_t off = 0;
+        if (p.force_splits > 0 ||
+            ranges_need(s, p.Q, p.d, p.k, copied, &off) > p.scratch_bytes) {
+            s.ranges = TileRanges();
+        } else {
+            s.splits = s.range_lists;
+            part_off = off;
+        }
+    }
     unsigned char *sb = static_cast<unsigned char *>(p.scratch);
     unsigned long long *part = reinterpret_cast<unsigned long long *>(sb + part_off);
     unsigned long long *lb = reinterpret_cast<unsigned long long *>(sb + lb_off);
     const float *qry = p.qry;
     long long ldq = p.ldq;
-    if ((reinterpret_cast<uintptr_t>(qry) & 15) || ldq % 4) {
+    if (copied) {
         float *copy = static_cast<float *>(p.scratch);
         ldq = qcopy_pitch(p.Q);
         // rows on gridDim.y (at most 65535 of them a launch)
@@ -409,6 +514,7 @@ int launch_exact(const ExactProblem &p, cudaStream_t st) {
     a.d = p.d;
     a.n_rtiles = s.n_rtiles;
     a.n_splits = s.splits;
+    a.ranges = s.ranges;
     a.n_dchunks = s.n_dchunks;
     a.out_dist = p.out_dist;
     a.out_idx = p.out_idx;
@@ -439,7 +545,8 @@ int launch_exact(const ExactProblem &p, cudaStream_t st) {
         if (p.timer) p.timer->mark(st, kPhaseExactMain);
         if (s.splits > 1) {
             const int rc = launch_split_merge(a.part, s.splits, p.Q, a.k, p.out_dist, p.out_idx,
-                                              p.ld_out, st, row0, a.lb_out);
+                                              p.ld_out, st, row0, a.lb_out, QuerySubset(),
+                                              s.ranges);
             if (rc != kOk) return rc;
             if (p.timer) p.timer->mark(st, kPhaseExactMerge);
         }

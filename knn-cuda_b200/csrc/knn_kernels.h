@@ -59,6 +59,24 @@ struct PhaseTimer {
     }
 };
 
+// A problem cut into equal ranges of tiles instead of a grid of (query tile,
+// split): the n_rtiles reference tiles of every query tile laid end to end,
+// CTA c taking the tiles [begin(c), begin(c + 1)).  ctas = 0: not used.
+struct TileRanges {
+    int ctas = 0, bq = 0, n_rtiles = 0;
+    long long units = 0;   // tiles altogether, at least ctas
+    __host__ __device__ long long begin(int c) const { return units * c / ctas; }
+    // the CTA that tile u belongs to
+    __host__ __device__ int owner(long long u) const {
+        return (int)(((u + 1) * ctas - 1) / units);
+    }
+    // lists of query q: one from every CTA that has tiles of its query tile
+    __host__ __device__ int lists(int q) const {
+        const long long u = (long long)(q / bq) * n_rtiles;
+        return owner(u + n_rtiles - 1) - owner(u) + 1;
+    }
+};
+
 // Kernel-side arguments of the fused exact kernel.
 struct ExactArgs {
     int N, Q, d, k;
@@ -66,7 +84,7 @@ struct ExactArgs {
     float *out_dist;
     int *out_idx;
     long long ld_out;
-    unsigned long long *part;   // [n_splits][Q][k] keys when n_splits > 1
+    unsigned long long *part;   // [n_splits][Q][k] keys when n_splits > 1 or ranges
     int *status;                // device status word (DeviceStatus)
     // k > 256 runs in passes of up to 256 ranks: pass p selects keys >= lb[q]
     // (LB kernels only), writes output rows row0 .. row0 + k - 1 and, when
@@ -74,6 +92,7 @@ struct ExactArgs {
     const unsigned long long *lb;
     unsigned long long *lb_out;
     int row0;
+    TileRanges ranges;   // instead of the grid of (query tile, split)
 };
 
 // One exact k-NN problem on device-resident, dim x n row-major inputs.
@@ -143,8 +162,11 @@ int launch_space(const ExactProblem &p, cudaStream_t st, QuerySubset *far);
 int launch_split_merge(const unsigned long long *part, int S, int Q, int k, float *out_dist,
                        int *out_idx, long long ld_out, cudaStream_t st, int row0 = 0,
                        unsigned long long *lb_out = nullptr,
-                       const QuerySubset &subset = QuerySubset());
+                       const QuerySubset &subset = QuerySubset(),
+                       const TileRanges &ranges = TileRanges());
 size_t exact_scratch_bytes(int N, int Q, int d, int k, int num_sms);
+// What the exact path can make use of, where the memory is there: up to 64 MB more.
+size_t exact_scratch_wanted(int N, int Q, int d, int k, int num_sms);
 int exact_plan_splits(int N, int Q, int d, int k, int num_sms);
 int launch_exact(const ExactProblem &p, cudaStream_t st);
 
