@@ -351,6 +351,7 @@ int enqueue(Workspace &ws, const ExactProblem &p0, int method, cudaStream_t st,
     t.force_kind = g_force_kind;
     t.point_sample = true;   // the whole set is prepared before pass 1
     t.probe_event = ws.probe;
+    t.clear_status = !ref_prepared;   // with the first chunk
     if (ws.bound_check) {
         if (cudaMemsetAsync(ws.bound.ptr, 0, 16, st) != cudaSuccess) return kErrCuda;
         t.bound_stat = static_cast<unsigned *>(ws.bound.ptr);
@@ -523,6 +524,7 @@ int enqueue_tc_streamed(Workspace &ws, const ExactProblem &p, const float *ref_h
     t.num_sms = p.num_sms;
     t.timer = nullptr;
     t.host_tmp = ws.tc_stats + 2;
+    t.clear_status = true;
     t.adaptive = false;   // pass 2 starts before the whole set has arrived
     // the translation comes from every fourth sample tile; the query prep
     // (in tc_run_begin) needs it
@@ -775,7 +777,8 @@ bool host_entry(int wanted, const float *ref, int ref_nb, const float *query, in
                                  cols * sizeof(float), dim, cudaMemcpyHostToDevice, st);
     };
     cudaError_t e0 = streamed ? cudaSuccess : copy_in(ref, ref_nb, ref_d, ldr, ref_nb);
-    cudaError_t e2 = cudaMemsetAsync(ws->status.ptr, 0, sizeof(int), st);
+    // (the tensor path clears the status word itself)
+    cudaError_t e2 = tc ? cudaSuccess : cudaMemsetAsync(ws->status.ptr, 0, sizeof(int), st);
     if (e0 != cudaSuccess || e2 != cudaSuccess) {
         std::printf("ERROR: Unable to copy data from host to device\n");
         cudaGetLastError();
@@ -939,7 +942,9 @@ int knnb200_knn_device(const float *ref, int ref_nb, long long ref_ld, const flo
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // Calls on one device share the workspace scratch: order them.
     if (cudaStreamWaitEvent(st, ws->last_done, 0) != cudaSuccess) return KNNB200_ECUDA;
-    if (cudaMemsetAsync(ws->status.ptr, 0, sizeof(int), st) != cudaSuccess) return KNNB200_ECUDA;
+    // (the tensor path clears the status word itself)
+    if (!tc && cudaMemsetAsync(ws->status.ptr, 0, sizeof(int), st) != cudaSuccess)
+        return KNNB200_ECUDA;
     long long stats[3] = {0, 0, 0};
     for (int q0 = 0; q0 < query_nb && rc == kOk; q0 += qc) {
         ExactProblem p;

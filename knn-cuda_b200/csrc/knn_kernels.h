@@ -243,9 +243,10 @@ struct TcProblem {
     // event for the read-back of the overflow prediction (launch_tc): with it
     // the main scan is queued before the host knows whether it runs in BF16
     cudaEvent_t probe_event = nullptr;
-    // pinned, 2 ints: [0] the device status word, copied with the last
-    // read-back of a run, [1] whether nothing was queued after that copy
+    // pinned, 2 ints: [0] the device status word, written with the run's
+    // counters, [1] whether nothing was queued after that
     int *host_status = nullptr;
+    bool clear_status = false;   // the run clears the status word itself
 };
 
 // A sample of the 256-point tiles: `run` consecutive tiles out of every

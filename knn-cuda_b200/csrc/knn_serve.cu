@@ -137,7 +137,6 @@ int run_refset(knnb200_refset *rs, Slot &slot, const float *query, int Q, long l
     if (!exact_supported_k(k)) return kErrUnsupported;
     if (!slot.scratch.ensure(scratch_need(rs, method, Q, k))) return kErrNoMemory;
     slot.host_stats[9] = 0;
-    if (cudaMemsetAsync(slot.status.ptr, 0, sizeof(int), st) != cudaSuccess) return kErrCuda;
     if (use_tc_for(rs, method, Q, k)) {
         TcProblem t;
         t.ref = static_cast<const float *>(rs->ref.ptr);
@@ -161,8 +160,10 @@ int run_refset(knnb200_refset *rs, Slot &slot, const float *query, int Q, long l
         t.point_sample = true;   // the resident set was prepared as a whole
         t.probe_event = slot.probe;
         t.host_status = slot.host_stats + 8;
+        t.clear_status = true;
         return launch_tc(t, rs->tc, st, slot.host_stats);
     }
+    if (cudaMemsetAsync(slot.status.ptr, 0, sizeof(int), st) != cudaSuccess) return kErrCuda;
     ExactProblem p;
     p.ref = static_cast<const float *>(rs->ref.ptr);
     p.N = rs->N;

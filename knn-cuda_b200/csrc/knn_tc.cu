@@ -706,11 +706,21 @@ KNN_DI void write_norm_row(__nv_bfloat16 *parts, int p, float s) {
 // queries, d = 768, and 39 at 16384, d = 256, next to the packing kernel's 5; this
 // one takes 18 and 11.5 for both.)
 constexpr int TC_QP_WARPS = 8;
+// Counters of a run: [0] uncertified queries, [1] those with an overflowing list,
+// [2..3] candidates (64-bit), [4..5] predicted overflows (BF16, FP8), [6] the
+// queries' largest coordinate (float bits, FP8), [7] the
+// certification's ticket (last_block)
+constexpr int TC_CTL = 8;
 __global__ void __launch_bounds__(32 * TC_QP_WARPS, 3)
     tc_prep_query_kernel(const float *__restrict__ x, int n, long long ld, int d, int d_pad,
                          const float *__restrict__ center, float *__restrict__ nrm,
                          unsigned *__restrict__ absmax_bits, __nv_bfloat16 *__restrict__ xb,
-                         __nv_bfloat16 *__restrict__ xlo) {
+                         __nv_bfloat16 *__restrict__ xlo, int *__restrict__ clear_ctl,
+                         int *__restrict__ clear_status) {
+    if (blockIdx.x == 0) {
+        if (clear_ctl && threadIdx.x < TC_CTL) clear_ctl[threadIdx.x] = 0;
+        if (clear_status && threadIdx.x == 0) *clear_status = 0;
+    }
     __shared__ float tile_all[TC_QP_WARPS][32][33], part[TC_QP_WARPS][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float(*tile)[33] = tile_all[warp];
@@ -1013,6 +1023,27 @@ __global__ void tc_pack_f8_kernel(const float *__restrict__ x, int n, long long 
     }
 }
 
+// What the certification's last block writes for the host.
+struct TcReport {
+    const int *ctl = nullptr;   // counters [0..3] to host[0..3]
+    int *ticket = nullptr;
+    volatile int *host = nullptr;
+    const int *status = nullptr;          // the status word to host_status[0]
+    volatile int *host_status = nullptr;
+};
+
+// Whether this block is the last of its grid to come here (one thread a block,
+// after the block's work and a __syncthreads; *ticket starts at 0).  What the
+// host needs of a kernel's results the last block writes to pinned memory
+// itself: a copy between two kernels of a stream held the second one up by 15 to
+// 18 us, and two copies at the end of a call took 13; the write costs its kernel 3.
+KNN_DI bool last_block(int *ticket) {
+    __threadfence();
+    if (atomicAdd(ticket, 1) != (int)gridDim.x - 1) return false;
+    __threadfence();
+    return true;
+}
+
 // Emission threshold: the KS-th smallest of the per-split pass-1 lists plus
 // the error bound E_q (so that the k-th exact distance only has to lie below
 // the sample's KS-th approximate one to certify); resets candidate counts.
@@ -1024,7 +1055,8 @@ __global__ void tc_pack_f8_kernel(const float *__restrict__ x, int n, long long 
 // above the sample's smallest values, so a band [T, T + E] wider than
 // [L_0, T] holds many times that; n_wide[0] counts them for probe0 (BF16:
 // switch to split BF16), n_wide[1] for probe1 (FP8: whether an FP8 pass 2
-// pays).
+// pays).  With host_wide (pinned) only n_wide[0] is wanted: the last block writes
+// it there.
 // One warp per query: the lists' values pass through a sorted list of KS keys
 // that lies across its lanes (one thread per query read the up to 148 lists of
 // a small batch one after the other: 33 us at 13 queries, now 6.7).
@@ -1033,7 +1065,8 @@ __global__ void __launch_bounds__(32 * TC_THR_WARPS)
     tc_threshold_kernel(const float *__restrict__ p1, int S, int Q, const float *__restrict__ qn,
                         const unsigned *__restrict__ rmax_bits, TcBound bound, TcBound probe0,
                         TcBound probe1, float *__restrict__ thr, float *__restrict__ thr_raw,
-                        int *__restrict__ count, int *__restrict__ n_wide) {
+                        int *__restrict__ count, int *__restrict__ n_wide,
+                        volatile int *__restrict__ host_wide) {
     const int lane = threadIdx.x & 31;
     const int q = blockIdx.x * TC_THR_WARPS + (threadIdx.x >> 5);
     bool wide0 = false, wide1 = false;
@@ -1084,7 +1117,13 @@ __global__ void __launch_bounds__(32 * TC_THR_WARPS)
     }
     if (n_wide) {
         const int n0 = __syncthreads_count(wide0), n1 = __syncthreads_count(wide1);
-        if (threadIdx.x == 0) {
+        if (threadIdx.x == 0 && host_wide) {
+            // the blocks that have arrived count in the word above
+            const unsigned long long all =
+                atomicAdd(reinterpret_cast<unsigned long long *>(n_wide),
+                          (1ull << 32) | (unsigned)n0);
+            if ((unsigned)(all >> 32) == gridDim.x - 1) host_wide[0] = (int)(uint32_t)all + n0;
+        } else if (threadIdx.x == 0) {
             if (n0) atomicAdd(n_wide, n0);
             if (n1) atomicAdd(n_wide + 1, n1);
         }
@@ -1588,33 +1627,43 @@ __global__ void __launch_bounds__(32 * TC_RK_WARPS)
                              float *__restrict__ out_dist, int *__restrict__ out_idx,
                              long long ld_out, int *__restrict__ fail_list,
                              int *__restrict__ n_fail, float *__restrict__ retry,
-                             float *__restrict__ retry_f, float *__restrict__ retry_s) {
+                             float *__restrict__ retry_f, float *__restrict__ retry_s,
+                             TcReport report) {
     // KCAP keys per warp; one warp per block with room for cmax keys when lists
     // may be longer than TC_RK_REG
     extern __shared__ unsigned long long keys_all[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int q = blockIdx.x * (blockDim.x >> 5) + warp;
-    if (q >= Q) return;
-    const int n = nsel[q];
-    if (n < 0) return;
-    const unsigned long long *cq = cand + (size_t)q * cmax;
-    unsigned long long *keys = keys_all + (size_t)warp * KCAP;
-    if (n <= 256) {
-        rr_sorted<8, KCAP>(cq, n, k, keys, lane);
-    } else if (n <= 512) {
-        rr_sorted<16, KCAP>(cq, n, k, keys, lane);
-    } else if (n <= TC_RK_REG) {
-        rr_sorted<32, KCAP>(cq, n, k, keys, lane);
-    } else {
-        int P = 32;
-        while (P < n) P <<= 1;
-        for (int t = lane; t < P; t += 32) keys[t] = t < n ? cq[t] : kKeyInf;
-        __syncwarp();
-        warp_bitonic_sort(keys, P, lane);
+    auto certify = [&] {
+        if (q >= Q) return;
+        const int n = nsel[q];
+        if (n < 0) return;
+        const unsigned long long *cq = cand + (size_t)q * cmax;
+        unsigned long long *keys = keys_all + (size_t)warp * KCAP;
+        if (n <= 256) {
+            rr_sorted<8, KCAP>(cq, n, k, keys, lane);
+        } else if (n <= 512) {
+            rr_sorted<16, KCAP>(cq, n, k, keys, lane);
+        } else if (n <= TC_RK_REG) {
+            rr_sorted<32, KCAP>(cq, n, k, keys, lane);
+        } else {
+            int P = 32;
+            while (P < n) P <<= 1;
+            for (int t = lane; t < P; t += 32) keys[t] = t < n ? cq[t] : kKeyInf;
+            __syncwarp();
+            warp_bitonic_sort(keys, P, lane);
+        }
+        rr_certify(keys, q, qn[q], __uint_as_float(*rmax_bits), thr[q], d_pad, k, rb, out_dist,
+                   out_idx, ld_out, fail_list, n_fail, retry, retry_f, retry_s, count[q] > cmax,
+                   lane);
+    };
+    certify();
+    if (!report.host) return;
+    __syncthreads();
+    if (threadIdx.x == 0 && last_block(report.ticket)) {
+        for (int i = 0; i < 4; ++i) report.host[i] = __ldcg(report.ctl + i);
+        if (report.host_status) report.host_status[0] = __ldcg(report.status);
     }
-    rr_certify(keys, q, qn[q], __uint_as_float(*rmax_bits), thr[q], d_pad, k, rb, out_dist,
-               out_idx, ld_out, fail_list, n_fail, retry, retry_f, retry_s, count[q] > cmax,
-               lane);
 }
 
 // Incremental re-rank for a reference set that arrives in pieces (the
@@ -2226,7 +2275,8 @@ TcBound run_bound(const TcRun &r, int kind) {
 // (from a scan of `kind`) have stride cmax.
 int rerank(const TcRun &r, cudaStream_t st, int kind, int Q, int cmax, const float *qry,
            long long ldq, const float *qn, const float *thr, const float *thr_raw,
-           float *out_dist, int *out_idx, long long ld_out, int *fail, bool final_pass) {
+           float *out_dist, int *out_idx, long long ld_out, int *fail, bool final_pass,
+           const TcReport &report = TcReport()) {
     const TcProblem &P = r.P;
     // (clear at the start of a run)
     if (final_pass && cudaMemsetAsync(r.nfail, 0, 2 * sizeof(int), st) != cudaSuccess)
@@ -2263,7 +2313,7 @@ int rerank(const TcRun &r, cudaStream_t st, int kind, int Q, int cmax, const flo
                                  r.cand, r.nsel, cmax, Q, P.bound_stat);
     certify<<<(Q + cwarps - 1) / cwarps, 32 * cwarps, csmem, st>>>(
         r.cand, r.nsel, r.count, cmax, Q, P.k, r.d_pad, qn, r.R.rmax_bits, thr, rb, out_dist,
-        out_idx, ld_out, fail, r.nfail, r.retry, r.retry_f, r.retry_s);
+        out_idx, ld_out, fail, r.nfail, r.retry, r.retry_f, r.retry_s, report);
     return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 
@@ -2326,7 +2376,7 @@ int tc_run_begin(const TcProblem &P, const TcRefView &R, cudaStream_t st, TcRun 
     r.fail = cv.take<int>(P.Q);
     r.fail2 = cv.take<int>(P.Q);
     r.nsel = cv.take<int>(P.Q);
-    r.ctl = cv.take<int>(8);
+    r.ctl = cv.take<int>(TC_CTL);
     r.nfail = r.ctl;
     r.cand_total = reinterpret_cast<unsigned long long *>(r.ctl + 2);
     r.nwide = r.ctl + 4;
@@ -2345,10 +2395,13 @@ int tc_run_begin(const TcProblem &P, const TcRefView &R, cudaStream_t st, TcRun 
     r.done = nullptr;
 
     // queries: norms (and their largest |q - c|) + BF16 K-major copy of -2 q
-    if (cudaMemsetAsync(r.ctl, 0, 8 * sizeof(int), st) != cudaSuccess) return kErrCuda;
+    // and, in the same launch, the run's counters cleared (with FP8 the kernel
+    // uses one of them itself) and the status word
+    if (fp8 && cudaMemsetAsync(r.ctl, 0, TC_CTL * sizeof(int), st) != cudaSuccess) return kErrCuda;
     tc_prep_query_kernel<<<(P.Q + 31) / 32, 32 * TC_QP_WARPS, 0, st>>>(
         P.qry, P.Q, P.ldq, P.d, p.d_pad, R.center, r.qn,
-        fp8 ? reinterpret_cast<unsigned *>(r.nwide + 2) : nullptr, r.qB, nullptr);
+        fp8 ? reinterpret_cast<unsigned *>(r.nwide + 2) : nullptr, r.qB, nullptr,
+        fp8 ? nullptr : r.ctl, P.clear_status ? P.status : nullptr);
     if (cudaGetLastError() != cudaSuccess) return kErrLaunch;
     r.want_fp8 = false;
     if (fp8) {
@@ -2372,7 +2425,8 @@ static int switch_to_split(TcRun &r, cudaStream_t st) {
     const int rc = ensure_ref_lo(r, st);
     if (rc != kOk) return rc;
     tc_prep_query_kernel<<<(P.Q + 31) / 32, 32 * TC_QP_WARPS, 0, st>>>(
-        P.qry, P.Q, P.ldq, P.d, r.d_pad, r.R.center, nullptr, nullptr, r.qB, r.qBlo);
+        P.qry, P.Q, P.ldq, P.d, r.d_pad, r.R.center, nullptr, nullptr, r.qB, r.qBlo,
+        nullptr, nullptr);
     tc_rethreshold_kernel<<<(P.Q + 255) / 256, 256, 0, st>>>(r.thr_raw, P.Q, r.qn, r.R.rmax_bits,
                                                             run_bound(r, kTcBf16x3),
                                                             run_bound(r, kTcBf16), 0, r.thr);
@@ -2396,21 +2450,19 @@ int tc_run_pass1(TcRun &r, cudaStream_t st) {
     const bool forced = (force == kTcBf16) || (force == kTcBf16x3 && lo_ok) ||
                         (force == kTcFp8 && r.want_fp8);
     const bool probe = !forced && P.host_tmp && ((P.adaptive && lo_ok) || r.want_fp8);
+    // BF16 unless most lists would overflow: launch_tc queues the BF16 scan,
+    // which looks at the count itself, before the host knows it
+    const bool undecided = probe && P.probe_event && !r.want_fp8;
     const TcBound b16 = run_bound(r, kTcBf16);
     tc_threshold_kernel<<<(P.Q + TC_THR_WARPS - 1) / TC_THR_WARPS, 32 * TC_THR_WARPS, 0, st>>>(
         r.p1, TP_LISTS * r.splits1, P.Q, r.qn, r.R.rmax_bits, b16, b16,
         r.want_fp8 ? run_bound(r, kTcFp8) : b16, r.thr, r.thr_raw, r.count,
-        probe ? r.nwide : nullptr);
+        probe ? r.nwide : nullptr, undecided ? P.host_tmp : nullptr);
     if (cudaGetLastError() != cudaSuccess) return kErrLaunch;
     r.kind = kTcBf16;
     int wide16 = 0, wide8 = 0;
-    if (probe && P.probe_event && !r.want_fp8) {
-        // BF16 unless most lists would overflow: launch_tc queues the BF16
-        // scan, which looks at the count itself, before the host knows it
-        if (cudaMemcpyAsync(P.host_tmp, r.nwide, sizeof(int), cudaMemcpyDeviceToHost, st) !=
-                cudaSuccess ||
-            cudaEventRecord(P.probe_event, st) != cudaSuccess)
-            return kErrCuda;
+    if (undecided) {
+        if (cudaEventRecord(P.probe_event, st) != cudaSuccess) return kErrCuda;
         r.undecided = true;
         if (P.timer) P.timer->mark(st, kPhaseTcThreshold);
         return kOk;
@@ -2512,7 +2564,8 @@ int tc_run_finish(TcRun &r, cudaStream_t st, int *host_stats) {
     host_stats[4] = host_stats[5] = 0;
     host_stats[6] = r.kind;
     host_stats[7] = -1;
-    int rc = kOk;
+    if (P.host_status) P.host_status[1] = 0;
+    int rc = kOk, nf = 0;
     if (r.pieces) {
         // every candidate was re-ranked piece by piece: certify
         RrBounds rb;
@@ -2524,25 +2577,22 @@ int tc_run_finish(TcRun &r, cudaStream_t st, int *host_stats) {
             r.d_pad, P.out_dist, P.out_idx, P.ld_out, r.fail, r.nfail, r.retry, r.retry_f,
             r.retry_s, r.cand_total);
         if (cudaGetLastError() != cudaSuccess) return kErrLaunch;
+        if (tm) tm->mark(st, kPhaseTcRerank);
+        if ((rc = read_count(r.ctl, host_tmp, st, nf, 4)) != kOk) return rc;
     } else {
+        const TcReport report = {r.ctl, r.ctl + 7, host_tmp, P.status, P.host_status};
         rc = rerank(r, st, r.kind, P.Q, r.cmax, P.qry, P.ldq, r.qn, r.thr, r.thr_raw, P.out_dist,
-                    P.out_idx, P.ld_out, r.fail, false);
+                    P.out_idx, P.ld_out, r.fail, false, report);
+        if (rc != kOk) return rc;
+        if (tm) tm->mark(st, kPhaseTcRerank);
+        if (cudaStreamSynchronize(st) != cudaSuccess) return kErrCuda;
+        nf = host_tmp[0];
     }
-    if (rc != kOk) return rc;
-    if (tm) tm->mark(st, kPhaseTcRerank);
-    // nfail[0..1] and cand_total land in host_stats[2..5]
-    if (P.host_status) {
-        P.host_status[1] = 0;
-        if (cudaMemcpyAsync(P.host_status, P.status, sizeof(int), cudaMemcpyDeviceToHost, st) !=
-            cudaSuccess)
-            return kErrCuda;
-    }
-    int nf = 0;
-    if ((rc = read_count(r.ctl, host_tmp, st, nf, 4)) != kOk) return rc;
+    // nfail[0..1] and cand_total are in host_stats[2..5]
     const int n_over = host_tmp[1];
     host_stats[0] = nf;
     if (nf == 0) {
-        if (P.host_status) P.host_status[1] = 1;
+        if (P.host_status && !r.pieces) P.host_status[1] = 1;
         return kOk;
     }
 
@@ -2559,7 +2609,7 @@ int tc_run_finish(TcRun &r, cudaStream_t st, int *host_stats) {
                                                                        nf, r.qsub, r.ldf);
     tc_prep_query_kernel<<<(nf + 31) / 32, 32 * TC_QP_WARPS, 0, st>>>(
         r.qsub, nf, r.ldf, P.d, r.d_pad, r.R.center, r.qn, nullptr, r.qB,
-        kind2 == kTcBf16x3 ? r.qBlo : nullptr);
+        kind2 == kTcBf16x3 ? r.qBlo : nullptr, nullptr, nullptr);
     tc_retry_prep_kernel<<<(nf + 255) / 256, 256, 0, st>>>(
         r.fail, nf, r.retry, r.retry_f, r.retry_s, r.qn, r.R.rmax_bits, run_bound(r, kind2), r.thr,
         r.count);
