@@ -282,6 +282,19 @@ KNN_DI void select_finish(unsigned long long *wl, unsigned long long *wt, unsign
         buf_finish<KCAP>(wl + i * REGION, wt + i, nbuf_get(nb, i), k, lane);
 }
 
+// How many keys more than k a selection may leave: up to KCAP + 32 - k fit beside
+// the next half tile's survivors.  Few make a lower threshold, which later tiles
+// pass less often, for a step or two more of the bisection: with k / 8 + 3, 18783
+// -> 18540 us for a batch of 512 problems (k to 64), 560 -> 536 at 100000 x 4736, d = 5
+// and 894 -> 863 at d = 20 (k = 20), 926 -> 914 at 65536 x 2048, d = 64, k = 200, 609 ->
+// 610.6 at 16384 x 4096, d = 128, k = 16; k / 4 + 4 to k / 3 + 3 give two thirds of that.
+// Lists of 128 keys (100 of them wanted) leave 60 as they did: 9854 us at 131072 x
+// 4736, d = 256, against 9964.
+template <int KCAP>
+KNN_DI int select_slack(int k) {
+    return KCAP == 128 ? KCAP + 32 - k : min(KCAP + 32 - k, k / 8 + 3);
+}
+
 // Filter one half tile (4 reference points per lane) against the thresholds of
 // the queries in hitq and append the survivors to their buffers.  A query
 // whose buffer was selected here is tested again with its new threshold: of a
@@ -324,7 +337,7 @@ KNN_DI void select_half_lb(unsigned long long *wl, unsigned long long *wt,
         for (int i = 0; i < QPW; ++i)
             if ((full_mask >> i) & 1u)
                 nb = nbuf_set(nb, i, buf_select<KCAP>(wl + i * REGION, wt + i, nbuf_get(nb, i), k,
-                                                      KCAP + 32 - k, lane));
+                                                      select_slack<KCAP>(k), lane));
 #pragma unroll
         for (int i = 0; i < QPW; ++i)
             if ((full_mask >> i) & 1u) pm[i] = passing(i);
