@@ -164,7 +164,8 @@ typedef struct knnb200_problem {
 typedef struct knnb200_batched_plan knnb200_batched_plan;
 /* Build a plan: problem table, TMA descriptors and scratch on the current
  * device (this call allocates and synchronises).  item_stages sets the work-
- * item granularity in pipeline stages (<= 0: 256); see the autotuner. */
+ * item granularity in pipeline stages (<= 0: by the size of the batch); see
+ * the autotuner. */
 KNNB200_API int knnb200_batched_plan_create(const knnb200_problem *problems, int count,
                                             int item_stages, knnb200_batched_plan **out);
 /* Queue the plan's work on `stream`: one persistent exact kernel over a
@@ -186,8 +187,8 @@ KNNB200_API void knnb200_graph_destroy(void *graph_exec);
 KNNB200_API int knnb200_batched_autotune(const knnb200_problem *problems, int count,
                                          void *stream, int *best_item_stages, float *best_ms);
 
-/* Plan configuration: the work-item size in pipeline stages (<= 0: 256),
- * the queries per consumer warp of the persistent kernel (its query tile is
+/* Plan configuration: the work-item size in pipeline stages (<= 0: by the
+ * size of the batch), the queries per consumer warp of the persistent kernel (its query tile is
  * 16 x that: 4 -> 64-query tiles, 2 -> 32-query tiles for small query
  * counts; 0: 4, or 2 when some k > 128), and whether problems with dim <= 4
  * and k <= 16 run the low-dimension kernel in launches of their own

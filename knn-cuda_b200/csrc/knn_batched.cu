@@ -333,7 +333,7 @@ long long round_up(long long x, long long m) { return (x + m - 1) / m * m; }
 
 struct knnb200_batched_plan {
     int device = 0, num_sms = 148;
-    int kcap = 32, qpw = 4, item_stages = 256;
+    int kcap = 32, qpw = 4, item_stages = 0;
     int count = 0, n_rows = 0, n_split_probs = 0;   // count: problems of the persistent launch
     std::vector<ExactProblem> lowdim;                // problems routed to the low-d kernel
     long long n_items = 0, n_tasks = 0;
@@ -395,14 +395,12 @@ int knnb200_batched_plan_create_config(const knnb200_problem *all, int n_all,
         cudaGetLastError();
         return KNNB200_ENODEV;
     }
-    const int item_stages = cfg && cfg->item_stages > 0 ? cfg->item_stages : 256;
     const int want_qpw = cfg ? cfg->queries_per_warp : 0;
     if (want_qpw != 0 && want_qpw != 2 && want_qpw != 4) return KNNB200_EINVAL;
     const bool route_lowdim = cfg && cfg->lowdim_kernel;
     knnb200_batched_plan *pl = new knnb200_batched_plan();
     cudaGetDevice(&pl->device);
     cudaDeviceGetAttribute(&pl->num_sms, cudaDevAttrMultiProcessorCount, pl->device);
-    pl->item_stages = item_stages;
     // problem classes: d <= 4, k <= 16 to the low-d kernel (when asked),
     // the rest to the persistent launch
     std::vector<knnb200_problem> persist;
@@ -421,7 +419,26 @@ int knnb200_batched_plan_create_config(const knnb200_problem *all, int n_all,
     pl->qpw = pl->kcap == 256 ? EX_QPW_K256 : (want_qpw ? want_qpw : EX_QPW);
     const int bq = pl->qpw * EX_WARPS;
 
-    // records, cut into items of about `item_stages` pipeline stages
+    // Records, cut into items of about `item_stages` pipeline stages.  Where the
+    // caller leaves the size open it follows from an SM's share of the batch: items
+    // that are a large part of it leave SMs idle at the end, and each warms up and
+    // sorts its lists, which costs about nine stages.  Against 256 stages always:
+    // 814 -> 466 us for 16 problems of 131 stages an SM together, 1374 -> 1121 at 377;
+    // 2824 -> 2785 at 1080, 6051 -> 5865 at 2406, 17636 -> 17060 at 6696 (512 problems).
+    // From 400 to 1000 neither a third nor two fifths is better than 256 throughout
+    // (0.94 to 1.08 of its time over six batches).
+    int item_stages = cfg ? cfg->item_stages : 0;
+    if (item_stages <= 0) {
+        long long share = 0;
+        for (const knnb200_problem &q : persist)
+            share += (long long)((q.ref_nb + EX_BR - 1) / EX_BR) *
+                     ((q.dim + EX_BD - 1) / EX_BD) * ((q.query_nb + bq - 1) / bq);
+        share /= pl->num_sms;
+        item_stages = (int)(share < 400    ? std::max(64ll, share / 3)
+                            : share < 1000 ? 256
+                                           : std::min(2048ll, share * 2 / 5));
+    }
+    pl->item_stages = item_stages;
     std::vector<BatchProb> recs(count);
     std::vector<double> cost(count);
     for (int i = 0; i < count; ++i) {
