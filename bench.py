@@ -442,20 +442,40 @@ def run_ours(args, D: Dist):
     achieved = flops / (pass2_ms * 1e-3) if pass2_ms else None
     peak = peaks["bf16_tflops"] * 1e12
     fb = head["uncertified_queries_per_step"]
-    # reference prep 3 (center, prep, sample rows) + query prep 2 + pass 1 +
-    # threshold + pass 2 + re-rank 3 (select, gather, certify); second scan
-    # 7 more; exact fallback 5 more (gather, query copy, fused kernel, split
-    # merge, scatter)
-    launches = 11 + (7 if fb["second_scan"] > 0 else 0) + (5 if fb["exact"] > 0 else 0)
+    kinds = head.get("scan_kinds", {})
+    if tensor_path:
+        # reference prep 3 (center, prep, sample rows) + query prep + pass 1 +
+        # threshold + pass 2 + re-rank 3 (select, gather, certify); a first scan
+        # in split BF16 adds 4 (the BF16 scan that finds nothing to do, lo
+        # parts, query prep, thresholds); second scan 8 more, and 1 for the lo
+        # parts if only it needs them; exact fallback 4 more (gather, fused
+        # kernel, split merge, scatter)
+        split = kinds.get("pass2") == "bf16x3"
+        launches = 10 + (4 if split else 0) + (4 if fb["exact"] > 0 else 0)
+        if fb["second_scan"] > 0:
+            launches += 8 + (1 if kinds.get("second_scan") == "bf16x3" and not split else 0)
+    else:
+        # the exact kernel and, with splits, the merge (a point-cloud search
+        # launches more)
+        launches = 1 + (1 if knncuda.plan_splits(N, qn, dim, k) > 1 else 0)
     ex = tiers["exact_fp32"]
     ex_ms = ex["phase_ms"].get("exact_main", ex["ms_per_step"])
     fp32_peak = knncuda.measure_fp32_peak(8192)
-    ex["roofline"] = {"bound": "fp32", "kernel": "knn_exact_kernel<4,128> (fused exact FP32)",
-                      "achieved": 3.0 * dim * N * qn / (ex_ms * 1e-3) / 1e12,
-                      "peak": fp32_peak / 1e12, "unit": "TFLOP/s",
-                      "frac": 3.0 * dim * N * qn / (ex_ms * 1e-3) / fp32_peak,
-                      "algorithmic": "3*dim flops per (query, reference) pair",
-                      "peak_source": "FP32 FMA throughput measured in this run"}
+    if dim <= 4:
+        # most pairs are never formed: the bytes that a call cannot do without
+        need = 4.0 * dim * (N + qn) + 8.0 * k * qn
+        ex["roofline"] = {"bound": "latency", "kernel": "sp_search_kernel (points ordered in "
+                          "space, boxes skipped)",
+                          "achieved": need / (ex_ms * 1e-3) / 1e9, "peak": peaks["hbm_gbs"],
+                          "unit": "GB/s", "frac": need / (ex_ms * 1e-3) / 1e9 / peaks["hbm_gbs"],
+                          "algorithmic": "both sets read once, the results written"}
+    else:
+        ex["roofline"] = {"bound": "fp32", "kernel": "knn_exact_kernel<4,128> (fused exact FP32)",
+                          "achieved": 3.0 * dim * N * qn / (ex_ms * 1e-3) / 1e12,
+                          "peak": fp32_peak / 1e12, "unit": "TFLOP/s",
+                          "frac": 3.0 * dim * N * qn / (ex_ms * 1e-3) / fp32_peak,
+                          "algorithmic": "3*dim flops per (query, reference) pair",
+                          "peak_source": "FP32 FMA throughput measured in this run"}
 
     line = {
         "metric": METRIC, "value": head["value"], "unit": UNIT, "n_gpus": D.world,
@@ -468,7 +488,7 @@ def run_ours(args, D: Dist):
                        tier=("bf16_rerank: tcgen05 BF16 scan + exact FP32 re-rank (knn_cublas)"
                              if tensor_path else
                              "bf16_rerank tier (knn_cublas): this shape runs the exact FP32 "
-                             "kernels (tensor path needs 16 <= dim and ref_nb >= 32768)"),
+                             "kernels (tensor path needs 16 <= dim and enough work)"),
                        parallelism=f"query-sharded replicas x{D.world}",
                        l2=l2_note),
         "e2e": {"value": D.world * qn / e2e["bf16_rerank"], "unit": UNIT,

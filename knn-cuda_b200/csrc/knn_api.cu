@@ -649,8 +649,7 @@ int plan_query_chunk(Workspace &ws, int Q, size_t fixed, F per_chunk) {
 
 // The scratch of a call.  Where it has to be allocated anyway and no cap is set,
 // it is taken with the room that the exact kernel can make use of (at most 64 MB
-// more); a call that the held scratch is enough for never allocates, so that
-// what was run once can be captured.
+// more); a call that the held scratch is enough for does not allocate.
 bool ensure_scratch(Workspace &ws, int method, int N, int Q, int d, int k) {
     const size_t need = scratch_for(method, N, Q, d, k, ws.num_sms);
     if (need <= ws.scratch.bytes) return true;
