@@ -56,7 +56,9 @@ KNNB200_API int knnb200_cublas(const float *ref, int ref_nb, const float *query,
 
 /* Device-resident variant of the same computation: every pointer is device
  * memory on the current device, work is queued on `stream` (a cudaStream_t,
- * NULL = legacy default stream) and the call returns without synchronising.
+ * NULL = legacy default stream) and the call returns without synchronising
+ * (but for the expansion methods where they run the tensor path, which waits
+ * for the certification: from 32768 points on, and below where it is faster).
  * It replaces the compute part of the reference host bodies
  * (code/knncuda.cu:352-394 and :709-805) for callers whose data already
  * lives in HBM.  ref_ld / query_ld are row pitches in elements (multiples of
@@ -77,7 +79,7 @@ KNNB200_API int knnb200_knn_device(const float *ref, int ref_nb, long long ref_l
  * outputs are caller-owned device memory as for knnb200_knn_device; the
  * scratch is a static 64 MiB device array inside this library, held on
  * every GPU that loads it until exit.  A call needs the exact path's whole
- * scratch there: the duplicated query copy (dim * round_up(query_nb, 32) * 8
+ * scratch there: room for two query copies (dim * round_up(query_nb, 32) * 8
  * bytes), 256 bytes, and the per-split lists (splits * query_nb *
  * min(k, 256) * 8 bytes when the reference set is split; query_nb * 8 more
  * for k > 256).

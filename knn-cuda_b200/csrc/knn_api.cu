@@ -745,6 +745,7 @@ bool host_entry(int wanted, const float *ref, int ref_nb, const float *query, in
         return false;
     }
     cudaStream_t st = ws->stream;
+    ws->stage_slot = 0;   // small input allocates and keeps no more than it fills
     // The scratch and the status word are shared with the device entry, whose
     // last call may still be running on its caller's stream: this call waits
     // for it, and the next one for this call, however it ends.

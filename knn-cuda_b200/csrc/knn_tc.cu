@@ -17,11 +17,11 @@
 //             FP32 point-major copy of the reference set (for re-ranking),
 //             the reference norm parts, FP32 query norms and the largest
 //             reference norm.
-//   pass 1    tensor scan of a 1/G sample of the reference tiles (runs of
-//             consecutive tiles, one run every G runs' worth); each
-//             epilogue thread keeps the KS smallest a of its query row in
-//             registers -> threshold T_q (KS-th smallest over the sample;
-//             over the full set about KS*G points lie below it).
+//   pass 1    tensor scan of a 1/G sample of the reference set (every G-th
+//             point, or runs of consecutive tiles); each epilogue thread keeps
+//             the KS smallest of the minima of groups of four a of its query
+//             row in registers -> threshold T_q (KS-th smallest over the
+//             sample; over the full set about KS*G points lie below it).
 //   pass 2    tensor scan of all reference tiles; the epilogue emits every
 //             reference with a < T_q into the query's candidate list.
 //   rerank    exact FP32 direct-form distances of the candidates, in the same
@@ -818,8 +818,9 @@ __global__ void __launch_bounds__(256)
 // four warps per tile).  A warp owns 32 points (one per lane) and walks the
 // dimensions in chunks of 32: each lane loads its point's 32 values of the
 // chunk (coalesced rows, the next chunk's loads in flight meanwhile),
-// accumulates its squared norm in increasing d with FP32 fma, and the chunk is transposed through a padded
-// shared tile so that every store writes four points' 128-byte rows.
+// accumulates its squared norm in increasing d with FP32 fma, and the chunk is
+// transposed through a padded shared tile so that every store writes four
+// points' 128-byte rows.
 constexpr int TC_PREP_WARPS = 4;
 constexpr int TC_PREP_LD = 36;   // floats per point row of the transpose tile
 __global__ void __launch_bounds__(32 * TC_PREP_WARPS)
@@ -1167,9 +1168,10 @@ KNN_DI void warp_bitonic_sort(unsigned long long *keys, int P, int lane) {
 
 // Exact FP32 re-rank of each query's candidates + certification, in three
 // kernels of one warp per query: select (tc_rerank_select_kernel: the k-th
-// smallest a by radix selection, the pruning below, the kept candidates
-// compacted in place), gather (tc_rerank_gather_kernel: their exact
-// distances) and certify (tc_rerank_certify_kernel: sort, check, output).
+// smallest a by bisection, the pruning below, the kept candidates compacted
+// in place), gather (tc_rerank_gather_kernel: their exact
+// distances) and certify (tc_rerank_certify_kernel: the k smallest sorted, check,
+// output).
 // The gather, which moves the bytes, then runs with nothing but its staging
 // ring and the query in shared memory, so the SM holds about twice the warps
 // (copies in flight) of one kernel that also keeps the sort keys there.
@@ -1191,9 +1193,8 @@ KNN_DI void warp_bitonic_sort(unsigned long long *keys, int P, int lane) {
 // copies (cp.async, several rows per instruction, coalesced), through a ring
 // of TC_RR_NBUF buffers so the next chunks are in flight while each lane
 // runs its candidate's FMA chain in increasing d -- the fused exact kernel's
-// arithmetic and order, so distances are identical.  The (distance, index)
-// keys are bitonic-sorted by the warp.  One warp per block: the gather is
-// latency-bound, and single-warp blocks let the SM hold as many warps as
+// arithmetic and order, so distances are identical.  One warp per block of the
+// gather: it is latency-bound, and single-warp blocks let the SM hold as many warps as
 // its shared memory allows.
 //
 // An uncertified query is appended to fail_list and retry[q] receives a
@@ -1988,7 +1989,7 @@ bool tc_pays(int N, int Q, int d, int k) {
     // Models in us.  The exact kernel: 13e6 coordinates of pairs a us.  The tensor
     // path: its launches and read-backs, and for each query the selection and
     // the gather of about 1.7 k + 20 rows.  Exact / tensor measured at (points,
-    // queries, dimensions, k): 674 / 206 (16384, 4096, 128, 10), 719 / 354 (16384,
+    // queries, dimensions, k): 609 / 207 (16384, 4096, 128, 16), 719 / 354 (16384,
     // 4096, 128, 100), 389 / 343 (8192, 4096, 128, 100), 649 / 280 (4096, 4096, 512,
     // 10), 2400 / 515 (16384, 16384, 128, 10), 185 / 128 (30000, 1000, 64, 10), 114 /
     // 126 (30000, 200, 128, 10), 813 / 742 (16384, 16384, 16, 100 and 10).  The line
