@@ -814,15 +814,17 @@ __global__ void __launch_bounds__(256)
 // Reference-set prep in one pass over the input: point-major BF16 and FP32
 // copies (zero-padded to d_pad; the BF16 one of x - center, the FP32 one of
 // x itself) plus the norm-step row and the largest squared norm of
-// x - center, for the 256-point tiles tile0 + tiles.tile(u) (two blocks of
+// x - center, for the 256-point tiles tile0 + tiles.tile(u) (2 SPLIT blocks of
 // four warps per tile).  A warp owns 32 points (one per lane) and walks the
-// dimensions in chunks of 32: each lane loads its point's 32 values of the
+// dimensions, or one of SPLIT parts of them (the parts' norms are added in
+// order), in chunks of 32: each lane loads its point's 32 values of the
 // chunk (coalesced rows, the next chunk's loads in flight meanwhile),
 // accumulates its squared norm in increasing d with FP32 fma, and the chunk is
 // transposed through a padded shared tile so that every store writes four
 // points' 128-byte rows.
 constexpr int TC_PREP_WARPS = 4;
 constexpr int TC_PREP_LD = 36;   // floats per point row of the transpose tile
+template <int SPLIT>
 __global__ void __launch_bounds__(32 * TC_PREP_WARPS)
     tc_prep_ref_kernel(const float *__restrict__ x, int n, long long ld, int d, int d_pad,
                        int tile0, TileRuns tiles, const float *__restrict__ center,
@@ -832,20 +834,27 @@ __global__ void __launch_bounds__(32 * TC_PREP_WARPS)
     __shared__ __align__(16) float tile_all[TC_PREP_WARPS][32 * TC_PREP_LD];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float *tt = tile_all[warp];
-    const int p0 = (tile0 + tiles.tile((int)(blockIdx.x >> 1))) * TP_BN +
-                   (int)(blockIdx.x & 1) * (TP_BN / 2) + warp * 32;
+    // a block takes 32 TC_PREP_WARPS / SPLIT points
+    constexpr int BPT = TP_BN / 32 * SPLIT / TC_PREP_WARPS;   // blocks a tile
+    const int part = warp % SPLIT;
+    const int p0 = (tile0 + tiles.tile((int)blockIdx.x / BPT)) * TP_BN +
+                   (int)blockIdx.x % BPT * (TP_BN / BPT) + warp / SPLIT * 32;
     const int p = p0 + lane;       // this lane's point (loads, norm)
     const bool pin = p < n;
     float s = 0.f;                 // squared norm of x_p - c
     float am = 0.f;                // largest |x - c| this lane wrote
+    // this warp's dimensions
+    const int d_lo = SPLIT == 1 ? 0 : d_pad / 32 * part / SPLIT * 32;
+    const int d_hi = SPLIT == 1 ? d_pad : d_pad / 32 * (part + 1) / SPLIT * 32;
     float cur[32], nxt[32];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) cur[j] = (j < d && pin) ? x[(size_t)j * ld + p] : 0.f;
+    for (int j = 0; j < 32; ++j)
+        cur[j] = (d_lo + j < d && pin) ? x[(size_t)(d_lo + j) * ld + p] : 0.f;
     // write-out roles: 8 rounds of 4 points, lane -> point 4 r + lane / 8,
     // dimensions 4 (lane % 8) .. + 3
     const int wp = lane >> 3, wm = lane & 7;
-    for (int d0 = 0; d0 < d_pad; d0 += 32) {
-        if (d0 + 32 < d_pad) {
+    for (int d0 = d_lo; d0 < d_hi; d0 += 32) {
+        if (d0 + 32 < d_hi) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
                 const int dd = d0 + 32 + j;
@@ -887,7 +896,7 @@ __global__ void __launch_bounds__(32 * TC_PREP_WARPS)
             }
         }
         __syncwarp();
-        if (d0 + 32 < d_pad) {
+        if (d0 + 32 < d_hi) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) cur[j] = nxt[j];
         }
@@ -897,6 +906,13 @@ __global__ void __launch_bounds__(32 * TC_PREP_WARPS)
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) ma = max(ma, __shfl_xor_sync(0xffffffffu, ma, o));
         if (lane == 0) atomicMax(absmax_bits, ma);
+    }
+    if constexpr (SPLIT > 1) {
+        __shared__ float sums[TC_PREP_WARPS][32];
+        sums[warp][lane] = s;
+        __syncthreads();
+        if (part) return;
+        for (int i = 1; i < SPLIT; ++i) s += sums[warp + i][lane];
     }
     if (pin) write_norm_row(parts, p, s);
     unsigned m = pin ? __float_as_uint(s) : 0u;
@@ -2064,9 +2080,18 @@ int tc_prepare_ref_tiles(const TcRefView &v, const float *ref, int N, long long 
     if (tiles.units <= 0) return kOk;
     if (tiles.run < 1 || tiles.period < tiles.run) return kErrInvalid;
     const int d_pad = (d + 63) / 64 * 64;
-    tc_prep_ref_kernel<<<tiles.units * 2, 32 * TC_PREP_WARPS, 0, st>>>(
-        ref, N, ldr, d, d_pad, tile0, tiles, v.center, v.refB, v.refT, v.refN, v.rmax_bits,
-        v.absmax_bits);
+    auto go = [&](auto kern, int split) {
+        kern<<<tiles.units * 2 * split, 32 * TC_PREP_WARPS, 0, st>>>(
+            ref, N, ldr, d, d_pad, tile0, tiles, v.center, v.refB, v.refT, v.refN, v.rmax_bits,
+            v.absmax_bits);
+    };
+    // 512 dimensions and more: a block takes a quarter of the points, so that the
+    // blocks of a medium set, four of which an SM holds, do not leave most SMs
+    // idle in their last wave: 188 -> 150 us at 100003 x 768 (782 blocks before), 307
+    // -> 277 at 300000 x 512.  Shorter points give a warp too few chunks to keep
+    // loads in flight: 538 -> 554 at 2^20 x 256 with two parts, 612 with four.
+    if (d_pad >= 512) go(tc_prep_ref_kernel<4>, 4);
+    else go(tc_prep_ref_kernel<1>, 1);
     return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
 
