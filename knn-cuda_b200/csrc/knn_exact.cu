@@ -426,33 +426,31 @@ int launch_split_merge(const unsigned long long *part, int S, int Q, int k, floa
 // the allocation-free entry plan with), 256 bytes of alignment, the per-split
 // key lists of one pass when the reference set is split, and for k > 256 the
 // per-query lower-bound keys of the passes.
-static size_t exact_need(const ExactShape &s, int Q, int d, int k, size_t *part_off,
-                         size_t *lb_off) {
+static size_t exact_need(const ExactShape &s, int Q, int d, int k) {
     const int kp = std::min(k, kPassRanks);
     const size_t dup = (size_t)d * qcopy_pitch(Q) * 2 * sizeof(float);
-    const size_t off = (dup + 255) & ~size_t(255);
     const size_t part = s.splits > 1 ? (size_t)s.splits * Q * kp * 8 : 0;
     const size_t lb = k > kPassRanks ? (size_t)Q * 8 : 0;
-    if (part_off) *part_off = off;
-    if (lb_off) *lb_off = off + part;
-    return std::max(dup + 256, off) + part + lb;
+    return dup + 256 + part + lb;
+}
+
+// Where a call's lists lie in its scratch: after the copy of the queries, if
+// there is one.
+static size_t lists_offset(int Q, int d, bool copied) {
+    return copied ? ((size_t)d * qcopy_pitch(Q) * sizeof(float) + 255) & ~size_t(255) : 0;
 }
 
 size_t exact_scratch_bytes(int N, int Q, int d, int k, int num_sms) {
     if (lowdim_applies(N, Q, d, k)) return lowdim_scratch_bytes(N, Q, d, k, num_sms);
     ExactShape s;
     if (!choose_shape(N, Q, d, k, num_sms, s)) return 0;
-    return exact_need(s, Q, d, k, nullptr, nullptr);
+    return exact_need(s, Q, d, k);
 }
 
-// Scratch of the ranges: their lists, after the copy of the queries if there is
-// one.  The room of the copies holds them in most cases.
-static size_t ranges_need(const ExactShape &s, int Q, int d, int k, bool copied,
-                          size_t *part_off) {
-    const size_t off = copied ? ((size_t)d * qcopy_pitch(Q) * sizeof(float) + 255) & ~size_t(255)
-                              : 0;
-    if (part_off) *part_off = off;
-    return off + (size_t)s.range_lists * Q * k * 8;
+// Scratch of the ranges: their lists, after the copy of the queries.  The room of
+// the copies holds them in most cases.
+static size_t ranges_need(const ExactShape &s, int Q, int d, int k, bool copied) {
+    return lists_offset(Q, d, copied) + (size_t)s.range_lists * Q * k * 8;
 }
 
 size_t exact_scratch_wanted(int N, int Q, int d, int k, int num_sms) {
@@ -460,7 +458,7 @@ size_t exact_scratch_wanted(int N, int Q, int d, int k, int num_sms) {
     ExactShape s;
     if (lowdim_applies(N, Q, d, k) || !choose_shape(N, Q, d, k, num_sms, s) || !s.ranges.ctas)
         return need;
-    const size_t want = ranges_need(s, Q, d, k, true, nullptr);
+    const size_t want = ranges_need(s, Q, d, k, true);
     return want > need + (size_t(64) << 20) ? need : std::max(need, want);
 }
 
@@ -471,20 +469,27 @@ int launch_exact(const ExactProblem &p, cudaStream_t st) {
     ExactShape s;
     if (!choose_shape(p.N, p.Q, p.d, p.k, p.num_sms, s)) return kErrUnsupported;
     if (p.force_splits > 0) s.splits = std::min(p.force_splits, std::min(s.n_rtiles, 256));
-    size_t part_off = 0, lb_off = 0;
-    if (exact_need(s, p.Q, p.d, p.k, &part_off, &lb_off) > p.scratch_bytes) return kErrScratch;
     const bool copied = (reinterpret_cast<uintptr_t>(p.qry) & 15) || p.ldq % 4;
+    const size_t part_off = lists_offset(p.Q, p.d, copied);
+    const size_t lb_bytes = p.k > kPassRanks ? (size_t)p.Q * 8 : 0;
+    if (part_off + lb_bytes > p.scratch_bytes) return kErrScratch;
+    // not where the split is given, or the scratch has no room for the lists
+    if (s.ranges.ctas &&
+        (p.force_splits > 0 || ranges_need(s, p.Q, p.d, p.k, copied) > p.scratch_bytes))
+        s.ranges = TileRanges();
     if (s.ranges.ctas) {
-        // not where the split is given, or the scratch has no room for the lists
-        size_t off = 0;
-        if (p.force_splits > 0 ||
-            ranges_need(s, p.Q, p.d, p.k, copied, &off) > p.scratch_bytes) {
-            s.ranges = TileRanges();
-        } else {
-            s.splits = s.range_lists;
-            part_off = off;
-        }
+        s.splits = s.range_lists;
+    } else {
+        // as many splits as the scratch holds lists of: it may have been sized for
+        // more queries than these (the last chunk of a call, the queries that the
+        // tensor path leaves over), whose plan has fewer
+        const size_t per_split = (size_t)p.Q * std::min(p.k, kPassRanks) * 8;
+        const size_t fit = (p.scratch_bytes - part_off - lb_bytes) / per_split;
+        s.splits = (int)std::min<size_t>(s.splits, std::max<size_t>(1, fit));
     }
+    const size_t lb_off = part_off + (s.splits > 1 ? (size_t)s.splits * p.Q *
+                                                         std::min(p.k, kPassRanks) * 8
+                                                   : 0);
     unsigned char *sb = static_cast<unsigned char *>(p.scratch);
     unsigned long long *part = reinterpret_cast<unsigned long long *>(sb + part_off);
     unsigned long long *lb = reinterpret_cast<unsigned long long *>(sb + lb_off);

@@ -2670,10 +2670,6 @@ int tc_run_finish(TcRun &r, cudaStream_t st, int *host_stats) {
             if (cudaGetLastError() != cudaSuccess) return kErrLaunch;
         }
         const int nx = narrow ? nf2 : nf;
-        const long long per_split = (long long)nx * std::min(P.k, 256) * 8;
-        const int splits = (int)std::max<long long>(
-            1, std::min<long long>(exact_plan_splits(P.N, nx, P.d, P.k, P.num_sms),
-                                   (long long)(r.xcap / per_split)));
         ExactProblem x;
         x.ref = P.ref;
         x.N = P.N;
@@ -2690,7 +2686,8 @@ int tc_run_finish(TcRun &r, cudaStream_t st, int *host_stats) {
         x.scratch_bytes = r.xcap;
         x.status = P.status;
         x.num_sms = P.num_sms;
-        x.force_splits = splits;
+        // (lowered where the scratch does not hold that many lists)
+        x.force_splits = exact_plan_splits(P.N, nx, P.d, P.k, P.num_sms);
         x.timer = nullptr;
         if ((rc = launch_exact(x, st)) != kOk) return rc;
         if (narrow) {
