@@ -242,8 +242,10 @@ int launch_lowdim(const ExactProblem &p, cudaStream_t st) {
         s.wpq = 1;
         s.splits = s.max_splits;
     }
-    const size_t need = s.splits > 1 ? (size_t)s.splits * p.Q * p.k * 8 : 0;
-    if (need > p.scratch_bytes) return kErrScratch;
+    // as many splits as the scratch holds lists of (it may have been sized for the
+    // larger first chunk of a call, whose plan has fewer)
+    s.splits = (int)std::min<size_t>(
+        s.splits, std::max<size_t>(1, p.scratch_bytes / ((size_t)p.Q * p.k * 8)));
     unsigned long long *part = static_cast<unsigned long long *>(p.scratch);
     cudaError_t e;
     switch (p.d) {

@@ -55,3 +55,22 @@ def test_small_last_chunk_under_a_memory_cap(knncuda, gpu, k, last):
         knncuda.set_memory_cap(0)
     assert np.array_equal(d.view(np.uint32), want_d.view(np.uint32))
     assert np.array_equal(i, want_i)
+
+
+@pytest.mark.parametrize("n,dim,chunk,last", [(9385, 4, 237568, 2), (7955, 4, 232704, 67),
+                                              (7970, 3, 302592, 38)])
+def test_small_last_chunk_of_a_point_cloud(knncuda, gpu, n, dim, chunk, last):
+    """The large chunk needs no lists at all, the last one would like two a query."""
+    k, q = 1, chunk + last
+    rng = np.random.default_rng(last)
+    ref, query = rng.random((dim, n), dtype=np.float32), rng.random((dim, q), dtype=np.float32)
+    want_d, want_i = knncuda.knn(ref, query, k, "global")
+    knncuda.lib().knnb200_release_workspace()
+    knncuda.set_memory_cap(knncuda.call_bytes(n, chunk, dim, k, "global", host=True))
+    try:
+        d, i = knncuda.knn(ref, query, k, "global")
+        assert knncuda.last_query_chunks() == 2
+    finally:
+        knncuda.set_memory_cap(0)
+    assert np.array_equal(d.view(np.uint32), want_d.view(np.uint32))
+    assert np.array_equal(i, want_i)
