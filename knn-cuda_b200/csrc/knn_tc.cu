@@ -2137,7 +2137,8 @@ int ensure_ref_lo(const TcRun &r, cudaStream_t st) {
     return kOk;
 }
 
-// The FP8 scales of the reference set, once per prepared set: reads back
+// The FP8 scales of the reference set, once per prepared set (kErrUnsupported: it
+// has none -- all points are their mean, some coordinate is not finite): reads back
 // the set's largest |r - c| and ||r - c||^2 (one synchronisation) for the
 // scale s_r = 2^floor(log2(448 / max|r - c|)) and the norm-step unit
 // kappa = 2^ceil(log2(s_r max||r - c||^2 / 896)) (so the norm needs at most
@@ -2159,6 +2160,7 @@ int ensure_ref_f8_scale(const TcRun &r, cudaStream_t st, unsigned *host_tmp) {
     s->r2max = r2;
     s->s_r = pow2_floor(448.0 / am);
     s->kappa = pow2_ceil(std::max(1e-30, (double)s->s_r * r2 / 896.0));
+    if (!std::isfinite(s->s_r) || !std::isfinite(s->kappa)) return kErrUnsupported;
     s->resid8 = 0.f;
     s->f8_scaled = true;
     return kOk;
@@ -2345,7 +2347,7 @@ int rerank(const TcRun &r, cudaStream_t st, int kind, int Q, int cmax, const flo
 
 // FP8 query scale (reads back the batch's largest |q - c|): s_q =
 // 2^floor(log2(min(224 / max|q - c|, 256 / kappa))), so that -2 s_q q and
-// the ones value c1 = s_q kappa both fit e4m3.
+// the ones value c1 = s_q kappa both fit e4m3 (kErrUnsupported: none does).
 int fp8_query_scale(TcRun &r, cudaStream_t st, unsigned *dev_absmax, unsigned *host_tmp) {
     if (cudaMemcpyAsync(host_tmp, dev_absmax, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
@@ -2357,6 +2359,7 @@ int fp8_query_scale(TcRun &r, cudaStream_t st, unsigned *dev_absmax, unsigned *h
     r.s_q = pow2_floor(lim);
     const double c1 = (double)r.s_q * s->kappa;
     if (!(c1 >= 1.0 / 512.0) || !std::isfinite(aq)) return kErrUnsupported;
+    if (!std::isfinite(r.s_q * s->s_r)) return kErrUnsupported;
     r.scale = r.s_q * s->s_r;
     return kOk;
 }
@@ -2437,8 +2440,9 @@ int tc_run_begin(const TcProblem &P, const TcRefView &R, cudaStream_t st, TcRun 
         unsigned *host_tmp = reinterpret_cast<unsigned *>(P.host_tmp);
         int rc = ensure_ref_f8_scale(r, st, host_tmp);
         if (rc == kOk) rc = fp8_query_scale(r, st, reinterpret_cast<unsigned *>(r.nwide + 2), host_tmp);
-        if (rc != kOk) return rc;
-        r.want_fp8 = true;
+        // where the data has no FP8 scale the request goes on as a BF16 one
+        if (rc != kOk && rc != kErrUnsupported) return rc;
+        r.want_fp8 = rc == kOk;
     }
     if (P.timer) P.timer->mark(st, kPhaseTcPrepQuery);
     return kOk;
@@ -2712,7 +2716,9 @@ int tc_prepare_extras(const TcRefView &v, int N, int d, cudaStream_t st, int *ho
     r.d_pad = (d + 63) / 64 * 64;
     r.d_pad8 = (d + 127) / 128 * 128;
     int rc = v.refBlo ? ensure_ref_lo(r, st) : kOk;
+    // (a set without an FP8 scale, one of equal points say, goes without that copy)
     if (rc == kOk && v.ref8) rc = ensure_ref_f8(r, st, reinterpret_cast<unsigned *>(host_tmp));
+    if (rc == kErrUnsupported) rc = kOk;
     if (rc == kOk && cudaStreamSynchronize(st) != cudaSuccess) rc = kErrCuda;
     return rc;
 }
