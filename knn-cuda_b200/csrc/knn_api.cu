@@ -295,7 +295,12 @@ bool valid_sizes(int ref_nb, int query_nb, int dim, int k) {
 // all its query chunks.
 int route(int method, int N, int Q, int d, int k) {
     if (method != KNNB200_METHOD_CUBLAS && method != KNNB200_METHOD_FP8) return method;
-    return tc_pays(N, Q, d, k) ? method : KNNB200_METHOD_GLOBAL;
+    if (!tc_pays(N, Q, d, k)) return KNNB200_METHOD_GLOBAL;
+    // Small sets run in BF16: an FP8 scan takes little less there, its set-up reads
+    // two scales back, and the candidates within its wider bound can overflow the
+    // lists: 257 us against 224 at 16384 x 4096, d = 128, k = 16, uniform data, 1631
+    // against 223 on 256 clusters (the exact kernel 609).
+    return N < kTcAlwaysPoints ? KNNB200_METHOD_CUBLAS : method;
 }
 
 // Whether a routed method runs the tensor path.

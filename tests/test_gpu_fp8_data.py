@@ -47,3 +47,25 @@ def test_fp8_request(knncuda, gpu, size, kind):
     finally:
         rs.close()
     assert torch.equal(d.view(torch.int32), wd.view(torch.int32)) and torch.equal(i, wi)
+
+
+@pytest.mark.parametrize("n,q,dim,k", [(16384, 4096, 128, 16), (32767, 2000, 64, 10)])
+def test_small_sets_are_not_scanned_in_fp8(knncuda, gpu, n, q, dim, k):
+    """Clusters whose candidates FP8's error bound does not tell apart."""
+    import torch
+
+    g = torch.Generator(device=gpu)
+    g.manual_seed(n)
+    centres = torch.randn((dim, 256), device=gpu, generator=g)
+    centres /= centres.norm(dim=0, keepdim=True)
+
+    def points(m):
+        of = torch.randint(256, (32768,), device=gpu, generator=g)
+        noise = torch.randn((dim, 32768), device=gpu, generator=g)
+        return (centres[:, of] + 0.05 * noise)[:, :m]
+
+    r, x = points(n), points(q)
+    d, i = knncuda.knn_device(r, x, k, "fp8")
+    assert knncuda.last_tc_kinds()[0] == "bf16"
+    wd, wi = knncuda.knn_device(r, x, k, "global")
+    assert torch.equal(d, wd) and torch.equal(i, wi)
