@@ -357,6 +357,9 @@ int enqueue(Workspace &ws, const ExactProblem &p0, int method, cudaStream_t st,
     t.point_sample = true;   // the whole set is prepared before pass 1
     t.probe_event = ws.probe;
     t.clear_status = !ref_prepared;   // with the first chunk
+    // (small sets took the exact kernel before: data that defeats the lists costs
+    // them no more than the sample)
+    t.may_leave = p.N < kTcAlwaysPoints;
     if (ws.bound_check) {
         if (cudaMemsetAsync(ws.bound.ptr, 0, 16, st) != cudaSuccess) return kErrCuda;
         t.bound_stat = static_cast<unsigned *>(ws.bound.ptr);

@@ -247,6 +247,10 @@ struct TcProblem {
     // counters, [1] whether nothing was queued after that
     int *host_status = nullptr;
     bool clear_status = false;   // the run clears the status word itself
+    // launch_tc may hand the whole call to the exact kernel after the threshold
+    // sample, where too many queries' lists are predicted to overflow in every
+    // scan (needs probe_event and point_sample)
+    bool may_leave = false;
 };
 
 // A sample of the 256-point tiles: `run` consecutive tiles out of every
@@ -311,12 +315,16 @@ struct TcRun {
     float *qn, *thr, *thr_raw, *retry, *retry_f, *retry_s, *p1, *qsub, *sd;
     // control words, cleared together at the start: nfail [0] uncertified
     // queries, [1] overflowing lists; cand_total; nwide [0], [1] predicted
-    // overflows, [2] query max |q - c| bits.  The first four are read back
-    // together.
+    // overflows, [2] query max |q - c| bits (FP8) or lost queries (may_leave).
+    // The first four are read back together.
     int *ctl;
     int *count, *fail, *fail2, *nfail, *si, *nwide, *nsel;
     unsigned long long *cand_total, *cand;
     bool undecided;         // the overflow prediction is on its way (probe_event)
+    bool may_switch;        // ... and may switch the run to split BF16
+    bool may_leave;         // ... or end it (TcProblem::may_leave)
+    int lost;               // queries predicted to overflow every scan, where the
+                            // run ended for that reason (else 0)
     unsigned char *xs;
     size_t xcap;
     // incremental re-rank (tc_run_rerank_piece): running k smallest exact
@@ -362,7 +370,10 @@ int tc_prepare_extras(const TcRefView &v, int N, int d, cudaStream_t st, int *ho
 // scratch, [4..5] total first-scan candidates (64-bit), [6] kind of the
 // first scan's pass 2, [7] kind of the second scan (-1: none); kinds are
 // 0 BF16, 1 split BF16, 2 FP8 (an FP8 request whose BF16 sample pass
-// predicts overflowing FP8 lists runs BF16 and reports that).
+// predicts overflowing FP8 lists runs BF16 and reports that).  A call handed to
+// the exact kernel after the sample (may_leave) reports [0] 0, [1] all queries,
+// [4..5] the candidates that the lost queries would have had, at least, and no
+// kinds.
 int launch_tc(const TcProblem &P, const TcRefView &R, cudaStream_t st, int *host_stats);
 
 }  // namespace knnb200

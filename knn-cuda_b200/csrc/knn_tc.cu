@@ -299,7 +299,15 @@ struct TpArgs {
     int *status;
     const int *n_wide;      // queries predicted to overflow: the scan does nothing
                             // when they are more than half (nullptr: always runs)
+    const int *n_lost;      // likewise when these are too many (too_many_lost)
 };
+
+// Whether a call is better handed to the exact kernel as a whole, given the
+// queries whose lists will overflow every scan (tc_threshold_kernel).  A lost query
+// costs an emission of whole tiles into its list, a second scan and the exact
+// kernel: constant data took 2201 us at 16384 x 4096 x 128 where the exact kernel
+// takes 609.
+__host__ __device__ inline bool too_many_lost(int n_lost, int Q) { return n_lost > Q / 8; }
 
 // Norm step and one ring item's MMAs for each kind, issued by the even
 // CTA's MMA thread.  K steps advance the descriptors by 32 bytes (2 in
@@ -348,6 +356,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
 
     // (both CTAs of a pair read the same word: they leave together)
     if (a.n_wide && 2 * *a.n_wide > a.Q) return;
+    if (a.n_lost && too_many_lost(*a.n_lost, a.Q)) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const bool lead = rank == 0;
@@ -708,8 +717,8 @@ KNN_DI void write_norm_row(__nv_bfloat16 *parts, int p, float s) {
 constexpr int TC_QP_WARPS = 8;
 // Counters of a run: [0] uncertified queries, [1] those with an overflowing list,
 // [2..3] candidates (64-bit), [4..5] predicted overflows (BF16, FP8), [6] the
-// queries' largest coordinate (float bits, FP8), [7] the
-// certification's ticket (last_block)
+// queries' largest coordinate (float bits, FP8) or the lost queries
+// (tc_threshold_kernel), [7] the certification's ticket (last_block)
 constexpr int TC_CTL = 8;
 __global__ void __launch_bounds__(32 * TC_QP_WARPS, 3)
     tc_prep_query_kernel(const float *__restrict__ x, int n, long long ld, int d, int d_pad,
@@ -1074,19 +1083,29 @@ KNN_DI bool last_block(int *ticket) {
 // switch to split BF16), n_wide[1] for probe1 (FP8: whether an FP8 pass 2
 // pays).  With host_wide (pinned) only n_wide[0] is wanted: the last block writes
 // it there.
+// With lost.count also counts, for host_wide[1], the queries whose list will
+// overflow the second scan too, as far as the sample shows: those where E_q under
+// the finest kind's bound is wider than [L_0, T] and either lost.near of the values
+// in the lists (or all, where they hold fewer) are within T + E_q, or some list's
+// last one is within T (a run of equal points: its further ones are not known).
 // One warp per query: the lists' values pass through a sorted list of KS keys
 // that lies across its lanes (one thread per query read the up to 148 lists of
 // a small batch one after the other: 33 us at 13 queries, now 6.7).
 constexpr int TC_THR_WARPS = 4;
+struct TcLost {
+    int *count = nullptr;
+    int near = 0;
+    TcBound bound = {0.f, 0.f, 0.f, 0.f, 0.f};
+};
 __global__ void __launch_bounds__(32 * TC_THR_WARPS)
     tc_threshold_kernel(const float *__restrict__ p1, int S, int Q, const float *__restrict__ qn,
                         const unsigned *__restrict__ rmax_bits, TcBound bound, TcBound probe0,
                         TcBound probe1, float *__restrict__ thr, float *__restrict__ thr_raw,
                         int *__restrict__ count, int *__restrict__ n_wide,
-                        volatile int *__restrict__ host_wide) {
+                        volatile int *__restrict__ host_wide, TcLost lost) {
     const int lane = threadIdx.x & 31;
     const int q = blockIdx.x * TC_THR_WARPS + (threadIdx.x >> 5);
-    bool wide0 = false, wide1 = false;
+    bool wide0 = false, wide1 = false, is_lost = false;
     if (q < Q) {
         unsigned long long mine = kKeyInf, tau = kKeyInf;
         auto key_of = [&](int s, int i) {
@@ -1131,15 +1150,42 @@ __global__ void __launch_bounds__(32 * TC_THR_WARPS)
             wide0 = tc_error_bound(qn[q], r2, T, probe0) > spread;
             wide1 = tc_error_bound(qn[q], r2, T, probe1) > spread;
         }
+        if (lost.count) {
+            // (comparisons that fail for NaN count the query as lost)
+            const float E = tc_error_bound(qn[q], __uint_as_float(*rmax_bits), T, lost.bound);
+            if (!(E < T - L0)) {
+                int near = 0;
+                bool full = false;
+                for (int t = lane; t < S * TC_KS; t += 32) {
+                    const float v = p1[((size_t)(t / TC_KS) * Q + q) * TC_KS + t % TC_KS];
+                    near += !(v > T + E) ? 1 : 0;
+                    full = full || (!(v > T) && t % TC_KS == TC_KS - 1);
+                }
+                near = (int)__reduce_add_sync(0xffffffffu, (unsigned)near);
+                is_lost = (near >= min(lost.near, S * TC_KS) ||
+                           __any_sync(0xffffffffu, full)) && lane == 0;
+            }
+        }
     }
     if (n_wide) {
         const int n0 = __syncthreads_count(wide0), n1 = __syncthreads_count(wide1);
+        const int nl = lost.count ? __syncthreads_count(is_lost) : 0;
         if (threadIdx.x == 0 && host_wide) {
+            if (nl) {
+                atomicAdd(lost.count, nl);
+                __threadfence();   // before this block's arrival
+            }
             // the blocks that have arrived count in the word above
             const unsigned long long all =
                 atomicAdd(reinterpret_cast<unsigned long long *>(n_wide),
                           (1ull << 32) | (unsigned)n0);
-            if ((unsigned)(all >> 32) == gridDim.x - 1) host_wide[0] = (int)(uint32_t)all + n0;
+            if ((unsigned)(all >> 32) == gridDim.x - 1) {
+                host_wide[0] = (int)(uint32_t)all + n0;
+                if (lost.count) {
+                    __threadfence();
+                    host_wide[1] = __ldcg(lost.count);
+                }
+            }
         } else if (threadIdx.x == 0) {
             if (n0) atomicAdd(n_wide, n0);
             if (n1) atomicAdd(n_wide + 1, n1);
@@ -2196,7 +2242,7 @@ template <int MODE>
 int launch_scan(const TcRun &r, cudaStream_t st, int kind, const __nv_bfloat16 *qB,
                 const __nv_bfloat16 *qBlo, const unsigned char *q8, int Q, const float *thr,
                 int cmax, int tile_base, const TileRuns &tiles, int n_splits,
-                const int *n_wide = nullptr) {
+                const int *n_wide = nullptr, const int *n_lost = nullptr) {
     const TcProblem &P = r.P;
     if (!kind_fits(kind, r.d_pad, r.d_pad8)) return kErrUnsupported;
     const TcOp op = tc_op(kind, r.d_pad, r.d_pad8);
@@ -2258,6 +2304,7 @@ int launch_scan(const TcRun &r, cudaStream_t st, int kind, const __nv_bfloat16 *
     a.cmax = cmax;
     a.status = P.status;
     a.n_wide = n_wide;
+    a.n_lost = n_lost;
     const dim3 grid(2 * ((Q + TC_QT - 1) / TC_QT), n_splits);
     auto go = [&](auto kern) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2275,7 +2322,7 @@ int launch_scan(const TcRun &r, cudaStream_t st, int kind, const __nv_bfloat16 *
 
 // Emission scan of the reference tiles [tb, te).
 int emit_scan(const TcRun &r, cudaStream_t st, int kind, int Q, const float *thr, int cmax,
-              int tb, int te, const int *n_wide = nullptr) {
+              int tb, int te, const int *n_wide = nullptr, const int *n_lost = nullptr) {
     const int qtiles = (Q + TC_QT - 1) / TC_QT;
     // reference bytes a tile streams (operand rows + norm-step rows); a
     // split holds at most kSplitBytes of them: measured at 2^20 x 256 BF16
@@ -2290,7 +2337,7 @@ int emit_scan(const TcRun &r, cudaStream_t st, int kind, int Q, const float *thr
     const int splits =
         choose_splits(qtiles, te - tb, 2, 2.0, std::max(1, r.P.num_sms / 2), max_tiles);
     return launch_scan<1>(r, st, kind, r.qB, r.qBlo, r.q8, Q, thr, cmax, tb,
-                          contiguous_tiles(te - tb), splits, n_wide);
+                          contiguous_tiles(te - tb), splits, n_wide, n_lost);
 }
 
 TcBound run_bound(const TcRun &r, int kind) {
@@ -2409,7 +2456,8 @@ int tc_run_begin(const TcProblem &P, const TcRefView &R, cudaStream_t st, TcRun 
     r.nfail = r.ctl;
     r.cand_total = reinterpret_cast<unsigned long long *>(r.ctl + 2);
     r.nwide = r.ctl + 4;
-    r.undecided = false;
+    r.undecided = r.may_switch = r.may_leave = false;
+    r.lost = 0;
     r.p1 = cv.take<float>((size_t)TP_LISTS * p.splits1 * P.Q * TC_KS);
     r.cand = cv.take<unsigned long long>((size_t)P.Q * p.cmax);
     r.ldf = (P.Q + 3) / 4 * 4;   // second-chance buffers, sized for all queries
@@ -2479,15 +2527,26 @@ int tc_run_pass1(TcRun &r, cudaStream_t st) {
     const int force = P.force_kind;
     const bool forced = (force == kTcBf16) || (force == kTcBf16x3 && lo_ok) ||
                         (force == kTcFp8 && r.want_fp8);
-    const bool probe = !forced && P.host_tmp && ((P.adaptive && lo_ok) || r.want_fp8);
+    r.may_leave = !forced && P.may_leave && P.probe_event && r.p1_every > 0 &&
+                  P.request == kTcReqBf16;
+    const bool probe =
+        !forced && P.host_tmp && ((P.adaptive && lo_ok) || r.want_fp8 || r.may_leave);
     // BF16 unless most lists would overflow: launch_tc queues the BF16 scan,
     // which looks at the count itself, before the host knows it
     const bool undecided = probe && P.probe_event && !r.want_fp8;
+    r.may_switch = P.adaptive && lo_ok;
     const TcBound b16 = run_bound(r, kTcBf16);
+    TcLost lost;
+    if (r.may_leave) {
+        const int every = TC_SAMPLE_EVERY * r.p1_every;   // points a sample row stands for
+        lost.count = r.nwide + 2;
+        lost.near = (r.cmax + every - 1) / every;
+        lost.bound = lo_ok ? run_bound(r, kTcBf16x3) : b16;
+    }
     tc_threshold_kernel<<<(P.Q + TC_THR_WARPS - 1) / TC_THR_WARPS, 32 * TC_THR_WARPS, 0, st>>>(
         r.p1, TP_LISTS * r.splits1, P.Q, r.qn, r.R.rmax_bits, b16, b16,
         r.want_fp8 ? run_bound(r, kTcFp8) : b16, r.thr, r.thr_raw, r.count,
-        probe ? r.nwide : nullptr, undecided ? P.host_tmp : nullptr);
+        probe ? r.nwide : nullptr, undecided ? P.host_tmp : nullptr, lost);
     if (cudaGetLastError() != cudaSuccess) return kErrLaunch;
     r.kind = kTcBf16;
     int wide16 = 0, wide8 = 0;
@@ -2533,11 +2592,16 @@ int tc_run_pass2(TcRun &r, int tile_begin, int tile_end, cudaStream_t st) {
     int rc = kOk;
     if (r.undecided) {
         // the host's wait for the prediction hides behind this scan
-        rc = emit_scan(r, st, r.kind, r.P.Q, r.thr, r.cmax, tile_begin, tile_end, r.nwide);
+        rc = emit_scan(r, st, r.kind, r.P.Q, r.thr, r.cmax, tile_begin, tile_end,
+                       r.may_switch ? r.nwide : nullptr, r.may_leave ? r.nwide + 2 : nullptr);
         if (rc != kOk) return rc;
         if (cudaEventSynchronize(r.P.probe_event) != cudaSuccess) return kErrCuda;
         r.undecided = false;
-        const bool wide = 2 * (long long)r.P.host_tmp[0] > r.P.Q;
+        if (r.may_leave && too_many_lost(r.P.host_tmp[1], r.P.Q)) {
+            r.lost = r.P.host_tmp[1];
+            return kOk;
+        }
+        const bool wide = r.may_switch && 2 * (long long)r.P.host_tmp[0] > r.P.Q;
         if (!wide || (rc = switch_to_split(r, st)) != kOk) {
             if (rc == kOk && r.P.timer) r.P.timer->mark(st, kPhaseTcPass2);
             return rc;
@@ -2723,6 +2787,37 @@ int tc_prepare_extras(const TcRefView &v, int N, int d, cudaStream_t st, int *ho
     return rc;
 }
 
+// The whole call by the exact kernel, after the sample (may_leave): the scratch,
+// which includes the exact kernel's for all queries, is free again.
+static int leave_tc(const TcRun &r, cudaStream_t st, int *host_stats) {
+    const TcProblem &P = r.P;
+    ExactProblem x;
+    x.ref = P.ref;
+    x.N = P.N;
+    x.ldr = P.ldr;
+    x.qry = P.qry;
+    x.Q = P.Q;
+    x.ldq = P.ldq;
+    x.d = P.d;
+    x.k = P.k;
+    x.out_dist = P.out_dist;
+    x.out_idx = P.out_idx;
+    x.ld_out = P.ld_out;
+    x.scratch = P.scratch;
+    x.scratch_bytes = P.scratch_bytes;
+    x.status = P.status;
+    x.num_sms = P.num_sms;
+    x.force_splits = 0;
+    x.timer = P.timer;
+    const long long candidates = (long long)r.lost * r.cmax;
+    std::memcpy(host_stats + 4, &candidates, sizeof(candidates));
+    host_stats[0] = 0;
+    host_stats[1] = P.Q;
+    host_stats[6] = host_stats[7] = -1;
+    if (P.host_status) P.host_status[1] = 0;
+    return launch_exact(x, st);
+}
+
 int launch_tc(const TcProblem &P, const TcRefView &R, cudaStream_t st, int *host_stats) {
     TcRun r;
     TcProblem p = P;
@@ -2730,6 +2825,7 @@ int launch_tc(const TcProblem &P, const TcRefView &R, cudaStream_t st, int *host
     int rc = tc_run_begin(p, R, st, r);
     if (rc == kOk) rc = tc_run_pass1(r, st);
     if (rc == kOk) rc = tc_run_pass2(r, 0, r.n_tiles2, st);
+    if (rc == kOk && r.lost) return leave_tc(r, st, host_stats);
     if (rc == kOk) rc = tc_run_finish(r, st, host_stats);
     return rc;
 }
