@@ -49,6 +49,7 @@ __global__ void __launch_bounds__(32 * LD_WARPS)
                       unsigned long long *__restrict__ part, QuerySubset subset) {
     constexpr int GROUPS = LD_WARPS / WPQ, QPB = GROUPS * QPW;
     __shared__ unsigned long long lists[LD_WARPS][QPW][32], merged[GROUPS][QPW][32];
+    __shared__ unsigned long long keys[LD_WARPS][LD_STEP];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int group = warp / WPQ;
     // with a subset: its queries, and the blocks loop over the (query block,
@@ -116,10 +117,8 @@ __global__ void __launch_bounds__(32 * LD_WARPS)
                 const float m = fminf(fminf(d4[0], d4[1]), fminf(d4[2], d4[3]));
                 // (strictly: a step's indices are above all earlier ones)
                 if (!__any_sync(0xffffffffu, m < key_dist2(tau[i]))) continue;
-                const uint32_t idx = (uint32_t)(s * LD_STEP + lane * 4);
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    lane_list_add(mine[i], tau[i], finite_key(d4[j], idx + j), k, lane);
+                lane_list_add4(mine[i], tau[i], d4, m, (uint32_t)(s * LD_STEP + lane * 4), k,
+                               lane, keys[warp]);
             }
         }
         if (WPQ > 1) {
@@ -183,13 +182,27 @@ bool lowdim_shape(int N, int Q, int d, int k, int num_sms, LowdimShape &s) {
         }
     }
     s.max_splits = best;
-    // four queries a warp share its loads where that still leaves every SM
-    // its warps; few queries take a whole block each
-    const int want = num_sms * 24;   // warps that keep the GPU busy
-    s.qpw = Q >= 4 * want ? 4 : 1;
-    s.wpq = Q < want ? LD_WARPS : 1;
+    // Few queries take a whole block each.  More queries to a warp share its loads,
+    // but the code that adds to their lists no longer fits the instruction cache
+    // with four: that pays only where few points enter a list, in large problems (at
+    // d = 3, k = 8, two / four queries a warp: 1074 / 1153 us at 8000 x 200000, 185 /
+    // 216 at 16384 x 14000, 506 / 488 at 65536 x 14000, 1768 / 1477 at 262144 x 14000;
+    // one: 2418 there, 45 / 46 with two at 4000 x 4000).
+    const int want = num_sms * 48;   // warps that keep the GPU busy
+    s.wpq = 1;
+    if (Q < 300 || (Q < 1200 && N < 131072)) {
+        s.qpw = 1;
+        if (N >= 1000) s.wpq = LD_WARPS;
+    } else if (N < 32768) {
+        s.qpw = Q < 5000 ? 1 : 2;
+    } else {
+        s.qpw = (double)N * Q >= 1e9 ? 4 : 2;
+    }
+    // splits of 8192 points and more: each starts its lists anew
     const long long warps = ((long long)Q + s.qpw - 1) / s.qpw * s.wpq;
-    s.splits = (int)std::min<long long>(s.max_splits, std::max<long long>(1, 2 * want / warps));
+    const long long fill = s.wpq > 1 ? want / 2 / warps : (want + warps - 1) / warps;
+    s.splits = (int)std::max<long long>(
+        1, std::min({(long long)s.max_splits, fill, (long long)N / 8192}));
     return true;
 }
 
@@ -207,6 +220,7 @@ cudaError_t launch_ld(const ExactProblem &p, const LowdimShape &s, unsigned long
     };
     if (s.wpq > 1) return go(knn_lowdim_kernel<D, 1, LD_WARPS>, 1);
     if (s.qpw == 4) return go(knn_lowdim_kernel<D, 4, 1>, 4 * LD_WARPS);
+    if (s.qpw == 2) return go(knn_lowdim_kernel<D, 2, 1>, 2 * LD_WARPS);
     return go(knn_lowdim_kernel<D, 1, 1>, LD_WARPS);
 }
 
