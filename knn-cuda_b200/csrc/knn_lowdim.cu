@@ -23,10 +23,15 @@
 // the GPU idle at smaller sizes: 244 -> 126 us at 1000 x 50000, d = 1, k = 8; 855 ->
 // 79 at 7000 x 7000, d = 3, k = 16; 438 -> 71 at 2^20 x 50, d = 1, k = 8.
 //
+// Many queries against few points run one thread a pair of queries
+// (knn_lowdim_thread_kernel): a warp's list costs it the same few thousand cycles
+// a query however few the points are.
+//
 // Large clouds are searched in space (knn_space.cu) where the caller has the
 // scratch for it; this kernel then answers the few queries that search leaves
 // over.
 #include <algorithm>
+#include <cmath>
 
 #include "knn_exact_core.cuh"
 #include "knn_kernels.h"
@@ -155,13 +160,133 @@ __global__ void __launch_bounds__(32 * LD_WARPS)
     }
 }
 
+// Every thread holds two queries (packed for sub.f32x2 / fma.f32x2) and their sorted
+// lists of K in registers; the block streams the reference points through a
+// double-buffered tile of shared memory, each coordinate stored twice, (r, r), so
+// that a 64-bit load is a packed operand, and every thread scans the tile in the
+// order of the indices: a point enters a list if it is strictly nearer than the
+// last entry and passes only strictly farther ones, so equal distances keep the
+// lower index first.  Bound by issue: the insertions of a warp's 64 lists diverge,
+// about 100 of the 150 instructions a point costs a warp at 128 points (K = 8).
+// One warp a query took 880 us for 3 10^6 queries against 16 points (d = 1, k = 1),
+// this kernel 127; 1043 and 299 for 10^6 against 128 (d = 3, k = 8), 3166 and 883
+// for 3 10^6 against 64 (d = 4, k = 16).  (Four queries a thread: 0 to 30 % slower.)
+constexpr int LT_THREADS = 256;
+constexpr int LT_TILE = 512;   // reference points per shared tile
+template <int D, int K>
+__global__ void __launch_bounds__(LT_THREADS, 2)
+    knn_lowdim_thread_kernel(const float *__restrict__ ref, int N, long long ldr,
+                             const float *__restrict__ qry, int Q, long long ldq, int k,
+                             float *__restrict__ out_dist, int *__restrict__ out_idx,
+                             long long ld_out) {
+    __shared__ float2 tile[2][D][LT_TILE];
+    const int tid = threadIdx.x;
+    const int qid[2] = {(int)blockIdx.x * 2 * LT_THREADS + tid,
+                        (int)blockIdx.x * 2 * LT_THREADS + LT_THREADS + tid};
+    f32x2_t q[D];
+#pragma unroll
+    for (int dd = 0; dd < D; ++dd)
+        q[dd] = f2_pack(qid[0] < Q ? qry[(size_t)dd * ldq + qid[0]] : 0.f,
+                        qid[1] < Q ? qry[(size_t)dd * ldq + qid[1]] : 0.f);
+    float ld[2][K];
+    int li[2][K];
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            ld[m][j] = INFINITY;
+            li[m][j] = -1;
+        }
+    constexpr int PER = LT_TILE / LT_THREADS;   // points per thread per tile load
+    float pre[D][PER];
+    auto fetch = [&](int t) {
+#pragma unroll
+        for (int dd = 0; dd < D; ++dd)
+#pragma unroll
+            for (int u = 0; u < PER; ++u) {
+                const long long r = (long long)t * LT_TILE + u * LT_THREADS + tid;
+                pre[dd][u] = r < N ? ref[(size_t)dd * ldr + r] : 0.f;
+            }
+    };
+    auto stash = [&](int buf) {
+#pragma unroll
+        for (int dd = 0; dd < D; ++dd)
+#pragma unroll
+            for (int u = 0; u < PER; ++u)
+                tile[buf][dd][u * LT_THREADS + tid] = make_float2(pre[dd][u], pre[dd][u]);
+    };
+    const int tiles = (int)(((long long)N + LT_TILE - 1) / LT_TILE);
+    fetch(0);
+    stash(0);
+    __syncthreads();
+    for (int t = 0; t < tiles; ++t) {
+        if (t + 1 < tiles) fetch(t + 1);
+        const int rbase = t * LT_TILE, valid = min(LT_TILE, N - rbase);
+        for (int j = 0; j < valid; ++j) {
+            f32x2_t acc;
+#pragma unroll
+            for (int dd = 0; dd < D; ++dd) {
+                const f32x2_t x = f2_sub(*reinterpret_cast<const f32x2_t *>(&tile[t & 1][dd][j]),
+                                         q[dd]);
+                acc = f2_fma(x, x, dd ? acc : 0ull);
+            }
+            const float d2[2] = {f2_lo(acc), f2_hi(acc)};
+            if (!(d2[0] < ld[0][K - 1] || d2[1] < ld[1][K - 1])) continue;
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                if (!(d2[m] < ld[m][K - 1])) continue;
+#pragma unroll
+                for (int i = K - 1; i > 0; --i) {
+                    const bool past = d2[m] < ld[m][i - 1], here = d2[m] < ld[m][i];
+                    ld[m][i] = past ? ld[m][i - 1] : here ? d2[m] : ld[m][i];
+                    li[m][i] = past ? li[m][i - 1] : here ? rbase + j : li[m][i];
+                }
+                if (d2[m] < ld[m][0]) {
+                    ld[m][0] = d2[m];
+                    li[m][0] = rbase + j;
+                }
+            }
+        }
+        if (t + 1 < tiles) stash((t + 1) & 1);
+        __syncthreads();
+    }
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        if (qid[m] >= Q) continue;
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            if (j >= k) break;
+            out_dist[(size_t)j * ld_out + qid[m]] = sqrtf(ld[m][j]);
+            out_idx[(size_t)j * ld_out + qid[m]] = li[m][j];
+        }
+    }
+}
+
 namespace {
 
 // Splits that callers' scratch is sized for, and the kernel's own choice.
 struct LowdimShape {
     int max_splits;
+    bool thread;   // knn_lowdim_thread_kernel
     int qpw, wpq, splits;
 };
+
+// Whether one thread a pair of queries takes less than warps, in us.  A thread's
+// points cost 0.22 (lists of 8; 16: 0.37) each while the blocks are one an SM, then
+// in proportion to the queries, less for more points, of which fewer enter a list.
+// A warp's query costs about as much up to 128 points, then more slowly than in
+// proportion.  Fitted to 1236 problems of 16 to 16000 points, 1000 to 3 10^6 queries
+// and k = 1 to 16; thread / warp measured at d = 3, k = 8: 24 / 50 with 16 x 50000,
+// 34 / 48 with 64 x 50000, 48 / 46 with 128 x 50000, 145 / 223 with 128 x 400000, 108 /
+// 80 with 512 x 50000, 831 / 1143 with 512 x 10^6.
+bool thread_pays(int N, int Q, int k) {
+    if (N > 1024) return false;
+    const double few = 128.0 / std::max(N, 128);
+    const double point = k <= 8 ? std::max(0.22, 0.12 + 2.0e-6 * Q * std::pow(few, 0.2))
+                                : std::max(0.37, 0.2 + 4.4e-6 * Q * std::pow(few, 0.12));
+    const double query = (0.25e-3 + 0.035e-3 * k) * std::pow(few, -0.55);
+    return N * point < Q * query;
+}
 
 bool lowdim_shape(int N, int Q, int d, int k, int num_sms, LowdimShape &s) {
     if (d < 1 || d > 4 || k < 1 || k > LD_MAX_K) return false;
@@ -203,6 +328,7 @@ bool lowdim_shape(int N, int Q, int d, int k, int num_sms, LowdimShape &s) {
     const long long fill = s.wpq > 1 ? want / 2 / warps : (want + warps - 1) / warps;
     s.splits = (int)std::max<long long>(
         1, std::min({(long long)s.max_splits, fill, (long long)N / 8192}));
+    s.thread = thread_pays(N, Q, k);
     return true;
 }
 
@@ -218,6 +344,15 @@ cudaError_t launch_ld(const ExactProblem &p, const LowdimShape &s, unsigned long
                                                        part, subset);
         return cudaGetLastError();
     };
+    if (s.thread) {
+        const unsigned blocks = (unsigned)(((long long)p.Q + 2 * LT_THREADS - 1) /
+                                           (2 * LT_THREADS));
+        const auto kern = p.k <= 8 ? knn_lowdim_thread_kernel<D, 8>
+                                   : knn_lowdim_thread_kernel<D, LD_MAX_K>;
+        kern<<<blocks, LT_THREADS, 0, st>>>(p.ref, p.N, p.ldr, p.qry, p.Q, p.ldq, p.k, p.out_dist,
+                                            p.out_idx, p.ld_out);
+        return cudaGetLastError();
+    }
     if (s.wpq > 1) return go(knn_lowdim_kernel<D, 1, LD_WARPS>, 1);
     if (s.qpw == 4) return go(knn_lowdim_kernel<D, 4, 1>, 4 * LD_WARPS);
     if (s.qpw == 2) return go(knn_lowdim_kernel<D, 2, 1>, 2 * LD_WARPS);
@@ -252,10 +387,12 @@ int launch_lowdim(const ExactProblem &p, cudaStream_t st) {
     if (p.space && space_applies(p.N, p.Q, p.d, p.k)) {
         const int rc = launch_space(p, st, &sub);
         if (rc != kOk) return rc;
+        s.thread = false;
         s.qpw = 4;
         s.wpq = 1;
         s.splits = s.max_splits;
     }
+    if (s.thread) s.splits = 1;
     // as many splits as the scratch holds lists of (it may have been sized for the
     // larger first chunk of a call, whose plan has fewer)
     s.splits = (int)std::min<size_t>(

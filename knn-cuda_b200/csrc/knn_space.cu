@@ -524,8 +524,13 @@ bool space_applies(int N, int Q, int d, int k) {
     // 1000, 56 / 48 and 90 / 87 with 7000 x 7000, 73 / 50 and 116 / 91 with 25000 x
     // 2000, 71 / 79 and 101 / 189 with 2^20 x 50, 173 / 100 and 256 / 197 with 2^20 x
     // 200, 736 / 82 and 1449 / 195 with 2^20 x 1600.
+    // A search never costs less than about 0.6 us a thousand queries (d = 1, k = 1; 1.9
+    // at d = 4, k = 16), so few points are searched by brute force however many the
+    // queries are: 831 / 1297 with 512 x 10^6 at d = 3, k = 8, 1258 / 1349 with 1000 x
+    // 10^6 (1846 / 1351 where the points are sorted); in one dimension 498 / 694 with
+    // 256 x 10^6, 791 / 720 with 512 x 10^6 (k = 8).
     return d >= 1 && d <= 4 && k >= 1 && k <= 16 && N <= (1 << 30) &&
-           (double)N * Q >= 5e7 + 100.0 * N;
+           (double)N * Q >= 5e7 + 100.0 * N && N >= (d == 1 ? 400 : 700);
 }
 
 size_t space_bytes(int N, int Q, int d, int k) {
