@@ -317,7 +317,7 @@ bool lowdim_shape(int N, int Q, int d, int k, int num_sms, LowdimShape &s) {
     s.wpq = 1;
     if (Q < 300 || (Q < 1200 && N < 131072)) {
         s.qpw = 1;
-        if (N >= 1000) s.wpq = LD_WARPS;
+        if (N >= (Q <= 512 ? 256 : 1000)) s.wpq = LD_WARPS;
     } else if (N < 32768) {
         s.qpw = Q < 5000 ? 1 : 2;
     } else {
