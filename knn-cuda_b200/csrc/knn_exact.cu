@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(32 * MG_WARPS)
     __shared__ unsigned long long lists[MG_WARPS][KCAP], scratch[MG_WARPS][KCAP];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nq = subset.count ? *subset.count : Q;
-    if (subset.count) S = QuerySubset::splits(nq, S);
+    if (subset.count) S = subset.splits(nq, S);
     if (subset.count && S == 1) return;   // written without lists
     for (int q0 = blockIdx.x * QPB; q0 < nq; q0 += gridDim.x * QPB) {
         const int q = q0 + warp / WPQ;

@@ -123,13 +123,20 @@ struct ExactProblem {
 struct QuerySubset {
     const int *list = nullptr;
     const int *count = nullptr;
-    // Splits of the reference set for nq queries, of at most max_splits: as
-    // many as give 7104 warps (24 an SM, twice) of four queries each.  The
-    // kernels that work on a subset call it with the count they find.
-    static __host__ __device__ int splits(int nq, int max_splits) {
-        const int warps = (nq + 3) / 4;
-        const int s = warps > 0 ? 7104 / warps : 1;
-        return s < 1 ? 1 : s < max_splits ? s : max_splits;
+    int slots = 1, steps = 1;   // blocks that run at once; steps over the whole set
+    // Splits of the reference set for nq queries, 32 a block, of at most max_splits
+    // (and 64): those whose waves of blocks end soonest, a block taking its share of
+    // the steps and about 90 more to fill its lists anew.  The kernels that work on a
+    // subset call it with the count they find, a whole warp together.
+    __device__ int splits(int nq, int max_splits) const {
+        if (nq <= 0) return 1;
+        unsigned best = 0xffffffffu;
+        for (int s = (int)(threadIdx.x & 31u) + 1; s <= 64; s += 32) {
+            const float waves = ceilf((float)((nq + 31) / 32) * (float)s / (float)slots);
+            const float t = waves * ((float)steps / (float)s + 90.0f);
+            if (s <= max_splits) best = min(best, (__float_as_uint(t) & ~63u) | (unsigned)(s - 1));
+        }
+        return (int)(__reduce_min_sync(0xffffffffu, best) & 63u) + 1;
     }
 };
 

@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(32 * LD_WARPS)
     // with a subset: its queries, and the blocks loop over the (query block,
     // split) pairs; otherwise one pair per block
     const int nq = subset.count ? *subset.count : Q;
-    if (subset.count) n_splits = QuerySubset::splits(nq, n_splits);
+    if (subset.count) n_splits = subset.splits(nq, n_splits);
     const long long n_items = (long long)((nq + QPB - 1) / QPB) * n_splits;
     const long long steps = ((long long)N + LD_STEP - 1) / LD_STEP;
     for (long long item = blockIdx.x; item < n_items; item += gridDim.x) {
@@ -391,6 +391,8 @@ int launch_lowdim(const ExactProblem &p, cudaStream_t st) {
         s.qpw = 4;
         s.wpq = 1;
         s.splits = s.max_splits;
+        sub.slots = 2 * p.num_sms;
+        sub.steps = (p.N + LD_STEP - 1) / LD_STEP;
     }
     if (s.thread) s.splits = 1;
     // as many splits as the scratch holds lists of (it may have been sized for the
