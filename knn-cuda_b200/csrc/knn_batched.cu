@@ -20,7 +20,9 @@
 // knnb200_batched_autotune picks by timing candidate plans.
 #include <algorithm>
 #include <cstdio>
+#include <functional>
 #include <numeric>
+#include <queue>
 #include <vector>
 
 #include "../../include/knn_b200.h"
@@ -365,6 +367,74 @@ bool needs_copy(const knnb200_problem &q) {
     return (reinterpret_cast<uintptr_t>(q.query) & 15) || q.query_ld % 4;
 }
 
+// Splits of a problem of `stages` pipeline stages a query tile in items of about
+// `item_stages`.
+int item_splits(long long stages, int n_rtiles, int k, int item_stages) {
+    const long long s = std::max<long long>(1, (stages + item_stages / 2) / item_stages);
+    return (int)std::max<long long>(
+        1, std::min({s, (long long)n_rtiles, 256ll, (long long)(kMaxListKeys / k)}));
+}
+
+// The item size of a batch that leaves it open: the one whose items, given out
+// largest first to the SM that is free first, end soonest.  An item costs its
+// stages and 14 more (it fills and sorts its lists), down to half of that where it
+// is a query tile's last and has few queries.  Where an SM gets a dozen items or
+// more the schedule comes out even but for a part of the smallest.  Over 39 batches
+// of 1 to 1000 problems the choice takes 1.00 to 1.02 times the time of the best of
+// the eleven sizes; 256 stages always take up to 2.9 times (227 us, 546 with 256,
+// for 14 problems of up to 32768 points), and sizes in proportion to an SM's share
+// of the batch up to 1.37 (5536 us for 170 problems of 24000 x 64, d = 256, whose two
+// items each make three waves; 4440 with 256 stages).
+int choose_item_stages(const std::vector<knnb200_problem> &probs, int bq, int num_sms) {
+    static const int sizes[] = {64, 96, 128, 192, 256, 384, 512, 768, 1024, 1536, 2048};
+    struct Part {
+        double stages;        // of an item
+        double last;          // cost of the last query tile's items, of a whole one's
+        long long tiles, splits;
+    };
+    int best = 256;
+    double best_t = 1e300;
+    std::vector<Part> parts(probs.size());
+    for (const int size : sizes) {
+        double total = 0;
+        long long items = 0;
+        for (size_t i = 0; i < probs.size(); ++i) {
+            const knnb200_problem &q = probs[i];
+            const int n_rtiles = (q.ref_nb + EX_BR - 1) / EX_BR;
+            const long long stages = (long long)n_rtiles * ((q.dim + EX_BD - 1) / EX_BD);
+            Part &p = parts[i];
+            p.splits = item_splits(stages, n_rtiles, q.k, size);
+            p.stages = (double)stages / p.splits;
+            p.tiles = ((long long)q.query_nb + bq - 1) / bq;
+            p.last = std::max(0.5, (double)(q.query_nb - (p.tiles - 1) * bq) / bq);
+            items += p.tiles * p.splits;
+            total += (p.stages + 14.0) * ((double)(p.tiles - 1) + p.last) * p.splits;
+        }
+        std::stable_sort(parts.begin(), parts.end(),
+                         [](const Part &a, const Part &b) { return a.stages > b.stages; });
+        double t = total / num_sms + 0.5 * (parts.back().stages + 14.0);
+        if (items <= 12ll * num_sms) {
+            std::priority_queue<double, std::vector<double>, std::greater<double>> free_at(
+                std::greater<double>(), std::vector<double>(num_sms, 0.0));
+            t = 0;
+            for (const Part &p : parts)
+                for (long long s = 0; s < p.splits; ++s)
+                    for (long long tile = 0; tile < p.tiles; ++tile) {
+                        const double end = free_at.top() + (p.stages + 14.0) *
+                                                               (tile + 1 < p.tiles ? 1.0 : p.last);
+                        free_at.pop();
+                        free_at.push(end);
+                        t = std::max(t, end);
+                    }
+        }
+        if (t < best_t) {
+            best_t = t;
+            best = size;
+        }
+    }
+    return best;
+}
+
 int validate(const knnb200_problem &q) {
     if (!q.ref || !q.query || !q.knn_dist || !q.knn_index) return KNNB200_EINVAL;
     if (q.ref_nb < 1 || q.query_nb < 1 || q.dim < 1 || q.k < 1 || q.k > q.ref_nb)
@@ -419,25 +489,10 @@ int knnb200_batched_plan_create_config(const knnb200_problem *all, int n_all,
     pl->qpw = pl->kcap == 256 ? EX_QPW_K256 : (want_qpw ? want_qpw : EX_QPW);
     const int bq = pl->qpw * EX_WARPS;
 
-    // Records, cut into items of about `item_stages` pipeline stages.  Where the
-    // caller leaves the size open it follows from an SM's share of the batch: items
-    // that are a large part of it leave SMs idle at the end, and each warms up and
-    // sorts its lists, which costs about nine stages.  Against 256 stages always:
-    // 814 -> 466 us for 16 problems of 131 stages an SM together, 1374 -> 1121 at 377;
-    // 2824 -> 2785 at 1080, 6051 -> 5865 at 2406, 17636 -> 17060 at 6696 (512 problems).
-    // From 400 to 1000 neither a third nor two fifths is better than 256 throughout
-    // (0.94 to 1.08 of its time over six batches).
+    // records, cut into items of about `item_stages` pipeline stages
     int item_stages = cfg ? cfg->item_stages : 0;
-    if (item_stages <= 0) {
-        long long share = 0;
-        for (const knnb200_problem &q : persist)
-            share += (long long)((q.ref_nb + EX_BR - 1) / EX_BR) *
-                     ((q.dim + EX_BD - 1) / EX_BD) * ((q.query_nb + bq - 1) / bq);
-        share /= pl->num_sms;
-        item_stages = (int)(share < 400    ? std::max(64ll, share / 3)
-                            : share < 1000 ? 256
-                                           : std::min(2048ll, share * 2 / 5));
-    }
+    if (item_stages <= 0)
+        item_stages = count > 0 ? choose_item_stages(persist, bq, pl->num_sms) : 256;
     pl->item_stages = item_stages;
     std::vector<BatchProb> recs(count);
     std::vector<double> cost(count);
@@ -452,9 +507,7 @@ int knnb200_batched_plan_create_config(const knnb200_problem *all, int n_all,
         P.n_dchunks = (q.dim + EX_BD - 1) / EX_BD;
         P.qtiles = (q.query_nb + bq - 1) / bq;
         const long long stages = (long long)P.n_rtiles * P.n_dchunks;
-        int S = (int)std::max<long long>(1, (stages + item_stages / 2) / item_stages);
-        S = std::min({S, P.n_rtiles, 256, kMaxListKeys / q.k});
-        P.n_splits = std::max(1, S);
+        P.n_splits = item_splits(stages, P.n_rtiles, q.k, item_stages);
         P.qry = q.query;
         P.ldq = q.query_ld;
         P.ldc = round_up(q.query_nb, 32);
