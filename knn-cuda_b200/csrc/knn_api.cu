@@ -170,9 +170,17 @@ class HostPool {
 // of the others are in flight.  A piece holds several ranges where they are
 // short: with a gather of its own for each 0.25 MB run of the threshold sample
 // the sample of 2^18 x 128 took 3.1 ms and the call 11.3, now 7.5.
+// Page-locking memory takes about 0.65 ms and 0.37 a megabyte, and the staging saves
+// 0.07 ms a megabyte, so a program that calls once or twice is better off without:
+// the buffers come once the calls so far would have saved what they cost (input
+// of kStagePays times their size), two of them at first, no larger than their
+// piece.  (The first call of a process at 16384 x 4096 x 128 took 20 ms with two whole
+// buffers taken at once, 3.4 by the driver's copy.)
 constexpr int kStageSlots = 4;
 constexpr size_t kStageBytes = 16u << 20;
 constexpr size_t kStageMinBytes = 1u << 20;   // smaller input is left to the driver
+constexpr size_t kStagePays = 6;
+constexpr size_t kStageAllSlots = 1u << 30;   // input before there are more than two
 
 // count floats from src to a 16-byte aligned dst with non-temporal stores:
 // the staging buffer is read next by the copy engine, not by this core, so
@@ -231,23 +239,32 @@ struct Workspace {
     cudaStream_t copy_stream = nullptr;          // host entry: reference copies
     cudaEvent_t copied[1 + kStreamChunks] = {};  // sample, then each chunk
     float *stage[kStageSlots] = {};              // pinned staging for pageable input
+    size_t stage_bytes[kStageSlots] = {};
+    size_t pageable_seen = 0;                    // pageable input of all calls so far
     cudaEvent_t stage_done[kStageSlots] = {};    // the copies out of each stage have ended
     int stage_slot = 0;
     std::unique_ptr<HostPool> pool;              // gathers into the staging buffers
 
-    // Staging buffer `slot` and the pool, on first use.
-    bool ensure_staging(int slot) {
+    // Staging buffer `slot` of `bytes` at least, and the pool, on first use.  (No copy
+    // out of the buffer is in flight.)
+    bool ensure_staging(int slot, size_t bytes) {
         if (!stage_done[slot] &&
             cudaEventCreateWithFlags(&stage_done[slot], cudaEventDisableTiming) != cudaSuccess) {
             stage_done[slot] = nullptr;
             cudaGetLastError();
             return false;
         }
-        if (!stage[slot] && cudaMallocHost(reinterpret_cast<void **>(&stage[slot]), kStageBytes) !=
-                                cudaSuccess) {
-            stage[slot] = nullptr;
-            cudaGetLastError();
-            return false;
+        if (stage_bytes[slot] < bytes) {
+            if (stage[slot]) cudaFreeHost(stage[slot]);
+            stage_bytes[slot] = 0;
+            const size_t mb = size_t(1) << 20;
+            const size_t want = std::min(kStageBytes, (bytes + bytes / 4 + mb - 1) / mb * mb);
+            if (cudaMallocHost(reinterpret_cast<void **>(&stage[slot]), want) != cudaSuccess) {
+                stage[slot] = nullptr;
+                cudaGetLastError();
+                return false;
+            }
+            stage_bytes[slot] = want;
         }
         if (!pool) {
             const unsigned hc = std::thread::hardware_concurrency();
@@ -389,9 +406,11 @@ int copy_staged(Workspace &ws, const std::vector<Range> &ranges, const float *sr
         auto flush = [&]() -> int {
             if (piece.empty()) return kOk;
             const int slot = ws.stage_slot;
-            if (!ws.ensure_staging(slot)) return kErrNoMemory;
-            ws.stage_slot = (ws.stage_slot + 1) % kStageSlots;
-            if (cudaEventSynchronize(ws.stage_done[slot]) != cudaSuccess) return kErrCuda;
+            if (ws.stage_done[slot] && cudaEventSynchronize(ws.stage_done[slot]) != cudaSuccess)
+                return kErrCuda;
+            if (!ws.ensure_staging(slot, held * nr * fb)) return kErrNoMemory;
+            ws.stage_slot =
+                (ws.stage_slot + 1) % (ws.pageable_seen < kStageAllSlots ? 2 : kStageSlots);
             float *buf = ws.stage[slot];
             const size_t pitch = held;
             // a single long range of few rows: parts of a row
@@ -754,6 +773,10 @@ bool host_entry(int wanted, const float *ref, int ref_nb, const float *query, in
     }
     cudaStream_t st = ws->stream;
     ws->stage_slot = 0;   // small input allocates and keeps no more than it fills
+    const size_t input_bytes = ((size_t)ref_nb + query_nb) * dim * sizeof(float);
+    if (input_bytes >= kStageMinBytes && host_pageable(ref)) ws->pageable_seen += input_bytes;
+    const bool stage_pays =
+        ws->stage[0] || ws->pageable_seen >= kStagePays * std::min(input_bytes, 2 * kStageBytes);
     // The scratch and the status word are shared with the device entry, whose
     // last call may still be running on its caller's stream: this call waits
     // for it, and the next one for this call, however it ends.
@@ -777,7 +800,7 @@ bool host_entry(int wanted, const float *ref, int ref_nb, const float *query, in
     // buffers too: the driver copies it with one thread (8.4 MB in 400 to
     // 700 us; a call at 16384 x 4096 x 128 takes 0.58 ms instead of 0.83)
     auto copy_in = [&](const float *src, size_t src_ld, float *dst, size_t dst_ld, size_t cols) {
-        if (cols * dim * sizeof(float) >= kStageMinBytes && host_pageable(src)) {
+        if (stage_pays && cols * dim * sizeof(float) >= kStageMinBytes && host_pageable(src)) {
             const int r = copy_staged(*ws, {Range{0, cols}}, src, src_ld, dst, dst_ld, dim, st);
             if (r != kErrNoMemory) return r == kOk ? cudaSuccess : cudaErrorUnknown;
         }
