@@ -17,6 +17,7 @@
 #include <functional>
 #include <memory>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -102,7 +103,11 @@ struct Buffer {
 class HostPool {
   public:
     explicit HostPool(int threads) {
-        for (int t = 0; t < threads; ++t) workers_.emplace_back([this] { loop(); });
+        // (with fewer threads, or none, where the system has no more)
+        try {
+            for (int t = 0; t < threads; ++t) workers_.emplace_back([this] { loop(); });
+        } catch (const std::system_error &) {
+        }
     }
     ~HostPool() {
         {
