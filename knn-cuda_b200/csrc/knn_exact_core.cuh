@@ -3,6 +3,8 @@
 // launch: knn_batched.cu).  See knn_exact.cu for the algorithm.
 #pragma once
 
+#include <atomic>
+
 #include "knn_common.cuh"
 
 namespace knnb200 {
@@ -24,15 +26,21 @@ constexpr int EX_LAUNCH_REGS = 96, EX_PRODUCER_REGS = 24, EX_CONSUMER_REGS = 112
 static_assert(128 * EX_PRODUCER_REGS + EX_WARPS * 32 * EX_CONSUMER_REGS <=
                   EX_THREADS * EX_LAUNCH_REGS,
               "the consumers' registers come from the block's own");
-// Whether `kern` is launched with the registers that the split counts on (asked
-// once for each kernel; a build with fewer would leave its consumers waiting).
+// Whether `kern` is launched with the registers that the split counts on (a build
+// with fewer would leave its consumers waiting).  Only a good answer is kept: a
+// failure to ask, for want of memory to load the kernel say, is this call's alone.
 template <auto kern>
 bool launch_regs_ok() {
-    static const bool ok = [] {
-        cudaFuncAttributes a;
-        return cudaFuncGetAttributes(&a, kern) == cudaSuccess && a.numRegs >= EX_LAUNCH_REGS;
-    }();
-    return ok;
+    static std::atomic<bool> known{false};
+    if (known.load(std::memory_order_relaxed)) return true;
+    cudaFuncAttributes a;
+    if (cudaFuncGetAttributes(&a, kern) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (a.numRegs < EX_LAUNCH_REGS) return false;
+    known.store(true, std::memory_order_relaxed);
+    return true;
 }
 KNN_DI void producer_regs() {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(EX_PRODUCER_REGS));
