@@ -755,7 +755,7 @@ __global__ void __launch_bounds__(32 * TC_QP_WARPS, 3)
         for (int r = 0; r < 8; ++r) {
             const int pp = 4 * r + wp;
             if (p0 + pp >= n) continue;
-            __nv_bfloat16 hi[4], lo[4];
+            __align__(8) __nv_bfloat16 hi[4], lo[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const float y = tile[4 * wm + e][pp] * -2.0f;
@@ -892,7 +892,7 @@ __global__ void __launch_bounds__(32 * TC_PREP_WARPS)
             const float4 v = *reinterpret_cast<const float4 *>(tt + pp * TC_PREP_LD + 4 * wm);
             if (q < n) {
                 const float ve[4] = {v.x, v.y, v.z, v.w};
-                __nv_bfloat16 yb[4];
+                __align__(8) __nv_bfloat16 yb[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const float y = dd + e < d ? ve[e] - c4[e] : 0.f;
@@ -959,7 +959,7 @@ __global__ void tc_ref_lo_kernel(const float *__restrict__ xt, long long n_elems
     if (e0 >= n_elems) return;
     const float4 v = *reinterpret_cast<const float4 *>(xt + e0);
     const float vv[4] = {v.x, v.y, v.z, v.w};
-    __nv_bfloat16 out[4];
+    __align__(8) __nv_bfloat16 out[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int dd = (int)((e0 + i) % d_pad);
@@ -1008,7 +1008,7 @@ __global__ void tc_pack_ref_f8_kernel(const float *__restrict__ xt, int n, int d
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) {
         double rem = (double)s * (double)s_r / (double)kappa;
-        unsigned char row8[32];
+        __align__(16) unsigned char row8[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) row8[j] = 0;
 #pragma unroll
