@@ -225,6 +225,19 @@ KNNB200_API size_t knnb200_scratch_bytes(int ref_nb, int query_nb, int dim, int 
 /* Number of reference splits the exact kernel uses for this shape. */
 KNNB200_API int knnb200_plan_splits(int ref_nb, int query_nb, int dim, int k);
 
+/* How the exact form computes this shape (for tests and measurements): the fused
+ * kernel on a grid of (query tile, split) or on one range of tiles a CTA; for dim <=
+ * 4 and k <= 16 the brute force, a warp or a thread a query, or the spatial search.
+ * The ranges' lists and the search's memory may not be there in a call (the
+ * allocation-free entry, a memory limit), which then takes the grid or the brute
+ * force.  -1 for invalid sizes. */
+#define KNNB200_ROUTE_GRID 0
+#define KNNB200_ROUTE_RANGES 1
+#define KNNB200_ROUTE_CLOUD_WARP 2
+#define KNNB200_ROUTE_CLOUD_THREAD 3
+#define KNNB200_ROUTE_CLOUD_SPACE 4
+KNNB200_API int knnb200_plan_route(int ref_nb, int query_nb, int dim, int k);
+
 /* Memory admission of the host and device entry points (the reference's
  * legacy code split the queries by free memory,
  * legacy/KNN.CUDA.with.indexes/knn_cuda_with_indexes.cu:348-349, :406-444):

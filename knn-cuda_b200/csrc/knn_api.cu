@@ -1070,6 +1070,16 @@ int knnb200_plan_splits(int ref_nb, int query_nb, int dim, int k) {
     return exact_plan_splits(ref_nb, query_nb, dim, k, sms);
 }
 
+int knnb200_plan_route(int ref_nb, int query_nb, int dim, int k) {
+    if (!valid_sizes(ref_nb, query_nb, dim, k)) return -1;
+    int sms = 148;
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess)
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaGetLastError();
+    return exact_plan_route(ref_nb, query_nb, dim, k, sms);
+}
+
 void knnb200_release_workspace(void) {
     Workspace *ws = nullptr;
     if (current_workspace(ws) != kOk) return;

@@ -40,6 +40,7 @@
 #include <cstdio>
 #include <type_traits>
 
+#include "../../include/knn_b200.h"
 #include "knn_exact_core.cuh"
 #include "knn_kernels.h"
 
@@ -563,6 +564,13 @@ int exact_plan_splits(int N, int Q, int d, int k, int num_sms) {
     if (lowdim_applies(N, Q, d, k)) return lowdim_plan_splits(N, Q, d, k, num_sms);
     ExactShape s;
     return choose_shape(N, Q, d, k, num_sms, s) ? s.splits : 0;
+}
+
+int exact_plan_route(int N, int Q, int d, int k, int num_sms) {
+    if (lowdim_applies(N, Q, d, k)) return lowdim_plan_route(N, Q, d, k, num_sms);
+    ExactShape s;
+    if (!choose_shape(N, Q, d, k, num_sms, s)) return -1;
+    return s.ranges.ctas ? KNNB200_ROUTE_RANGES : KNNB200_ROUTE_GRID;
 }
 
 }  // namespace knnb200

@@ -156,6 +156,7 @@ bool exact_supported_k(int k);
 bool lowdim_applies(int N, int Q, int d, int k);
 size_t lowdim_scratch_bytes(int N, int Q, int d, int k, int num_sms);
 int lowdim_plan_splits(int N, int Q, int d, int k, int num_sms);
+int lowdim_plan_route(int N, int Q, int d, int k, int num_sms);   // KNNB200_ROUTE_*
 int launch_lowdim(const ExactProblem &p, cudaStream_t st);
 // Spatial search of large low-dimension problems (knn_space.cu): used by
 // launch_lowdim where it applies and p.space holds space_bytes (0: does not
@@ -175,6 +176,7 @@ size_t exact_scratch_bytes(int N, int Q, int d, int k, int num_sms);
 // What the exact path can make use of, where the memory is there: up to 64 MB more.
 size_t exact_scratch_wanted(int N, int Q, int d, int k, int num_sms);
 int exact_plan_splits(int N, int Q, int d, int k, int num_sms);
+int exact_plan_route(int N, int Q, int d, int k, int num_sms);    // KNNB200_ROUTE_*
 int launch_exact(const ExactProblem &p, cudaStream_t st);
 
 // Host-side state of a prepared reference set: which of the optional

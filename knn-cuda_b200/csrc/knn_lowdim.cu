@@ -33,6 +33,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "../../include/knn_b200.h"
 #include "knn_exact_core.cuh"
 #include "knn_kernels.h"
 #include "knn_lane_list.cuh"
@@ -375,6 +376,14 @@ size_t lowdim_scratch_bytes(int N, int Q, int d, int k, int num_sms) {
 int lowdim_plan_splits(int N, int Q, int d, int k, int num_sms) {
     LowdimShape s;
     return lowdim_shape(N, Q, d, k, num_sms, s) ? s.max_splits : 0;
+}
+
+int lowdim_plan_route(int N, int Q, int d, int k, int num_sms) {
+    LowdimShape s;
+    if (!lowdim_shape(N, Q, d, k, num_sms, s)) return -1;
+    return space_applies(N, Q, d, k) ? KNNB200_ROUTE_CLOUD_SPACE
+           : s.thread                ? KNNB200_ROUTE_CLOUD_THREAD
+                                     : KNNB200_ROUTE_CLOUD_WARP;
 }
 
 int launch_lowdim(const ExactProblem &p, cudaStream_t st) {

@@ -57,7 +57,7 @@ C_SYMBOLS = (
     "knnb200_set_bound_check", "knnb200_last_bound_check", "knnb200_set_memory_cap",
     "knnb200_last_query_chunks", "knnb200_call_bytes", "knnb200_last_tc_kinds",
     "knnb200_batched_plan_create_config", "knnb200_batched_plan_config",
-    "knnb200_batched_autotune_config", "knnb200_set_tc_kind_override",
+    "knnb200_batched_autotune_config", "knnb200_set_tc_kind_override", "knnb200_plan_route",
 )
 
 
@@ -110,6 +110,8 @@ def lib():
         L.knnb200_scratch_bytes.argtypes = [ctypes.c_int] * 5
         L.knnb200_plan_splits.restype = ctypes.c_int
         L.knnb200_plan_splits.argtypes = [ctypes.c_int] * 4
+        L.knnb200_plan_route.restype = ctypes.c_int
+        L.knnb200_plan_route.argtypes = [ctypes.c_int] * 4
         L.knnb200_release_workspace.restype = None
         L.knnb200_release_workspace.argtypes = []
         L.knnb200_status_string.restype = ctypes.c_char_p
@@ -533,6 +535,16 @@ def scratch_bytes(ref_nb, query_nb, dim, k, method="global") -> int:
 
 def plan_splits(ref_nb, query_nb, dim, k) -> int:
     return lib().knnb200_plan_splits(ref_nb, query_nb, dim, k)
+
+
+ROUTES = ("grid", "ranges", "cloud_warp", "cloud_thread", "cloud_space")
+
+
+def plan_route(ref_nb, query_nb, dim, k):
+    """How the exact form computes this shape where it has the memory: one of ROUTES,
+    None for invalid sizes."""
+    r = lib().knnb200_plan_route(ref_nb, query_nb, dim, k)
+    return ROUTES[r] if r >= 0 else None
 
 
 def selftest_wait_timeout(limit_ns: int = 50_000_000) -> int:

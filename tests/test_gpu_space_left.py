@@ -43,18 +43,19 @@ def test_queries_left_to_the_brute_force(knncuda, oracle, gpu, dim, k, inside):
     assert np.allclose(d.cpu().numpy()[:, some], gt_d, rtol=1e-6, atol=0)
 
 
-def test_resident_cloud_equals_brute_force(knncuda, gpu):
+@pytest.mark.parametrize("n,q,dim,k", [(100000, 5000, 3, 8), (4000036, 132, 2, 16)])
+def test_resident_cloud_equals_brute_force(knncuda, gpu, n, q, dim, k):
     import torch
 
-    n, q, k = 100000, 5000, 8
     rng = np.random.default_rng(3)
-    r = torch.from_numpy(rng.random((3, n), dtype=np.float32)).to(gpu)
-    x = torch.from_numpy(rng.random((3, q), dtype=np.float32)).to(gpu)
+    r = torch.from_numpy(rng.random((dim, n), dtype=np.float32)).to(gpu)
+    x = torch.from_numpy(rng.random((dim, q), dtype=np.float32)).to(gpu)
+    assert knncuda.plan_route(n, q, dim, k) == "cloud_space"
     rs = knncuda.RefSet(r)
     d, i = rs.knn(x, k, "global")
     bd, bi = torch.empty_like(d), torch.empty_like(i)
     rc = knncuda.lib().knnb200_knn_device_noalloc(
-        r.data_ptr(), n, n, x.data_ptr(), q, q, 3, k, bd.data_ptr(), bi.data_ptr(), q,
+        r.data_ptr(), n, n, x.data_ptr(), q, q, dim, k, bd.data_ptr(), bi.data_ptr(), q,
         ctypes.c_void_p(torch.cuda.current_stream(gpu).cuda_stream))
     assert rc == 0
     assert torch.equal(d, bd) and torch.equal(i, bi)
