@@ -40,8 +40,9 @@ extern "C" {
 #define KNNB200_METHOD_CUBLAS 2   /* expansion method (knn_cublas) */
 #define KNNB200_METHOD_FP8 3      /* expansion method with an FP8 (e4m3) candidate scan; same
                                      exact results; as CUBLAS where the FP8 scan does not apply
-                                     (d > 1024) or where its sample pass predicts that most
-                                     candidate lists would overflow */
+                                     (d > 1024, sets below 32768 points, data without
+                                     an FP8 scale) or where its sample pass predicts that
+                                     most candidate lists would overflow */
 
 /* C-linkage aliases of the three drop-in entry points of knncuda.h.
  * Replace knn_cuda_global / knn_cuda_texture / knn_cublas,
@@ -279,7 +280,10 @@ KNNB200_API int knnb200_selftest_wait_timeout(long long limit_ns, void *stream);
  * number of candidates the first tensor-core scan emitted (*candidates), the
  * number of queries that failed the first certification and were scanned a
  * second time (*second_scan), and of those the number recomputed by the
- * exact kernel (*exact).  All 0 when the call ran the exact kernel only.
+ * exact kernel (*exact).  All 0 when the call ran the exact kernel only.  A call on a
+ * set below 32768 points that went to the exact kernel after its threshold sample
+ * reports all its queries as exact, none scanned a second time, and the candidates
+ * that the queries counted there would have had, at least.
  * Any pointer may be NULL. */
 KNNB200_API void knnb200_last_tc_stats(long long *candidates, int *second_scan, int *exact);
 

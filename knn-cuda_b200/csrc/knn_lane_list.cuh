@@ -6,7 +6,6 @@
 
 namespace knnb200 {
 
-constexpr int LL_MAX_K = 32;
 // An entry without a point: distance +inf, index -1.
 constexpr unsigned long long kKeyNone = (0x7f800000ull << 32) | 0xffffffffull;
 

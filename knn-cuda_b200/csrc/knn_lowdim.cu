@@ -19,9 +19,9 @@
 //
 // Bound by the FP32 pipe: 24 lane operations per four points at d = 3.  One
 // thread per query with register lists, the layout before this one, took 29.1
-// ms at 2^20 x 65536, d = 3, k = 8, where this one takes 22.9, and left most of
-// the GPU idle at smaller sizes: 244 -> 126 us at 1000 x 50000, d = 1, k = 8; 855 ->
-// 79 at 7000 x 7000, d = 3, k = 16; 438 -> 71 at 2^20 x 50, d = 1, k = 8.
+// ms at 2^20 x 65536, d = 3, k = 8, where this one takes 22.2, and left most of
+// the GPU idle at smaller sizes (d = 3, k = 8): 267 -> 32 us at 1000 x 4000, 527 -> 55
+// at 65536 x 400, 2179 -> 134 at 2^20 x 100, 1566 -> 851 at 2^18 x 8192.
 //
 // Many queries against few points run one thread a pair of queries
 // (knn_lowdim_thread_kernel): a warp's list costs it the same few thousand cycles

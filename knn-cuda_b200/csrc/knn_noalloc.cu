@@ -13,9 +13,10 @@
 // Limits and sharing:
 //   * the static area is 64 MiB of device memory, held on every GPU that
 //     loads this library until the process exits;
-//   * a call needs the exact path's whole scratch in it: the query set
-//     duplicated into (q, q) pairs (dim * round_up(query_nb, 32) * 8 bytes),
-//     256 bytes of alignment and, when the planner splits the reference set,
+//   * a call needs the exact path's whole scratch in it: room for two copies of the
+//     query set (dim * round_up(query_nb, 32) * 8 bytes; one is made, where the
+//     queries cannot be read in place), 256 bytes and, when the planner splits the
+//     reference set,
 //     splits * query_nb * min(k, 256) * 8 bytes of per-split lists (for
 //     k > 256 also query_nb * 8 bytes of lower-bound keys).  knnb200_scratch_bytes(...,
 //     KNNB200_METHOD_GLOBAL) gives the exact figure; a call needing more

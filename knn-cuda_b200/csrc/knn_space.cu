@@ -1,4 +1,4 @@
-// knn_space.cu -- exact FP32 k-NN for point clouds (d <= 4, k <= 32) that are
+// knn_space.cu -- exact FP32 k-NN for point clouds (d <= 4, k <= 16) that are
 // large enough to be put in spatial order first.
 //
 // In a few dimensions nearly all pairs of a brute force are far from each
@@ -23,7 +23,9 @@
 // order separates them badly a query gives up after `cap` leaves, or at once
 // where a quarter of the points share a cell (a few outliers that stretch the
 // grid), and joins a list that the brute-force kernel answers, on the device,
-// with no read-back.
+// with no read-back.  Such a query pays for both: points on a sphere and queries near
+// its centre take 0.32 to 0.96 of the brute force that ran before the search, all
+// queries exactly at the centre up to 1.06 (2^20 points, 4096 queries).
 //
 // At 2^20 points, d = 3, 65536 queries and k = 8 a call takes 314 us against 22.9
 // ms for the brute force: 76 us to order the points (counting and scattering 24

@@ -1523,9 +1523,10 @@ KNN_DI int keep_below(const unsigned long long (&key)[SL], unsigned long long cu
 }
 
 // Select: reject lists that cannot be re-ranked, find the k-th smallest entry
-// key (a bisection over the order-preserving bits of a, key_cut) and compact the entries with a <= the pruning limit
-// to the front of the list (in place: an entry moves only to a position already
-// read).  nsel[q] = their number, or -1 for a rejected list.
+// key (a bisection over the order-preserving bits of a, key_cut) and compact the
+// entries with a <= the pruning limit to the front of the list (in place: an entry
+// moves only to a position already read).  nsel[q] = their number, or -1 for a
+// rejected list.
 //
 // The list sits in registers, SL keys a lane.  Against an 8-bit radix selection
 // in shared memory that read the list six times: 66 -> 42 us at 16384 queries of
@@ -2616,11 +2617,11 @@ int tc_run_rerank_piece(TcRun &r, cudaStream_t st) {
     const TcProblem &P = r.P;
     if (!r.pieces) {
         // the running lists take the exact-fallback scratch, which nothing
-        // uses before the certification.  tc_scratch_bytes sizes that
-        // scratch for the fallback's query copy (d * Q floats) and result
-        // keys (k * Q), so Q * k keys plus Q flags always fit; the check
-        // only guards a caller-sized scratch, for which the full re-rank
-        // then runs in tc_run_finish instead
+        // uses before the certification: room for two copies of the queries
+        // (2 d floats a query) and the fallback's split lists.  Q * k keys and Q
+        // flags fit there for k up to about d, and for larger k where the
+        // fallback splits the set; where they do not, the full re-rank runs
+        // in tc_run_finish instead
         Carve cv{r.xs, 0, r.xcap};
         unsigned long long *keys = cv.take<unsigned long long>((size_t)P.Q * P.k);
         int *done = cv.take<int>(P.Q);
