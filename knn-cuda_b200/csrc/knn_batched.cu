@@ -396,7 +396,7 @@ int choose_item_stages(const std::vector<knnb200_problem> &probs, int bq, int nu
     double best_t = 1e300;
     std::vector<Part> parts(probs.size());
     for (const int size : sizes) {
-        double total = 0;
+        double total = 0, least = 1e300;
         long long items = 0;
         for (size_t i = 0; i < probs.size(); ++i) {
             const knnb200_problem &q = probs[i];
@@ -408,12 +408,13 @@ int choose_item_stages(const std::vector<knnb200_problem> &probs, int bq, int nu
             p.tiles = ((long long)q.query_nb + bq - 1) / bq;
             p.last = std::max(0.5, (double)(q.query_nb - (p.tiles - 1) * bq) / bq);
             items += p.tiles * p.splits;
+            least = std::min(least, p.stages);
             total += (p.stages + 14.0) * ((double)(p.tiles - 1) + p.last) * p.splits;
         }
-        std::stable_sort(parts.begin(), parts.end(),
-                         [](const Part &a, const Part &b) { return a.stages > b.stages; });
-        double t = total / num_sms + 0.5 * (parts.back().stages + 14.0);
+        double t = total / num_sms + 0.5 * (least + 14.0);
         if (items <= 12ll * num_sms) {
+            std::stable_sort(parts.begin(), parts.end(),
+                             [](const Part &a, const Part &b) { return a.stages > b.stages; });
             std::priority_queue<double, std::vector<double>, std::greater<double>> free_at(
                 std::greater<double>(), std::vector<double>(num_sms, 0.0));
             t = 0;

@@ -62,11 +62,12 @@ __global__ void __launch_bounds__(32 * LD_WARPS)
     // split) pairs; otherwise one pair per block
     const int nq = subset.count ? *subset.count : Q;
     if (subset.count) n_splits = subset.splits(nq, n_splits);
-    const long long n_items = (long long)((nq + QPB - 1) / QPB) * n_splits;
+    const long long n_items = ((long long)nq + QPB - 1) / QPB * n_splits;
     const long long steps = ((long long)N + LD_STEP - 1) / LD_STEP;
     for (long long item = blockIdx.x; item < n_items; item += gridDim.x) {
         const int split = (int)(item % n_splits);
-        const int q0 = (int)(item / n_splits) * QPB + group * QPW;
+        // (unsigned: the last block's queries may lie beyond the largest int)
+        const unsigned q0 = (unsigned)(item / n_splits) * QPB + group * QPW;
         // this warp's steps
         const long long parts = (long long)n_splits * WPQ;
         const long long mypart = (long long)split * WPQ + warp % WPQ;
@@ -75,8 +76,8 @@ __global__ void __launch_bounds__(32 * LD_WARPS)
         unsigned long long mine[QPW], tau[QPW];
 #pragma unroll
         for (int i = 0; i < QPW; ++i) {
-            const int qi = q0 + i;
-            const int col = qi < nq ? (subset.list ? subset.list[qi] : qi) : -1;
+            const unsigned qi = q0 + i;
+            const int col = qi < (unsigned)nq ? (subset.list ? subset.list[qi] : (int)qi) : -1;
 #pragma unroll
             for (int dd = 0; dd < D; ++dd) q[i][dd] = col >= 0 ? qry[(size_t)dd * ldq + col] : 0.f;
             mine[i] = kKeyNone;
@@ -145,11 +146,11 @@ __global__ void __launch_bounds__(32 * LD_WARPS)
         if (warp % WPQ == 0) {
 #pragma unroll
             for (int i = 0; i < QPW; ++i) {
-                const int qi = q0 + i;
-                if (qi >= nq || lane >= k) continue;
+                const unsigned qi = q0 + i;
+                if (qi >= (unsigned)nq || lane >= k) continue;
                 const unsigned long long key = WPQ > 1 ? merged[group][i][lane] : mine[i];
                 if (n_splits == 1) {
-                    const int col = subset.list ? subset.list[qi] : qi;
+                    const int col = subset.list ? subset.list[qi] : (int)qi;
                     out_dist[(size_t)lane * ld_out + col] = sqrtf(key_dist2(key));
                     out_idx[(size_t)lane * ld_out + col] = key_index(key);
                 } else {
@@ -182,13 +183,15 @@ __global__ void __launch_bounds__(LT_THREADS, 2)
                              long long ld_out) {
     __shared__ float2 tile[2][D][LT_TILE];
     const int tid = threadIdx.x;
-    const int qid[2] = {(int)blockIdx.x * 2 * LT_THREADS + tid,
-                        (int)blockIdx.x * 2 * LT_THREADS + LT_THREADS + tid};
+    // (unsigned: the last block's may lie beyond the largest int)
+    const unsigned qid[2] = {blockIdx.x * 2 * LT_THREADS + tid,
+                             blockIdx.x * 2 * LT_THREADS + LT_THREADS + tid};
+    const unsigned nq = (unsigned)Q;
     f32x2_t q[D];
 #pragma unroll
     for (int dd = 0; dd < D; ++dd)
-        q[dd] = f2_pack(qid[0] < Q ? qry[(size_t)dd * ldq + qid[0]] : 0.f,
-                        qid[1] < Q ? qry[(size_t)dd * ldq + qid[1]] : 0.f);
+        q[dd] = f2_pack(qid[0] < nq ? qry[(size_t)dd * ldq + qid[0]] : 0.f,
+                        qid[1] < nq ? qry[(size_t)dd * ldq + qid[1]] : 0.f);
     float ld[2][K];
     int li[2][K];
 #pragma unroll
@@ -253,7 +256,7 @@ __global__ void __launch_bounds__(LT_THREADS, 2)
     }
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
-        if (qid[m] >= Q) continue;
+        if (qid[m] >= nq) continue;
 #pragma unroll
         for (int j = 0; j < K; ++j) {
             if (j >= k) break;
@@ -337,7 +340,7 @@ template <int D>
 cudaError_t launch_ld(const ExactProblem &p, const LowdimShape &s, unsigned long long *part,
                       const QuerySubset &subset, cudaStream_t st) {
     auto go = [&](auto kern, int qpb) {
-        const long long items = (long long)((p.Q + qpb - 1) / qpb) * s.splits;
+        const long long items = ((long long)p.Q + qpb - 1) / qpb * s.splits;
         // a subset is usually small or empty: blocks that loop
         const long long grid = subset.count ? std::min<long long>(items, 4 * p.num_sms) : items;
         kern<<<(unsigned)grid, 32 * LD_WARPS, 0, st>>>(p.ref, p.N, p.ldr, p.qry, p.Q, p.ldq, p.k,

@@ -403,8 +403,9 @@ __global__ void __launch_bounds__(32 * SP_WARPS)
     __shared__ SpaceGrid g;
     sp_load_grid(g, v.grid);
     const int lane = threadIdx.x & 31;
-    const int qi = blockIdx.x * SP_WARPS + (threadIdx.x >> 5);
-    if (qi >= Q) return;
+    // (unsigned: the last block's queries may lie beyond the largest int)
+    const unsigned qi = blockIdx.x * SP_WARPS + (threadIdx.x >> 5);
+    if (qi >= (unsigned)Q) return;
     float q[D];
     bool finite = true;
 #pragma unroll
@@ -463,7 +464,7 @@ __global__ void __launch_bounds__(32 * SP_WARPS)
         }
     }
     if (visits > cap) {
-        if (lane == 0) v.far[atomicAdd(v.nfar, 1)] = qi;
+        if (lane == 0) v.far[atomicAdd(v.nfar, 1)] = (int)qi;
         return;
     }
     if (lane < k) {
@@ -524,7 +525,8 @@ int launch_space_d(const ExactProblem &p, const SpaceView &v, cudaStream_t st) {
     sp_leaf_kernel<D><<<v.n[1], 1024, 0, st>>>(v, p.N);
     sp_top_kernel<D><<<(v.n[2] + 3) / 4, 128, 0, st>>>(v);
     const int cap = std::max(256, v.n[0] / 64);
-    sp_search_kernel<D><<<(p.Q + SP_WARPS - 1) / SP_WARPS, 32 * SP_WARPS, 0, st>>>(
+    sp_search_kernel<D><<<(unsigned)(((long long)p.Q + SP_WARPS - 1) / SP_WARPS), 32 * SP_WARPS,
+                          0, st>>>(
         p.qry, p.Q, p.ldq, p.N, p.k, cap, v, p.out_dist, p.out_idx, p.ld_out);
     return cudaGetLastError() == cudaSuccess ? kOk : kErrLaunch;
 }
