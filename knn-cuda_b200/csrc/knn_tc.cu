@@ -2709,9 +2709,15 @@ int tc_run_finish(TcRun &r, cudaStream_t st, int *host_stats) {
         r.fail, nf, r.retry, r.retry_f, r.retry_s, r.qn, r.R.rmax_bits, run_bound(r, kind2), r.thr,
         r.count);
     if (cudaGetLastError() != cudaSuccess) return kErrLaunch;
-    // the compacted queries share the whole list buffer (Q * cmax entries)
-    const int cmax2 = (int)std::min<long long>(
-        kTcCmaxRetry, std::max<long long>(r.cmax, (long long)P.Q * r.cmax / nf));
+    // The compacted queries share the whole list buffer (Q * cmax entries).  A small
+    // set's lists stay as long as they were: one warp works through a list, about 0.14
+    // us an entry, and the exact kernel answers a few queries in 50 to 160 us (one
+    // query among 8192 equal points of 16384 x 128, 4096 queries: 1743 us with
+    // longer lists).
+    const int cmax2 =
+        P.may_leave ? r.cmax
+                    : (int)std::min<long long>(
+                          kTcCmaxRetry, std::max<long long>(r.cmax, (long long)P.Q * r.cmax / nf));
     if ((rc = emit_scan(r, st, kind2, nf, r.thr, cmax2, 0, r.n_tiles2)) != kOk) return rc;
     if (tm) tm->mark(st, kPhaseTcRetryScan);
     rc = rerank(r, st, kind2, nf, cmax2, r.qsub, r.ldf, r.qn, r.thr, nullptr, r.sd, r.si, r.ldf,
