@@ -332,8 +332,8 @@ struct TcRun {
     bool undecided;         // the overflow prediction is on its way (probe_event)
     bool may_switch;        // ... and may switch the run to split BF16
     bool may_leave;         // ... or end it (TcProblem::may_leave)
-    int lost;               // queries predicted to overflow every scan, where the
-                            // run ended for that reason (else 0)
+    int max_lost;           // more queries predicted to overflow every scan end it
+    int lost;               // their number, where the run ended for that reason (else 0)
     unsigned char *xs;
     size_t xcap;
     // incremental re-rank (tc_run_rerank_piece): running k smallest exact

@@ -299,15 +299,9 @@ struct TpArgs {
     int *status;
     const int *n_wide;      // queries predicted to overflow: the scan does nothing
                             // when they are more than half (nullptr: always runs)
-    const int *n_lost;      // likewise when these are too many (too_many_lost)
+    const int *n_lost;      // likewise when these are more than max_lost
+    int max_lost;
 };
-
-// Whether a call is better handed to the exact kernel as a whole, given the
-// queries whose lists will overflow every scan (tc_threshold_kernel).  A lost query
-// costs an emission of whole tiles into its list, a second scan and the exact
-// kernel: constant data took 2201 us at 16384 x 4096 x 128 where the exact kernel
-// takes 609.
-__host__ __device__ inline bool too_many_lost(int n_lost, int Q) { return n_lost > Q / 8; }
 
 // Norm step and one ring item's MMAs for each kind, issued by the even
 // CTA's MMA thread.  K steps advance the descriptors by 32 bytes (2 in
@@ -356,7 +350,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TP_THREADS, 1)
 
     // (both CTAs of a pair read the same word: they leave together)
     if (a.n_wide && 2 * *a.n_wide > a.Q) return;
-    if (a.n_lost && too_many_lost(*a.n_lost, a.Q)) return;
+    if (a.n_lost && *a.n_lost > a.max_lost) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const bool lead = rank == 0;
@@ -2040,6 +2034,28 @@ float pow2_ceil(double x) { return (float)std::ldexp(1.0, (int)std::ceil(std::lo
 
 }  // namespace
 
+// Models for sets below kTcAlwaysPoints, in us.  The exact kernel: 13e6 coordinates
+// of pairs a us.  The tensor path: its launches and read-backs, and for each query
+// the selection and the gather of about 1.7 k + 20 rows.
+static double exact_us(int N, int Q, int d) {
+    return 30.0 + (double)N * Q * std::max(d, 32) / 13e6;
+}
+static double tensor_us(int Q, int d, int k) {
+    return 150.0 + Q * (0.025 + (1.7 * k + 20) * d * 8e-7 + 0.00015 * k);
+}
+
+// How many queries may be lost (tc_threshold_kernel) before a call is better handed
+// to the exact kernel as a whole.  The first ones cost about 350 us (whole tiles
+// emitted into their lists, re-ranked in vain, a second scan), and each its part of
+// the exact kernel's time.  With every 100th, 12th and 8th query lost, against the
+// exact kernel: 683, 713 and 749 against 690 us at 16384 x 4096 x 128, k = 16 (line at
+// 6 %), 884, 1030 and 985 against 1250 at 8192 x 8192 x 256, k = 32 (32 %), 1146, 1345
+// and 1503 against 2590 at 12000 x 6000 x 512, k = 50 (40 %).
+static int most_lost(int N, int Q, int d, int k) {
+    const double share = (1.0 - (tensor_us(Q, d, k) + 350.0) / exact_us(N, Q, d)) / 1.1;
+    return (int)(Q * std::min(0.4, std::max(1.0 / 64, share)));
+}
+
 bool tc_supported(int N, int Q, int d, int k) {
     // (256 sample rows at least: the threshold is the 16th of their minima)
     return d >= 16 && d <= kTcMaxDim && k >= 1 && k <= kTcMaxK && Q >= 1 &&
@@ -2049,19 +2065,14 @@ bool tc_supported(int N, int Q, int d, int k) {
 bool tc_pays(int N, int Q, int d, int k) {
     if (!tc_supported(N, Q, d, k)) return false;
     if (N >= kTcAlwaysPoints) return true;
-    // Models in us.  The exact kernel: 13e6 coordinates of pairs a us.  The tensor
-    // path: its launches and read-backs, and for each query the selection and
-    // the gather of about 1.7 k + 20 rows.  Exact / tensor measured at (points,
+    // Exact / tensor measured, in us, at (points,
     // queries, dimensions, k): 609 / 207 (16384, 4096, 128, 16), 719 / 354 (16384,
     // 4096, 128, 100), 389 / 343 (8192, 4096, 128, 100), 649 / 280 (4096, 4096, 512,
     // 10), 2400 / 515 (16384, 16384, 128, 10), 185 / 128 (30000, 1000, 64, 10), 114 /
     // 126 (30000, 200, 128, 10), 813 / 742 (16384, 16384, 16, 100 and 10).  The line
     // leaves ties and small gains to the exact kernel, whose time does not
     // depend on the data.
-    const double exact = 30.0 + (double)N * Q * std::max(d, 32) / 13e6;
-    const double tensor =
-        150.0 + Q * (0.025 + (1.7 * k + 20) * d * 8e-7 + 0.00015 * k);
-    return exact > 1.2 * tensor;
+    return exact_us(N, Q, d) > 1.2 * tensor_us(Q, d, k);
 }
 
 bool tc_fp8_supported(int d) {
@@ -2306,6 +2317,7 @@ int launch_scan(const TcRun &r, cudaStream_t st, int kind, const __nv_bfloat16 *
     a.status = P.status;
     a.n_wide = n_wide;
     a.n_lost = n_lost;
+    a.max_lost = r.max_lost;
     const dim3 grid(2 * ((Q + TC_QT - 1) / TC_QT), n_splits);
     auto go = [&](auto kern) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2458,7 +2470,7 @@ int tc_run_begin(const TcProblem &P, const TcRefView &R, cudaStream_t st, TcRun 
     r.cand_total = reinterpret_cast<unsigned long long *>(r.ctl + 2);
     r.nwide = r.ctl + 4;
     r.undecided = r.may_switch = r.may_leave = false;
-    r.lost = 0;
+    r.lost = r.max_lost = 0;
     r.p1 = cv.take<float>((size_t)TP_LISTS * p.splits1 * P.Q * TC_KS);
     r.cand = cv.take<unsigned long long>((size_t)P.Q * p.cmax);
     r.ldf = (P.Q + 3) / 4 * 4;   // second-chance buffers, sized for all queries
@@ -2539,6 +2551,7 @@ int tc_run_pass1(TcRun &r, cudaStream_t st) {
     const TcBound b16 = run_bound(r, kTcBf16);
     TcLost lost;
     if (r.may_leave) {
+        r.max_lost = most_lost(P.N, P.Q, P.d, P.k);
         const int every = TC_SAMPLE_EVERY * r.p1_every;   // points a sample row stands for
         lost.count = r.nwide + 2;
         lost.near = (r.cmax + every - 1) / every;
@@ -2598,7 +2611,7 @@ int tc_run_pass2(TcRun &r, int tile_begin, int tile_end, cudaStream_t st) {
         if (rc != kOk) return rc;
         if (cudaEventSynchronize(r.P.probe_event) != cudaSuccess) return kErrCuda;
         r.undecided = false;
-        if (r.may_leave && too_many_lost(r.P.host_tmp[1], r.P.Q)) {
+        if (r.may_leave && r.P.host_tmp[1] > r.max_lost) {
             r.lost = r.P.host_tmp[1];
             return kOk;
         }
