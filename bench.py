@@ -455,9 +455,13 @@ def run_ours(args, D: Dist):
         if fb["second_scan"] > 0:
             launches += 8 + (1 if kinds.get("second_scan") == "bf16x3" and not split else 0)
     else:
-        # the exact kernel and, with splits, the merge (a point-cloud search
-        # launches more)
-        launches = 1 + (1 if knncuda.plan_splits(N, qn, dim, k) > 1 else 0)
+        # the exact kernel and, with splits or ranges of tiles, the merge; a
+        # point-cloud search launches eight kernels before the brute force for the
+        # queries it leaves over
+        route = knncuda.plan_route(N, qn, dim, k)
+        merged = route == "ranges" or knncuda.plan_splits(N, qn, dim, k) > 1
+        launches = ((8 if route == "cloud_space" else 0) + 1 +
+                    (1 if merged and route != "cloud_thread" else 0))
     ex = tiers["exact_fp32"]
     ex_ms = ex["phase_ms"].get("exact_main", ex["ms_per_step"])
     fp32_peak = knncuda.measure_fp32_peak(8192)

@@ -2047,7 +2047,7 @@ static double tensor_us(int Q, int d, int k) {
 // How many queries may be lost (tc_threshold_kernel) before a call is better handed
 // to the exact kernel as a whole.  The first ones cost about 350 us (whole tiles
 // emitted into their lists, re-ranked in vain, a second scan), and each its part of
-// the exact kernel's time.  With every 100th, 12th and 8th query lost, against the
+// the exact kernel's time.  With every 100th, 11th and 8th query lost, against the
 // exact kernel: 683, 713 and 749 against 690 us at 16384 x 4096 x 128, k = 16 (line at
 // 6 %), 884, 1030 and 985 against 1250 at 8192 x 8192 x 256, k = 32 (32 %), 1146, 1345
 // and 1503 against 2590 at 12000 x 6000 x 512, k = 50 (40 %).
