@@ -1135,17 +1135,18 @@ __global__ void __launch_bounds__(32 * TC_THR_WARPS)
         }
         const float T = ord_float((uint32_t)(tau >> 32));
         const float L0 = ord_float((uint32_t)(__shfl_sync(0xffffffffu, mine, 0) >> 32));
+        bool unsure = false;   // (comparisons that fail for NaN count the query as lost)
         if (lane == 0) {
             const float r2 = __uint_as_float(*rmax_bits);
             thr[q] = T + tc_error_bound(qn[q], r2, T, bound);
             thr_raw[q] = T;
             count[q] = 0;
-            const float spread = T - L0;
-            wide0 = tc_error_bound(qn[q], r2, T, probe0) > spread;
-            wide1 = tc_error_bound(qn[q], r2, T, probe1) > spread;
+            const float spread = T - L0, e0 = tc_error_bound(qn[q], r2, T, probe0);
+            wide0 = e0 > spread;
+            if (lost.count) unsure = !(e0 < spread);
+            else wide1 = tc_error_bound(qn[q], r2, T, probe1) > spread;
         }
-        if (lost.count) {
-            // (comparisons that fail for NaN count the query as lost)
+        if (lost.count && __any_sync(0xffffffffu, unsure)) {
             const float E = tc_error_bound(qn[q], __uint_as_float(*rmax_bits), T, lost.bound);
             if (!(E < T - L0)) {
                 int near = 0;
@@ -1162,11 +1163,12 @@ __global__ void __launch_bounds__(32 * TC_THR_WARPS)
         }
     }
     if (n_wide) {
-        const int n0 = __syncthreads_count(wide0), n1 = __syncthreads_count(wide1);
-        const int nl = lost.count ? __syncthreads_count(is_lost) : 0;
+        // (a run that counts lost queries asks for no FP8)
+        const int n0 = __syncthreads_count(wide0);
+        const int n1 = __syncthreads_count(lost.count ? is_lost : wide1);
         if (threadIdx.x == 0 && host_wide) {
-            if (nl) {
-                atomicAdd(lost.count, nl);
+            if (lost.count && n1) {
+                atomicAdd(lost.count, n1);
                 __threadfence();   // before this block's arrival
             }
             // the blocks that have arrived count in the word above
